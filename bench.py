@@ -261,7 +261,7 @@ def run_ours(args):
 
     gs = [cvo.upload(s) for s, _, _ in pairs]
     gt = [cvo.upload(t) for _, t, _ in pairs]
-    # association cell size picked by the autotuner on the first pair (untimed setup)
+    # division of the candidate test picked by the autotuner on the first pair (untimed setup)
     tune = None
     if not args.no_autotune:
         # at the pose and lengthscale the refinement starts from: the network's first hypothesis
@@ -401,7 +401,7 @@ def run_ours(args):
             traffic = round(per_pair * pair_passes / prof["assoc_launches"])
         roof = {"bound": "hbm", "achieved": round(achieved, 2), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 5), "traffic": traffic, "peak_source": peak_kind,
-                "kernel": "k_assoc_cta + k_select + k_rescan + k_rowsum", "launches": prof["assoc_launches"],
+                "kernel": "k_cand + k_rows", "launches": prof["assoc_launches"],
                 "avg_launch_us": round(avg_s * 1e6, 3), "algorithmic_bytes_per_launch": round(per_launch_bytes),
                 "iteration_kernel_ms": {k: round(v, 3) for k, v in prof["kernel_ms"].items()},
                 "association_phase_ms": {k: round(v, 3) for k, v in prof.get("assoc_split_ms", {}).items()}}
@@ -700,7 +700,7 @@ def run_component(args):
             batch = pairs[b0:b0 + args.pairs]
             gs = [cvo.upload(s) for s, _, _ in batch]
             gt = [cvo.upload(t) for _, t, _ in batch]
-            if b0 == 0:                       # warm-up of both paths (graphs, grid levels)
+            if b0 == 0:                       # warm-up of both paths (graphs)
                 learned(gs, gt)
                 grid(gs, gt)
             torch.cuda.synchronize()
@@ -928,7 +928,7 @@ def main():
                     help="complete CPU registrations the reference arm's value is measured on")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--refine", type=int, default=1, help="hypotheses refined per pair (1..8)")
-    ap.add_argument("--no-autotune", action="store_true", help="keep the default association cell size")
+    ap.add_argument("--no-autotune", action="store_true", help="keep the default division of the candidate test")
     ap.add_argument("--refine-ell", type=float, default=0.4,
                     help="lengthscale the hypotheses' refinement starts at (0: ell_init of the yaml)")
     ap.add_argument("--fallback-cos", type=float, default=0.0,

@@ -299,14 +299,15 @@ int cvo_register_hypotheses_dev(cvo_handle *h, cvo_gpu_cloud *src, cvo_gpu_cloud
                                 float T_out[16], int *best, float *cos_out, double *secs);
 
 /* ------------------------------------------------------------ autotuner */
-/* The association's grid cell size for search radius r and source tiles of diagonal
- * ext is max(r / div_r, (ext + 2 r) / div_ext).  cvo_autotune_dev times one
+/* How finely the association's candidate test divides the targets among warps: the splits
+ * per tile of 32 source rows are the default ones times (div_r / 4) (div_ext / 8).
+ * cvo_autotune_dev times one
  * association pass of (src, tgt) at pose T and lengthscale ell (<= 0: ell_init) for
  * each candidate (div_r in {2, 3, 4, 6} x div_ext in {4, 8, 16}; median of reps), then
- * the best of these with 1 to 3 resident blocks per SM, and keeps the fastest for every
- * later batch with the same (F, C, log2 rows) key (the arrays list all 15 candidates).  The
- * kernel matrix does not depend on the choice (kept pairs are defined by index order);
- * only the candidate work per row does.  Arrays (max_configs entries, may be NULL)
+ * the best of these with work items for 1 to 3 blocks of four warps per SM, and keeps the
+ * fastest for every later batch with the same (F, C, log2 rows) key (the arrays list all
+ * 15 candidates).  The kernel matrix does not depend on the choice (kept pairs are defined
+ * by index order); only how the work spreads does.  Arrays (max_configs entries, may be NULL)
  * receive every candidate and its time in ms; best its index.  No reference
  * counterpart: the reference's block size and kd-tree are compile-time choices
  * (CMakeLists.txt:473-558, src/experiments/cuda_performance_tune.cu:3-45). */
@@ -316,13 +317,13 @@ int cvo_autotune_dev(cvo_handle *h, cvo_gpu_cloud *src, cvo_gpu_cloud *tgt, cons
  * CVO_ERR_INVALID_ARG and the defaults (4, 8) for a key that was never tuned. */
 int cvo_tune_set(cvo_handle *h, int F, int C, int64_t rows, float div_r, float div_ext);
 int cvo_tune_get(const cvo_handle *h, int F, int C, int64_t rows, float *div_r, float *div_ext);
-/* The same with the launch dimension: after the 12 cell sizes, cvo_autotune_launch_dev
- * times the best one with 1, 2 and 3 resident association blocks per SM (0 = as many as
- * the occupancy allows, the default) and keeps the fastest of all 15; blocks_per_sm
- * receives each candidate's value.  Like the cell size, the choice changes no result.
- * The cell size applies to later batches of pairs of the key's size; the blocks per SM
- * only to batches with as many work items (128 source rows each) as the tuned pair, i.e.
- * single-pair batches of that size (batches of many pairs keep the occupancy default).
+/* The same with the launch dimension: after the 12 divisions, cvo_autotune_launch_dev
+ * times the best one with work items for 1, 2 and 3 blocks of four warps per SM (0 = about
+ * two items per resident warp, the default) and keeps the fastest of all 15; blocks_per_sm
+ * receives each candidate's value.  Like the division, the choice changes no result.
+ * The division applies to later batches of pairs of the key's size; the blocks per SM
+ * only to batches of about as many source rows as the tuned pair, i.e.
+ * single-pair batches of that size (batches of many pairs keep the default).
  * No reference counterpart (its block sizes are compile-time, CMakeLists.txt:473-558). */
 int cvo_autotune_launch_dev(cvo_handle *h, cvo_gpu_cloud *src, cvo_gpu_cloud *tgt, const float T[16], float ell,
                             int reps, int max_configs, int *n_configs, float *div_r, float *div_ext,

@@ -54,51 +54,16 @@ __device__ __forceinline__ float xform_row(const float *r, float t, float x, flo
   return fa(fa(fa(fm(r[0], x), fm(r[1], y)), fm(r[2], z)), t);
 }
 
-__host__ __device__ __forceinline__ unsigned long long cell_key(int cx, int cy, int cz) {
-  return ((unsigned long long)(unsigned)cx << 42) | ((unsigned long long)(unsigned)cy << 21) |
-         (unsigned long long)(unsigned)cz;
+// Order-preserving map between floats and ints (its own inverse), for the warp's integer
+// minimum and maximum instructions.  A NaN becomes an extreme value and comes back a NaN.
+__device__ __forceinline__ int float_order(int i) { return i ^ ((i >> 31) & 0x7FFFFFFF); }
+__device__ __forceinline__ float warp_fmin(float v) {
+  return __int_as_float(float_order(__reduce_min_sync(FULLMASK, float_order(__float_as_int(v)))));
 }
-
-__host__ __device__ __forceinline__ unsigned long long cell_hash(unsigned long long k) {
-  k ^= k >> 33;
-  k *= 0xff51afd7ed558ccdull;
-  k ^= k >> 33;
-  k *= 0xc4ceb9fe1a85ec53ull;
-  k ^= k >> 33;
-  return k;
-}
-
-// Returns (start, count) of a grid cell, (0, 0) if empty or outside the grid.
-__device__ __forceinline__ int2 grid_lookup(const GridDesc &g, int cx, int cy, int cz) {
-  if (cx < 0 || cy < 0 || cz < 0 || cx >= g.dimx || cy >= g.dimy || cz >= g.dimz) return make_int2(0, 0);
-  unsigned long long key = cell_key(cx, cy, cz);
-  unsigned int mask = (1u << g.tbits) - 1u;
-  unsigned int slot = (unsigned int)cell_hash(key) & mask;
-  for (unsigned int probe = 0; probe <= mask; probe++) {
-    unsigned long long k = __ldg(&g.keys[slot]);
-    if (k == key) return make_int2(__ldg(&g.cstart[slot]), __ldg(&g.ccount[slot]));
-    if (k == kEmptyKey) return make_int2(0, 0);
-    slot = (slot + 1u) & mask;
-  }
-  return make_int2(0, 0);
-}
-
-__device__ __forceinline__ float warp_min(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(FULLMASK, v, o));
-  return v;
-}
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(FULLMASK, v, o));
-  return v;
+__device__ __forceinline__ float warp_fmax(float v) {
+  return __int_as_float(float_order(__reduce_max_sync(FULLMASK, float_order(__float_as_int(v)))));
 }
 __device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULLMASK, v, o);
-  return v;
-}
-__device__ __forceinline__ float warp_sumf(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULLMASK, v, o);
   return v;
@@ -108,12 +73,6 @@ __device__ __forceinline__ int warp_sumi(int v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULLMASK, v, o);
   return v;
 }
-__device__ __forceinline__ int warp_maxi(int v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(FULLMASK, v, o));
-  return v;
-}
-
 // Shared-memory address of a generic pointer (for ldmatrix).
 __device__ __forceinline__ uint32_t smem_addr(const void *p) {
   return (uint32_t)__cvta_generic_to_shared(p);

@@ -13,7 +13,6 @@
 #include <cstdio>
 #include "cvo_internal.h"
 #include "cvo_kernels.cuh"
-#include "cvo_assoc_cta.cuh"
 #include "cvo_lie.cuh"
 
 namespace cvo_gb {
@@ -21,93 +20,6 @@ namespace cvo_gb {
 namespace {
 
 constexpr int kChunk = 8;
-
-// ------------------------------------------------------------------ reduce
-// Per-pair FP64 sums of the per-row partials written by k_rowsum.
-__global__ void __launch_bounds__(kReduceThreads) k_reduce(BatchDev B, KParams K) {
-  __shared__ double sh[kReduceThreads / 32][10];
-  __shared__ bool last;
-  const int blk = blockIdx.x;
-  if (blk >= B.total_rblocks) return;
-  const int p = find_segment(B.rblk_off, B.npairs, blk);
-  PairDev *P = &B.pairs[p];
-  if (P->done) return;
-  const int b = blk - B.rblk_off[p];
-  const int nb = B.rblk_off[p + 1] - B.rblk_off[p];
-  const int n = P->n;
-  double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  int mx = 0;
-  for (int r = b * kReduceRows + threadIdx.x; r < min(n, (b + 1) * kReduceRows); r += kReduceThreads) {
-    const float4 *rs = reinterpret_cast<const float4 *>(P->row_sums + (size_t)r * 8);
-    float4 a0 = rs[0], a1 = rs[1];
-    acc[0] += a0.x; acc[1] += a0.y; acc[2] += a0.z; acc[3] += a0.w;
-    acc[4] += a1.x; acc[5] += a1.y; acc[6] += a1.z;
-    int z = P->nnz_row[r];
-    acc[7] += (double)z;
-    mx = max(mx, z);
-  }
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < 8; k++) acc[k] = warp_sum(acc[k]);
-  mx = warp_maxi(mx);
-  if (lane == 0) {
-    for (int k = 0; k < 8; k++) sh[w][k] = acc[k];
-    sh[w][8] = (double)mx;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double out[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int ww = 0; ww < kReduceThreads / 32; ww++) {
-      for (int k = 0; k < 8; k++) out[k] += sh[ww][k];
-      out[8] = fmax(out[8], sh[ww][8]);
-    }
-    for (int k = 0; k < 9; k++) P->part[(size_t)b * kPartStride + k] = out[k];
-    __threadfence();
-    unsigned prev = atomicAdd(&P->counter[0], 1u);
-    last = (prev == (unsigned)(nb - 1));
-  }
-  __syncthreads();
-  if (!last || threadIdx.x != 0) return;
-  __threadfence();
-  double tot[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  volatile double *pv = P->part;
-  for (int bb = 0; bb < nb; bb++) {
-    for (int k = 0; k < 8; k++) tot[k] += pv[(size_t)bb * kPartStride + k];
-    tot[8] = fmax(tot[8], pv[(size_t)bb * kPartStride + 8]);
-  }
-  P->counter[0] = 0;
-  // algorithmic bytes of this pair's association pass: every source and target
-  // record once, the per-row count, and the ELL entries when they are written
-  atomicAdd(B.assoc_bytes, (double)(P->n + P->m) * B.record_bytes + 4.0 * P->n +
-                               (P->mode != MODE_IP ? 8.0 * tot[7] : 0.0));
-  for (int k = 0; k < 6; k++) P->grad[k] = tot[k];
-  P->asum = tot[6];
-  P->nnz_sum = (long long)tot[7];
-  P->max_row = (int)tot[8];
-  if (P->mode == MODE_ALIGN) {
-    // float normalisation of the stacked gradient (CvoGPU.cu:2096-2104)
-    float f[6];
-    for (int k = 0; k < 6; k++) f[k] = (float)tot[k];
-    float s = 0.f;
-    for (int k = 0; k < 6; k++) s = fa(s, fm(f[k], f[k]));
-    if (s > 0.f) {
-      float nr = __fsqrt_rn(s);
-      for (int k = 0; k < 6; k++) f[k] = __fdiv_rn(f[k], nr);
-    }
-    for (int k = 0; k < 6; k++) P->xi[k] = f[k];
-  }
-}
-
-// Picks the finest grid level whose cells serve the largest search radius.
-__device__ void choose_level(PairDev *P, const KParams &K, float max_norm) {
-  float l = range_ell(P->ell, max_norm);
-  float r = K.use_geo ? sqrtf(geo_d2_thres(l, K.log_geo)) : 0.f;
-  int lv = P->nlevels - 1;
-  for (int i = 0; i < P->nlevels; i++)
-    if (P->level_r[i] >= r) { lv = i; break; }
-  P->level = lv;
-  P->rq_max = r;
-}
 
 __device__ void pose_to_rinv(PairDev *P) {
   for (int r = 0; r < 3; r++)
@@ -148,14 +60,13 @@ __device__ bool indicator_update(PairDev *P, const KParams &K, float ind) {
 }
 
 // Scalar tail of one iteration of align_impl (src/cvo/CvoGPU.cu:1339-1433).
-__device__ void finalize_iteration(BatchDev &B, PairDev *P, const KParams &K, float src_max_norm) {
+__device__ void finalize_iteration(BatchDev &B, PairDev *P, const KParams &K) {
   const int k = P->iter;
   double step = step_from_terms(P->bcde, (double)K.min_step, (double)K.max_step);
   P->step = step;
   const float *xi = P->xi;
   float wn = __fsqrt_rn(fa(fa(fm(xi[0], xi[0]), fm(xi[1], xi[1])), fm(xi[2], xi[2])));
   float vn = __fsqrt_rn(fa(fa(fm(xi[3], xi[3]), fm(xi[4], xi[4])), fm(xi[5], xi[5])));
-  P->level_used = P->level;
   if ((double)wn < (double)K.eps && (double)vn < (double)K.eps) {
     if (wn < 1e-8f && vn < 1e-8f) P->ret = -1;
     P->done = 1;
@@ -205,16 +116,14 @@ __device__ void finalize_iteration(BatchDev &B, PairDev *P, const KParams &K, fl
   if (P->iter >= K.max_iter) {
     P->done = 1;
     atomicSub(B.active, 1);
-    return;
   }
-  choose_level(P, K, src_max_norm);
 }
 
 // -------------------------------------------------------------------- step
 // Taylor step-size terms (compute_step_size_xi + compute_step_size_poly_coeff,
 // src/cvo/CvoGPU.cu:333-462) per ELL row in FP32, FP64 across rows; the last
 // block of a pair finishes the iteration.
-__global__ void __launch_bounds__(kStepThreads) k_step(BatchDev B, KParams K, const float *src_max_norm) {
+__global__ void __launch_bounds__(kStepThreads) k_step(BatchDev B, KParams K) {
   __shared__ double sh[kStepThreads / 32][4];
   __shared__ bool last;
   const int blk = blockIdx.x;
@@ -294,7 +203,7 @@ __global__ void __launch_bounds__(kStepThreads) k_step(BatchDev B, KParams K, co
     for (int k = 0; k < 4; k++) tot[k] += pv[(size_t)bb * kPartStride + k];
   P->counter[1] = 0;
   for (int k = 0; k < 4; k++) P->bcde[k] = tot[k];
-  finalize_iteration(B, P, K, src_max_norm[p]);
+  finalize_iteration(B, P, K);
 }
 
 // ----------------------------------------------------- association export
@@ -312,55 +221,37 @@ __global__ void k_export(const PairDev *P, const int *row_start, int *cols, floa
 }
 
 // --------------------------------------------------------- template dispatch
-using AssocFn = void (*)(BatchDev, KParams);
+using CandFn = void (*)(BatchDev, KParams);
+using RowsFn = void (*)(BatchDev, KParams, int);
+
+struct AssocKernels {
+  CandFn cand = nullptr;
+  RowsFn rows = nullptr;
+};
 
 // Feature rows are stored as ceil(F/4) float4 chunks; label rows as 5 or 9
 // chunks (C <= 20 or C <= 36, padded at upload), so the chunk counts below are
 // the storage strides of the clouds.
 template <int FC, int LC, bool G>
-static int pick_assoc(AssocFn &a, AssocFn &rs, size_t &smem, int &per_sm) {
-  a = k_assoc_cta<FC, LC, G>;
-  rs = k_rescan<FC, LC, G>;
-  smem = CtaSmem<FC, LC, G>::kBytes;
-  // opt in above the 48 KB default once per device (setting it twice is harmless)
-  static unsigned long long set_mask = 0;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return CVO_ERR_CUDA; }
-  const unsigned long long bit = 1ull << (dev & 63);
-  if (!(set_mask & bit)) {
-    if (cudaFuncSetAttribute(a, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-      cudaGetLastError();
-      return CVO_ERR_CUDA;
-    }
-    // the selection keeps kSelBlocksPerSm blocks of static shared memory resident: ask
-    // for the largest shared-memory share of the unified L1 (a hint; failure is harmless)
-    if (cudaFuncSetAttribute(k_select, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess)
-      cudaGetLastError();
-    set_mask |= bit;
+static int pick_assoc(AssocKernels *a) {
+  a->cand = k_cand<FC>;
+  a->rows = k_rows<FC, LC, G>;
+  // opt in above the 48 KB default (setting it again is harmless)
+  if (cudaFuncSetAttribute(a->rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem_bytes(kRowWindow)) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    return CVO_ERR_CUDA;
   }
-  static int occ[64] = {0};
-  if (occ[dev & 63] == 0) {
-    int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, a, kCtaRows, smem) != cudaSuccess || nb < 1) {
-      cudaGetLastError();
-      nb = 1;
-    }
-    occ[dev & 63] = nb;
-  }
-  per_sm = occ[dev & 63];
   return 0;
 }
 
-int select_kernels(const KParams &K, int F, int C, AssocFn &a, AssocFn &rs, size_t &smem, int &per_sm) {
+int select_kernels(const KParams &K, int F, int C, AssocKernels *a) {
   int fch = K.use_int ? (F + 3) / 4 : 0;
   int lch = K.use_sem ? label_chunks(C) : 0;
   bool gt = K.use_gtype != 0;
   if (fch > 2 || lch > 9) return CVO_ERR_UNSUPPORTED;
-#define CVO_PICK(FC, LC)                                       \
-  if (fch == FC && lch == LC) {                                \
-    return gt ? pick_assoc<FC, LC, true>(a, rs, smem, per_sm) : pick_assoc<FC, LC, false>(a, rs, smem, per_sm); \
-  }
+#define CVO_PICK(FC, LC) \
+  if (fch == FC && lch == LC) return gt ? pick_assoc<FC, LC, true>(a) : pick_assoc<FC, LC, false>(a);
   CVO_PICK(0, 0) CVO_PICK(1, 0) CVO_PICK(2, 0)
   CVO_PICK(0, 5) CVO_PICK(1, 5) CVO_PICK(2, 5)
   CVO_PICK(0, 9) CVO_PICK(1, 9) CVO_PICK(2, 9)
@@ -459,11 +350,13 @@ KParams make_kparams(const cvo_params &p) {
   k.two_c2 = 2.0 * (double)k.c2;
   // Kernel value bound: a <= sigma^2 c_sigma^2 s_sigma^2 exp(-(d2/(2l^2) + d2c/(2c^2))) (the geometric-type
   // factor is <= 1), so a > sp_thres needs the exponent below ln(sigma^2 c_sigma^2 s_sigma^2 / sp_thres).
+  // Without the geometric kernel the colour term alone bounds the value.
   k.use_mma = 0;
   k.mma_tau = 0.f;
-  if (k.use_geo && p.sp_thres > 0.f && k.sigma2 > 0.f && (!k.use_int || k.c_sigma2 > 0.f) &&
+  if ((k.use_geo || k.use_int) && p.sp_thres > 0.f && (!k.use_geo || k.sigma2 > 0.f) && (!k.use_int || k.c_sigma2 > 0.f) &&
       (!k.use_sem || k.s_sigma_sq > 0.f)) {
-    double lb = std::log((double)k.sigma2) - std::log((double)p.sp_thres);
+    double lb = -std::log((double)p.sp_thres);
+    if (k.use_geo) lb += std::log((double)k.sigma2);
     if (k.use_int) lb += std::log((double)k.c_sigma2);
     if (k.use_sem) lb += std::log((double)k.s_sigma_sq);
     if (k.val_scale > 0.f) lb += std::log((double)k.val_scale);
@@ -473,31 +366,12 @@ KParams make_kparams(const cvo_params &p) {
   return k;
 }
 
-// Cell size for search radius r and source tiles of diagonal ext: small against r
-// (the distance test on cells then trims the query box towards the union of balls)
-// while keeping a tile's box at about 8 cells per axis.
-static float cell_for_radius(float r, float ext, const TuneConfig &c) {
-  return std::max(r / c.cell_div_r, (ext + 2.f * r) / c.cell_div_ext);
-}
-// Largest radius a cell of size hc serves (inverse of cell_for_radius).
-static float radius_for_cell(float hc, float ext, const TuneConfig &c) {
-  return std::max(0.f, std::min(c.cell_div_r * hc, 0.5f * (c.cell_div_ext * hc - ext)));
-}
-
-long long tune_items(long long rows) { return (rows + 32 * kCtaWarps - 1) / (32 * kCtaWarps); }
+long long tune_items(long long rows) { return (rows + 127) / 128; }
 
 long long tune_key(int F, int C, long long rows) {
   int b = 0;
   while ((1LL << (b + 1)) <= rows && b < 40) b++;
   return ((long long)F << 32) | ((long long)C << 16) | b;
-}
-
-static float host_range_ell(float ell, float dist) { return (float)(((double)dist / 500.0 + 1.0) * (double)ell); }
-static float host_radius(const KParams &K, float ell, float norm) {
-  if (!K.use_geo) return INFINITY;
-  float l = host_range_ell(ell, norm);
-  float d2t = (float)(-2.0 * (double)l * (double)l * (double)K.log_geo);
-  return std::sqrt(std::max(d2t, 0.f));
 }
 
 // ------------------------------------------------------------ batch setup
@@ -506,15 +380,18 @@ namespace {
 struct BatchHost {
   BatchDev B;
   std::vector<PairDev> pairs;
-  std::vector<int> tile_off, row_off, tgt_off, rblk_off, sblk_off;
-  float *src_max_norm = nullptr;
-  AssocFn assoc = nullptr, rescan = nullptr;
-  size_t assoc_smem = 0;
-  int sel_blocks = 0;
-  int ov = 0;
-  int assoc_per_sm = 1;
-  int assoc_blocks = 0, xform_blocks = 0;
+  std::vector<int> item_off, tgt_off, rblk_off, sblk_off;
+  AssocKernels fn;
+  int cand_blocks = 0, xform_blocks = 0;
+  int window_words = 0;
+  size_t row_smem = 0;
 };
+
+// Work items that keep the candidate test's warps busy: about two per resident warp slot,
+// so that tiles of uneven cost even out.  Fewer tiles than that are split over their
+// targets (each split repeats the tile's setup, some 400 instructions against 5,000 or
+// more for a tile of a 50k cloud).
+constexpr long long kCandItems = 10240;
 
 // Lays out every device buffer of a batch in the handle's workspace.
 int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs, const std::vector<DevCloud *> &tgts,
@@ -526,134 +403,105 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     if (srcs[p]->F != F || tgts[p]->F != F || srcs[p]->C != C || tgts[p]->C != C) return CVO_ERR_INVALID_ARG;
     if (K.use_gtype && (!srcs[p]->has_geo || !tgts[p]->has_geo)) return CVO_ERR_INVALID_ARG;
   }
-  int rc = select_kernels(K, F, C, bh->assoc, bh->rescan, bh->assoc_smem, bh->assoc_per_sm);
+  int rc = select_kernels(K, F, C, &bh->fn);
   if (rc) return rc;
-  // cell-size configuration: forced by the autotuner, else the tuned one for this key, else the default
-  // The cell size is keyed by the pairs' size (it sets the work per row); the blocks per
-  // SM by the batch's number of work items (it sets how the items spread over the SMs),
-  // so a value tuned on one pair does not carry over to a batch of many.
+  // division of the candidate test: forced by the autotuner, else the tuned one for this
+  // key, else the default.  The splits are keyed by the pairs' size (it sets the work per
+  // tile); the items per SM by the batch's number of work items (it sets how they spread
+  // over the SMs), so a value tuned on one pair does not carry over to a batch of many.
   TuneConfig tc;
+  long long tiles = 0, maxn = 0;
+  int maxm = 1;
+  for (int p = 0; p < np; p++) {
+    tiles += group_count(srcs[p]->n);
+    maxn = std::max<long long>(maxn, srcs[p]->n);
+    maxm = std::max(maxm, tgts[p]->n);
+  }
   if (h->tune_force) {
     tc = *h->tune_force;
   } else {
-    long long maxn = 0, items = 0;
-    for (int p = 0; p < np; p++) {
-      maxn = std::max<long long>(maxn, srcs[p]->n);
-      items += (srcs[p]->n + 32 * kCtaWarps - 1) / (32 * kCtaWarps);
-    }
+    long long items = 0;
+    for (int p = 0; p < np; p++) items += tune_items(srcs[p]->n);
     auto it = h->tuned.find(tune_key(F, C, maxn));
     if (it != h->tuned.end()) tc = it->second;
     tc.blocks_per_sm = 0;
     auto ib = h->tuned_bps.find(tune_key(F, C, items));
     if (ib != h->tuned_bps.end()) tc.blocks_per_sm = ib->second;
   }
-  // grid levels per pair
-  std::vector<std::vector<GridDesc>> lv(np);
-  std::vector<std::vector<float>> lr(np);
-  for (int p = 0; p < np; p++) {
-    DevCloud *t = tgts[p];
-    const float ext = srcs[p]->tile_ext;
-    std::vector<int> exps;
-    if (!K.use_geo) {
-      exps.push_back(1000);
-    } else {
-      float ell_hi = ell0[p];
-      float ell_lo = (mode == MODE_ALIGN) ? std::min(K.ell_min, ell_hi) : ell_hi;
-      float r_hi = host_radius(K, ell_hi, srcs[p]->max_norm);
-      float r_lo = host_radius(K, ell_lo, 0.f);
-      int e_hi = level_for_radius(cell_for_radius(r_hi, ext, tc)), e_lo = level_for_radius(cell_for_radius(r_lo, ext, tc));
-      if (e_hi - e_lo + 1 > 24) e_lo = e_hi - 23;
-      for (int e = e_lo; e <= e_hi; e++) exps.push_back(e);
-    }
-    for (int e : exps) {
-      GridDesc g;
-      if ((rc = cloud_level(h, t, e, &g))) return rc;
-      lv[p].push_back(g);
-      lr[p].push_back(e >= 1000 ? INFINITY : radius_for_cell(g.h, ext, tc));
-    }
-  }
+  const int sms = h->num_sms > 0 ? h->num_sms : 152;
+  const double want = (tc.blocks_per_sm > 0 ? 4.0 * tc.blocks_per_sm * sms : (double)kCandItems) *
+                      (tc.cell_div_r / 4.0) * (tc.cell_div_ext / 8.0);
+  const int splits = (int)std::min<double>(kMaxSplits, std::max(1.0, std::ceil(want / (double)std::max<long long>(tiles, 1))));
   // sizes
-  bh->tile_off.assign(np + 1, 0);
-  bh->row_off.assign(np + 1, 0);
+  bh->item_off.assign(np + 1, 0);
   bh->tgt_off.assign(np + 1, 0);
   bh->rblk_off.assign(np + 1, 0);
   bh->sblk_off.assign(np + 1, 0);
   size_t bytes = 0;
   auto add = [&](size_t b) { bytes += (b + 255) & ~(size_t)255; };
-  int max_part_blocks = 0;
-  // spill-list entries per row (kept pairs beyond cap, row-major): up to kSelMax, at most 16 GB for the
-  // batch (only the entries rows actually spill are ever written; a row that overflows its list is
-  // rescanned in index order, which costs far more than the memory)
+  // candidate entries per row: one per target group, at most 16 GB for the batch (a row
+  // that needs more is evaluated by an index-ordered scan of the targets)
   long long rows_all = 0;
   for (int p = 0; p < np; p++) rows_all += srcs[p]->n;
-  int ov = kSelMax;
-  if (rows_all > 0) ov = (int)std::min<long long>(ov, (16ll << 30) / (8ll * rows_all));
-  ov &= ~3;   // spill rows start 16-byte aligned (k_select reads them with 16-byte loads)
-  bh->ov = ov;
+  const int most = rows_all > 0 ? (int)std::min<long long>(1 << 20, (16ll << 30) / (8ll * rows_all)) : 1;
   const int ell_ld = (std::max(capmax, 1) + 3) & ~3;   // 16-byte aligned ELL rows
+  const bool ell = mode != MODE_IP;                    // an inner product needs no kernel matrix
+  std::vector<int> sp(np), caps(np);
   for (int p = 0; p < np; p++) {
     int n = srcs[p]->n, m = tgts[p]->n;
-    // tiles per pair padded to whole association blocks (kCtaWarps tiles of one pair)
-    bh->tile_off[p + 1] = bh->tile_off[p] + ((n + 32 * kCtaWarps - 1) / (32 * kCtaWarps)) * kCtaWarps;
-    bh->row_off[p + 1] = bh->row_off[p] + n;
+    const int ns = group_count(group_count(m));
+    sp[p] = std::max(1, std::min(splits, ns));
+    caps[p] = std::max(1, std::min(kGroup * ((ns + sp[p] - 1) / sp[p]), most / sp[p]));
+    if (!K.use_mma) sp[p] = caps[p] = 1;
+    bh->item_off[p + 1] = bh->item_off[p] + group_count(n) * sp[p];
     bh->tgt_off[p + 1] = bh->tgt_off[p] + m;
-    int rb = (n + kReduceRows - 1) / kReduceRows, sb = (n + kStepThreads - 1) / kStepThreads;
+    int rb = (n + kRowsPerBlock - 1) / kRowsPerBlock, sb = (n + kStepThreads - 1) / kStepThreads;
     bh->rblk_off[p + 1] = bh->rblk_off[p] + rb;
     bh->sblk_off[p + 1] = bh->sblk_off[p] + sb;
-    max_part_blocks = std::max(max_part_blocks, std::max(rb, sb));
     add(sizeof(float4) * m);                                     // ycur
     add(sizeof(float4) * m);                                     // yorig
-    add(sizeof(int) * (size_t)n * ell_ld);                       // ELL (every mode: the row selection uses it)
-    add(sizeof(float) * (size_t)n * ell_ld);
-    add(sizeof(int2) * (size_t)n * ov);                          // spill lists
+    add(ell ? sizeof(int) * (size_t)n * ell_ld : 0);             // ELL
+    add(ell ? sizeof(float) * (size_t)n * ell_ld : 0);
+    add(sizeof(uint2) * (size_t)n * sp[p] * caps[p]);            // candidate entries
+    add(sizeof(int2) * (size_t)n * sp[p]);                       // entry counts
     add(sizeof(int) * n);                                        // nnz_row
-    add(sizeof(float) * 8 * (size_t)n);                          // row_sums
     add(sizeof(double) * kPartStride * (size_t)std::max(rb, sb)); // partials
     add(sizeof(unsigned) * 2);
-    add(sizeof(GridDesc) * lv[p].size());
+    bytes += 9 * 256;                                            // room for empty pieces
   }
-  const int total_rows = bh->row_off[np];
   add(sizeof(PairDev) * np);
-  add(sizeof(int) * (np + 1) * 5);
-  add(sizeof(int) * 7);
-  add(sizeof(float) * np);
-  add(sizeof(int4) * (size_t)total_rows);                        // selection list
-  add(sizeof(int4) * (size_t)total_rows);                        // rescan list
-  const int n_items = bh->tile_off[np] / kCtaWarps;
-  add(sizeof(int) * (size_t)std::max(n_items, 1) * kCtaWarps);   // work-item order (split items: 4 entries)
-  add(sizeof(int) * (size_t)std::max(n_items, 1));               // work-item cost
-  add(sizeof(int));                                              // entries of the order
+  add(sizeof(int) * (np + 1) * 4);
+  add(sizeof(int) * 4);
+  add(sizeof(double));
   if ((rc = ensure_workspace(h, bytes))) return rc;
   Arena ar;
   ar.base = h->ws->dev;
   ar.cap = h->ws->dev_cap;
   bh->pairs.assign(np, PairDev());
-  std::vector<GridDesc *> lvdev(np);
-  std::vector<std::pair<void *, std::pair<const void *, size_t>>> uploads;
+  int active = 0;
   for (int p = 0; p < np; p++) {
     PairDev &P = bh->pairs[p];
     memset(&P, 0, sizeof(P));
     DevCloud *s = srcs[p], *t = tgts[p];
     P.n = s->n; P.m = t->n; P.F = F; P.C = C;
-    P.xs = s->spos; P.xf = s->sfeat; P.xl = s->slab; P.xg = s->sgeo; P.sperm = s->sperm;
+    P.xs = s->spos; P.xf = s->sfeat; P.xl = s->slab; P.xg = s->sgeo; P.sbox = s->gbox;
+    P.tpos = t->spos; P.tperm = t->sperm; P.tfs = t->sfeat; P.tbox = t->gbox; P.tsup = t->sbox;
+    P.groups = group_count(t->n);
     P.ycur = ar.take<float4>(t->n);
     P.yorig = ar.take<float4>(t->n);
-    P.A_j = ar.take<int>((size_t)s->n * ell_ld);
-    P.A_v = ar.take<float>((size_t)s->n * ell_ld);
+    P.A_j = ar.take<int>(ell ? (size_t)s->n * ell_ld : 0);
+    P.A_v = ar.take<float>(ell ? (size_t)s->n * ell_ld : 0);
     P.ld = ell_ld;
-    P.ovf = ar.take<int2>((size_t)s->n * ov);
-    P.ov = ov;
+    P.splits = sp[p];
+    P.cap_split = caps[p];
+    P.cand_pitch = sp[p] * caps[p];
+    P.cand = ar.take<uint2>((size_t)s->n * P.cand_pitch);
+    P.cand_cnt = ar.take<int2>((size_t)s->n * sp[p]);
     P.tf = t->feat; P.tl = t->lab; P.tg = t->geo;
     P.nnz_row = ar.take<int>(s->n);
-    P.row_sums = ar.take<float>(8 * (size_t)s->n);
     int rb = bh->rblk_off[p + 1] - bh->rblk_off[p], sb = bh->sblk_off[p + 1] - bh->sblk_off[p];
     P.part = ar.take<double>(kPartStride * (size_t)std::max(rb, sb));
     P.counter = ar.take<unsigned>(2);
-    lvdev[p] = ar.take<GridDesc>(lv[p].size());
-    uploads.push_back({lvdev[p], {lv[p].data(), sizeof(GridDesc) * lv[p].size()}});
-    P.levels = lvdev[p];
-    P.nlevels = (int)lv[p].size();
-    for (int i = 0; i < P.nlevels && i < 24; i++) P.level_r[i] = lr[p][i];
     P.capmax = capmax;
     P.mode = mode;
     for (int r = 0; r < 3; r++) {
@@ -669,87 +517,48 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     }
     P.ell = ell0[p];
     P.cap = capmax;
-    // initial level
-    float r0 = host_radius(K, P.ell, s->max_norm);
-    P.level = P.nlevels - 1;
-    for (int i = 0; i < P.nlevels; i++)
-      if (P.level_r[i] >= r0) { P.level = i; break; }
-    P.level_used = P.level;
-    P.rq_max = r0;
     P.done = (s->n == 0 || t->n == 0) ? 1 : 0;
+    if (!P.done) active++;
   }
   PairDev *pairs_d = ar.take<PairDev>(np);
-  int *offs_d = ar.take<int>((size_t)(np + 1) * 5);
-  int *ctr_d = ar.take<int>(7);
+  int *offs_d = ar.take<int>((size_t)(np + 1) * 4);
+  int *ctr_d = ar.take<int>(4);
   double *bytes_d = ar.take<double>(1);
-  bh->src_max_norm = ar.take<float>(np);
-  int4 *sel_list_d = ar.take<int4>(total_rows);
-  int4 *scan_list_d = ar.take<int4>(total_rows);
-  int *item_order_d = ar.take<int>((size_t)std::max(n_items, 1) * kCtaWarps);
-  int *item_cost_d = ar.take<int>((size_t)std::max(n_items, 1));
-  int *n_order_d = ar.take<int>(1);
-  {
-    // first pass: every item whole, in index order
-    std::vector<int> ord(std::max(n_items, 1));
-    for (int i = 0; i < (int)ord.size(); i++) ord[i] = (i << 3) | kItemWhole;
-    CVO_CUDA_TRY(h, cudaMemcpyAsync(item_order_d, ord.data(), sizeof(int) * ord.size(), cudaMemcpyHostToDevice,
-                                    h->stream));
-    CVO_CUDA_TRY(h, cudaMemsetAsync(item_cost_d, 0, sizeof(int) * ord.size(), h->stream));
-    const int n_ord = n_items;
-    CVO_CUDA_TRY(h, cudaMemcpyAsync(n_order_d, &n_ord, sizeof(int), cudaMemcpyHostToDevice, h->stream));
-  }
   // zero counters of every pair
   for (int p = 0; p < np; p++) CVO_CUDA_TRY(h, cudaMemsetAsync(bh->pairs[p].counter, 0, 2 * sizeof(unsigned), h->stream));
-  for (auto &u : uploads) CVO_CUDA_TRY(h, cudaMemcpyAsync(u.first, u.second.first, u.second.second, cudaMemcpyHostToDevice, h->stream));
   CVO_CUDA_TRY(h, cudaMemcpyAsync(pairs_d, bh->pairs.data(), sizeof(PairDev) * np, cudaMemcpyHostToDevice, h->stream));
   std::vector<int> offs;
-  for (auto *v : {&bh->tile_off, &bh->row_off, &bh->tgt_off, &bh->rblk_off, &bh->sblk_off}) offs.insert(offs.end(), v->begin(), v->end());
+  for (auto *v : {&bh->item_off, &bh->tgt_off, &bh->rblk_off, &bh->sblk_off}) offs.insert(offs.end(), v->begin(), v->end());
   CVO_CUDA_TRY(h, cudaMemcpyAsync(offs_d, offs.data(), sizeof(int) * offs.size(), cudaMemcpyHostToDevice, h->stream));
-  std::vector<float> mn(np);
-  int active = 0;
-  for (int p = 0; p < np; p++) { mn[p] = srcs[p]->max_norm; if (!bh->pairs[p].done) active++; }
-  CVO_CUDA_TRY(h, cudaMemcpyAsync(bh->src_max_norm, mn.data(), sizeof(float) * np, cudaMemcpyHostToDevice, h->stream));
-  int ctr_h[7] = {0, 0, active, 0, 0, 0, 0};
+  int ctr_h[4] = {0, 0, active, 0};
   CVO_CUDA_TRY(h, cudaMemcpyAsync(ctr_d, ctr_h, sizeof(ctr_h), cudaMemcpyHostToDevice, h->stream));
   CVO_CUDA_TRY(h, cudaMemsetAsync(bytes_d, 0, sizeof(double), h->stream));
   CVO_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   BatchDev &B = bh->B;
   memset(&B, 0, sizeof(B));
   B.npairs = np;
-  B.total_warps = bh->tile_off[np];
-  B.total_rows = total_rows;
+  B.total_items = bh->item_off[np];
+  B.total_rows = (int)rows_all;
   B.total_targets = bh->tgt_off[np];
   B.pairs = pairs_d;
-  B.tile_off = offs_d;
-  B.row_off = offs_d + (np + 1);
-  B.tgt_off = offs_d + 2 * (np + 1);
-  B.rblk_off = offs_d + 3 * (np + 1);
-  B.sblk_off = offs_d + 4 * (np + 1);
+  B.item_off = offs_d;
+  B.tgt_off = offs_d + (np + 1);
+  B.rblk_off = offs_d + 2 * (np + 1);
+  B.sblk_off = offs_d + 3 * (np + 1);
   B.total_rblocks = bh->rblk_off[np];
   B.total_sblocks = bh->sblk_off[np];
   B.err = ctr_d + 1;
   B.active = ctr_d + 2;
   B.active_iters = ctr_d + 3;
   B.assoc_bytes = bytes_d;
-  B.sel_list = sel_list_d;
-  B.scan_list = scan_list_d;
-  B.sel_count = ctr_d + 4;
-  B.scan_count = ctr_d + 5;
-  B.assoc_next = ctr_d + 6;
-  B.n_items = n_items;
-  B.item_order = item_order_d;
-  B.item_cost = item_cost_d;
-  B.n_order = n_order_d;
   {
     int fch = K.use_int ? (F + 3) / 4 : 0, lch = K.use_sem ? label_chunks(C) : 0;
     B.record_bytes = 16 + 16 * fch + 16 * lch + (K.use_gtype ? 8 : 0);
   }
-  // persistent association blocks: one wave of resident blocks (work items are taken from a counter),
-  // at most the tuned number per SM
-  const int per_sm = tc.blocks_per_sm > 0 ? std::min(tc.blocks_per_sm, bh->assoc_per_sm) : bh->assoc_per_sm;
-  bh->assoc_blocks = std::max(1, std::min(B.total_warps / kCtaWarps, per_sm * (h->num_sms > 0 ? h->num_sms : 152)));
+  bh->cand_blocks = K.use_mma ? (B.total_items + kCandWarps - 1) / kCandWarps : 0;
   bh->xform_blocks = (B.total_targets + 255) / 256;
-  bh->sel_blocks = std::max(1, std::min(kSelBlocksPerSm * (h->num_sms > 0 ? h->num_sms : 152), (total_rows + 3) / 4));
+  bh->window_words = row_window_words(maxm);
+  bh->row_smem = row_smem_bytes(maxm);
   return 0;
 }
 
@@ -759,36 +568,47 @@ inline void mark(Handle *h, const cudaEvent_t *ev, int k) {
   if (ev) cudaEventRecordWithFlags(ev[k], h->stream, cudaEventRecordExternal);
 }
 
-// ev (optional): 7 events: 0-4 bracket transform, association phase, reduce and step;
-// 5 and 6 split the association phase into the association kernel (+ item order),
-// the selection (k_select + k_rescan) and the row sums.
+// ev (optional): 7 events: 0-4 bracket transform, association phase, (empty) reduce and
+// step; 5 and 6 split the association phase into the candidate test, the row pass and
+// nothing (the row pass sums the gradient).
 void launch_association(Handle *h, BatchHost *bh, const KParams &K, const cudaEvent_t *ev = nullptr) {
   BatchDev &B = bh->B;
   mark(h, ev, 0);
   k_transform<<<std::max(bh->xform_blocks, 1), 256, 0, h->stream>>>(B);
   mark(h, ev, 1);
-  bh->assoc<<<std::max(bh->assoc_blocks, 1), kAssocThreads, bh->assoc_smem, h->stream>>>(B, K);
-  if (B.n_items > 1) {
-    k_order_items<<<1, 1024, 0, h->stream>>>(B.n_items, std::max(bh->assoc_blocks, 1), B.item_cost, B.item_order,
-                                             B.n_order);
+  if (bh->cand_blocks > 0) {
+    bh->fn.cand<<<bh->cand_blocks, 32 * kCandWarps, 0, h->stream>>>(B, K);
     h->launches++;
   }
   mark(h, ev, 5);
-  k_select<<<bh->sel_blocks, kSelThreads, 0, h->stream>>>(B, K);
-  bh->rescan<<<bh->sel_blocks, kSelThreads, 0, h->stream>>>(B, K);
+  bh->fn.rows<<<std::max(B.total_rblocks, 1), 32 * kRowWarps, bh->row_smem, h->stream>>>(B, K, bh->window_words);
   mark(h, ev, 6);
-  k_rowsum<<<std::max((B.total_rows + 255) / 256, 1), 256, 0, h->stream>>>(B, K);
   mark(h, ev, 2);
-  k_reduce<<<std::max(B.total_rblocks, 1), kReduceThreads, 0, h->stream>>>(B, K);
   mark(h, ev, 3);
-  h->launches += 6;
+  h->launches += 2;
 }
 
 void launch_iteration(Handle *h, BatchHost *bh, const KParams &K, const cudaEvent_t *ev = nullptr) {
   launch_association(h, bh, K, ev);
-  k_step<<<std::max(bh->B.total_sblocks, 1), kStepThreads, 0, h->stream>>>(bh->B, K, bh->src_max_norm);
+  k_step<<<std::max(bh->B.total_sblocks, 1), kStepThreads, 0, h->stream>>>(bh->B, K);
   mark(h, ev, 4);
   h->launches += 1;
+}
+
+// What a captured launch sequence of a batch depends on.
+void append_launch_key(const Handle *h, const BatchHost &bh, const KParams &K, std::vector<unsigned char> *key) {
+  auto add = [&](const void *p, size_t n) {
+    const unsigned char *c = static_cast<const unsigned char *>(p);
+    key->insert(key->end(), c, c + n);
+  };
+  add(&bh.B, sizeof(bh.B));
+  add(&K, sizeof(K));
+  add(&bh.fn, sizeof(bh.fn));
+  add(&bh.cand_blocks, sizeof(bh.cand_blocks));
+  add(&bh.xform_blocks, sizeof(bh.xform_blocks));
+  add(&bh.window_words, sizeof(bh.window_words));
+  add(&bh.row_smem, sizeof(bh.row_smem));
+  add(&h->stream, sizeof(h->stream));
 }
 
 int read_pairs(Handle *h, BatchHost *bh) {
@@ -886,22 +706,7 @@ int run_align_batch(Handle *h, const std::vector<DevCloud *> &srcs, const std::v
   constexpr int kEv = 7;
   std::vector<cudaEvent_t> pev;
   std::vector<unsigned char> key;
-  {
-    auto add = [&](const void *p, size_t n) {
-      const unsigned char *c = static_cast<const unsigned char *>(p);
-      key.insert(key.end(), c, c + n);
-    };
-    add(&bh.B, sizeof(bh.B));
-    add(&K, sizeof(K));
-    add(&bh.assoc, sizeof(bh.assoc));
-    add(&bh.rescan, sizeof(bh.rescan));
-    add(&bh.assoc_smem, sizeof(bh.assoc_smem));
-    add(&bh.assoc_blocks, sizeof(bh.assoc_blocks));
-    add(&bh.xform_blocks, sizeof(bh.xform_blocks));
-    add(&bh.sel_blocks, sizeof(bh.sel_blocks));
-    add(&bh.src_max_norm, sizeof(bh.src_max_norm));
-    add(&h->stream, sizeof(h->stream));
-  }
+  append_launch_key(h, bh, K, &key);
   Workspace *ws = h->ws;
   const bool reuse = !h->prof.on && ws->align_exec && ws->align_key == key;
   long long per_chunk = 0;
@@ -1034,8 +839,8 @@ int run_inner_product_pairs(Handle *h, const std::vector<DevCloud *> &srcs, cons
 int autotune_association(Handle *h, DevCloud *src, DevCloud *tgt, const float T[16], float ell, int reps,
                          std::vector<TuneConfig> *configs, std::vector<float> *ms, int *best) {
   NvtxRange nvtx_range("autotune");
-  // candidates: cells of r/2 .. r/6 against the radius, tile-box terms of 4 .. 16 cells,
-  // all with the occupancy's blocks per SM; then 1 .. 3 blocks per SM with the best cells
+  // candidates: 1/4 .. 3 times the default division of the targets among warps, then 4 to
+  // 12 work items per SM with the fastest one's divisors
   const float div_r[] = {2.f, 3.f, 4.f, 6.f};
   const float div_ext[] = {4.f, 8.f, 16.f};
   configs->clear();
@@ -1058,7 +863,7 @@ int autotune_association(Handle *h, DevCloud *src, DevCloud *tgt, const float T[
   for (size_t k = 0; k < configs->size() && !rc; k++) {
     h->tune_force = &(*configs)[k];
     std::vector<double> asum;
-    rc = run_inner_product_pairs(h, {src}, {tgt}, Tv, ell, cap, &asum);   // builds this configuration's levels
+    rc = run_inner_product_pairs(h, {src}, {tgt}, Tv, ell, cap, &asum);   // sizes the workspace
     std::vector<float> t;
     for (int r = 0; r < reps && !rc; r++) {
       cudaEventRecord(e0, h->stream);
@@ -1075,8 +880,7 @@ int autotune_association(Handle *h, DevCloud *src, DevCloud *tgt, const float T[
       if ((*ms)[k] < (*ms)[bi]) bi = (int)k;
     }
   }
-  // then the launch: resident blocks per SM for the fastest cell size (fewer blocks give
-  // each one more items, which can even out a pass whose items differ widely in cost)
+  // then the launch: few work items per SM (less setup, but tiles of uneven cost even out less)
   const int per_sm_max = 4;
   for (int bps = 1; bps < per_sm_max && !rc; bps++) {
     TuneConfig c = (*configs)[bi];
@@ -1167,20 +971,9 @@ int replay_association(Handle *h, BatchHost *bh, const KParams &K, AssocGraph *g
     g->pin_pairs = np;
   }
   std::vector<unsigned char> key;
-  auto add = [&](const void *p, size_t n) {
-    const unsigned char *c = static_cast<const unsigned char *>(p);
-    key.insert(key.end(), c, c + n);
-  };
-  add(&bh->B, sizeof(bh->B));
-  add(&K, sizeof(K));
-  add(&bh->assoc, sizeof(bh->assoc));
-  add(&bh->rescan, sizeof(bh->rescan));
-  add(&bh->assoc_smem, sizeof(bh->assoc_smem));
-  add(&bh->assoc_blocks, sizeof(bh->assoc_blocks));
-  add(&bh->xform_blocks, sizeof(bh->xform_blocks));
-  add(&bh->sel_blocks, sizeof(bh->sel_blocks));
-  add(&g->pin_in, sizeof(g->pin_in));
-  add(&h->stream, sizeof(h->stream));
+  append_launch_key(h, *bh, K, &key);
+  key.insert(key.end(), reinterpret_cast<const unsigned char *>(&g->pin_in),
+             reinterpret_cast<const unsigned char *>(&g->pin_in) + sizeof(g->pin_in));
   if (!g->exec || g->key != key) {
     if (g->exec) cudaGraphExecDestroy(g->exec);
     g->exec = nullptr;
@@ -1220,8 +1013,7 @@ int replay_association(Handle *h, BatchHost *bh, const KParams &K, AssocGraph *g
 }  // namespace
 
 int run_association_edges(Handle *h, const std::vector<DevCloud *> &srcs, const std::vector<DevCloud *> &tgts,
-                          const std::vector<const float4 *> &src_world, const std::vector<float> &src_world_norm,
-                          const std::vector<float> &tgt_pose, const std::vector<float> &ells,
+                          const std::vector<const float4 *> &src_world, const std::vector<float> &tgt_pose, const std::vector<float> &ells,
                           const std::vector<int> &caps, int capmax, std::vector<EdgeAssoc> *out,
                           const KParams *kparams, AssocGraph *graph) {
   NvtxRange nvtx_range("association_edges");
@@ -1248,11 +1040,6 @@ int run_association_edges(Handle *h, const std::vector<DevCloud *> &srcs, const 
     for (int r = 0; r < 3; r++)
       for (int c = 0; c < 3; c++) P.R[3 * r + c] = Q[4 * c + r];
     for (int r = 0; r < 3; r++) P.T[r] = -(P.R[3 * r] * Q[3] + P.R[3 * r + 1] * Q[7] + P.R[3 * r + 2] * Q[11]);
-    float rw = host_radius(K, ells[e], src_world_norm[e]);
-    P.level = P.nlevels - 1;
-    for (int i = 0; i < P.nlevels; i++)
-      if (P.level_r[i] >= rw) { P.level = i; break; }
-    P.level_used = P.level;
   }
   if (graph && !h->prof.on) {
     if ((rc = replay_association(h, &bh, K, graph))) return rc;

@@ -1,9 +1,10 @@
-// cvo_grid.cu -- device clouds: packed SoA upload, source tile (Morton) order,
-// and spatial-hash grid levels over target clouds.
+// cvo_grid.cu -- device clouds: packed SoA upload, tile (Morton) order, and bounding
+// boxes of the groups of 32 tile-order points.
 //
 // Replaces CvoPointCloud_to_gpu (src/cvo/CvoGPU_impl.cu:220-289) and the kd-tree
-// association structure (thirdparty/cugicp/cukdtree/cukdtree.cuh:236-509): a
-// radius query becomes a scan of the hash cells that overlap the query box.
+// association structure (thirdparty/cugicp/cukdtree/cukdtree.cuh:236-509): the boxes do
+// not depend on the lengthscale, so one build serves every call, and they bound the
+// features as well as the positions.
 #include <cmath>
 #include <cstring>
 #include <algorithm>
@@ -11,18 +12,6 @@
 #include "cvo_device.cuh"
 
 namespace cvo_gb {
-
-float level_cell_size(int e) { return exp2f(0.5f * (float)e); }
-
-// Smallest quantised cell size h = 2^(e/2) with h >= r.
-int level_for_radius(float r) {
-  if (!(r > 0.f)) return -60;
-  if (!std::isfinite(r)) return 1000;
-  int e = (int)std::ceil(2.0 * std::log2((double)r));
-  while (level_cell_size(e) < r) e++;
-  while (e > -60 && level_cell_size(e - 1) >= r) e--;
-  return e;
-}
 
 namespace {
 
@@ -63,22 +52,6 @@ __global__ void k_morton(const float4 *pos, int n, float ox, float oy, float oz,
   vals[i] = i;
 }
 
-// Bounding-box diagonal of each block of 128 consecutive tile-order points (one
-// thread per block of points).
-__global__ void k_tile_extent(const float4 *spos, int n, float *ext) {
-  const int tile = blockIdx.x * blockDim.x + threadIdx.x;
-  const int tiles = (n + 127) / 128;
-  if (tile >= tiles) return;
-  float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  for (int s = tile * 128; s < min(n, tile * 128 + 128); s++) {
-    const float4 p = spos[s];
-    lo[0] = fminf(lo[0], p.x); lo[1] = fminf(lo[1], p.y); lo[2] = fminf(lo[2], p.z);
-    hi[0] = fmaxf(hi[0], p.x); hi[1] = fmaxf(hi[1], p.y); hi[2] = fmaxf(hi[2], p.z);
-  }
-  const float dx = hi[0] - lo[0], dy = hi[1] - lo[1], dz = hi[2] - lo[2];
-  ext[tile] = sqrtf(dx * dx + dy * dy + dz * dz);
-}
-
 __global__ void k_gather_source(const int *perm, int n, const float4 *pos, const float *feat, int FP, const float *lab,
                                 int CP, const float2 *geo, float4 *spos, float *sfeat, float *slab, float2 *sgeo) {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -90,43 +63,29 @@ __global__ void k_gather_source(const int *perm, int n, const float4 *pos, const
   if (geo) sgeo[s] = geo[i];
 }
 
-__global__ void k_hash_insert(const float4 *pos, int n, float ox, float oy, float oz, float inv_h, int dimx, int dimy,
-                              int dimz, unsigned long long *keys, int *ccount, int tbits, unsigned int *slot_of,
-                              int *vals, int *err) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  float4 p = pos[j];
-  int cx = min(max((int)floorf((p.x - ox) * inv_h), 0), dimx - 1);
-  int cy = min(max((int)floorf((p.y - oy) * inv_h), 0), dimy - 1);
-  int cz = min(max((int)floorf((p.z - oz) * inv_h), 0), dimz - 1);
-  unsigned long long key = cell_key(cx, cy, cz);
-  unsigned int mask = (1u << tbits) - 1u;
-  unsigned int slot = (unsigned int)cell_hash(key) & mask;
-  for (unsigned int probe = 0; probe <= mask; probe++) {
-    unsigned long long prev = atomicCAS(&keys[slot], kEmptyKey, key);
-    if (prev == kEmptyKey || prev == key) {
-      atomicAdd(&ccount[slot], 1);
-      slot_of[j] = slot;
-      vals[j] = j;
-      return;
+// Bounding boxes of 32 consecutive items, one warp per box.  LEVEL 0: points (tile-order
+// positions and features); LEVEL 1: boxes of LEVEL 0.  Planes as in cvo_kernels.cuh.
+template <int LEVEL>
+__global__ void __launch_bounds__(128) k_boxes(const float4 *pos, const float4 *feat, int stride, int count, int chunks,
+                                               float4 *out, int boxes) {
+  const int lane = threadIdx.x & 31, g = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (g >= boxes) return;
+  const int i = min(32 * g + lane, count - 1);      // spare lanes repeat the last item
+  for (int k = 0; k < 1 + chunks; k++) {
+    float4 lo, hi;
+    if (LEVEL == 0) {
+      lo = hi = k == 0 ? pos[i] : feat[(size_t)i * stride + k - 1];
+    } else {
+      lo = pos[(size_t)(k == 0 ? 0 : 1 + k) * count + i];
+      hi = pos[(size_t)(k == 0 ? 1 : 1 + chunks + k) * count + i];
     }
-    slot = (slot + 1u) & mask;
+    lo = make_float4(warp_fmin(lo.x), warp_fmin(lo.y), warp_fmin(lo.z), warp_fmin(lo.w));
+    hi = make_float4(warp_fmax(hi.x), warp_fmax(hi.y), warp_fmax(hi.z), warp_fmax(hi.w));
+    if (lane == 0) {
+      out[(size_t)(k == 0 ? 0 : 1 + k) * boxes + g] = lo;
+      out[(size_t)(k == 0 ? 1 : 1 + chunks + k) * boxes + g] = hi;
+    }
   }
-  atomicExch(err, 1);   // table full: cannot happen with load factor <= 1/2
-  slot_of[j] = 0;
-  vals[j] = j;
-}
-
-__global__ void k_gather_target(const int *perm, int n, const float4 *pos, const float *feat, int FP, const float *lab,
-                                int CP, const float2 *geo, float4 *tpos, float *tfeat, float *tlab, float4 *tgeo) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  int j = perm[t];
-  float4 p = pos[j];
-  tpos[t] = make_float4(p.x, p.y, p.z, __int_as_float(j));
-  for (int k = 0; k < FP; k++) tfeat[(size_t)t * FP + k] = feat[(size_t)j * FP + k];
-  for (int k = 0; k < CP; k++) tlab[(size_t)t * CP + k] = lab[(size_t)j * CP + k];
-  if (geo) { float2 g = geo[j]; tgeo[t] = make_float4(g.x, g.y, 0.f, 0.f); }
 }
 
 template <typename T>
@@ -174,7 +133,7 @@ static int cloud_build(Handle *h, DevCloud *d, const float *xyz_d, int stride, c
   if (d->has_geo)
     CVO_CUDA_TRY(h, cudaMemcpyAsync(d->geo, geo_in, sizeof(float2) * n, cudaMemcpyDeviceToDevice, h->stream));
 
-  // source tile order: Morton order of a 1024^3 lattice over the bounding box
+  // tile order: Morton order of a 1024^3 lattice over the bounding box
   if ((rc = dalloc(h, &keys, n)) || (rc = dalloc(h, &keys_tmp, n)) || (rc = dalloc(h, &perm_vals, n)) ||
       (rc = dalloc(h, &perm_tmp, n)))
     return rc;
@@ -187,17 +146,14 @@ static int cloud_build(Handle *h, DevCloud *d, const float *xyz_d, int stride, c
   k_gather_source<<<(n + 255) / 256, 256, 0, h->stream>>>(d->sperm, n, d->pos, d->feat, d->FP, d->lab, d->CP, d->geo,
                                                          d->spos, d->sfeat, d->slab, d->sgeo);
   h->launches++;
-  // mean bounding-box diagonal of the 128-point source blocks (sizes the grid cells)
-  const int tiles = (n + 127) / 128;
-  float *ext_d = reinterpret_cast<float *>(keys);
-  k_tile_extent<<<(tiles + 127) / 128, 128, 0, h->stream>>>(d->spos, n, ext_d);
-  h->launches++;
-  std::vector<float> ext_h(tiles);
-  CVO_CUDA_TRY(h, cudaMemcpyAsync(ext_h.data(), ext_d, sizeof(float) * tiles, cudaMemcpyDeviceToHost, h->stream));
+  // boxes of the groups and supergroups
+  const int ng = group_count(n), ns = group_count(ng), ch = box_chunks(d->FP);
+  if ((rc = dalloc(h, &d->gbox, (size_t)(2 + 2 * ch) * ng)) || (rc = dalloc(h, &d->sbox, (size_t)(2 + 2 * ch) * ns))) return rc;
+  k_boxes<0><<<(ng + 3) / 4, 128, 0, h->stream>>>(d->spos, reinterpret_cast<const float4 *>(d->sfeat), d->FP / 4, n, ch,
+                                                  d->gbox, ng);
+  k_boxes<1><<<(ns + 3) / 4, 128, 0, h->stream>>>(d->gbox, nullptr, 0, ng, ch, d->sbox, ns);
+  h->launches += 2;
   CVO_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-  double es = 0.0;
-  for (float e : ext_h) es += e;
-  d->tile_ext = tiles > 0 ? (float)(es / tiles) : 0.f;
   cudaFree(keys); cudaFree(keys_tmp); cudaFree(perm_vals); cudaFree(perm_tmp);
   return 0;
 }
@@ -328,80 +284,8 @@ void cloud_free(DevCloud *d) {
   if (!d) return;
   cudaFree(d->pos); cudaFree(d->feat); cudaFree(d->lab); cudaFree(d->geo);
   cudaFree(d->sperm); cudaFree(d->spos); cudaFree(d->sfeat); cudaFree(d->slab); cudaFree(d->sgeo);
-  for (void *p : d->level_allocs) cudaFree(p);
-  for (auto &kv : d->levels_dev) cudaFree(kv.second);
+  cudaFree(d->gbox); cudaFree(d->sbox);
   delete d;
-}
-
-// Builds (or returns the cached) grid level with cell size 2^(e/2) over the
-// target cloud.  e >= 1000 selects a single cell holding every point (used
-// when the geometric kernel is disabled and every target is a candidate).
-int cloud_level(Handle *h, DevCloud *d, int e, GridDesc *host_desc) {
-  auto it = d->levels_host.find(e);
-  if (it != d->levels_host.end()) { *host_desc = it->second; return 0; }
-  int n = d->n;
-  GridDesc g;
-  memset(&g, 0, sizeof(g));
-  float ext[3];
-  for (int k = 0; k < 3; k++) ext[k] = d->bbmax[k] - d->bbmin[k];
-  float hsz = (e >= 1000) ? INFINITY : level_cell_size(e);
-  // keep at most 2^20 cells per axis
-  float emax = std::max(std::max(ext[0], ext[1]), ext[2]);
-  if (std::isfinite(hsz) && emax / hsz > 1048000.f) hsz = emax / 1048000.f;
-  g.h = hsz;
-  g.inv_h = std::isfinite(hsz) ? 1.f / hsz : 0.f;
-  g.ox = d->bbmin[0]; g.oy = d->bbmin[1]; g.oz = d->bbmin[2];
-  g.dimx = std::isfinite(hsz) ? (int)std::floor(ext[0] * g.inv_h) + 1 : 1;
-  g.dimy = std::isfinite(hsz) ? (int)std::floor(ext[1] * g.inv_h) + 1 : 1;
-  g.dimz = std::isfinite(hsz) ? (int)std::floor(ext[2] * g.inv_h) + 1 : 1;
-  int tbits = 10;
-  while ((1 << tbits) < 2 * std::max(n, 1)) tbits++;
-  g.tbits = tbits;
-  size_t T = (size_t)1 << tbits;
-  unsigned long long *keys = nullptr;
-  int *cstart = nullptr, *ccount = nullptr, *perm = nullptr, *vals_tmp = nullptr, *err = nullptr;
-  unsigned int *slot_of = nullptr, *slot_tmp = nullptr;
-  float4 *tpos = nullptr;
-  float *tfeat = nullptr, *tlab = nullptr;
-  float4 *tgeo = nullptr;   // 16-byte records so that bulk copies stay aligned
-  int rc = 0;
-  if ((rc = dalloc(h, &keys, T)) || (rc = dalloc(h, &cstart, T)) || (rc = dalloc(h, &ccount, T)) ||
-      (rc = dalloc(h, &perm, n)) || (rc = dalloc(h, &tpos, n)) || (rc = dalloc(h, &tfeat, (size_t)n * d->FP)) ||
-      (rc = dalloc(h, &tlab, (size_t)n * d->CP)) || (rc = dalloc(h, &slot_of, n)) || (rc = dalloc(h, &slot_tmp, n)) ||
-      (rc = dalloc(h, &vals_tmp, n)) || (rc = dalloc(h, &err, 1)))
-    return rc;
-  if (d->has_geo && (rc = dalloc(h, &tgeo, n))) return rc;
-  size_t scr = scan_scratch_ints((int)T);
-  int *scan_scr = nullptr;
-  if ((rc = dalloc(h, &scan_scr, scr))) return rc;
-  CVO_CUDA_TRY(h, cudaMemsetAsync(keys, 0xFF, sizeof(unsigned long long) * T, h->stream));
-  CVO_CUDA_TRY(h, cudaMemsetAsync(ccount, 0, sizeof(int) * T, h->stream));
-  CVO_CUDA_TRY(h, cudaMemsetAsync(err, 0, sizeof(int), h->stream));
-  if (n > 0) {
-    k_hash_insert<<<(n + 255) / 256, 256, 0, h->stream>>>(d->pos, n, g.ox, g.oy, g.oz, g.inv_h, g.dimx, g.dimy, g.dimz,
-                                                          keys, ccount, tbits, slot_of, perm, err);
-    h->launches++;
-    if ((rc = radix_sort_pairs(h, slot_of, perm, slot_tmp, vals_tmp, n, tbits))) return rc;
-  }
-  exclusive_scan_int(h, ccount, cstart, (int)T, scan_scr, (int)scr);
-  if (n > 0) {
-    k_gather_target<<<(n + 255) / 256, 256, 0, h->stream>>>(perm, n, d->pos, d->feat, d->FP, d->lab, d->CP, d->geo,
-                                                           tpos, tfeat, tlab, tgeo);
-    h->launches++;
-  }
-  int herr = 0;
-  CVO_CUDA_TRY(h, cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-  CVO_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-  cudaFree(slot_of); cudaFree(slot_tmp); cudaFree(vals_tmp); cudaFree(err); cudaFree(scan_scr);
-  if (herr) return CVO_ERR_CAPACITY;
-  g.keys = keys; g.cstart = cstart; g.ccount = ccount; g.perm = perm;
-  g.pos = tpos; g.feat = tfeat; g.lab = tlab; g.geo = tgeo;
-  for (void *p : {(void *)keys, (void *)cstart, (void *)ccount, (void *)perm, (void *)tpos, (void *)tfeat,
-                  (void *)tlab, (void *)tgeo})
-    if (p) d->level_allocs.push_back(p);
-  d->levels_host[e] = g;
-  *host_desc = g;
-  return 0;
 }
 
 }  // namespace cvo_gb

@@ -6,8 +6,9 @@
 //   features  : n * FP floats, FP = F rounded up to 4 (float4 loads)
 //   labels    : n * CP floats, CP = C rounded up to 4
 //   geom_type : float2
-// A source cloud is additionally kept in "tile order" (Morton order, 32 points per
-// warp tile); a target cloud keeps one spatial-hash grid per cell size ("level").
+// Every cloud is additionally kept in "tile order" (Morton order): 32 consecutive points
+// are a source tile of the association and a target group of it, with a bounding box in
+// position and features; 32 consecutive groups are a supergroup, with a box of its own.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -23,49 +24,31 @@ namespace cvo_gb {
 constexpr int kWarp = 32;
 constexpr int kMaxIndicatorWindow = 128;
 constexpr int kMaxTargetBits = 22;          // targets per cloud <= 4M
-constexpr unsigned long long kEmptyKey = 0xFFFFFFFFFFFFFFFFull;
+constexpr int kGroup = 32;                  // points of a group, groups of a supergroup
 
-// ------------------------------------------------------------------ grid
-// One spatial-hash grid over a target cloud at cell size h.  Cells are keyed by
-// integer coordinates relative to the cloud's bounding-box minimum; the table
-// uses linear probing.  Points are stored sorted by (table slot, original index),
-// so the members of one cell are contiguous and in ascending original index.
-struct GridDesc {
-  float h, inv_h;
-  float ox, oy, oz;
-  int dimx, dimy, dimz;         // number of cells per axis over the bounding box
-  int tbits;                    // table size = 1 << tbits
-  const unsigned long long *keys;
-  const int *cstart;
-  const int *ccount;
-  const int *perm;              // sorted position -> original index
-  const float4 *pos;            // sorted copy: x, y, z, original index (int bits)
-  const float *feat;            // sorted copy, n * FP
-  const float *lab;             // sorted copy, n * CP
-  const float4 *geo;            // sorted copy {g0, g1, 0, 0} (may be null)
-};
+inline int group_count(int n) { return (n + kGroup - 1) / kGroup; }
+// Feature chunks (float4) of a bounding box: the association takes at most two.
+inline int box_chunks(int FP) { return FP / 4 < 2 ? FP / 4 : 2; }
 
 struct DevCloud {
   int n = 0, F = 0, C = 0, FP = 0, CP = 0;
   bool has_geo = false;
   float bbmin[3] = {0, 0, 0}, bbmax[3] = {0, 0, 0};
   float max_norm = 0.f;
-  float tile_ext = 0.f;          // mean bounding-box diagonal of 128 consecutive tile-order points
   // original order
   float4 *pos = nullptr;
   float *feat = nullptr;
   float *lab = nullptr;
   float2 *geo = nullptr;
-  // source tile order
-  int *sperm = nullptr;
+  // tile order
+  int *sperm = nullptr;          // tile-order position -> original index
   float4 *spos = nullptr;
   float *sfeat = nullptr;
   float *slab = nullptr;
   float2 *sgeo = nullptr;
-  // target grids keyed by quantised cell-size exponent
-  std::map<int, GridDesc *> levels_dev;   // device copies of descriptors
-  std::map<int, GridDesc> levels_host;
-  std::vector<void *> level_allocs;
+  // bounding boxes of the groups, then of the supergroups: float4 planes (position low,
+  // high, feature low, feature high; box_planes of them) of one entry per group
+  float4 *gbox = nullptr, *sbox = nullptr;
 };
 
 // ----------------------------------------------------------- kernel params
@@ -80,8 +63,8 @@ struct KParams {
   int ell_decay_start, indicator_window_size, max_iter, nn_max, use_range_ell_step;
   int use_geo, use_int, use_sem, use_gtype;
   float inv2c2;          // 1 / (2 c_ell^2), rounded once (IEEE division)
-  // Tensor-core prefilter: a kept pair needs d2/(2l^2) + d2c/(2c_ell^2) < mma_tau
-  // (mma_tau = ln(sigma^2 c_sigma^2 s_sigma^2 / sp_thres) + slack), see k_assoc.
+  // Candidate test: a kept pair needs d2/(2l^2) + d2c/(2c_ell^2) < mma_tau
+  // (mma_tau = ln(sigma^2 c_sigma^2 s_sigma^2 / sp_thres) + slack), see k_cand.
   float mma_tau;
   int use_mma;
   // Value scale (1 on the two-view path; c_sigma for the adaptive path's geometric-only
@@ -98,21 +81,27 @@ struct PairDev {
   const float4 *xs;               // source, tile order (x,y,z,||x||)
   const float *xf, *xl;
   const float2 *xg;
-  const int *sperm;
-  const GridDesc *levels;         // device array of grid levels of the target
-  int nlevels;
-  float level_r[24];              // largest search radius each level serves
-  float4 *ycur;                   // transformed targets, current level order
+  const float4 *sbox;             // source tiles' boxes
+  // target, tile order
+  const float4 *tpos;
+  const int *tperm;               // tile-order position -> original index
+  const float *tfs;
+  const float4 *tbox, *tsup;      // boxes of groups and supergroups
+  int groups;
+  float4 *ycur;                   // transformed targets, tile order
   float4 *yorig;                  // transformed targets, original order
   int *A_j; float *A_v;           // ELL, row-major: entry c of row s at [s * ld + c] (original target index)
   int ld;                         // ELL row pitch (capmax rounded up to a multiple of 4)
-  int2 *ovf;                      // spill lists: kept pair cap + t of row s at [s * ov + t] = {j, bits of a}
-  int ov;                         // row-list entries per row
+  // candidates: entry e of split q of row s at [s * cand_pitch + q * cap_split + e] =
+  // {group, bits of its 32 points}; cand_cnt[q * n + s] = {entries, candidates} (more than
+  // cap_split entries: not all stored)
+  uint2 *cand;
+  int2 *cand_cnt;
+  int splits, cap_split, cand_pitch;
   const float *tf, *tl;           // target features / labels, original order (float4 chunks)
   const float2 *tg;               // target geometric types, original order
   int *nnz_row;                   // n
-  float *row_sums;                // n * 8: omega(3)/c, v(3)/d, asum, count
-  double *part;                   // reduce partials
+  double *part;                   // block partials
   unsigned int *counter;          // last-block counters [2]
   int F, C;                       // feature / label dimensions (source and target agree)
   int capmax;
@@ -122,7 +111,6 @@ struct PairDev {
   float Ri[9], Ti[3];             // target transform R^T, -R^T T
   float ell;
   int cap;
-  int level, level_used;
   int iter, done, ret;
   float xi[6];
   double grad[6];
@@ -131,7 +119,6 @@ struct PairDev {
   int max_row;
   double bcde[4];
   double step, dist;
-  float rq_max;                   // largest search radius of this iteration
   // indicator queues (ring buffers)
   float qs[kMaxIndicatorWindow], qe[kMaxIndicatorWindow];
   int qs_head, qs_len, qe_head, qe_len;
@@ -142,34 +129,20 @@ struct PairDev {
 // Batch of pairs processed together by every kernel launch.
 struct BatchDev {
   int npairs;
-  int total_warps;                // association tiles over all pairs
+  int total_items;                // work items of k_cand over all pairs (tiles x splits)
   int total_rows;                 // sum of n
   int total_targets;              // sum of m
   PairDev *pairs;                 // device array
-  const int *tile_off;            // npairs + 1 (prefix of tile counts)
-  const int *row_off;             // npairs + 1 (prefix of n)
+  const int *item_off;            // npairs + 1 (prefix of work items)
   const int *tgt_off;             // npairs + 1 (prefix of m)
   int *err;                       // error word (0 ok)
-  const int *rblk_off;            // reduce blocks per pair (prefix)
+  const int *rblk_off;            // row-pass blocks per pair (prefix)
   const int *sblk_off;            // step blocks per pair (prefix)
   int total_rblocks, total_sblocks;
   int *active;                    // number of pairs not done
   int *active_iters;              // iterations that started with an active pair
   double *assoc_bytes;            // algorithmic bytes of the association passes
   int record_bytes;               // packed bytes of one target record
-  // rows with more than `cap` kept pairs, {pair, row, kept count, 0}; reset by k_transform
-  int4 *sel_list;                 // cap < count <= ov: select from the row list
-  int *sel_count;
-  int4 *scan_list;                // count > ov: index-ordered rescan of the row
-  int *scan_count;
-  int *assoc_next;                // next association work item (persistent blocks); reset by k_transform
-  // work items (four tiles of one pair) in the order the persistent blocks take them:
-  // heaviest first by the cost each took in the previous pass (SM clock / 256); an
-  // entry is (item << 3) | mode, mode 4 = whole item, 0-3 = one tile of a split item
-  int n_items;
-  int *item_order;                // up to 4 n_items entries
-  int *item_cost;
-  int *n_order;                   // entries of item_order
 };
 
 // ------------------------------------------------------------- host side
@@ -185,11 +158,11 @@ struct Profile {
   long long iterations = 0;
 };
 
-// Association tuning: grid cell size h = max(r / cell_div_r, (ext + 2 r) / cell_div_ext)
-// for search radius r and source tiles of diagonal ext, and the resident association
-// blocks per SM of the persistent launch (0: as many as the occupancy allows).  Results
-// do not depend on either (the kept pairs are defined by index order), only the work per
-// row and how the work items spread over the SMs do.
+// Association tuning: how finely the candidate test divides the targets among warps.
+// The splits per source tile scale with (cell_div_r / 4) (cell_div_ext / 8), and
+// blocks_per_sm > 0 asks for that many times four work items per SM instead of the
+// default.  Results do not depend on any of them (k_rows orders the candidates), only how
+// the work spreads over the SMs does.
 struct TuneConfig {
   float cell_div_r = 4.f;
   float cell_div_ext = 8.f;
@@ -206,7 +179,7 @@ struct Handle {
   long long launches = 0;
   std::string last_error;
   Workspace *ws = nullptr;
-  std::map<long long, TuneConfig> tuned;    // (F, C, log2 rows) -> fastest cell size
+  std::map<long long, TuneConfig> tuned;    // (F, C, log2 rows) -> fastest division
   std::map<long long, int> tuned_bps;       // (F, C, log2 work items of a batch) -> blocks per SM
   const TuneConfig *tune_force = nullptr;   // set while the autotuner times a configuration
 };
@@ -235,9 +208,6 @@ int cloud_upload(Handle *h, const cvo_cloud *c, DevCloud **out);
 int cloud_from_device(Handle *h, int n, int F, int C, const float *xyz_d, const float *feat_d, const float *lab_d,
                       const float2 *geo_d, DevCloud **out);
 void cloud_free(DevCloud *c);
-int cloud_level(Handle *h, DevCloud *c, int level_exp, GridDesc *host_desc);
-float level_cell_size(int level_exp);
-int level_for_radius(float r);
 
 // radix sort / scan (cvo_sort.cu)
 int radix_sort_pairs(Handle *h, unsigned int *keys, int *vals, unsigned int *keys_tmp, int *vals_tmp,
@@ -300,8 +270,7 @@ struct AssocGraph {
   ~AssocGraph();
 };
 int run_association_edges(Handle *h, const std::vector<DevCloud *> &srcs, const std::vector<DevCloud *> &tgts,
-                          const std::vector<const float4 *> &src_world, const std::vector<float> &src_world_norm,
-                          const std::vector<float> &tgt_pose, const std::vector<float> &ells,
+                          const std::vector<const float4 *> &src_world, const std::vector<float> &tgt_pose, const std::vector<float> &ells,
                           const std::vector<int> &caps, int capmax, std::vector<EdgeAssoc> *out,
                           const KParams *kparams = nullptr, AssocGraph *graph = nullptr);
 

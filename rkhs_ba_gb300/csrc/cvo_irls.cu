@@ -467,21 +467,17 @@ int run_align_multi(Handle *h, int nf, DevCloud *const *clouds, double *poses, c
     for (int t = 0; t < 12 * nf; t++) fpose[t] = (float)poses[t];
     if (cudaMemcpyAsync(pose_d, fpose.data(), sizeof(float) * 12 * nf, cudaMemcpyHostToDevice, h->stream) !=
         cudaSuccess) { cleanup(); return CVO_ERR_CUDA; }
-    std::vector<float> wnorm(nf, 0.f);
     for (int f = 0; f < nf; f++) {
       int n = clouds[f]->n;
       if (n > 0) {
         k_world<<<(n + 255) / 256, 256, 0, h->stream>>>(clouds[f]->spos, n, pose_d + 12 * f, world[f]);
         h->launches++;
       }
-      double tn = std::sqrt(poses[12 * f + 3] * poses[12 * f + 3] + poses[12 * f + 7] * poses[12 * f + 7] +
-                            poses[12 * f + 11] * poses[12 * f + 11]);
-      wnorm[f] = (float)(clouds[f]->max_norm + tn) * 1.0001f;
     }
     // association of every edge in one batch
     std::vector<DevCloud *> es(ne), et(ne);
     std::vector<const float4 *> ew(ne);
-    std::vector<float> enorm(ne), epose(12 * (size_t)ne), eell(ne);
+    std::vector<float> epose(12 * (size_t)ne), eell(ne);
     for (int e = 0; e < ne; e++) {
       int f1 = edges[2 * e], f2 = edges[2 * e + 1];
       nz_last[e] = prev_nnz[e];
@@ -489,12 +485,11 @@ int run_align_multi(Handle *h, int nf, DevCloud *const *clouds, double *poses, c
       es[e] = clouds[f1];
       et[e] = clouds[f2];
       ew[e] = world[f1];
-      enorm[e] = wnorm[f1];
       for (int t = 0; t < 12; t++) epose[12 * e + t] = fpose[12 * f2 + t];
       eell[e] = (float)ell[e];
     }
     std::vector<EdgeAssoc> EA;
-    if ((rc = run_association_edges(h, es, et, ew, enorm, epose, eell, nn, init_nn, &EA, nullptr, &ag))) {
+    if ((rc = run_association_edges(h, es, et, ew, epose, eell, nn, init_nn, &EA, nullptr, &ag))) {
       cleanup();
       return rc;
     }

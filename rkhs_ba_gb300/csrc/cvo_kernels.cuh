@@ -1,16 +1,14 @@
-// cvo_kernels.cuh -- per-iteration kernels of the batched CVO engine.
+// cvo_kernels.cuh -- association kernels of the batched CVO engine.
 //
 // One iteration of the reference's align loop (src/cvo/CvoGPU.cu:1303-1433) is a
 // fixed sequence of launches over every active pair of a batch:
 //   k_transform  target transform y' = R^T (y - T)            (CvoGPU_impl.cu:32-83)
-//   k_assoc_cta  association: grid candidates -> tensor-core prefilter -> exact kernel
-//                value -> threshold -> ELL row (first cap) + spill list (the rest)
-//                (cvo_assoc_cta.cuh; per-warp path assoc_warp below)
-//                                                               (CvoGPU.cu:951-1099)
-//   k_select / k_rescan  rows with more than cap kept pairs: their cap smallest indices
-//   k_rowsum     per-row gradient partials from the final ELL    (CvoGPU.cu:2001-2062)
-//   k_reduce     per-pair FP64 sums of the row partials; gradient normalisation
-//                                                               (CvoGPU.cu:2065-2120)
+//   k_cand       candidates: source tiles against target groups by bounding boxes in
+//                position and colour, then a tensor-core test of the 32 x 32 pairs of
+//                the groups that remain; one bit per pair that may be kept
+//   k_rows       each row's candidates in ascending target index: exact kernel value,
+//                threshold, the first cap kept ones to the ELL row, gradient sums
+//                                            (CvoGPU.cu:951-1099, 2001-2120)
 //   k_step       Taylor step-size terms over the ELL rows; the last block of each pair
 //                runs the scalar tail of the iteration: cubic roots, step clamp,
 //                Exp_SEK3 pose update, SE(3) distance, lengthscale schedule, cap update
@@ -22,9 +20,6 @@
 namespace cvo_gb {
 
 enum { MODE_ALIGN = 0, MODE_IP = 1, MODE_EXPORT = 2 };
-constexpr int kAssocThreads = 128;
-constexpr int kReduceRows = 1024;
-constexpr int kReduceThreads = 256;
 constexpr int kStepThreads = 256;
 constexpr int kPartStride = 12;
 
@@ -36,8 +31,8 @@ constexpr int kPartStride = 12;
 template <int FCH, int LCH, bool GT>
 __device__ __forceinline__ bool eval_pair(const KParams &K, int F, int C, bool pre, float l, float d2t, float inv2l2,
                                           const float4 &x, const float4 (&xf)[FCH > 0 ? FCH : 1],
-                                          const float4 (&xl)[LCH > 0 ? LCH : 1], float2 xg, const float4 &y,
-                                          const float4 *yfp, const float4 *ylp, const float4 *ygp, float &a) {
+                                          const float4 *xl, float2 xg, const float4 &y,
+                                          const float4 (&yf)[FCH > 0 ? FCH : 1], const float4 *ylp, float2 yg, float &a) {
   bool pass = pre;
   float d2 = 0.f;
   if (K.use_geo) {
@@ -47,7 +42,6 @@ __device__ __forceinline__ bool eval_pair(const KParams &K, int F, int C, bool p
   if (!__any_sync(FULLMASK, pass)) return false;
   float geo = 1.f;
   if (GT) {
-    float4 yg = *ygp;
     float n2a = fa(fm(xg.x, xg.x), fm(xg.y, xg.y));
     float n2b = fa(fm(yg.x, yg.x), fm(yg.y, yg.y));
     float dab = fa(fm(xg.x, yg.x), fm(xg.y, yg.y));
@@ -58,9 +52,8 @@ __device__ __forceinline__ bool eval_pair(const KParams &K, int F, int C, bool p
   if (FCH > 0 && K.use_int) {
 #pragma unroll
     for (int q = 0; q < FCH; q++) {
-      float4 yf = yfp[q];
       float av[4] = {xf[q].x, xf[q].y, xf[q].z, xf[q].w};
-      float bv[4] = {yf.x, yf.y, yf.z, yf.w};
+      float bv[4] = {yf[q].x, yf[q].y, yf[q].z, yf[q].w};
 #pragma unroll
       for (int r = 0; r < 4; r++)
         if (4 * q + r < F) { float t = fs(av[r], bv[r]); d2c = fa(d2c, fm(t, t)); }
@@ -73,8 +66,9 @@ __device__ __forceinline__ bool eval_pair(const KParams &K, int F, int C, bool p
   if (LCH > 0 && K.use_sem) {
 #pragma unroll
     for (int q = 0; q < LCH; q++) {
-      float4 yl = ylp[q];
-      float av[4] = {xl[q].x, xl[q].y, xl[q].z, xl[q].w};
+      float4 yl = pass ? __ldg(ylp + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+      float4 xq = xl[q];
+      float av[4] = {xq.x, xq.y, xq.z, xq.w};
       float bv[4] = {yl.x, yl.y, yl.z, yl.w};
 #pragma unroll
       for (int r = 0; r < 4; r++)
@@ -97,163 +91,62 @@ __device__ __forceinline__ bool eval_pair(const KParams &K, int F, int C, bool p
 
 // Per-source-point kernel constants.
 struct RowConst {
-  float l, d2t, inv2l2, rq;
+  float l, d2t, inv2l2;
 };
 
-__device__ __forceinline__ RowConst row_const(const KParams &K, float ell, float norm, float Tn) {
+__device__ __forceinline__ RowConst row_const(const KParams &K, float ell, float norm) {
   RowConst rc;
   rc.l = range_ell(ell, norm);
   rc.d2t = K.use_geo ? geo_d2_thres(rc.l, K.log_geo) : INFINITY;
   rc.inv2l2 = __frcp_rn(fm(fm(2.f, rc.l), rc.l));
-  rc.rq = K.use_geo ? sqrtf(rc.d2t) * 1.00001f + 1e-5f * (norm + Tn + sqrtf(rc.d2t)) + 1e-6f : 0.f;
   return rc;
 }
 
-// Cell range of the box [lo, hi] in grid g; returns false if empty.
-__device__ __forceinline__ bool cell_range(const GridDesc &g, float lox, float loy, float loz, float hix, float hiy,
-                                           float hiz, int &x0, int &y0, int &z0, int &nx, int &ny, int &nz) {
-  if (g.dimx == 1 && g.dimy == 1 && g.dimz == 1 && g.inv_h == 0.f) {
-    x0 = y0 = z0 = 0; nx = ny = nz = 1;
-    return true;
-  }
-  float a0 = floorf((lox - g.ox) * g.inv_h), a1 = floorf((hix - g.ox) * g.inv_h);
-  float b0 = floorf((loy - g.oy) * g.inv_h), b1 = floorf((hiy - g.oy) * g.inv_h);
-  float c0 = floorf((loz - g.oz) * g.inv_h), c1 = floorf((hiz - g.oz) * g.inv_h);
-  if (!(a1 >= 0.f && b1 >= 0.f && c1 >= 0.f)) return false;
-  if (!(a0 < (float)g.dimx && b0 < (float)g.dimy && c0 < (float)g.dimz)) return false;
-  x0 = (int)fmaxf(a0, 0.f); int x1 = (int)fminf(a1, (float)(g.dimx - 1));
-  y0 = (int)fmaxf(b0, 0.f); int y1 = (int)fminf(b1, (float)(g.dimy - 1));
-  z0 = (int)fmaxf(c0, 0.f); int z1 = (int)fminf(c1, (float)(g.dimz - 1));
-  nx = x1 - x0 + 1; ny = y1 - y0 + 1; nz = z1 - z0 + 1;
-  return nx > 0 && ny > 0 && nz > 0;
-}
-
 // ------------------------------------------------------------- transform
-// Writes the transformed targets twice: in grid order (read by the association
-// scan) and in original order (gathered by index from the ELL rows).
+// Writes the transformed targets twice: in tile order (read by k_cand) and in
+// original order (gathered by index by k_rows and k_step).
 __global__ void k_transform(BatchDev B) {
   int gt = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gt == 0) {
-    if (*B.active > 0) *B.active_iters += 1;
-    *B.sel_count = 0;
-    *B.scan_count = 0;
-    *B.assoc_next = 0;
-  }
+  if (gt == 0 && *B.active > 0) *B.active_iters += 1;
   if (gt >= B.total_targets) return;
   int p = find_segment(B.tgt_off, B.npairs, gt);
   PairDev *P = &B.pairs[p];
   if (P->done) return;
   int t = gt - B.tgt_off[p];
-  const GridDesc &G = P->levels[P->level];
-  float4 y = __ldg(&G.pos[t]);
+  float4 y = __ldg(&P->tpos[t]);
   float o0 = xform_row(&P->Ri[0], P->Ti[0], y.x, y.y, y.z);
   float o1 = xform_row(&P->Ri[3], P->Ti[1], y.x, y.y, y.z);
   float o2 = xform_row(&P->Ri[6], P->Ti[2], y.x, y.y, y.z);
-  float4 o = make_float4(o0, o1, o2, y.w);
+  float4 o = make_float4(o0, o1, o2, 0.f);
   P->ycur[t] = o;
-  P->yorig[__float_as_int(y.w)] = o;
+  P->yorig[__ldg(&P->tperm[t])] = o;
 }
 
-// -------------------------------------------------------- row selection
-// The reference keeps the first `cap` kept pairs of a row in ascending target
-// index (its scan stops at `cap`, src/cvo/CvoGPU.cu:994-996).  Here candidates
-// arrive in grid order, so k_assoc writes the first `cap` kept pairs of a row to
-// its ELL slots and the first `ov` to the row's list (row-major); a row that kept
-// more than `cap` is listed, and k_select (count <= ov) or k_rescan (count > ov)
-// rewrites its ELL row with the `cap` smallest kept indices, i.e. the
-// reference's set.
-struct EllRow {
-  int *j;
-  float *v;
-  size_t stride;
-  __device__ __forceinline__ int &J(int c) const { return j[(size_t)c * stride]; }
-  __device__ __forceinline__ float &V(int c) const { return v[(size_t)c * stride]; }
-};
-
-// ------------------------------------------------------- candidate staging
-// A chunk of up to CH candidate targets in shared memory.  The grid stores the
-// members of one cell contiguously (positions, features, labels, geometric
-// types); the warp fills a chunk from consecutive cells with 16-byte loads.
-template <int FCH, int LCH, bool GT>
-struct __align__(16) StageBuf {
-  static constexpr int CH = (LCH > 5) ? 16 : 32;
-  float4 pos[CH];
-  float4 feat[CH * (FCH > 0 ? FCH : 1)];
-  float4 lab[CH * (LCH > 0 ? LCH : 1)];
-  float4 geo[GT ? CH : 1];
-};
-
-// Copies the nk grid-order candidates t0 .. t0+nk-1 into slots at .. at+nk-1 of a
-// staging buffer; the warp copies each array (positions, features, labels,
-// geometric types) as one contiguous run of 16-byte vectors.
-template <int FCH, int LCH, bool GT>
-__device__ __forceinline__ void stage_piece(StageBuf<FCH, LCH, GT> &buf, const float4 *ycur, const GridDesc &G,
-                                            int at, int t0, int nk, int lane) {
-#pragma unroll 1
-  for (int i = lane; i < nk; i += 32) buf.pos[at + i] = __ldg(ycur + t0 + i);
-  if (FCH > 0) {
-    const float4 *src = reinterpret_cast<const float4 *>(G.feat) + (size_t)t0 * FCH;
-#pragma unroll 1
-    for (int i = lane; i < nk * FCH; i += 32) buf.feat[at * FCH + i] = __ldg(src + i);
-  }
-  if (LCH > 0) {
-    const float4 *src = reinterpret_cast<const float4 *>(G.lab) + (size_t)t0 * LCH;
-#pragma unroll 1
-    for (int i = lane; i < nk * LCH; i += 32) buf.lab[at * LCH + i] = __ldg(src + i);
-  }
-  if (GT) {
-#pragma unroll 1
-    for (int i = lane; i < nk; i += 32) buf.geo[at + i] = __ldg(G.geo + t0 + i);
-  }
-}
-
-// ------------------------------------------------- tensor-core prefilter
+// ---------------------------------------------------------- candidate test
 // A kept pair satisfies  u = g_s |x - y|^2 + c |xc - yc|^2 < tau  with
 // g_s = 1/(2 l_s^2), c = 1/(2 c_ell^2), tau = ln(sigma^2 c_sigma^2 s_sigma^2 / sp_thres)
 // (+ slack): the kernel value is at most the product of the three scales times
-// exp(-u), and the geometric-type factor is at most 1.  Around a per-warp centre
-// p (x~ = x - p, y~ = y - p) u is the inner product of two 16-vectors,
-//   A_s = [-2 g x~ | -2 c xc | g | c | g|x~|^2 + c|xc|^2 | -kappa |A_s| | 0]
-//   B_t = [ y~     |  yc     | |y~|^2 | |yc|^2 | 1       |  |B_t|        | 0]
-// so a 32-source x 32-candidate tile of u is a 32x32x16 GEMM.  Each vector is
-// split into f16 hi + lo parts and the tile is Ahi*Bhi + Ahi*Blo + Alo*Bhi
-// (mma.sync m16n8k16, FP32 accumulation): the error is below 2^-16 |A||B|, and
-// the -kappa |A||B| column (kappa = 2^-12) lowers u by more than that, so the
-// test "u < tau" never rejects a pair the exact evaluation keeps.  Only pairs
-// that pass go through the exact per-pair arithmetic (eval_pair), in the same
-// candidate order as an unfiltered scan, so the kernel matrix is unchanged.
-constexpr float kMmaKappa = 1.f / 4096.f;
-constexpr float kMmaMaxAbs = 6.0e4f;    // larger components would leave the f16 range: no filtering
-
-struct __align__(16) MmaTile {
-  uint4 a[4][32];   // source rows:  [hi k0-7, hi k8-15, lo k0-7, lo k8-15][row]
-  uint4 b[4][32];   // candidates:   same layout
-};
+// exp(-u), and the geometric-type factor is at most 1.  With g the smallest g_s of a
+// tile of 32 source rows, a = [sqrt(g) (x - p), sqrt(c) (xc - q)] and b likewise for a
+// candidate (p, q: a point near the tile), u >= |a - b|^2.  a and b are rounded to
+// f16 (a^, b^); then |a^ - b^| <= |a - b| + 2^-11 (|a| + |b|), and a kept pair has
+// |b| <= |a| + sqrt(tau), so with A the largest |a^| of the tile the test
+//   |a^ - b^|^2 < (sqrt(tau) + 2^-11 (2 A + sqrt(tau)))^2 + rounding
+// never rejects a kept pair.  |a^ - b^|^2 minus that bound is one 16-wide product:
+//   [-2 a^ (11) | (|a^|^2 - bound) hi | lo | 1 | 1 | 0] . [b^ | 1 | 1 | |b^|^2 hi | lo | 0]
+// (squares split into two f16), one mma.sync.m16n8k16 per 16 x 8 pairs, and the sign
+// of the accumulator is the answer.  The bound is within 1-2 % of tau for tiles a few
+// lengthscales wide.  Only candidates go through the exact per-pair arithmetic
+// (eval_pair), so the kernel matrix does not depend on the test.
+constexpr float kCandWide = 200.f;      // largest |a^| the f16 squares serve
+constexpr float kCandFar = 60000.f;     // |b^|^2 beyond which a candidate is rejected outright
 
 __device__ __forceinline__ float f4_at(const float4 &v, int i) {
   return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w));
 }
 
-// Splits v into f16 hi + lo and stores entry `idx` of the 4 planes (plane p at
-// dst + p * stride); returns false
-// if a component is outside the f16-safe range (or not finite).
-__device__ __forceinline__ bool mma_store_vec(const float (&v)[16], uint4 *dst, int stride, int idx) {
-  uint32_t hw[8], lw[8];
-  bool ok = true;
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    float v0 = v[2 * i], v1 = v[2 * i + 1];
-    ok = ok && (fabsf(v0) <= kMmaMaxAbs) && (fabsf(v1) <= kMmaMaxAbs);
-    __half h0 = __float2half_rn(v0), h1 = __float2half_rn(v1);
-    __half l0 = __float2half_rn(v0 - __half2float(h0)), l1 = __float2half_rn(v1 - __half2float(h1));
-    hw[i] = (uint32_t)__half_as_ushort(h0) | ((uint32_t)__half_as_ushort(h1) << 16);
-    lw[i] = (uint32_t)__half_as_ushort(l0) | ((uint32_t)__half_as_ushort(l1) << 16);
-  }
-  dst[idx] = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-  dst[stride + idx] = make_uint4(hw[4], hw[5], hw[6], hw[7]);
-  dst[2 * stride + idx] = make_uint4(lw[0], lw[1], lw[2], lw[3]);
-  dst[3 * stride + idx] = make_uint4(lw[4], lw[5], lw[6], lw[7]);
-  return ok;
+__device__ __forceinline__ uint32_t pack_h2(__half a, __half b) {
+  return (uint32_t)__half_as_ushort(a) | ((uint32_t)__half_as_ushort(b) << 16);
 }
 
 __device__ __forceinline__ void ldsm_x4(const void *p, uint32_t &r0, uint32_t &r1, uint32_t &r2, uint32_t &r3) {
@@ -266,743 +159,626 @@ __device__ __forceinline__ void ldsm_x4(const void *p, uint32_t &r0, uint32_t &r
 __device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile(
       "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
-      "{%0, %1, %2, %3};\n"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+      "{%10, %10, %10, %10};\n"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
 }
 
-// Row partials as k_reduce reads them: omega / c, v / d (align mode only), sum of a.
-__device__ __forceinline__ void write_row_sums(float *rs, int mode, const KParams &K, float w0, float w1, float w2,
-                                               float v0, float v1, float v2, float as) {
-  if (mode == MODE_ALIGN) {
-    rs[0] = __fdiv_rn(w0, K.c); rs[1] = __fdiv_rn(w1, K.c); rs[2] = __fdiv_rn(w2, K.c);
-    rs[3] = __fdiv_rn(v0, K.d); rs[4] = __fdiv_rn(v1, K.d); rs[5] = __fdiv_rn(v2, K.d);
-  } else {
-    rs[0] = rs[1] = rs[2] = rs[3] = rs[4] = rs[5] = 0.f;
-  }
-  rs[6] = as;
+// The operand of one point: scaled coordinates v[11] rounded to f16, and the four
+// square / one columns.  Planes 0 and 1 hold k 0-7 and 8-15 (16 bytes each).
+__device__ __forceinline__ void cand_store(const __half (&v)[11], __half c11, __half c12, __half c13, __half c14,
+                                           uint4 (*pl)[32], int idx) {
+  pl[0][idx] = make_uint4(pack_h2(v[0], v[1]), pack_h2(v[2], v[3]), pack_h2(v[4], v[5]), pack_h2(v[6], v[7]));
+  pl[1][idx] = make_uint4(pack_h2(v[8], v[9]), pack_h2(v[10], c11), pack_h2(c12, c13), pack_h2(c14, __float2half_rn(0.f)));
 }
 
-// The warp's 32 source rows, for lanes that evaluate another lane's row.
-template <int FCH, int LCH>
-struct __align__(16) SrcRows {
-  float4 x[32];                                // position, ||x||
-  float4 rc[32];                               // l, d2 threshold, 1 / (2 l^2), geometric type g0
-  float4 f[32 * (FCH > 0 ? FCH : 1)];
-  float4 l[32 * (LCH > 0 ? LCH : 1)];
-  float g1[32];                                // geometric type g1
-};
-
-// Position of the (n+1)-th set bit of m (n >= 0, m has more than n set bits):
-// a binary search on population counts of the low halves, fixed latency.
-__device__ __forceinline__ int nth_set_bit(uint32_t m, int n) {
-  int pos = 0;
+// Scaled coordinates of a point relative to the tile's centre.
+template <int FCH>
+__device__ __forceinline__ void cand_coords(float (&v)[11], const float4 &y, const float4 (&yf)[FCH > 0 ? FCH : 1],
+                                            const float (&pc)[3], const float (&fc)[8], float sg, float sc) {
+  v[0] = (y.x - pc[0]) * sg;
+  v[1] = (y.y - pc[1]) * sg;
+  v[2] = (y.z - pc[2]) * sg;
 #pragma unroll
-  for (int w = 16; w > 0; w >>= 1) {
-    const uint32_t low = (m >> pos) & ((1u << w) - 1u);
-    const int c = __popc(low);
-    if (n >= c) {
-      n -= c;
-      pos += w;
+  for (int f = 0; f < 8; f++) v[3 + f] = FCH * 4 > f ? (f4_at(yf[FCH > 0 ? (f >> 2) % FCH : 0], f & 3) - fc[f]) * sc : 0.f;
+}
+
+// Column of the 32 x 32 tile that answers for bit p of a row's mask: the sign bits of
+// the accumulators are shifted together in this order (see k_cand), so candidate p is
+// staged in column cand_col(p).
+__device__ __forceinline__ int cand_col(int p) {
+  const int q = 7 - (p & 7);
+  return 8 * (q >> 1) + 2 * (p >> 3) + (q & 1);
+}
+
+// Squared distance of the intervals [alo, ahi] and [blo, bhi] (0 if they meet).
+__device__ __forceinline__ float gap2(float alo, float ahi, float blo, float bhi) {
+  const float d = fmaxf(fmaxf(blo - ahi, alo - bhi), 0.f);
+  return d * d;
+}
+
+// Bounding boxes of groups (or of 32 groups): float4 planes of `count` entries each --
+// position low, high, feature low (FCH chunks), feature high (FCH chunks).
+// Whether some pair between the tile and box i may be kept.
+template <int FCH>
+__device__ __forceinline__ bool box_near(const float4 *box, int count, int i, const float (&qlo)[3], const float (&qhi)[3],
+                                         const float (&flo)[8], const float (&fhi)[8], float g, float cw, float tau,
+                                         float dc_max) {
+  const float4 lo = __ldg(box + i), hi = __ldg(box + count + i);
+  const float dp = gap2(qlo[0], qhi[0], lo.x, hi.x) + gap2(qlo[1], qhi[1], lo.y, hi.y) + gap2(qlo[2], qhi[2], lo.z, hi.z);
+  float dc = 0.f;
+#pragma unroll
+  for (int q = 0; q < FCH; q++) {
+    const float4 a = __ldg(box + (size_t)(2 + q) * count + i), b = __ldg(box + (size_t)(2 + FCH + q) * count + i);
+    dc += gap2(flo[4 * q], fhi[4 * q], a.x, b.x) + gap2(flo[4 * q + 1], fhi[4 * q + 1], a.y, b.y) +
+          gap2(flo[4 * q + 2], fhi[4 * q + 2], a.z, b.z) + gap2(flo[4 * q + 3], fhi[4 * q + 3], a.w, b.w);
+  }
+  // written so that a NaN bound keeps the group
+  return !(g * dp + cw * dc > tau) && !(dc > dc_max);
+}
+
+// One warp per work item: a tile of 32 source rows (Morton order) and every S-th of the
+// target's supergroups (32 groups of 32 points).  The warp tests the supergroups' boxes,
+// then the groups' boxes of those near it (one box per lane), and runs the tensor-core
+// test on the groups that remain.  A row's answer for a group is a 32-bit mask, appended
+// to the row's entries {group, mask} of this split; k_rows puts the entries in index
+// order, so neither the number of splits nor their order matters.
+// Bounds: issue (box tests 25-45 instructions per 32 groups, 70 to stage a group's 32
+// candidates, 60 for the product and its mask).  Boxes in position and colour leave
+// 3-14 % of all 32 x 32 tiles on the stereo scenes, four times fewer than boxes in
+// position alone, which is why the cells of a position grid are not used here.
+constexpr int kCandWarps = 4;
+
+template <int FCH>
+__global__ void __launch_bounds__(32 * kCandWarps) k_cand(BatchDev B, KParams K) {
+  __shared__ __align__(16) uint4 apl_all[kCandWarps][2][32];
+  __shared__ __align__(16) uint4 bpl_all[kCandWarps][2][32];
+  constexpr int FP = FCH > 0 ? FCH : 1;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint4(*apl)[32] = apl_all[w];
+  uint4(*bpl)[32] = bpl_all[w];
+  const int gw = blockIdx.x * kCandWarps + w;
+  if (gw >= B.total_items) return;
+  const int p = find_segment(B.item_off, B.npairs, gw);
+  const PairDev *P = &B.pairs[p];
+  if (P->done) return;
+  const int S = P->splits, it = gw - B.item_off[p];
+  const int tile = it / S, sp = it - tile * S;
+  const int n = P->n, m = P->m;
+  const int s = tile * 32 + lane;
+  const bool valid = s < n;
+  const int si = valid ? s : n - 1;      // spare lanes repeat the last row for the boxes
+  const float4 x = __ldg(&P->xs[si]);
+  float4 xf[FP];
+#pragma unroll
+  for (int q = 0; q < FP; q++)
+    xf[q] = FCH > 0 ? __ldg(reinterpret_cast<const float4 *>(P->xf) + (size_t)si * FCH + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float tau = K.mma_tau;
+  const float cw = K.use_int ? K.inv2c2 : 0.f;
+  // the tile's smallest 1 / (2 l^2), and how far rounding can move a point between frames
+  const float l = range_ell(P->ell, x.w);
+  const float lmax = warp_fmax(l);
+  const float g = K.use_geo ? 1.f / (2.f * lmax * lmax) : 0.f;
+  const float Tn = fabsf(P->T[0]) + fabsf(P->T[1]) + fabsf(P->T[2]);
+  const float xn = warp_fmax(sqrtf(x.x * x.x + x.y * x.y + x.z * x.z));
+  const float slack = K.use_geo ? 4e-5f * (xn + Tn + lmax * sqrtf(2.f * fmaxf(tau, 0.f))) + 1e-6f : 0.f;
+  // box of the rows' positions in the target's own frame (q = R x + T)
+  const float *R = P->R;
+  const float qx = fmaf(R[0], x.x, fmaf(R[1], x.y, fmaf(R[2], x.z, P->T[0])));
+  const float qy = fmaf(R[3], x.x, fmaf(R[4], x.y, fmaf(R[5], x.z, P->T[1])));
+  const float qz = fmaf(R[6], x.x, fmaf(R[7], x.y, fmaf(R[8], x.z, P->T[2])));
+  const float qlo[3] = {warp_fmin(qx) - slack, warp_fmin(qy) - slack, warp_fmin(qz) - slack};
+  const float qhi[3] = {warp_fmax(qx) + slack, warp_fmax(qy) + slack, warp_fmax(qz) + slack};
+  // box of the rows' features (kept with the cloud) and the tile's centre
+  float flo[8], fhi[8], fc[8];
+#pragma unroll
+  for (int f = 0; f < 8; f++) flo[f] = fhi[f] = fc[f] = 0.f;
+  const int st = (n + 31) >> 5;
+#pragma unroll
+  for (int q = 0; q < FCH; q++) {
+    const float4 a = __ldg(P->sbox + (size_t)(2 + q) * st + tile), b = __ldg(P->sbox + (size_t)(2 + FCH + q) * st + tile);
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      flo[4 * q + r] = f4_at(a, r);
+      fhi[4 * q + r] = f4_at(b, r);
+      fc[4 * q + r] = 0.5f * (flo[4 * q + r] + fhi[4 * q + r]);
     }
   }
-  return pos;
-}
-
-// Kept count of a finished row; a row with more than cap kept pairs is listed for
-// k_select (its ELL row and its spill list hold them all) or k_rescan.
-__device__ __forceinline__ void finish_row(const BatchDev &B, PairDev *P, int p, int s, int cnt, int cap, int ov) {
-  P->nnz_row[s] = cnt < cap ? cnt : cap;
-  if (cnt > cap && cap > 0) {
-    if (cnt - cap <= ov) B.sel_list[atomicAdd(B.sel_count, 1)] = make_int4(p, s, cnt, 0);
-    else B.scan_list[atomicAdd(B.scan_count, 1)] = make_int4(p, s, cnt, 0);
+  const float pc[3] = {__shfl_sync(FULLMASK, x.x, 0), __shfl_sync(FULLMASK, x.y, 0), __shfl_sync(FULLMASK, x.z, 0)};
+  const float sg = sqrtf(g), sc = sqrtf(cw);
+  // the rows' operands
+  bool wide;
+  {
+    float v[11];
+    cand_coords<FCH>(v, x, xf, pc, fc, sg, sc);
+    __half h[11];
+    float sa = 0.f;
+#pragma unroll
+    for (int k = 0; k < 11; k++) {
+      h[k] = __float2half_rn(v[k]);
+      const float r = __half2float(h[k]);
+      sa = fmaf(r, r, sa);
+      h[k] = __float2half_rn(-2.f * r);
+    }
+    const float A = sqrtf(warp_fmax(sa)), rt = sqrtf(fmaxf(tau, 0.f));
+    wide = !(A <= kCandWide);
+    const float reach = 2.f * A + rt;
+    const float rb = rt + 4.95e-4f * reach + 2e-6f;
+    const float bound = rb * rb * 1.00001f + 4e-6f * reach * reach + 1e-6f;
+    const float d = valid ? sa - bound : kCandFar;
+    const __half hi = __float2half_rn(d), one = __float2half_rn(1.f);
+    cand_store(h, hi, __float2half_rn(d - __half2float(hi)), one, one, apl, lane);
   }
-}
-
-// Stores kept pair number `slot` of source row sidx: the first cap go to the row's
-// ELL slots, the next ov to its spill list (row-major), the rest are only counted.
-__device__ __forceinline__ void put_kept(PairDev *P, int ld, int cap, int ov, size_t sidx, int slot, int j, float a) {
-  if (slot < cap) {
-    P->A_j[sidx * ld + slot] = j;
-    P->A_v[sidx * ld + slot] = a;
-  } else if (slot - cap < ov) {
-    P->ovf[sidx * ov + (slot - cap)] = make_int2(j, __float_as_int(a));
-  }
-}
-
-// Dynamic shared memory of one k_assoc block: per warp two staging buffers, the
-// prefilter tile and the grid descriptor (16-byte aligned pieces).
-template <int FCH, int LCH, bool GT>
-struct AssocSmem {
-  static constexpr int kWarps = kAssocThreads / 32;
-  static constexpr size_t align16(size_t v) { return (v + 15) & ~(size_t)15; }
-  static constexpr size_t kStage = 0;
-  static constexpr size_t kMma = align16(kStage + sizeof(StageBuf<FCH, LCH, GT>) * 2 * kWarps);
-  static constexpr size_t kRows = align16(kMma + sizeof(MmaTile) * kWarps);
-  static constexpr size_t kGrid = align16(kRows + sizeof(SrcRows<FCH, LCH>) * kWarps);
-  static constexpr size_t kBytes = align16(kGrid + sizeof(GridDesc) * kWarps);
-};
-
-// Plane p of a row/candidate block: entry i at base[p * stride + i] (16 B = 8 halves).
-// A fragments (rows 16m..16m+15) of plane pair `hl` (0 = hi, 2 = lo).
-__device__ __forceinline__ void mma_load_a(const uint4 *a, int stride, int hl, int m, int lane, uint32_t (&r)[4]) {
-  const int mi = lane >> 3, r8 = lane & 7;
-  ldsm_x4(&a[(hl + (mi >> 1)) * stride + 16 * m + 8 * (mi & 1) + r8], r[0], r[1], r[2], r[3]);
-}
-
-// B fragments of candidate groups 2j and 2j+1 (candidates 16j..16j+15).
-__device__ __forceinline__ void mma_load_b(const uint4 *b, int stride, int hl, int j, int lane, uint32_t (&r)[4]) {
-  const int mi = lane >> 3, r8 = lane & 7;
-  ldsm_x4(&b[(hl + (mi & 1)) * stride + 16 * j + 8 * (mi >> 1) + r8], r[0], r[1], r[2], r[3]);
-}
-
-// u-tile of 32 rows (planes at a, stride as) against 32 candidates (planes at b,
-// stride bs); returns, for the lane's own row, the bit mask of candidates with
-// u < tau.  All lanes call it.
-__device__ __forceinline__ uint32_t mma_filter(const uint4 *a, int as, const uint4 *b, int bs, int lane, float tau) {
-  uint32_t word = 0;   // byte (2m + h), bit (2n + jj): row 16m + 8h + lane/4, column 8n + 2(lane%4) + jj
+  __syncwarp();
+  uint32_t af[2][4];
 #pragma unroll
-  for (int j = 0; j < 2; j++) {
-    uint32_t bh[4], bl[4];
-    mma_load_b(b, bs, 0, j, lane, bh);
-    mma_load_b(b, bs, 2, j, lane, bl);
+  for (int mm = 0; mm < 2; mm++)
+    ldsm_x4(&apl[lane >> 4][16 * mm + (lane & 15)], af[mm][0], af[mm][1], af[mm][2], af[mm][3]);
+  const float box_tau = tau * 1.0001f + 1e-5f, dc_max = K.use_int ? K.d2_c_thres * 1.0001f : INFINITY;
+  const int caps = P->cap_split;
+  uint2 *out = P->cand + (size_t)si * P->cand_pitch + (size_t)sp * caps;
+  const int ng = P->groups, ns = (ng + 31) >> 5;
+  int cnt = 0, cands = 0;
+  const int my_col = cand_col(lane);
+  const int src0 = 4 * (lane & 7);
+  const uint32_t sel = (uint32_t)(lane >> 3) | ((uint32_t)((lane >> 3) + 4) << 4);
+  const float4 *__restrict__ ycur = P->ycur;
+  const float4 *__restrict__ tfs = reinterpret_cast<const float4 *>(P->tfs);
+  const int mine = sp < ns ? (ns - sp + S - 1) / S : 0;      // supergroups sp, sp + S, ...
+  for (int u0 = 0; u0 < mine && tau > 0.f; u0 += 32) {
+    const int su = sp + S * (u0 + lane);
+    const bool snear = u0 + lane < mine && box_near<FCH>(P->tsup, ns, su, qlo, qhi, flo, fhi, g, cw, box_tau, dc_max);
+    uint32_t sm = __ballot_sync(FULLMASK, snear);
+    while (sm) {
+      const int g0 = 32 * (sp + S * (u0 + __ffs(sm) - 1));
+      sm &= sm - 1;
+      const bool gnear = g0 + lane < ng && box_near<FCH>(P->tbox, ng, g0 + lane, qlo, qhi, flo, fhi, g, cw, box_tau, dc_max);
+      uint32_t gm = __ballot_sync(FULLMASK, gnear);
+      float4 y = make_float4(0.f, 0.f, 0.f, 0.f), yf[FP];
 #pragma unroll
-    for (int m = 0; m < 2; m++) {
-      uint32_t ah[4], al[4];
-      mma_load_a(a, as, 0, m, lane, ah);
-      mma_load_a(a, as, 2, m, lane, al);
+      for (int q = 0; q < FP; q++) yf[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+      auto load = [&](uint32_t mk) {      // the next group's candidates, in flight while this one is tested
+        if (!mk) return;
+        const int t = min(32 * (g0 + __ffs(mk) - 1) + lane, m - 1);
+        y = __ldg(&ycur[t]);
 #pragma unroll
-      for (int q = 0; q < 2; q++) {
-        const int n = 2 * j + q;
-        float d[4] = {0.f, 0.f, 0.f, 0.f};
-        mma_16816(d, ah, bh[2 * q], bh[2 * q + 1]);
-        mma_16816(d, ah, bl[2 * q], bl[2 * q + 1]);
-        mma_16816(d, al, bh[2 * q], bh[2 * q + 1]);
-        word |= (d[0] < tau ? 1u : 0u) << (8 * (2 * m) + 2 * n);
-        word |= (d[1] < tau ? 1u : 0u) << (8 * (2 * m) + 2 * n + 1);
-        word |= (d[2] < tau ? 1u : 0u) << (8 * (2 * m + 1) + 2 * n);
-        word |= (d[3] < tau ? 1u : 0u) << (8 * (2 * m + 1) + 2 * n + 1);
+        for (int q = 0; q < FCH; q++) yf[q] = __ldg(tfs + (size_t)t * FCH + q);
+      };
+      load(gm);
+      while (gm) {
+        const int gi = g0 + __ffs(gm) - 1;
+        const bool has = 32 * gi + lane < m;
+        uint32_t mask = 0;
+        gm &= gm - 1;
+        if (!wide) {
+          float v[11];
+          cand_coords<FCH>(v, y, yf, pc, fc, sg, sc);
+          load(gm);
+          __half h[11];
+          float sb = 0.f;
+#pragma unroll
+          for (int k = 0; k < 11; k++) {
+            h[k] = __float2half_rn(v[k]);
+            const float r = __half2float(h[k]);
+            sb = fmaf(r, r, sb);
+          }
+          const bool far = !has || !(sb <= kCandFar);
+          const __half zero = __float2half_rn(0.f), one = __float2half_rn(1.f);
+          if (far) {
+#pragma unroll
+            for (int k = 0; k < 11; k++) h[k] = zero;
+            sb = kCandFar;
+          }
+          const __half hi = __float2half_rn(sb);
+          __syncwarp();      // the previous group's operands have been read
+          cand_store(h, one, one, hi, __float2half_rn(sb - __half2float(hi)), bpl, my_col);
+          __syncwarp();
+          uint32_t b0[4], b1[4];
+          ldsm_x4(&bpl[(lane >> 3) & 1][8 * (lane >> 4) + (lane & 7)], b0[0], b0[1], b0[2], b0[3]);
+          ldsm_x4(&bpl[(lane >> 3) & 1][16 + 8 * (lane >> 4) + (lane & 7)], b1[0], b1[1], b1[2], b1[3]);
+          uint32_t wb[4];      // byte 2 mm + hh: rows 16 mm + 8 hh + lane / 4
+#pragma unroll
+          for (int mm = 0; mm < 2; mm++) {
+            uint32_t w0 = 0, w1 = 0;
+#pragma unroll
+            for (int nn = 0; nn < 4; nn++) {
+              float d[4];
+              mma_16816(d, af[mm], nn < 2 ? b0[2 * nn] : b1[2 * nn - 4], nn < 2 ? b0[2 * nn + 1] : b1[2 * nn - 3]);
+              w0 = __funnelshift_l(__float_as_uint(d[0]), w0, 1);
+              w0 = __funnelshift_l(__float_as_uint(d[1]), w0, 1);
+              w1 = __funnelshift_l(__float_as_uint(d[2]), w1, 1);
+              w1 = __funnelshift_l(__float_as_uint(d[3]), w1, 1);
+            }
+            wb[2 * mm] = w0;
+            wb[2 * mm + 1] = w1;
+          }
+          const uint32_t word = __byte_perm(__byte_perm(wb[0], wb[1], 0x0040), __byte_perm(wb[2], wb[3], 0x0040), 0x5410);
+          if (!__any_sync(FULLMASK, word != 0)) continue;
+          uint32_t q4[4];
+#pragma unroll
+          for (int t = 0; t < 4; t++) q4[t] = __shfl_sync(FULLMASK, word, src0 + t);
+          mask = __byte_perm(__byte_perm(q4[0], q4[1], sel), __byte_perm(q4[2], q4[3], sel), 0x5410);
+        } else {
+          // a tile many lengthscales wide: the same test in FP32, candidate by candidate
+#pragma unroll 1
+          for (int k = 0; k < 32; k++) {
+            float d = 0.f, e = 0.f;
+            const float yx = __shfl_sync(FULLMASK, y.x, k), yy = __shfl_sync(FULLMASK, y.y, k), yz = __shfl_sync(FULLMASK, y.z, k);
+            d = (x.x - yx) * (x.x - yx) + (x.y - yy) * (x.y - yy) + (x.z - yz) * (x.z - yz);
+#pragma unroll
+            for (int f = 0; f < 4 * FCH; f++) {
+              const float t = f4_at(xf[FCH > 0 ? (f >> 2) % FCH : 0], f & 3) -
+                              __shfl_sync(FULLMASK, f4_at(yf[FCH > 0 ? (f >> 2) % FCH : 0], f & 3), k);
+              e += t * t;
+            }
+            if (!(g * d + cw * e > box_tau)) mask |= 1u << k;
+          }
+          const uint32_t there = __ballot_sync(FULLMASK, has);
+          mask &= there;
+          load(gm);
+        }
+        if (valid && mask) {
+          if (cnt < caps) out[cnt] = make_uint2((uint32_t)gi, mask);
+          cnt++;
+          cands += __popc(mask);
+        }
       }
     }
   }
-  // gather the lane's row: held by lanes 4 (row % 8) + t, t = 0..3
-  const int sh = 8 * (2 * (lane >> 4) + ((lane >> 3) & 1));
-  const int src0 = 4 * (lane & 7);
-  uint32_t mask = 0;
-#pragma unroll
-  for (int t = 0; t < 4; t++) {
-    const uint32_t w = __shfl_sync(FULLMASK, word, src0 + t);
-    const uint32_t bb = (w >> sh) & 0xFFu;
-    const uint32_t sp = (bb & 0x3u) | ((bb & 0xCu) << 6) | ((bb & 0x30u) << 12) | ((bb & 0xC0u) << 18);
-    mask |= sp << (2 * t);
-  }
-  return mask;
+  if (valid) P->cand_cnt[(size_t)sp * n + s] = make_int2(cnt, cands);
 }
 
-// Filter vector of a source row (A) or a candidate (B), relative to the centre p.
-template <int FCH>
-__device__ __forceinline__ void mma_row_vec(float (&av)[16], bool valid, const float4 &x, const float4 (&xf)[FCH > 0 ? FCH : 1],
-                                            int F, float g, float cw, float px, float py, float pz) {
-  const float tx = x.x - px, ty = x.y - py, tz = x.z - pz;
-  g = valid ? g : 0.f;
-  av[0] = -2.f * g * tx; av[1] = -2.f * g * ty; av[2] = -2.f * g * tz;
-  float xc2 = 0.f;
+// --------------------------------------------------------------- row pass
+// Sum of each of 8 values over the warp: lane l returns value l >> 2 (three folding
+// steps halve the values a lane carries, two more finish the sum).
+__device__ __forceinline__ float warp_sum8(const float (&v)[8], int lane) {
+  float a[4], b[2], c;
 #pragma unroll
-  for (int f = 0; f < 8; f++) {
-    float xv = 0.f;
-    if (FCH > 0 && (f >> 2) < FCH && f < F) xv = f4_at(xf[(f >> 2) < FCH ? (f >> 2) : 0], f & 3);
-    av[3 + f] = valid ? -2.f * cw * xv : 0.f;
-    xc2 += xv * xv;
+  for (int k = 0; k < 4; k++) {
+    const bool up = lane & 16;
+    const float keep = up ? v[k + 4] : v[k], give = up ? v[k] : v[k + 4];
+    a[k] = keep + __shfl_xor_sync(FULLMASK, give, 16);
   }
-  av[11] = g;
-  av[12] = valid ? cw : 0.f;
-  av[13] = valid ? g * (tx * tx + ty * ty + tz * tz) + cw * xc2 : 0.f;
-  float na = 0.f;
 #pragma unroll
-  for (int k = 0; k < 14; k++) na += av[k] * av[k];
-  av[14] = -kMmaKappa * sqrtf(na);
-  av[15] = 0.f;
+  for (int k = 0; k < 2; k++) {
+    const bool up = lane & 8;
+    const float keep = up ? a[k + 2] : a[k], give = up ? a[k] : a[k + 2];
+    b[k] = keep + __shfl_xor_sync(FULLMASK, give, 8);
+  }
+  {
+    const bool up = lane & 4;
+    const float keep = up ? b[1] : b[0], give = up ? b[0] : b[1];
+    c = keep + __shfl_xor_sync(FULLMASK, give, 4);
+  }
+  c += __shfl_xor_sync(FULLMASK, c, 2);
+  return c + __shfl_xor_sync(FULLMASK, c, 1);
 }
 
-template <int FCH>
-__device__ __forceinline__ void mma_cand_vec(float (&bv)[16], bool has, const float4 &y, const float4 *yf, int F,
-                                             float px, float py, float pz) {
-#pragma unroll
-  for (int q = 0; q < 16; q++) bv[q] = 0.f;
-  if (!has) return;
-  bv[0] = y.x - px; bv[1] = y.y - py; bv[2] = y.z - pz;
-  float yc2 = 0.f;
-#pragma unroll
-  for (int f = 0; f < 8; f++) {
-    float yv = 0.f;
-    if (FCH > 0 && (f >> 2) < FCH && f < F) yv = f4_at(yf[(f >> 2) < FCH ? (f >> 2) : 0], f & 3);
-    bv[3 + f] = yv;
-    yc2 += yv * yv;
-  }
-  bv[11] = bv[0] * bv[0] + bv[1] * bv[1] + bv[2] * bv[2];
-  bv[12] = yc2;
-  bv[13] = 1.f;
-  float nb = 0.f;
-#pragma unroll
-  for (int q = 0; q < 14; q++) nb += bv[q] * bv[q];
-  bv[14] = sqrtf(nb);
-}
-
-// Exact evaluation of the surviving pairs of one candidate group, 32 at a time:
-// pair number i of the warp (rows in order, each row's candidates ascending) goes
-// to lane i % 32, so a row's kept pairs still enter it in ascending candidate
-// order.  `cand` is the lane's own row mask, `cnt` its kept count (updated);
-// put(r, slot, j, a) stores kept pair number `slot` of row r.
-template <int FCH, int LCH, bool GT, class Put>
-__device__ __forceinline__ void eval_survivors(const KParams &K, int F, int C, int lane, uint32_t cand, int &cnt,
-                                               const SrcRows<FCH, LCH> &sr, const float4 *cpos, const float4 *cfeat,
-                                               const float4 *clab, const float4 *cgeo, Put put) {
-  const int cc = __popc(cand);
-  int incl = cc;
+__device__ __forceinline__ int warp_excl_scan(int v, int lane, int &total) {
+  int incl = v;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const int t = __shfl_up_sync(FULLMASK, incl, o);
     if (lane >= o) incl += t;
   }
-  const int excl = incl - cc;
-  const int total = __shfl_sync(FULLMASK, incl, 31);
-  for (int b0 = 0; b0 < total; b0 += 32) {
-    const int idx = b0 + lane;
-    const bool has = idx < total;
-    int r = 0;   // row of pair idx: the last row whose first pair is at or before idx
+  total = __shfl_sync(FULLMASK, incl, 31);
+  return incl - v;
+}
+
+// One block of four warps per source tile, one warp per row.  The row's candidates
+// (entries of k_cand) are put in ascending target index -- up to 32 of them by a sorting
+// network over the lanes, more through a bitmap over a window of target indices in shared
+// memory -- and evaluated 32 at a time with the exact arithmetic, the next 32 records in
+// flight.  The reference scans the targets by index and stops at cap kept pairs
+// (src/cvo/CvoGPU.cu:994-996): here the row stops there too, so no pair beyond cap is
+// evaluated or stored.  A row whose entries did not fit, or a call without a candidate
+// test, scans all targets in index order instead.  Gradient partials: FP32 per lane and
+// row, summed over the lanes, FP64 from there (CvoGPU.cu:2001-2062); the last block of a
+// pair adds the blocks' sums in a fixed order and normalises the gradient.
+// Bounds: latency of the dependent steps entry -> permutation -> bitmap -> record, hidden
+// by 16-28 resident warps per SM (the bitmap's shared memory sets the number).  The rows'
+// FP64 constants are computed 32 rows at a time: once per warp and row they took most of
+// a pass over rows without candidates.
+constexpr int kRowWarps = 4;
+constexpr int kRowsPerBlock = kGroup;
+constexpr int kMaxSplits = 16;
+constexpr int kRowWindow = 65536;       // most target indices of one bitmap window
+constexpr int kRowQueue = 512;          // sorted candidates of one round
+
+// Words of one warp's bitmap for targets of up to m points: an odd number per lane, so
+// that the lanes' runs start in different banks.
+__host__ __device__ inline int row_window_words(int m) {
+  return 32 * ((((m < kRowWindow ? m : kRowWindow) + 1023) / 1024) | 1);
+}
+__host__ __device__ inline size_t row_smem_bytes(int m) {
+  return (size_t)kRowWarps * sizeof(uint32_t) * (row_window_words(m) + kRowQueue);
+}
+
+// Block sums -> part; the last block of the pair finishes the pass.
+__device__ __forceinline__ void rows_finish(const BatchDev &B, const KParams &K, PairDev *P, int b, int nb, double lane_sum,
+                                            long long nnz, int mx) {
+  __shared__ double sh[kRowWarps][9];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if ((lane & 3) == 0 && lane < 28) sh[w][lane >> 2] = lane_sum;
+  if (lane == 0) {
+    sh[w][7] = (double)nnz;
+    sh[w][8] = (double)mx;
+  }
+  __syncthreads();
+  if (threadIdx.x < 9) {
+    double t = sh[0][threadIdx.x];
+    for (int q = 1; q < kRowWarps; q++) t = threadIdx.x < 8 ? t + sh[q][threadIdx.x] : fmax(t, sh[q][threadIdx.x]);
+    P->part[(size_t)b * kPartStride + threadIdx.x] = t;
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&P->counter[0], 1u) == (unsigned)(nb - 1);
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double t[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  for (int q = threadIdx.x; q < nb; q += 32 * kRowWarps) {
+    const double *pv = P->part + (size_t)q * kPartStride;
 #pragma unroll
-    for (int st = 16; st > 0; st >>= 1) {
-      const int e = __shfl_sync(FULLMASK, excl, r + st);
-      if (e <= idx) r += st;
+    for (int k = 0; k < 8; k++) t[k] += __ldcg(pv + k);
+    t[8] = fmax(t[8], __ldcg(pv + 8));
+  }
+#pragma unroll
+  for (int k = 0; k < 8; k++) t[k] = warp_sum(t[k]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t[8] = fmax(t[8], __shfl_xor_sync(FULLMASK, t[8], o));
+  if (lane == 0)
+    for (int k = 0; k < 9; k++) sh[w][k] = t[k];
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  double tot[9];
+  for (int k = 0; k < 9; k++) {
+    tot[k] = sh[0][k];
+    for (int q = 1; q < kRowWarps; q++) tot[k] = k < 8 ? tot[k] + sh[q][k] : fmax(tot[k], sh[q][k]);
+  }
+  P->counter[0] = 0;
+  // algorithmic bytes of this pair's association pass: every source and target
+  // record once, the per-row count, and the ELL entries when they are written
+  atomicAdd(B.assoc_bytes, (double)(P->n + P->m) * B.record_bytes + 4.0 * P->n +
+                               (P->mode != MODE_IP ? 8.0 * tot[7] : 0.0));
+  for (int k = 0; k < 6; k++) P->grad[k] = P->mode == MODE_ALIGN ? tot[k] : 0.0;
+  P->asum = tot[6];
+  P->nnz_sum = (long long)tot[7];
+  P->max_row = (int)tot[8];
+  if (P->mode == MODE_ALIGN) {
+    // float normalisation of the stacked gradient (CvoGPU.cu:2096-2104)
+    float f[6];
+    for (int k = 0; k < 6; k++) f[k] = (float)tot[k];
+    float s = 0.f;
+    for (int k = 0; k < 6; k++) s = fa(s, fm(f[k], f[k]));
+    if (s > 0.f) {
+      float nr = __fsqrt_rn(s);
+      for (int k = 0; k < 6; k++) f[k] = __fdiv_rn(f[k], nr);
     }
-    const int er = __shfl_sync(FULLMASK, excl, r);
-    const uint32_t mr = __shfl_sync(FULLMASK, cand, r);
-    const int cr = __shfl_sync(FULLMASK, cnt, r);
-    const int k = has ? nth_set_bit(mr, idx - er) : 0;
-    const float4 xr = sr.x[r];
-    const float4 rr = sr.rc[r];
-    float4 xfr[FCH > 0 ? FCH : 1];
-    float4 xlr[LCH > 0 ? LCH : 1];
-#pragma unroll
-    for (int q = 0; q < (FCH > 0 ? FCH : 1); q++) xfr[q] = sr.f[r * (FCH > 0 ? FCH : 1) + q];
-#pragma unroll
-    for (int q = 0; q < (LCH > 0 ? LCH : 1); q++) xlr[q] = sr.l[r * (LCH > 0 ? LCH : 1) + q];
-    const float2 xgr = make_float2(rr.w, sr.g1[r]);
-    const float4 y = cpos[k];
-    float a;
-    const bool acc = eval_pair<FCH, LCH, GT>(K, F, C, has, rr.x, rr.y, rr.z, xr, xfr, xlr, xgr, y,
-                                             &cfeat[k * (FCH > 0 ? FCH : 1)], &clab[k * (LCH > 0 ? LCH : 1)],
-                                             &cgeo[GT ? k : 0], a);
-    const uint32_t bal = __ballot_sync(FULLMASK, acc);
-    if (acc) {
-      const int lo = max(er - b0, 0);
-      const uint32_t before = bal & ((1u << lane) - 1u) & ~((1u << lo) - 1u);
-      put(r, cr + __popc(before), __float_as_int(y.w), a);
-    }
-    // row owners count their kept pairs of this group
-    const int lo = min(max(excl - b0, 0), 32), hi = min(max(incl - b0, 0), 32);
-    const uint32_t seg = (uint32_t)(((1ull << hi) - 1ull) & ~((1ull << lo) - 1ull));
-    cnt += __popc(bal & seg);
+    for (int k = 0; k < 6; k++) P->xi[k] = f[k];
   }
 }
 
-// ------------------------------------------------------------ association
-// One warp per tile of 32 spatially adjacent source points (Morton order).  The
-// warp scans the grid cells overlapping the union of its lanes' query boxes;
-// each candidate target is staged once per warp in shared memory and tested by
-// every lane against its own source point.  Chunks are double-buffered: the copy
-// of chunk k+1 is in flight while the lanes test chunk k.
 template <int FCH, int LCH, bool GT>
-__device__ __forceinline__ void assoc_warp(const BatchDev &B, const KParams &K, int gw, unsigned char *assoc_smem) {
-  using Buf = StageBuf<FCH, LCH, GT>;
-  using L = AssocSmem<FCH, LCH, GT>;
-  constexpr int CH = Buf::CH;
-  Buf(*stage_all)[2] = reinterpret_cast<Buf(*)[2]>(assoc_smem + L::kStage);
-  MmaTile *mma_all = reinterpret_cast<MmaTile *>(assoc_smem + L::kMma);
-  SrcRows<FCH, LCH> *rows_all = reinterpret_cast<SrcRows<FCH, LCH> *>(assoc_smem + L::kRows);
-  GridDesc *grid_all = reinterpret_cast<GridDesc *>(assoc_smem + L::kGrid);
-  const int lane = threadIdx.x & 31;
-  const int wib = threadIdx.x >> 5;
-  Buf *stage = stage_all[wib];
-  MmaTile &mt = mma_all[wib];
-  SrcRows<FCH, LCH> &sr = rows_all[wib];
-  if (gw >= B.total_warps) return;
-  const int p = find_segment(B.tile_off, B.npairs, gw);
+__global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams K, int window_words) {
+  extern __shared__ __align__(16) uint32_t row_smem[];
+  __shared__ float4 sh_rc[kRowsPerBlock];                  // l, d2 threshold, 1 / (2 l^2)
+  __shared__ int2 sh_cnt[kMaxSplits][kRowsPerBlock];       // entries and candidates per split
+  __shared__ int2 sh_tot[kRowsPerBlock];                   // of the row; entries < 0: scan all targets
+  __shared__ float4 sh_keep[kRowWarps][64];                // kept pairs by slot: y and value
+  __shared__ int sh_keepj[kRowWarps][64];
+  constexpr int FP = FCH > 0 ? FCH : 1;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint32_t *bits = row_smem + (size_t)w * (window_words + kRowQueue);
+  int *queue = reinterpret_cast<int *>(bits + window_words);
+  const int blk = blockIdx.x;
+  if (blk >= B.total_rblocks) return;
+  const int p = find_segment(B.rblk_off, B.npairs, blk);
   PairDev *P = &B.pairs[p];
   if (P->done) return;
-  if (lane == 0) grid_all[wib] = P->levels[P->level];
-  __syncwarp();
-  const GridDesc &G = grid_all[wib];
-  const int n = P->n;
-  const int s = (gw - B.tile_off[p]) * 32 + lane;
-  const bool valid = s < n;
-  const float ell = P->ell;
-  const int cap = P->cap;
-  const int F = P->F, C = P->C;
-  float4 x = valid ? __ldg(&P->xs[s]) : make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 xf[FCH > 0 ? FCH : 1];
-  float4 xl[LCH > 0 ? LCH : 1];
-  float2 xg = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int q = 0; q < (FCH > 0 ? FCH : 1); q++)
-    xf[q] = (FCH > 0 && valid) ? __ldg(reinterpret_cast<const float4 *>(P->xf) + (size_t)s * FCH + q)
-                               : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-  for (int q = 0; q < (LCH > 0 ? LCH : 1); q++)
-    xl[q] = (LCH > 0 && valid) ? __ldg(reinterpret_cast<const float4 *>(P->xl) + (size_t)s * LCH + q)
-                               : make_float4(0.f, 0.f, 0.f, 0.f);
-  if (GT && valid) xg = __ldg(&P->xg[s]);
-  const float Tn = fabsf(P->T[0]) + fabsf(P->T[1]) + fabsf(P->T[2]);
-  RowConst rc = row_const(K, ell, x.w, Tn);
-  // query box in the target's initial frame: q = R x + T
-  const float *R = P->R;
-  float qx = fmaf(R[0], x.x, fmaf(R[1], x.y, fmaf(R[2], x.z, P->T[0])));
-  float qy = fmaf(R[3], x.x, fmaf(R[4], x.y, fmaf(R[5], x.z, P->T[1])));
-  float qz = fmaf(R[6], x.x, fmaf(R[7], x.y, fmaf(R[8], x.z, P->T[2])));
-  float lox = valid ? qx - rc.rq : INFINITY, hix = valid ? qx + rc.rq : -INFINITY;
-  float loy = valid ? qy - rc.rq : INFINITY, hiy = valid ? qy + rc.rq : -INFINITY;
-  float loz = valid ? qz - rc.rq : INFINITY, hiz = valid ? qz + rc.rq : -INFINITY;
-  // own box of this lane (used when the warp's union box is too sparse)
-  int ox0 = 0, oy0 = 0, oz0 = 0, onx = 0, ony = 0, onz = 0;
-  long long own_cells = 0;
-  if (valid && cell_range(G, lox, loy, loz, hix, hiy, hiz, ox0, oy0, oz0, onx, ony, onz))
-    own_cells = (long long)onx * ony * onz;
-  long long own_sum = own_cells;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) own_sum += __shfl_xor_sync(FULLMASK, own_sum, o);
-  lox = warp_min(lox); loy = warp_min(loy); loz = warp_min(loz);
-  hix = warp_max(hix); hiy = warp_max(hiy); hiz = warp_max(hiz);
-  int ux0, uy0, uz0, unx, uny, unz;
-  const bool union_ok = cell_range(G, lox, loy, loz, hix, hiy, hiz, ux0, uy0, uz0, unx, uny, unz);
-  const long long union_cells = union_ok ? (long long)unx * uny * unz : 0;
-  // One pass over the union box of the tile, or, when that box is much larger
-  // than the lanes' own boxes together, one pass per lane over its own box.
-  const bool per_lane = union_cells > 64 && union_cells > 2 * own_sum;
-  const int npass = per_lane ? 32 : (union_ok ? 1 : 0);
-  // Tensor-core prefilter for the tile (one pass over the union box, F <= 8).
-  bool use_mma = K.use_mma && npass == 1 && !per_lane && F <= 8;
-  float pcx = 0.f, pcy = 0.f, pcz = 0.f;   // centre of the tile's valid source points
-  const float cw = K.use_int ? K.inv2c2 : 0.f;
-  if (use_mma) {
-    const int nv = warp_sumi(valid ? 1 : 0);
-    const float inv = 1.f / (float)max(nv, 1);
-    pcx = warp_sumf(valid ? x.x : 0.f) * inv;
-    pcy = warp_sumf(valid ? x.y : 0.f) * inv;
-    pcz = warp_sumf(valid ? x.z : 0.f) * inv;
-    float av[16];
-    mma_row_vec<FCH>(av, valid, x, xf, F, rc.inv2l2, cw, pcx, pcy, pcz);
-    const bool ok = mma_store_vec(av, &mt.a[0][0], 32, lane);
-    use_mma = __all_sync(FULLMASK, ok);
-    // this row's data for the lanes that evaluate its surviving pairs
-    sr.x[lane] = x;
-    sr.rc[lane] = make_float4(rc.l, rc.d2t, rc.inv2l2, xg.x);
-    sr.g1[lane] = xg.y;
-#pragma unroll
-    for (int q = 0; q < (FCH > 0 ? FCH : 1); q++) sr.f[lane * (FCH > 0 ? FCH : 1) + q] = xf[q];
-#pragma unroll
-    for (int q = 0; q < (LCH > 0 ? LCH : 1); q++) sr.l[lane * (LCH > 0 ? LCH : 1) + q] = xl[q];
-    __syncwarp();
-  }
-  int cnt = 0;
-  const float4 *__restrict__ ycur = P->ycur;
-  const int ov = P->ov;
-  const int tile0 = (gw - B.tile_off[p]) * 32;   // source index of lane 0's row
-  // kept pair number `slot` of row r enters its ELL slot (first cap) or its spill list
-  const int ld = P->ld;
-  auto put = [&](int r, int slot, int j, float a) { put_kept(P, ld, cap, ov, (size_t)(tile0 + r), slot, j, a); };
-  for (int pass = 0; pass < npass; pass++) {
-    int x0, y0, z0, nx, ny, nz;
-    bool me = valid;
-    if (per_lane) {
-      x0 = __shfl_sync(FULLMASK, ox0, pass); y0 = __shfl_sync(FULLMASK, oy0, pass);
-      z0 = __shfl_sync(FULLMASK, oz0, pass); nx = __shfl_sync(FULLMASK, onx, pass);
-      ny = __shfl_sync(FULLMASK, ony, pass); nz = __shfl_sync(FULLMASK, onz, pass);
-      if (__shfl_sync(FULLMASK, own_cells, pass) == 0) continue;
-      me = valid && lane == pass;
-    } else {
-      x0 = ux0; y0 = uy0; z0 = uz0; nx = unx; ny = uny; nz = unz;
-    }
-    // bounding box of this pass's query points and their largest search radius
-    float bl0 = qx, bl1 = qy, bl2 = qz, bh0 = qx, bh1 = qy, bh2 = qz, brq = valid ? rc.rq : 0.f;
-    if (per_lane) {
-      bl0 = bh0 = __shfl_sync(FULLMASK, qx, pass); bl1 = bh1 = __shfl_sync(FULLMASK, qy, pass);
-      bl2 = bh2 = __shfl_sync(FULLMASK, qz, pass); brq = __shfl_sync(FULLMASK, brq, pass);
-    } else {
-      bl0 = warp_min(valid ? qx : INFINITY); bl1 = warp_min(valid ? qy : INFINITY); bl2 = warp_min(valid ? qz : INFINITY);
-      bh0 = warp_max(valid ? qx : -INFINITY); bh1 = warp_max(valid ? qy : -INFINITY); bh2 = warp_max(valid ? qz : -INFINITY);
-      brq = warp_max(brq);
-    }
-    const float slack = 1e-3f * G.h;
-    const float prune_r2 = (brq + slack) * (brq + slack);
-    const int ncells = nx * ny * nz;
-    for (int cb = 0; cb < ncells; cb += 32) {
-      int ci = cb + lane;
-      int2 se = make_int2(0, 0);
-      if (ci < ncells) {
-        int cx = x0 + ci % nx, cy = y0 + (ci / nx) % ny, cz = z0 + ci / (nx * ny);
-        // skip cells farther than the largest radius from every query point of the pass
-        bool near = true;
-        if (G.inv_h != 0.f) {
-          const float c0 = fmaf((float)cx, G.h, G.ox), c1 = fmaf((float)cy, G.h, G.oy), c2 = fmaf((float)cz, G.h, G.oz);
-          const float dx = fmaxf(fmaxf(c0 - bh0, bl0 - (c0 + G.h)), 0.f);
-          const float dy = fmaxf(fmaxf(c1 - bh1, bl1 - (c1 + G.h)), 0.f);
-          const float dz = fmaxf(fmaxf(c2 - bh2, bl2 - (c2 + G.h)), 0.f);
-          near = dx * dx + dy * dy + dz * dz <= prune_r2;
-        }
-        if (near) se = grid_lookup(G, cx, cy, cz);
-      }
-      unsigned mk = __ballot_sync(FULLMASK, se.y > 0);
-      if (!mk) continue;
-      // Chunks of up to CH candidates filled from consecutive non-empty cells of this
-      // batch; the warp walks a cursor (cell, offset) in lockstep.
-      int c_start = 0, c_cnt = 0, c_off = 0;
-      auto fill = [&](int bi) -> int {
-        int filled = 0;
-        while (filled < CH) {
-          if (c_off >= c_cnt) {
-            if (!mk) break;
-            const int bb = __ffs(mk) - 1;
-            mk &= mk - 1;
-            c_start = __shfl_sync(FULLMASK, se.x, bb);
-            c_cnt = __shfl_sync(FULLMASK, se.y, bb);
-            c_off = 0;
-          }
-          const int take = min(CH - filled, c_cnt - c_off);
-          stage_piece<FCH, LCH, GT>(stage[bi], ycur, G, filled, c_start + c_off, take, lane);
-          filled += take;
-          c_off += take;
-        }
-        __syncwarp();   // the chunk is visible to every lane
-        return filled;
-      };
-      int cur = 0;
-      int nk = fill(cur);
-      while (nk > 0) {
-        const Buf &sb = stage[cur];
-        if (use_mma) {
-          // candidate vectors of this chunk (lane k builds candidate k; empty slots are zero)
-          float bv[16];
-          mma_cand_vec<FCH>(bv, lane < nk, sb.pos[lane], &sb.feat[lane * (FCH > 0 ? FCH : 1)], F, pcx, pcy, pcz);
-          const bool ok = __all_sync(FULLMASK, mma_store_vec(bv, &mt.b[0][0], 32, lane));
-          __syncwarp();
-          uint32_t cand = ok ? mma_filter(&mt.a[0][0], 32, &mt.b[0][0], 32, lane, K.mma_tau) : 0xFFFFFFFFu;
-          cand &= (nk >= 32) ? 0xFFFFFFFFu : ((1u << nk) - 1u);
-          if (!me) cand = 0u;
-          eval_survivors<FCH, LCH, GT>(K, F, C, lane, cand, cnt, sr, sb.pos, sb.feat, sb.lab, sb.geo, put);
-        } else {
-          for (int k = 0; k < nk; k++) {
-            const float4 y = sb.pos[k];
-            float a;
-            bool acc = eval_pair<FCH, LCH, GT>(K, F, C, me, rc.l, rc.d2t, rc.inv2l2, x, xf, xl, xg, y,
-                                               &sb.feat[k * (FCH > 0 ? FCH : 1)], &sb.lab[k * (LCH > 0 ? LCH : 1)],
-                                               &sb.geo[GT ? k : 0], a);
-            if (acc) { put(lane, cnt, __float_as_int(y.w), a); cnt++; }
-          }
-        }
-        __syncwarp();   // every lane is done with the chunk before the next one is staged
-        cur ^= 1;
-        nk = fill(cur);
-      }
-    }
-  }
-  if (valid) finish_row(B, P, p, s, cnt, cap, ov);
-}
-
-template <int FCH, int LCH, bool GT>
-__global__ void __launch_bounds__(kAssocThreads) k_assoc(BatchDev B, KParams K) {
-  extern __shared__ __align__(128) unsigned char assoc_smem[];
-  assoc_warp<FCH, LCH, GT>(B, K, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, assoc_smem);
-}
-
-// ------------------------------------------------------------ selection
-constexpr int kSelMax = 4096;      // kept pairs beyond cap one spill list can hold
-constexpr int kSelStage = 1024;    // rows up to this many entries are selected from shared memory
-constexpr int kSelThreads = 128;
-
-// Row partials of one source row from its final ELL entries, in slot order
-// (thread per row): omega = sum a (x cross y), v = sum a (y - x), sum a.
-// (CvoGPU.cu:2001-2062 computes the same sums from the sparse kernel matrix.)
-__global__ void __launch_bounds__(256) k_rowsum(BatchDev B, KParams K) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= B.total_rows) return;
-  const int p = find_segment(B.row_off, B.npairs, g);
-  const PairDev *P = &B.pairs[p];
-  if (P->done) return;
-  const int s = g - B.row_off[p];
-  const int z = P->nnz_row[s];
-  const float4 x = __ldg(&P->xs[s]);
-  float w0 = 0.f, w1 = 0.f, w2 = 0.f, v0 = 0.f, v1 = 0.f, v2 = 0.f, as = 0.f;
-  const int *__restrict__ Aj = P->A_j + (size_t)s * P->ld;
-  const float *__restrict__ Av = P->A_v + (size_t)s * P->ld;
+  const int b = blk - B.rblk_off[p], nb = B.rblk_off[p + 1] - B.rblk_off[p];
+  const int n = P->n, m = P->m, F = P->F, C = P->C, cap = P->cap, mode = P->mode, S = P->splits, caps = P->cap_split;
   const float4 *__restrict__ yorig = P->yorig;
-  auto add = [&](float a, const float4 &y) {
-    w0 = fmaf(a, fs(fm(x.y, y.z), fm(x.z, y.y)), w0);
-    w1 = fmaf(a, fs(fm(x.z, y.x), fm(x.x, y.z)), w1);
-    w2 = fmaf(a, fs(fm(x.x, y.y), fm(x.y, y.x)), w2);
-    v0 = fmaf(a, y.x - x.x, v0);
-    v1 = fmaf(a, y.y - x.y, v1);
-    v2 = fmaf(a, y.z - x.z, v2);
-    as += a;
-  };
-  int c = 0;
-  // four entries per 16-byte load (rows are 16-byte aligned); the sums keep slot order
-  for (; c + 4 <= z; c += 4) {
-    const int4 j4 = *reinterpret_cast<const int4 *>(Aj + c);
-    const float4 a4 = *reinterpret_cast<const float4 *>(Av + c);
-    const float4 y0 = __ldg(&yorig[j4.x]), y1 = __ldg(&yorig[j4.y]), y2 = __ldg(&yorig[j4.z]), y3 = __ldg(&yorig[j4.w]);
-    add(a4.x, y0);
-    add(a4.y, y1);
-    add(a4.z, y2);
-    add(a4.w, y3);
-  }
-  for (; c < z; c++) add(Av[c], __ldg(&yorig[Aj[c]]));
-  write_row_sums(P->row_sums + (size_t)s * 8, P->mode, K, w0, w1, w2, v0, v1, v2, as);
-}
-
-// One warp per listed row with cap < count <= cap + ov: its ELL slots hold the
-// first cap kept pairs and its spill list (row-major) the rest, in the order they
-// were kept.  The indices of a row of up to kSelStage entries are first staged in
-// shared memory (16-byte loads: many loads in flight per lane), so the radix passes
-// read no global memory; the values stay in global memory and are read once, by
-// the compaction, for the kept entries only.  A radix select over d = j - jmin
-// (jmin, jmax: the row's smallest and largest kept index; 9-bit digits from the
-// highest bit of jmax - jmin, warp-private histograms) finds the cap-th smallest
-// index r.  Offsetting by jmin spreads the indices over the bins, each lane counts
-// its own run of the list (so one instruction's increments come from different
-// grid cells and rarely collide), and a row whose indices span fewer than 512 values
-// needs one pass.  The entries with index <= r (exactly cap: indices are distinct)
-// are compacted in list order into the ELL slots, in place: an entry is read before
-// any write can reach its slot, and a __syncwarp between a chunk's reads and its
-// writes orders the lanes' accesses.  Longer rows read their indices from global
-// memory on every pass.  Eight blocks of four warps per SM: 6.2 KB of shared memory
-// per warp and at most 64 registers a thread keep 32 warps resident, which hide the
-// latency of the dependent passes of each warp's rows.
-constexpr int kSelBins = 512;
-constexpr int kSelDigit = 9;
-constexpr int kSelBlocksPerSm = 8;
-// bin b lives at b + b / 16: lane l's scan reads its 16 bins at stride 17 words, on
-// distinct banks
-constexpr int kSelHist = kSelBins + kSelBins / 16;
-__device__ __forceinline__ int sel_bin(int b) { return b + (b >> 4); }
-__global__ void __launch_bounds__(kSelThreads, kSelBlocksPerSm) k_select(BatchDev B, KParams K) {
-  __shared__ int jbuf_all[kSelThreads / 32][kSelStage];
-  __shared__ int hist_all[kSelThreads / 32][kSelHist];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int *jb = jbuf_all[w];
-  int *hist = hist_all[w];
-  const int count = *B.sel_count;
-  const int nwarps = gridDim.x * (kSelThreads / 32);
-  const int e0 = blockIdx.x * (kSelThreads / 32) + w;
-  int4 next = e0 < count ? B.sel_list[e0] : make_int4(0, 0, 0, 0);
-  for (int e = e0; e < count; e += nwarps) {
-    const int4 it = next;            // this row's list entry; the next one is loaded meanwhile
-    if (e + nwarps < count) next = B.sel_list[e + nwarps];
-    const PairDev *P = &B.pairs[it.x];
-    const int s = it.y, cap = P->cap, ov = P->ov;
-    const int E = it.z;
-    const int2 *lst = P->ovf + (size_t)s * ov;
-    int *Aj = P->A_j + (size_t)s * P->ld;
-    float *Av = P->A_v + (size_t)s * P->ld;
-    const bool staged = E <= kSelStage;
-    auto gidx = [&](int t) -> int { return t < cap ? Aj[t] : lst[t - cap].x; };
-    int jmin = 0x7FFFFFFF, jmax = -1;
-    if (staged) {
-      // ELL part: 4 indices per 16-byte load (rows are 16-byte aligned, the pitch covers
-      // the rounded-up chunk); spill part: 2 entries per 16-byte load (rows start 16-byte
-      // aligned).  Each lane issues up to 4 loads before it stores any: the loads go
-      // through generic pointers, which the compiler must not move past a shared-memory
-      // store, so loads and stores interleaved one by one would wait for memory in turn.
-      const int nq = (cap + 3) >> 2;
-      for (int q0 = lane; q0 < nq; q0 += 128) {
-        int4 j4[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-          if (q0 + 32 * u < nq) j4[u] = reinterpret_cast<const int4 *>(Aj)[q0 + 32 * u];
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const int q = q0 + 32 * u;
-          if (q < nq) {
-            const int jv[4] = {j4[u].x, j4[u].y, j4[u].z, j4[u].w};
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-              if (4 * q + i < cap) {
-                jb[4 * q + i] = jv[i];
-                jmin = min(jmin, jv[i]);
-                jmax = max(jmax, jv[i]);
-              }
-          }
-        }
+  const float4 *__restrict__ tf = reinterpret_cast<const float4 *>(P->tf);
+  const float4 *__restrict__ tl = reinterpret_cast<const float4 *>(P->tl);
+  const int *__restrict__ tperm = P->tperm;
+  {
+    const int s = b * kRowsPerBlock + lane;
+    if (w == 0) {
+      const RowConst rc = row_const(K, P->ell, s < n ? __ldg(&P->xs[s]).w : 0.f);
+      sh_rc[lane] = make_float4(rc.l, rc.d2t, rc.inv2l2, 0.f);
+    }
+    if (K.use_mma)
+      for (int q = w; q < S; q += kRowWarps) sh_cnt[q][lane] = s < n ? __ldg(&P->cand_cnt[(size_t)q * n + s]) : make_int2(0, 0);
+    __syncthreads();
+    if (w == 0) {
+      int2 t = make_int2(K.use_mma ? 0 : -1, 0);
+      bool fits = true;
+      for (int q = 0; q < S && K.use_mma; q++) {
+        const int2 c = sh_cnt[q][lane];
+        fits = fits && c.x <= caps;
+        t.x += c.x;
+        t.y += c.y;
       }
-      const int ns = E - cap, np = (ns + 1) >> 1;
-      for (int q0 = lane; q0 < np; q0 += 128) {
-        int4 v4[4];
+      if (!fits) t.x = -1;
+      if (cap <= 0 || s >= n) t.x = 0;
+      sh_tot[lane] = t;
+      if (s < n && t.x == 0) P->nnz_row[s] = 0;
+    }
+    __syncthreads();
+  }
+  double lane_sum = 0.0;
+  long long nnz = 0;
+  int mx = 0;
+  for (int r = w; r < kRowsPerBlock; r += kRowWarps) {
+    const int entries = sh_tot[r].x, cands = sh_tot[r].y;
+    if (entries == 0) continue;
+    const int s = b * kRowsPerBlock + r;
+    const float4 x = __ldg(&P->xs[s]);
+    float4 xf[FP];
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const int q = q0 + 32 * u;
-          if (2 * q + 1 < ns) v4[u] = reinterpret_cast<const int4 *>(lst)[q];
-          else if (2 * q < ns) v4[u] = make_int4(lst[2 * q].x, 0, -1, 0);
+    for (int q = 0; q < FP; q++)
+      xf[q] = FCH > 0 ? __ldg(reinterpret_cast<const float4 *>(P->xf) + (size_t)s * FCH + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 *xl = reinterpret_cast<const float4 *>(P->xl) + (size_t)s * LCH;
+    const float2 xg = GT ? __ldg(&P->xg[s]) : make_float2(0.f, 0.f);
+    const float4 rc = sh_rc[r];
+    const uint2 *ent = P->cand + (size_t)s * P->cand_pitch;
+    // entry e of the row, the splits' entries one after the other
+    auto entry = [&](int e) {
+      const uint2 *at = nullptr;
+      for (int q = 0; q < S; q++) {
+        const int c = sh_cnt[q][r].x;
+        if (e >= 0 && e < c) at = ent + (size_t)q * caps + e;
+        e -= c;
+      }
+      return at ? __ldg(at) : make_uint2(0u, 0u);
+    };
+    int kept = 0;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    // 32 kept pairs to the ELL row and the gradient: lane l takes slots l, l + 32, ..., so
+    // the sums depend on the kept pairs alone, not on the candidates beside them
+    int flushed = 0;
+    float4 *keep = sh_keep[w];
+    int *keepj = sh_keepj[w];
+    auto flush = [&](bool on) {
+      const float4 v = keep[(flushed + lane) & 63];
+      if (on) {
+        if (mode != MODE_IP) {
+          P->A_j[(size_t)s * P->ld + flushed + lane] = keepj[(flushed + lane) & 63];
+          P->A_v[(size_t)s * P->ld + flushed + lane] = v.w;
         }
+        acc[0] = fmaf(v.w, fs(fm(x.y, v.z), fm(x.z, v.y)), acc[0]);
+        acc[1] = fmaf(v.w, fs(fm(x.z, v.x), fm(x.x, v.z)), acc[1]);
+        acc[2] = fmaf(v.w, fs(fm(x.x, v.y), fm(x.y, v.x)), acc[2]);
+        acc[3] = fmaf(v.w, v.x - x.x, acc[3]);
+        acc[4] = fmaf(v.w, v.y - x.y, acc[4]);
+        acc[5] = fmaf(v.w, v.z - x.z, acc[5]);
+        acc[6] += v.w;
+      }
+      flushed += 32;
+      __syncwarp();
+    };
+    int w0 = 0, base = 0, total = 0, off = 0, bank = 0;      // bitmap window, rounds of its candidates
+    bool fresh = true;
+    const int wl = window_words >> 5;
+    while (true) {
+      int count = 0;
+      if (entries < 0) {
+        count = m;
+      } else if (cands <= 32) {
+        // every candidate in a lane, sorted by a bitonic network
+        const uint2 v = entry(lane);
+        int o = warp_excl_scan(__popc(v.y), lane, count);
+        for (uint32_t mk = v.y; mk; mk &= mk - 1) queue[o++] = __ldg(&tperm[32 * (int)v.x + __ffs(mk) - 1]);
+        __syncwarp();
+        int j = lane < count ? queue[lane] : 0x7FFFFFFF;
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const int q = q0 + 32 * u;
-          if (2 * q < ns) {
-            jb[cap + 2 * q] = v4[u].x;
-            jmin = min(jmin, v4[u].x);
-            jmax = max(jmax, v4[u].x);
-            if (2 * q + 1 < ns) {
-              jb[cap + 2 * q + 1] = v4[u].z;
-              jmin = min(jmin, v4[u].z);
-              jmax = max(jmax, v4[u].z);
+        for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll
+          for (int d = k >> 1; d > 0; d >>= 1) {
+            const int o2 = __shfl_xor_sync(FULLMASK, j, d);
+            const bool lower = ((lane & d) == 0) == ((lane & k) == 0 || k == 32);
+            j = lower ? min(j, o2) : max(j, o2);
+          }
+        queue[lane] = j;
+        __syncwarp();
+      } else {
+        if (fresh) {
+          for (int i = lane; i < window_words / 4; i += 32) reinterpret_cast<uint4 *>(bits)[i] = make_uint4(0u, 0u, 0u, 0u);
+          __syncwarp();
+          uint2 next = entry(lane);
+          for (int e0 = 0; e0 < entries; e0 += 32) {
+            const uint2 v = next;
+            if (e0 + 32 < entries) next = entry(e0 + 32 + lane);
+            const int here = min(32, entries - e0);
+#pragma unroll 8
+            for (int i = 0; i < here; i++) {
+              const uint32_t g = __shfl_sync(FULLMASK, v.x, i), mk = __shfl_sync(FULLMASK, v.y, i);
+              if ((mk >> lane) & 1u) {
+                const uint32_t k = (uint32_t)(__ldg(&tperm[32 * (int)g + lane]) - w0);
+                if (k < 32u * (uint32_t)window_words) atomicOr(&bits[k >> 5], 1u << (k & 31));
+              }
             }
           }
+          __syncwarp();
+          // lane l owns words l * wl .. : their candidates follow those of the lanes before
+          bank = 0;
+          for (int i = 0; i < wl; i++) bank += __popc(bits[lane * wl + i]);
+          off = warp_excl_scan(bank, lane, total);
+          base = 0;
+          fresh = false;
         }
-      }
-    } else {
-      for (int t = lane; t < E; t += 32) {
-        const int j = gidx(t);
-        jmin = min(jmin, j);
-        jmax = max(jmax, j);
-      }
-    }
-    jmin = __reduce_min_sync(FULLMASK, jmin);
-    jmax = __reduce_max_sync(FULLMASK, jmax);
-    __syncwarp();
-    auto entry = [&](int t) -> int { return staged ? jb[t] : gidx(t); };
-    const int span = jmax - jmin;
-    const int bits = span > 0 ? 32 - __clz(span) : 1;
-    // lane l counts the contiguous run of entries l * per .. : neighbouring entries of
-    // the list come from one grid cell and share their high index bits, so the 32
-    // increments of one instruction then go to different bins instead of colliding (an
-    // odd run length keeps the 32 lanes' shared-memory reads on distinct banks)
-    const int per = ((E + 31) >> 5) | 1;
-    const int t_lo = lane * per, t_hi = min(t_lo + per, E);
-    int prefix = 0, target = cap;
-    for (int hs = bits; hs > 0; hs -= kSelDigit) {
-      const int sh = max(hs - kSelDigit, 0), wd = hs - sh;
-      for (int b = lane; b < kSelHist; b += 32) hist[b] = 0;
-      __syncwarp();
-      const int want = prefix >> hs, mask = (1 << wd) - 1;
-#pragma unroll 4
-      for (int t = t_lo; t < t_hi; t++) {
-        const int d = entry(t) - jmin;
-        if ((d >> hs) == want) atomicAdd(&hist[sel_bin((d >> sh) & mask)], 1);
-      }
-      __syncwarp();
-      // lane l owns bins 16 l .. 16 l + 15: their total, an exclusive scan over the lanes,
-      // the lane L whose bins reach target, then the bin inside L's 16 (lanes 0..15 read
-      // one bin each and scan them)
-      constexpr int kPer = kSelBins / 32;
-      int loc = 0;
-#pragma unroll
-      for (int i = 0; i < kPer; i++) loc += hist[sel_bin(lane * kPer + i)];
-      int incl = loc;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(FULLMASK, incl, o);
-        if (lane >= o) incl += t;
-      }
-      int L = __ffs(__ballot_sync(FULLMASK, incl >= target)) - 1;
-      if (L < 0) L = 31;             // unreachable: the counted entries always reach target
-      const int before = __shfl_sync(FULLMASK, incl - loc, L);
-      const int hb = lane < kPer ? hist[sel_bin(L * kPer + lane)] : 0;
-      int hin = hb;
-#pragma unroll
-      for (int o = 1; o < kPer; o <<= 1) {
-        const int t = __shfl_up_sync(FULLMASK, hin, o);
-        if (lane >= o) hin += t;
-      }
-      int i_bin = __ffs(__ballot_sync(FULLMASK, lane < kPer && before + hin >= target)) - 1;
-      if (i_bin < 0) i_bin = kPer - 1;  // unreachable, as above
-      const int run = before + __shfl_sync(FULLMASK, hin - hb, i_bin);
-      prefix |= (L * kPer + i_bin) << sh;
-      target -= run;
-      __syncwarp();
-    }
-    const int r = jmin + prefix;   // the cap-th smallest kept index
-    // compaction, 128 entries per round: every lane reads its 4 entries (index, and the
-    // value of a kept one: 4 independent loads in flight), a __syncwarp orders these reads
-    // before the round's writes (which go to slots below the round's end), then the 4
-    // chunks are placed in list order
-    int base = 0;
-    for (int t0 = 0; t0 < E; t0 += 128) {
-      int j[4];
-      float a[4];
-      bool k[4];
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const int t = t0 + 32 * u + lane;
-        j[u] = t < E ? entry(t) : 0;
-        k[u] = t < E && j[u] <= r;
-        a[u] = 0.f;
-      }
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const int t = t0 + 32 * u + lane;
-        if (k[u]) a[u] = t < cap ? Av[t] : __int_as_float(lst[t - cap].y);
-      }
-      __syncwarp();
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const unsigned bal = __ballot_sync(FULLMASK, k[u]);
-        const int c = base + __popc(bal & ((1u << lane) - 1u));
-        if (k[u] && c < cap) {
-          Aj[c] = j[u];
-          Av[c] = a[u];
+        count = min(kRowQueue, total - base);
+        if (off < base + count && off + bank > base) {
+          int o = off - base;
+          for (int i = 0; i < wl && o < count; i++) {
+            uint32_t mk = bits[lane * wl + i];
+            if (o + __popc(mk) <= 0) {
+              o += __popc(mk);
+              continue;
+            }
+            for (; mk; mk &= mk - 1, o++)
+              if (o >= 0 && o < count) queue[o] = w0 + 32 * (lane * wl + i) + __ffs(mk) - 1;
+          }
         }
-        base += __popc(bal);
+        base += count;
+        __syncwarp();
+      }
+      // the round's candidates, 32 at a time
+      const bool direct = entries < 0;
+      float4 y = make_float4(0.f, 0.f, 0.f, 0.f), yf[FP];
+#pragma unroll
+      for (int q = 0; q < FP; q++) yf[q] = y;
+      int j = 0;
+      auto load = [&](int i) {
+        if (i >= count) return;
+        j = direct ? i : queue[i];
+        y = __ldg(&yorig[j]);
+#pragma unroll
+        for (int q = 0; q < FCH; q++) yf[q] = __ldg(tf + (size_t)j * FCH + q);
+      };
+      load(lane);
+      for (int i0 = 0; i0 < count && kept < cap; i0 += 32) {
+        const bool has = i0 + lane < count;
+        const float4 yc = y;
+        float4 fc[FP];
+#pragma unroll
+        for (int q = 0; q < FP; q++) fc[q] = yf[q];
+        const int jc = j;
+        load(i0 + 32 + lane);
+        const float2 yg = GT && has ? __ldg(&P->tg[jc]) : make_float2(0.f, 0.f);
+        float a = 0.f;
+        const bool k = eval_pair<FCH, LCH, GT>(K, F, C, has, rc.x, rc.y, rc.z, x, xf, xl, xg, yc, fc,
+                                               tl + (size_t)jc * LCH, yg, a);
+        const unsigned bal = __ballot_sync(FULLMASK, k);
+        const int c = kept + __popc(bal & ((1u << lane) - 1u));
+        if (k && c < cap) {
+          keep[c & 63] = make_float4(yc.x, yc.y, yc.z, a);
+          keepj[c & 63] = jc;
+        }
+        kept += __popc(bal);
+        __syncwarp();
+        if (min(kept, cap) - flushed >= 32) flush(true);
+      }
+      __syncwarp();
+      if (kept >= cap || entries < 0 || cands <= 32) break;
+      if (base >= total) {
+        w0 += 32 * window_words;
+        if (w0 >= m) break;
+        fresh = true;
       }
     }
-    __syncwarp();
+    const int z = min(kept, cap);
+    if (flushed < z) flush(lane < z - flushed);
+    if (lane == 0) P->nnz_row[s] = z;
+    nnz += z;
+    mx = max(mx, z);
+    const float sum = warp_sum8(acc, lane);
+    const int k = lane >> 2;
+    lane_sum += (double)(k < 3 ? __fdiv_rn(sum, K.c) : (k < 6 ? __fdiv_rn(sum, K.d) : sum));
   }
-}
-
-// One warp per listed row with count > cap + ov: the reference's own order, i.e. a
-// scan of the targets by ascending original index (32 per step, one per lane) that
-// stops once cap pairs are kept.  Same per-pair arithmetic as k_assoc.
-template <int FCH, int LCH, bool GT>
-__global__ void __launch_bounds__(kSelThreads) k_rescan(BatchDev B, KParams K) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int count = *B.scan_count;
-  const int nwarps = gridDim.x * (kSelThreads / 32);
-  for (int e = blockIdx.x * (kSelThreads / 32) + w; e < count; e += nwarps) {
-    const int4 it = B.scan_list[e];
-    const PairDev *P = &B.pairs[it.x];
-    const int s = it.y, m = P->m, cap = P->cap, F = P->F, C = P->C;
-    const float4 x = P->xs[s];
-    float4 xf[FCH > 0 ? FCH : 1];
-    float4 xl[LCH > 0 ? LCH : 1];
-#pragma unroll
-    for (int q = 0; q < (FCH > 0 ? FCH : 1); q++)
-      xf[q] = FCH > 0 ? __ldg(reinterpret_cast<const float4 *>(P->xf) + (size_t)s * FCH + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int q = 0; q < (LCH > 0 ? LCH : 1); q++)
-      xl[q] = LCH > 0 ? __ldg(reinterpret_cast<const float4 *>(P->xl) + (size_t)s * LCH + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float2 xg = GT ? __ldg(&P->xg[s]) : make_float2(0.f, 0.f);
-    const float Tn = fabsf(P->T[0]) + fabsf(P->T[1]) + fabsf(P->T[2]);
-    const RowConst rc = row_const(K, P->ell, x.w, Tn);
-    int taken = 0;
-    for (int j0 = 0; j0 < m && taken < cap; j0 += 32) {
-      const int j = j0 + lane;
-      const bool pre = j < m;
-      const int jj = pre ? j : 0;
-      const float4 y = __ldg(&P->yorig[jj]);
-      float4 yg = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (GT) { const float2 g2 = __ldg(&P->tg[jj]); yg.x = g2.x; yg.y = g2.y; }
-      const float4 *yfp = reinterpret_cast<const float4 *>(P->tf) + (size_t)jj * (FCH > 0 ? FCH : 1);
-      const float4 *ylp = reinterpret_cast<const float4 *>(P->tl) + (size_t)jj * (LCH > 0 ? LCH : 1);
-      float a = 0.f;
-      const bool k = eval_pair<FCH, LCH, GT>(K, F, C, pre, rc.l, rc.d2t, rc.inv2l2, x, xf, xl, xg, y, yfp, ylp, &yg, a);
-      const unsigned bal = __ballot_sync(FULLMASK, k);
-      if (k) {
-        const int c = taken + __popc(bal & ((1u << lane) - 1u));
-        if (c < cap) {
-          P->A_j[(size_t)s * P->ld + c] = j;
-          P->A_v[(size_t)s * P->ld + c] = a;
-        }
-      }
-      taken += __popc(bal);
-    }
-  }
+  rows_finish(B, K, P, b, nb, lane_sum, nnz, mx);
 }
 
 }  // namespace cvo_gb
