@@ -109,7 +109,7 @@ struct PairDev {
   // iteration state
   float R[9], T[3];               // internal pose
   float Ri[9], Ti[3];             // target transform R^T, -R^T T
-  float ell;
+  float ell, step_coef;           // step_coef: 1 / (2 ell^2), rounded from double
   int cap;
   int iter, done, ret;
   float xi[6];

@@ -21,6 +21,8 @@ namespace cvo_gb {
 
 enum { MODE_ALIGN = 0, MODE_IP = 1, MODE_EXPORT = 2 };
 constexpr int kStepThreads = 256;
+constexpr int kStepRows = 16;           // rows of a block of k_step
+constexpr int kStepLanes = 16;          // lanes sharing one of them
 constexpr int kPartStride = 12;
 
 // ------------------------------------------------------------ pair value
@@ -494,6 +496,11 @@ __host__ __device__ inline size_t row_smem_bytes(int m) {
   return (size_t)kRowWarps * sizeof(uint32_t) * (row_window_words(m) + kRowQueue);
 }
 
+// 1 / (2 l^2) of the step-size terms (compute_step_size_xi), in double, rounded once.
+__device__ __forceinline__ float step_coef(float l) {
+  return __double2float_rn(__ddiv_rn(1.0, dm(dm(2.0, (double)l), (double)l)));
+}
+
 // Block sums -> part; the last block of the pair finishes the pass.
 __device__ __forceinline__ void rows_finish(const BatchDev &B, const KParams &K, PairDev *P, int b, int nb, double lane_sum,
                                             long long nnz, int mx) {
@@ -557,6 +564,7 @@ __device__ __forceinline__ void rows_finish(const BatchDev &B, const KParams &K,
       for (int k = 0; k < 6; k++) f[k] = __fdiv_rn(f[k], nr);
     }
     for (int k = 0; k < 6; k++) P->xi[k] = f[k];
+    P->step_coef = step_coef(P->ell);   // FP64 division: once here, not per row
   }
 }
 
