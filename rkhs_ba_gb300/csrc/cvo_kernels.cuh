@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(32 * kCandWarps) k_cand(BatchDev B, KParams K)
   const float pc[3] = {__shfl_sync(FULLMASK, x.x, 0), __shfl_sync(FULLMASK, x.y, 0), __shfl_sync(FULLMASK, x.z, 0)};
   const float sg = sqrtf(g), sc = sqrtf(cw);
   // the rows' operands
-  bool wide;
+  bool wide, spread;
   {
     float v[11];
     cand_coords<FCH>(v, x, xf, pc, fc, sg, sc);
@@ -304,6 +304,7 @@ __global__ void __launch_bounds__(32 * kCandWarps) k_cand(BatchDev B, KParams K)
     }
     const float A = sqrtf(warp_fmax(sa)), rt = sqrtf(fmaxf(tau, 0.f));
     wide = !(A <= kCandWide);
+    spread = K.use_geo && A > 3.f * rt;
     const float reach = 2.f * A + rt;
     const float rb = rt + 4.95e-4f * reach + 2e-6f;
     const float bound = rb * rb * 1.00001f + 4e-6f * reach * reach + 1e-6f;
@@ -326,6 +327,14 @@ __global__ void __launch_bounds__(32 * kCandWarps) k_cand(BatchDev B, KParams K)
   const uint32_t sel = (uint32_t)(lane >> 3) | ((uint32_t)((lane >> 3) + 4) << 4);
   const float4 *__restrict__ ycur = P->ycur;
   const float4 *__restrict__ tfs = reinterpret_cast<const float4 *>(P->tfs);
+  // A tile much wider than the search radius (the Morton order jumps within it) has a box
+  // that meets almost everything: such a tile also asks whether a box is near one of its rows.
+  auto row_near = [&](const float4 *box, int count, int i) {
+    const float4 lo = __ldg(box + i), hi = __ldg(box + count + i);
+    const float d = gap2(qx - slack, qx + slack, lo.x, hi.x) + gap2(qy - slack, qy + slack, lo.y, hi.y) +
+                    gap2(qz - slack, qz + slack, lo.z, hi.z);
+    return __any_sync(FULLMASK, !(g * d > box_tau));
+  };
   const int mine = sp < ns ? (ns - sp + S - 1) / S : 0;      // supergroups sp, sp + S, ...
   for (int u0 = 0; u0 < mine && tau > 0.f; u0 += 32) {
     const int su = sp + S * (u0 + lane);
@@ -334,8 +343,14 @@ __global__ void __launch_bounds__(32 * kCandWarps) k_cand(BatchDev B, KParams K)
     while (sm) {
       const int g0 = 32 * (sp + S * (u0 + __ffs(sm) - 1));
       sm &= sm - 1;
+      if (spread && !row_near(P->tsup, ns, g0 >> 5)) continue;
       const bool gnear = g0 + lane < ng && box_near<FCH>(P->tbox, ng, g0 + lane, qlo, qhi, flo, fhi, g, cw, box_tau, dc_max);
       uint32_t gm = __ballot_sync(FULLMASK, gnear);
+      if (spread)
+        for (uint32_t left = gm; left; left &= left - 1) {
+          const int k = __ffs(left) - 1;
+          if (!row_near(P->tbox, ng, g0 + k)) gm &= ~(1u << k);
+        }
       float4 y = make_float4(0.f, 0.f, 0.f, 0.f), yf[FP];
 #pragma unroll
       for (int q = 0; q < FP; q++) yf[q] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -468,7 +483,7 @@ __device__ __forceinline__ int warp_excl_scan(int v, int lane, int &total) {
 }
 
 // One block of four warps per source tile, one warp per row.  The row's candidates
-// (entries of k_cand) are put in ascending target index -- up to 32 of them by a sorting
+// (entries of k_cand) are put in ascending target index -- up to 128 of them by a sorting
 // network over the lanes, more through a bitmap over a window of target indices in shared
 // memory -- and evaluated 32 at a time with the exact arithmetic, the next 32 records in
 // flight.  The reference scans the targets by index and stops at cap kept pairs
@@ -486,6 +501,7 @@ constexpr int kRowsPerBlock = kGroup;
 constexpr int kMaxSplits = 16;
 constexpr int kRowWindow = 65536;       // most target indices of one bitmap window
 constexpr int kRowQueue = 512;          // sorted candidates of one round
+constexpr int kRowSorted = 128;         // most candidates a sorting network puts in order
 
 // Words of one warp's bitmap for targets of up to m points: an odd number per lane, so
 // that the lanes' runs start in different banks.
@@ -499,6 +515,39 @@ __host__ __device__ inline size_t row_smem_bytes(int m) {
 // 1 / (2 l^2) of the step-size terms (compute_step_size_xi), in double, rounded once.
 __device__ __forceinline__ float step_coef(float l) {
   return __double2float_rn(__ddiv_rn(1.0, dm(dm(2.0, (double)l), (double)l)));
+}
+
+// Sorts queue[0 .. count), count <= 32 R, in ascending order: a bitonic network over element
+// 32 r + lane in register r of each lane.
+template <int R>
+__device__ __forceinline__ void warp_sort(int *queue, int count, int lane) {
+  int v[R];
+#pragma unroll
+  for (int r = 0; r < R; r++) v[r] = 32 * r + lane < count ? queue[32 * r + lane] : 0x7FFFFFFF;
+#pragma unroll
+  for (int k = 2; k <= 32 * R; k <<= 1)
+#pragma unroll
+    for (int d = k >> 1; d > 0; d >>= 1) {
+      if (d >= 32) {
+#pragma unroll
+        for (int r = 0; r < R; r++)
+          if ((r & (d >> 5)) == 0) {
+            const int a = v[r], b = v[r | (d >> 5)];
+            const bool up = ((32 * r) & k) == 0;
+            v[r] = up ? min(a, b) : max(a, b);
+            v[r | (d >> 5)] = up ? max(a, b) : min(a, b);
+          }
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          const int o = __shfl_xor_sync(FULLMASK, v[r], d);
+          const bool up = ((32 * r + lane) & k) == 0;
+          v[r] = ((lane & d) == 0) == up ? min(v[r], o) : max(v[r], o);
+        }
+      }
+    }
+#pragma unroll
+  for (int r = 0; r < R; r++) queue[32 * r + lane] = v[r];
 }
 
 // Block sums -> part; the last block of the pair finishes the pass.
@@ -674,22 +723,19 @@ __global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams 
       int count = 0;
       if (entries < 0) {
         count = m;
-      } else if (cands <= 32) {
-        // every candidate in a lane, sorted by a bitonic network
-        const uint2 v = entry(lane);
-        int o = warp_excl_scan(__popc(v.y), lane, count);
-        for (uint32_t mk = v.y; mk; mk &= mk - 1) queue[o++] = __ldg(&tperm[32 * (int)v.x + __ffs(mk) - 1]);
+      } else if (cands <= kRowSorted) {
+        // one to four candidates in a lane, sorted by a bitonic network
+        for (int e0 = 0; e0 < entries; e0 += 32) {
+          const uint2 v = entry(e0 + lane);
+          int o, add;
+          o = count + warp_excl_scan(__popc(v.y), lane, add);
+          for (uint32_t mk = v.y; mk; mk &= mk - 1) queue[o++] = __ldg(&tperm[32 * (int)v.x + __ffs(mk) - 1]);
+          count += add;
+        }
         __syncwarp();
-        int j = lane < count ? queue[lane] : 0x7FFFFFFF;
-#pragma unroll
-        for (int k = 2; k <= 32; k <<= 1)
-#pragma unroll
-          for (int d = k >> 1; d > 0; d >>= 1) {
-            const int o2 = __shfl_xor_sync(FULLMASK, j, d);
-            const bool lower = ((lane & d) == 0) == ((lane & k) == 0 || k == 32);
-            j = lower ? min(j, o2) : max(j, o2);
-          }
-        queue[lane] = j;
+        if (count <= 32) warp_sort<1>(queue, count, lane);
+        else if (count <= 64) warp_sort<2>(queue, count, lane);
+        else warp_sort<4>(queue, count, lane);
         __syncwarp();
       } else {
         if (fresh) {
@@ -770,7 +816,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams 
         if (min(kept, cap) - flushed >= 32) flush(true);
       }
       __syncwarp();
-      if (kept >= cap || entries < 0 || cands <= 32) break;
+      if (kept >= cap || entries < 0 || cands <= kRowSorted) break;
       if (base >= total) {
         w0 += 32 * window_words;
         if (w0 >= m) break;
