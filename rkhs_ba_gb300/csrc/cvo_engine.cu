@@ -21,6 +21,104 @@ namespace {
 
 constexpr int kChunk = 8;
 
+// ------------------------------------------------------------------ reduce
+// Sums of columns 0 .. NV-1 of the blocks' partials, each from block 0 upwards by one thread
+// (the order is part of the result); all threads bring the partials to shared memory first,
+// where a chain of loads costs 30 cycles a step instead of an L2 round trip.  Column NV-1 is a
+// maximum if MAX.  buf: kReduceThreads * NV doubles; out: NV.
+template <int NV, bool MAX>
+__device__ __forceinline__ void sum_partials(const double *part, int nb, double *buf, double *out) {
+  double t = 0.0;
+  for (int q0 = 0; q0 < nb; q0 += kReduceThreads) {
+    const int here = min(kReduceThreads, nb - q0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < here * NV; i += blockDim.x)
+      buf[i] = __ldcg(part + (size_t)(q0 + i / NV) * kPartStride + i % NV);
+    __syncthreads();
+    if (threadIdx.x < NV)
+      for (int q = 0; q < here; q++) {
+        const double v = buf[q * NV + threadIdx.x];
+        t = MAX && threadIdx.x == NV - 1 ? fmax(t, v) : t + v;
+      }
+  }
+  if (threadIdx.x < NV) out[threadIdx.x] = t;
+  __syncthreads();
+}
+
+// Per-pair FP64 sums of the per-row partials written by k_rowsum.
+__global__ void __launch_bounds__(kReduceThreads) k_reduce(BatchDev B, KParams K) {
+  __shared__ double sh[kReduceThreads / 32][10];
+  __shared__ double buf[kReduceThreads * 9], tot[9];
+  __shared__ bool last;
+  const int blk = blockIdx.x;
+  if (blk >= B.total_gblocks) return;
+  const int p = find_segment(B.gblk_off, B.npairs, blk);
+  PairDev *P = &B.pairs[p];
+  if (P->done) return;
+  const int b = blk - B.gblk_off[p];
+  const int nb = B.gblk_off[p + 1] - B.gblk_off[p];
+  const int n = P->n;
+  double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  int mx = 0;
+  for (int r = b * kReduceRows + threadIdx.x; r < min(n, (b + 1) * kReduceRows); r += kReduceThreads) {
+    const float4 *rs = reinterpret_cast<const float4 *>(P->row_sums + (size_t)r * 8);
+    float4 a0 = rs[0], a1 = rs[1];
+    acc[0] += a0.x; acc[1] += a0.y; acc[2] += a0.z; acc[3] += a0.w;
+    acc[4] += a1.x; acc[5] += a1.y; acc[6] += a1.z;
+    int z = P->nnz_row[r];
+    acc[7] += (double)z;
+    mx = max(mx, z);
+  }
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < 8; k++) acc[k] = warp_sum(acc[k]);
+  mx = __reduce_max_sync(FULLMASK, mx);
+  if (lane == 0) {
+    for (int k = 0; k < 8; k++) sh[w][k] = acc[k];
+    sh[w][8] = (double)mx;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double out[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    for (int ww = 0; ww < kReduceThreads / 32; ww++) {
+      for (int k = 0; k < 8; k++) out[k] += sh[ww][k];
+      out[8] = fmax(out[8], sh[ww][8]);
+    }
+    for (int k = 0; k < 9; k++) P->part[(size_t)b * kPartStride + k] = out[k];
+    __threadfence();
+    unsigned prev = atomicAdd(&P->counter[0], 1u);
+    last = (prev == (unsigned)(nb - 1));
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  sum_partials<9, true>(P->part, nb, buf, tot);
+  if (threadIdx.x != 0) return;
+  P->counter[0] = 0;
+  pass_finished(B, P, tot[6], tot[7], tot[8]);
+  for (int k = 0; k < 6; k++) P->grad[k] = tot[k];
+  // float normalisation of the stacked gradient (CvoGPU.cu:2096-2104)
+  float f[6];
+  for (int k = 0; k < 6; k++) f[k] = (float)tot[k];
+  float s = 0.f;
+  for (int k = 0; k < 6; k++) s = fa(s, fm(f[k], f[k]));
+  if (s > 0.f) {
+    float nr = __fsqrt_rn(s);
+    for (int k = 0; k < 6; k++) f[k] = __fdiv_rn(f[k], nr);
+  }
+  for (int k = 0; k < 6; k++) P->xi[k] = f[k];
+}
+
+// Picks the finest lattice whose cells serve the largest search radius.
+__device__ void choose_level(PairDev *P, const KParams &K) {
+  float l = range_ell(P->ell, P->src_norm);
+  float r = K.use_geo ? sqrtf(geo_d2_thres(l, K.log_geo)) : 0.f;
+  int lv = P->nlevels - 1;
+  for (int i = 0; i < P->nlevels; i++)
+    if (P->level_r[i] >= r) { lv = i; break; }
+  P->level = lv;
+}
+
 __device__ void pose_to_rinv(PairDev *P) {
   for (int r = 0; r < 3; r++)
     for (int c = 0; c < 3; c++) P->Ri[3 * r + c] = P->R[3 * c + r];
@@ -116,20 +214,19 @@ __device__ void finalize_iteration(BatchDev &B, PairDev *P, const KParams &K) {
   if (P->iter >= K.max_iter) {
     P->done = 1;
     atomicSub(B.active, 1);
+    return;
   }
+  choose_level(P, K);
 }
 
 // -------------------------------------------------------------------- step
 // Taylor step-size terms (compute_step_size_xi + compute_step_size_poly_coeff,
-// src/cvo/CvoGPU.cu:333-462): FP32 per ELL row, FP64 across rows; the last block of a
-// pair finishes the iteration.  Sixteen lanes share a row: rows hold 10 to cap entries, so a
-// thread per row leaves its warp waiting for the longest one, and a warp per row idles on
-// short ones (a 60-iteration align of 50k colour points took 67, 62 and 63 ms with 8, 16
-// and 32 lanes).  A block takes 16 rows, and the last one adds the blocks' sums with all
-// threads.  Bounds: L2 latency of entry -> target, then the scalar tail in FP64.  One
-// thread per row and one thread adding the blocks' sums took 150 us on the 50k colour pair.
+// src/cvo/CvoGPU.cu:333-462) per ELL row in FP32, one entry after the other (see k_rowsum),
+// FP64 across rows; the last block of a pair adds the blocks' sums and finishes the iteration.
+// Bounds: L2 latency of index -> position, then the scalar tail in FP64.
 __global__ void __launch_bounds__(kStepThreads) k_step(BatchDev B, KParams K) {
   __shared__ double sh[kStepThreads / 32][4];
+  __shared__ double buf[kReduceThreads * 4], tot[4];
   __shared__ bool last;
   const int blk = blockIdx.x;
   if (blk >= B.total_sblocks) return;
@@ -139,88 +236,56 @@ __global__ void __launch_bounds__(kStepThreads) k_step(BatchDev B, KParams K) {
   const int b = blk - B.sblk_off[p];
   const int nb = B.sblk_off[p + 1] - B.sblk_off[p];
   const int n = P->n;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, sub = threadIdx.x & (kStepLanes - 1);
-  const float w0 = P->xi[0], w1 = P->xi[1], w2 = P->xi[2];
-  const float u0v = P->xi[3], u1v = P->xi[4], u2v = P->xi[5];
-  const float4 *__restrict__ yorig = P->yorig;
-  double v[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int s0 = b * kStepRows; s0 < min(n, (b + 1) * kStepRows); s0 += kStepThreads / kStepLanes) {
-    const int s = s0 + threadIdx.x / kStepLanes;
-    const int z = s < n ? __ldg(&P->nnz_row[s]) : 0;
-    float Bs = 0.f, Cs = 0.f, Ds = 0.f, Es = 0.f;
-    if (z > 0) {
-      const float4 x = __ldg(&P->xs[s]);
-      const float coef = K.use_range_ell_step ? step_coef(range_ell(P->ell, x.w)) : P->step_coef;
-      const int *__restrict__ Aj = P->A_j + (size_t)s * P->ld;
-      const float *__restrict__ Av = P->A_v + (size_t)s * P->ld;
-#pragma unroll 4
-      for (int c = sub; c < z; c += kStepLanes) {
-        const float a = __ldg(Av + c);
-        const float4 y = __ldg(&yorig[__ldg(Aj + c)]);
-        float ux = w1 * y.z - w2 * y.y + u0v, uy = w2 * y.x - w0 * y.z + u1v, uz = w0 * y.y - w1 * y.x + u2v;
-        float px = w1 * uz - w2 * uy, py = w2 * ux - w0 * uz, pz = w0 * uy - w1 * ux;          // xi^2 z
-        float qx = w1 * pz - w2 * py, qy = w2 * px - w0 * pz, qz = w0 * py - w1 * px;          // xi^3 z
-        float rx = w1 * qz - w2 * qy, ry = w2 * qx - w0 * qz, rz = w0 * qy - w1 * qx;          // xi^4 z
-        float dx = x.x - y.x, dy = x.y - y.y, dz = x.z - y.z;
-        float normxiz2 = ux * ux + uy * uy + uz * uz;
-        float xiz_dot_xi2z = -(ux * px + uy * py + uz * pz);
-        float epsil_const = (px * px + py * py + pz * pz) + 2.f * (ux * qx + uy * qy + uz * qz);
-        float beta = -2.f * coef * (ux * dx + uy * dy + uz * dz);
-        float gamma = -coef * (normxiz2 + 2.f * (px * dx + py * dy + pz * dz));
-        float delta = 2.f * coef * (xiz_dot_xi2z - (qx * dx + qy * dy + qz * dz));
-        float epsil = -coef * (epsil_const + 2.f * (rx * dx + ry * dy + rz * dz));
-        float b2 = beta * beta;
-        Bs += a * beta;
-        Cs += a * (gamma + 0.5f * b2);
-        Ds += a * (delta + beta * gamma + b2 * beta * (1.f / 6.f));
-        Es += a * (epsil + beta * delta + 0.5f * b2 * gamma + 0.5f * gamma * gamma + b2 * b2 * (1.f / 24.f));
-      }
-    }
-#pragma unroll
-    for (int o = kStepLanes / 2; o > 0; o >>= 1) {
-      Bs += __shfl_xor_sync(FULLMASK, Bs, o);
-      Cs += __shfl_xor_sync(FULLMASK, Cs, o);
-      Ds += __shfl_xor_sync(FULLMASK, Ds, o);
-      Es += __shfl_xor_sync(FULLMASK, Es, o);
-    }
-    if (sub == 0) {
-      v[0] += (double)Bs;
-      v[1] += (double)Cs;
-      v[2] += (double)Ds;
-      v[3] += (double)Es;
-    }
+  const int s = b * kStepThreads + threadIdx.x;
+  float Bs = 0.f, Cs = 0.f, Ds = 0.f, Es = 0.f;
+  if (s < n) {
+    const float w0 = P->xi[0], w1 = P->xi[1], w2 = P->xi[2];
+    const float u0v = P->xi[3], u1v = P->xi[4], u2v = P->xi[5];
+    float4 x = __ldg(&P->xs[s]);
+    float tl = K.use_range_ell_step ? range_ell(P->ell, x.w) : P->ell;
+    float coef = __double2float_rn(__ddiv_rn(1.0, dm(dm(2.0, (double)tl), (double)tl)));
+    const int z = P->nnz_row[s];
+    auto add = [&](float a, const float4 &y) {
+      float ux = w1 * y.z - w2 * y.y + u0v, uy = w2 * y.x - w0 * y.z + u1v, uz = w0 * y.y - w1 * y.x + u2v;
+      float px = w1 * uz - w2 * uy, py = w2 * ux - w0 * uz, pz = w0 * uy - w1 * ux;          // xi^2 z
+      float qx = w1 * pz - w2 * py, qy = w2 * px - w0 * pz, qz = w0 * py - w1 * px;          // xi^3 z
+      float rx = w1 * qz - w2 * qy, ry = w2 * qx - w0 * qz, rz = w0 * qy - w1 * qx;          // xi^4 z
+      float dx = x.x - y.x, dy = x.y - y.y, dz = x.z - y.z;
+      float normxiz2 = ux * ux + uy * uy + uz * uz;
+      float xiz_dot_xi2z = -(ux * px + uy * py + uz * pz);
+      float epsil_const = (px * px + py * py + pz * pz) + 2.f * (ux * qx + uy * qy + uz * qz);
+      float beta = -2.f * coef * (ux * dx + uy * dy + uz * dz);
+      float gamma = -coef * (normxiz2 + 2.f * (px * dx + py * dy + pz * dz));
+      float delta = 2.f * coef * (xiz_dot_xi2z - (qx * dx + qy * dy + qz * dz));
+      float epsil = -coef * (epsil_const + 2.f * (rx * dx + ry * dy + rz * dz));
+      float b2 = beta * beta;
+      Bs += a * beta;
+      Cs += a * (gamma + 0.5f * b2);
+      Ds += a * (delta + beta * gamma + b2 * beta * (1.f / 6.f));
+      Es += a * (epsil + beta * delta + 0.5f * b2 * gamma + 0.5f * gamma * gamma + b2 * b2 * (1.f / 24.f));
+    };
+    row_entries(P, s, z, add);
   }
-  // v: zero but in the first lane of each row
-#pragma unroll
-  for (int k = 0; k < 4; k++)
-#pragma unroll
-    for (int o = kStepLanes; o < 32; o <<= 1) v[k] += __shfl_xor_sync(FULLMASK, v[k], o);
-  if (lane == 0)
-    for (int k = 0; k < 4; k++) sh[w][k] = v[k];
-  __syncthreads();
-  if (threadIdx.x < 4) {
-    double o = 0.0;
-    for (int ww = 0; ww < kStepThreads / 32; ww++) o += sh[ww][threadIdx.x];
-    P->part[(size_t)b * kPartStride + threadIdx.x] = o;
-    __threadfence();
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(&P->counter[1], 1u) == (unsigned)(nb - 1);
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-#pragma unroll
-  for (int k = 0; k < 4; k++) v[k] = 0.0;
-  for (int q = threadIdx.x; q < nb; q += kStepThreads) {
-    const double *pv = P->part + (size_t)q * kPartStride;
-#pragma unroll
-    for (int k = 0; k < 4; k++) v[k] += __ldcg(pv + k);
-  }
+  double v[4] = {Bs, Cs, Ds, Es};
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
   for (int k = 0; k < 4; k++) v[k] = warp_sum(v[k]);
   if (lane == 0)
     for (int k = 0; k < 4; k++) sh[w][k] = v[k];
   __syncthreads();
+  if (threadIdx.x == 0) {
+    double o[4] = {0, 0, 0, 0};
+    for (int ww = 0; ww < kStepThreads / 32; ww++)
+      for (int k = 0; k < 4; k++) o[k] += sh[ww][k];
+    for (int k = 0; k < 4; k++) P->part[(size_t)b * kPartStride + k] = o[k];
+    __threadfence();
+    unsigned prev = atomicAdd(&P->counter[1], 1u);
+    last = (prev == (unsigned)(nb - 1));
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  sum_partials<4, false>(P->part, nb, buf, tot);
   // The scalar tail is one thread's chain of dependent reads and writes of the pair's state:
   // in shared memory they cost 30 cycles instead of an L2 round trip each.
   __shared__ PairDev state;
@@ -230,11 +295,7 @@ __global__ void __launch_bounds__(kStepThreads) k_step(BatchDev B, KParams K) {
   __syncthreads();
   if (threadIdx.x == 0) {
     state.counter[1] = 0;
-    for (int k = 0; k < 4; k++) {
-      double t = 0.0;
-      for (int ww = 0; ww < kStepThreads / 32; ww++) t += sh[ww][k];
-      state.bcde[k] = t;
-    }
+    for (int k = 0; k < 4; k++) state.bcde[k] = tot[k];
     finalize_iteration(B, &state, K);
   }
   __syncthreads();
@@ -262,7 +323,7 @@ using RowsFn = void (*)(BatchDev, KParams, int);
 
 struct AssocKernels {
   CandFn cand = nullptr;
-  RowsFn rows = nullptr;
+  RowsFn rows = nullptr, align_rows = nullptr;
 };
 
 // Feature rows are stored as ceil(F/4) float4 chunks; label rows as 5 or 9
@@ -271,13 +332,14 @@ struct AssocKernels {
 template <int FC, int LC, bool G>
 static int pick_assoc(AssocKernels *a) {
   a->cand = k_cand<FC>;
-  a->rows = k_rows<FC, LC, G>;
+  a->rows = k_rows<FC, LC, G, ROWS_SUM>;
+  a->align_rows = k_rows<FC, LC, G, ROWS_ALIGN>;
   // opt in above the 48 KB default (setting it again is harmless)
-  if (cudaFuncSetAttribute(a->rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem_bytes(kRowWindow)) !=
-      cudaSuccess) {
-    cudaGetLastError();
-    return CVO_ERR_CUDA;
-  }
+  for (RowsFn f : {a->rows, a->align_rows})
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem_bytes(kRowWindow)) != cudaSuccess) {
+      cudaGetLastError();
+      return CVO_ERR_CUDA;
+    }
   return 0;
 }
 
@@ -402,6 +464,19 @@ KParams make_kparams(const cvo_params &p) {
   return k;
 }
 
+// The lattice for search radius r and source blocks of diagonal ext: cells small against r, a
+// block's box about 8 of them along each axis.
+static float cell_for_radius(float r, float ext) { return std::max(r / 4.f, (ext + 2.f * r) / 8.f); }
+// Largest radius a cell of size hc serves (inverse of cell_for_radius).
+static float radius_for_cell(float hc, float ext) { return std::max(0.f, std::min(4.f * hc, 0.5f * (8.f * hc - ext))); }
+static float host_range_ell(float ell, float dist) { return (float)(((double)dist / 500.0 + 1.0) * (double)ell); }
+static float host_radius(const KParams &K, float ell, float norm) {
+  if (!K.use_geo) return INFINITY;
+  float l = host_range_ell(ell, norm);
+  float d2t = (float)(-2.0 * (double)l * (double)l * (double)K.log_geo);
+  return std::sqrt(std::max(d2t, 0.f));
+}
+
 long long tune_items(long long rows) { return (rows + 127) / 128; }
 
 long long tune_key(int F, int C, long long rows) {
@@ -416,7 +491,7 @@ namespace {
 struct BatchHost {
   BatchDev B;
   std::vector<PairDev> pairs;
-  std::vector<int> item_off, tgt_off, rblk_off, sblk_off;
+  std::vector<int> item_off, tgt_off, row_off, rblk_off, gblk_off, sblk_off;
   AssocKernels fn;
   int cand_blocks = 0, xform_blocks = 0;
   int window_words = 0;
@@ -468,8 +543,32 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
   const double want = (tc.blocks_per_sm > 0 ? 4.0 * tc.blocks_per_sm * sms : (double)kCandItems) *
                       (tc.cell_div_r / 4.0) * (tc.cell_div_ext / 8.0);
   const int splits = (int)std::min<double>(kMaxSplits, std::max(1.0, std::ceil(want / (double)std::max<long long>(tiles, 1))));
+  // orders of the targets (align): the lattices of every radius the lengthscale may reach
+  std::vector<std::vector<RankLevel>> lv(np);
+  std::vector<std::vector<float>> lr(np);
+  for (int p = 0; p < np && mode == MODE_ALIGN; p++) {
+    const float ext = srcs[p]->tile_ext;
+    std::vector<int> exps;
+    if (!K.use_geo) {
+      exps.push_back(1000);
+    } else {
+      const float ell_hi = ell0[p], ell_lo = std::min(K.ell_min, ell_hi);
+      const float r_hi = host_radius(K, ell_hi, srcs[p]->max_norm), r_lo = host_radius(K, ell_lo, 0.f);
+      int e_hi = level_for_radius(cell_for_radius(r_hi, ext)), e_lo = level_for_radius(cell_for_radius(r_lo, ext));
+      if (e_hi - e_lo + 1 > 24) e_lo = e_hi - 23;
+      for (int e = e_lo; e <= e_hi; e++) exps.push_back(e);
+    }
+    if (tgts[p]->n == 0) continue;
+    if ((rc = cloud_ranks(h, tgts[p], exps))) return rc;
+    for (int e : exps) {
+      lv[p].push_back(tgts[p]->ranks[e]);
+      lr[p].push_back(e >= 1000 ? INFINITY : radius_for_cell(lv[p].back().h, ext));
+    }
+  }
   // sizes
   bh->item_off.assign(np + 1, 0);
+  bh->row_off.assign(np + 1, 0);
+  bh->gblk_off.assign(np + 1, 0);
   bh->tgt_off.assign(np + 1, 0);
   bh->rblk_off.assign(np + 1, 0);
   bh->sblk_off.assign(np + 1, 0);
@@ -481,32 +580,42 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
   for (int p = 0; p < np; p++) rows_all += srcs[p]->n;
   const int most = rows_all > 0 ? (int)std::min<long long>(1 << 20, (16ll << 30) / (8ll * rows_all)) : 1;
   const int ell_ld = (std::max(capmax, 1) + 3) & ~3;   // 16-byte aligned ELL rows
+  const int order_cap = rows_all > 0 ? (int)std::min<long long>(4096, (16ll << 30) / (8ll * rows_all)) & ~3 : 0;
   const bool ell = mode != MODE_IP;                    // an inner product needs no kernel matrix
-  std::vector<int> sp(np), caps(np);
+  std::vector<int> sp(np), caps(np), pitch(np);
   for (int p = 0; p < np; p++) {
     int n = srcs[p]->n, m = tgts[p]->n;
     const int ns = group_count(group_count(m));
     sp[p] = std::max(1, std::min(splits, ns));
     caps[p] = std::max(1, std::min(kGroup * ((ns + sp[p] - 1) / sp[p]), most / sp[p]));
     if (!K.use_mma) sp[p] = caps[p] = 1;
+    // an align row's kept entries pass through its candidate entries' place (order_row)
+    pitch[p] = std::max(sp[p] * caps[p], mode == MODE_ALIGN ? std::min(capmax, m) : 0);
     bh->item_off[p + 1] = bh->item_off[p] + group_count(n) * sp[p];
     bh->tgt_off[p + 1] = bh->tgt_off[p] + m;
-    int rb = (n + kRowsPerBlock - 1) / kRowsPerBlock, sb = (n + kStepRows - 1) / kStepRows;
+    int rb = (n + kRowsPerBlock - 1) / kRowsPerBlock, sb = (n + kStepThreads - 1) / kStepThreads;
     bh->rblk_off[p + 1] = bh->rblk_off[p] + rb;
+    const int gb = (n + kReduceRows - 1) / kReduceRows;
+    bh->row_off[p + 1] = bh->row_off[p] + n;
+    bh->gblk_off[p + 1] = bh->gblk_off[p] + gb;
     bh->sblk_off[p + 1] = bh->sblk_off[p] + sb;
     add(sizeof(float4) * m);                                     // ycur
     add(sizeof(float4) * m);                                     // yorig
     add(ell ? sizeof(int) * (size_t)n * ell_ld : 0);             // ELL
     add(ell ? sizeof(float) * (size_t)n * ell_ld : 0);
-    add(sizeof(uint2) * (size_t)n * sp[p] * caps[p]);            // candidate entries
+    add(sizeof(uint2) * (size_t)n * pitch[p]);                   // candidate entries
+    if (mode == MODE_ALIGN) {
+      add(sizeof(float) * 8 * (size_t)n);                        // row_sums
+      add(sizeof(RankLevel) * lv[p].size());
+    }
     add(sizeof(int2) * (size_t)n * sp[p]);                       // entry counts
     add(sizeof(int) * n);                                        // nnz_row
     add(sizeof(double) * kPartStride * (size_t)std::max(rb, sb)); // partials
     add(sizeof(unsigned) * 2);
-    bytes += 9 * 256;                                            // room for empty pieces
+    bytes += 12 * 256;                                           // room for empty pieces
   }
   add(sizeof(PairDev) * np);
-  add(sizeof(int) * (np + 1) * 4);
+  add(sizeof(int) * (np + 1) * 6);
   add(sizeof(int) * 4);
   add(sizeof(double));
   if ((rc = ensure_workspace(h, bytes))) return rc;
@@ -530,7 +639,7 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     P.ld = ell_ld;
     P.splits = sp[p];
     P.cap_split = caps[p];
-    P.cand_pitch = sp[p] * caps[p];
+    P.cand_pitch = pitch[p];
     P.cand = ar.take<uint2>((size_t)s->n * P.cand_pitch);
     P.cand_cnt = ar.take<int2>((size_t)s->n * sp[p]);
     P.tf = t->feat; P.tl = t->lab; P.tg = t->geo;
@@ -553,18 +662,32 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     }
     P.ell = ell0[p];
     P.cap = capmax;
+    P.order_cap = order_cap;
+    P.src_norm = s->max_norm;
+    if (mode == MODE_ALIGN) {
+      P.row_sums = ar.take<float>(8 * (size_t)s->n);
+      RankLevel *levels = ar.take<RankLevel>(lv[p].size());
+      CVO_CUDA_TRY(h, cudaMemcpyAsync(levels, lv[p].data(), sizeof(RankLevel) * lv[p].size(), cudaMemcpyHostToDevice, h->stream));
+      P.levels = levels;
+      P.nlevels = (int)lv[p].size();
+      for (int i = 0; i < P.nlevels && i < 24; i++) P.level_r[i] = lr[p][i];
+      const float r0 = host_radius(K, P.ell, s->max_norm);
+      P.level = P.nlevels - 1;
+      for (int i = 0; i < P.nlevels; i++)
+        if (P.level_r[i] >= r0) { P.level = i; break; }
+    }
     P.done = (s->n == 0 || t->n == 0) ? 1 : 0;
     if (!P.done) active++;
   }
   PairDev *pairs_d = ar.take<PairDev>(np);
-  int *offs_d = ar.take<int>((size_t)(np + 1) * 4);
+  int *offs_d = ar.take<int>((size_t)(np + 1) * 6);
   int *ctr_d = ar.take<int>(4);
   double *bytes_d = ar.take<double>(1);
   // zero counters of every pair
   for (int p = 0; p < np; p++) CVO_CUDA_TRY(h, cudaMemsetAsync(bh->pairs[p].counter, 0, 2 * sizeof(unsigned), h->stream));
   CVO_CUDA_TRY(h, cudaMemcpyAsync(pairs_d, bh->pairs.data(), sizeof(PairDev) * np, cudaMemcpyHostToDevice, h->stream));
   std::vector<int> offs;
-  for (auto *v : {&bh->item_off, &bh->tgt_off, &bh->rblk_off, &bh->sblk_off}) offs.insert(offs.end(), v->begin(), v->end());
+  for (auto *v : {&bh->item_off, &bh->tgt_off, &bh->rblk_off, &bh->sblk_off, &bh->row_off, &bh->gblk_off}) offs.insert(offs.end(), v->begin(), v->end());
   CVO_CUDA_TRY(h, cudaMemcpyAsync(offs_d, offs.data(), sizeof(int) * offs.size(), cudaMemcpyHostToDevice, h->stream));
   int ctr_h[4] = {0, 0, active, 0};
   CVO_CUDA_TRY(h, cudaMemcpyAsync(ctr_d, ctr_h, sizeof(ctr_h), cudaMemcpyHostToDevice, h->stream));
@@ -581,6 +704,9 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
   B.tgt_off = offs_d + (np + 1);
   B.rblk_off = offs_d + 2 * (np + 1);
   B.sblk_off = offs_d + 3 * (np + 1);
+  B.row_off = offs_d + 4 * (np + 1);
+  B.gblk_off = offs_d + 5 * (np + 1);
+  B.total_gblocks = bh->gblk_off[np];
   B.total_rblocks = bh->rblk_off[np];
   B.total_sblocks = bh->sblk_off[np];
   B.err = ctr_d + 1;
@@ -604,10 +730,10 @@ inline void mark(Handle *h, const cudaEvent_t *ev, int k) {
   if (ev) cudaEventRecordWithFlags(ev[k], h->stream, cudaEventRecordExternal);
 }
 
-// ev (optional): 7 events: 0-4 bracket transform, association phase, (empty) reduce and
-// step; 5 and 6 split the association phase into the candidate test, the row pass and
-// nothing (the row pass sums the gradient).
-void launch_association(Handle *h, BatchHost *bh, const KParams &K, const cudaEvent_t *ev = nullptr) {
+// ev (optional): 7 events: 0-4 bracket transform, association phase, reduce and step; 5 and 6
+// split the association phase into the candidate test, the row pass and the row sums (align
+// only: single passes sum in the row pass).
+void launch_association(Handle *h, BatchHost *bh, const KParams &K, bool align = false, const cudaEvent_t *ev = nullptr) {
   BatchDev &B = bh->B;
   mark(h, ev, 0);
   k_transform<<<std::max(bh->xform_blocks, 1), 256, 0, h->stream>>>(B);
@@ -617,15 +743,21 @@ void launch_association(Handle *h, BatchHost *bh, const KParams &K, const cudaEv
     h->launches++;
   }
   mark(h, ev, 5);
-  bh->fn.rows<<<std::max(B.total_rblocks, 1), 32 * kRowWarps, bh->row_smem, h->stream>>>(B, K, bh->window_words);
-  mark(h, ev, 6);
-  mark(h, ev, 2);
-  mark(h, ev, 3);
+  const RowsFn rows = align ? bh->fn.align_rows : bh->fn.rows;
+  rows<<<std::max(B.total_rblocks, 1), 32 * kRowWarps, bh->row_smem, h->stream>>>(B, K, bh->window_words);
   h->launches += 2;
+  mark(h, ev, 6);
+  if (align) {
+    k_rowsum<<<std::max((B.total_rows + 127) / 128, 1), 128, 0, h->stream>>>(B, K);
+    mark(h, ev, 2);
+    k_reduce<<<std::max(B.total_gblocks, 1), kReduceThreads, 0, h->stream>>>(B, K);
+    h->launches += 2;
+  }
+  mark(h, ev, 3);
 }
 
 void launch_iteration(Handle *h, BatchHost *bh, const KParams &K, const cudaEvent_t *ev = nullptr) {
-  launch_association(h, bh, K, ev);
+  launch_association(h, bh, K, true, ev);
   k_step<<<std::max(bh->B.total_sblocks, 1), kStepThreads, 0, h->stream>>>(bh->B, K);
   mark(h, ev, 4);
   h->launches += 1;

@@ -13,6 +13,18 @@
 
 namespace cvo_gb {
 
+float level_cell_size(int e) { return exp2f(0.5f * (float)e); }
+
+// Smallest quantised cell size h = 2^(e/2) with h >= r.
+int level_for_radius(float r) {
+  if (!(r > 0.f)) return -60;
+  if (!std::isfinite(r)) return 1000;
+  int e = (int)std::ceil(2.0 * std::log2((double)r));
+  while (level_cell_size(e) < r) e++;
+  while (e > -60 && level_cell_size(e - 1) >= r) e--;
+  return e;
+}
+
 namespace {
 
 __global__ void k_pack_positions(const float *xyz, int stride, int n, float4 *pos) {
@@ -88,6 +100,72 @@ __global__ void __launch_bounds__(128) k_boxes(const float4 *pos, const float4 *
   }
 }
 
+// Bounding-box diagonals of 128 consecutive tile-order points (four groups).
+__global__ void k_tile_extent(const float4 *box, int groups, int tiles, float *ext) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= tiles) return;
+  float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+  for (int g = 4 * t; g < min(4 * t + 4, groups); g++) {
+    const float4 a = box[g], b = box[groups + g];
+    lo[0] = fminf(lo[0], a.x); lo[1] = fminf(lo[1], a.y); lo[2] = fminf(lo[2], a.z);
+    hi[0] = fmaxf(hi[0], b.x); hi[1] = fmaxf(hi[1], b.y); hi[2] = fmaxf(hi[2], b.z);
+  }
+  const float dx = hi[0] - lo[0], dy = hi[1] - lo[1], dz = hi[2] - lo[2];
+  ext[t] = sqrtf(dx * dx + dy * dy + dz * dz);
+}
+
+// A lattice of rank level q of a joint build: cell c of axis k covers [o + c h, o + (c + 1) h).
+struct Lattice {
+  float ox, oy, oz, inv_h;
+  int dimx, dimy, dimz;
+};
+constexpr int kMaxLattices = 24;
+struct Lattices {
+  Lattice l[kMaxLattices];
+};
+
+__device__ __forceinline__ unsigned long long lattice_cell(const Lattice &L, const float4 &p) {
+  const int cx = min(max((int)floorf((p.x - L.ox) * L.inv_h), 0), L.dimx - 1);
+  const int cy = min(max((int)floorf((p.y - L.oy) * L.inv_h), 0), L.dimy - 1);
+  const int cz = min(max((int)floorf((p.z - L.oz) * L.inv_h), 0), L.dimz - 1);
+  return ((unsigned long long)cz * L.dimy + cy) * L.dimx + cx;
+}
+
+// Sort keys of `count` lattices at once: the lattice's number above `bits` bits of the cell.
+// hi (single lattice of more than 32 bits): the upper half of the cell number.
+__global__ void k_rank_keys(const float4 *pos, int n, Lattices L, int count, int bits, unsigned int *key, unsigned int *hi,
+                            int *val) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n * count) return;
+  const int q = t / n, j = t - q * n;
+  const unsigned long long c = lattice_cell(L.l[q], pos[j]);
+  key[t] = hi ? (unsigned int)c : ((unsigned int)q << bits) | (unsigned int)c;
+  if (hi) hi[t] = (unsigned int)(c >> 32);
+  val[t] = j;
+}
+
+__global__ void k_rank_upper(const unsigned int *hi, const int *val, int n, unsigned int *key) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t < n) key[t] = hi[val[t]];
+}
+
+// Sorted indices of `count` lattices -> the arrays of each (3 n ints: index, of_index, of_tile).
+__global__ void k_rank_arrays(const int *val, int n, int count, int *out) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n * count) return;
+  const int q = t / n, r = t - q * n, j = val[t];
+  int *o = out + 3 * (size_t)q * n;
+  o[r] = j;
+  o[n + j] = r;
+}
+__global__ void k_rank_tiles(const int *sperm, int n, int count, int *out) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n * count) return;
+  const int q = t / n, s = t - q * n;
+  int *o = out + 3 * (size_t)q * n;
+  o[2 * (size_t)n + s] = o[n + sperm[s]];
+}
+
 template <typename T>
 int dalloc(Handle *h, T **p, size_t count) {
   if (count == 0) count = 1;
@@ -152,8 +230,16 @@ static int cloud_build(Handle *h, DevCloud *d, const float *xyz_d, int stride, c
   k_boxes<0><<<(ng + 3) / 4, 128, 0, h->stream>>>(d->spos, reinterpret_cast<const float4 *>(d->sfeat), d->FP / 4, n, ch,
                                                   d->gbox, ng);
   k_boxes<1><<<(ns + 3) / 4, 128, 0, h->stream>>>(d->gbox, nullptr, 0, ng, ch, d->sbox, ns);
-  h->launches += 2;
+  const int tiles = (n + 127) / 128;
+  float *ext_d = reinterpret_cast<float *>(keys);
+  k_tile_extent<<<(tiles + 127) / 128, 128, 0, h->stream>>>(d->gbox, ng, tiles, ext_d);
+  h->launches += 3;
+  std::vector<float> ext_h(tiles);
+  CVO_CUDA_TRY(h, cudaMemcpyAsync(ext_h.data(), ext_d, sizeof(float) * tiles, cudaMemcpyDeviceToHost, h->stream));
   CVO_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+  double es = 0.0;
+  for (float e : ext_h) es += e;
+  d->tile_ext = tiles > 0 ? (float)(es / tiles) : 0.f;
   cudaFree(keys); cudaFree(keys_tmp); cudaFree(perm_vals); cudaFree(perm_tmp);
   return 0;
 }
@@ -285,7 +371,83 @@ void cloud_free(DevCloud *d) {
   cudaFree(d->pos); cudaFree(d->feat); cudaFree(d->lab); cudaFree(d->geo);
   cudaFree(d->sperm); cudaFree(d->spos); cudaFree(d->sfeat); cudaFree(d->slab); cudaFree(d->sgeo);
   cudaFree(d->gbox); cudaFree(d->sbox);
+  for (void *p : d->rank_allocs) cudaFree(p);
   delete d;
+}
+
+// Lattices whose cell numbers fit are sorted together (one radix sort over all of them, the
+// lattice's number in the top bits): an align wants the orders of every lengthscale it may
+// reach, and a sort of some 10^4 keys is launches, not work.
+int cloud_ranks(Handle *h, DevCloud *d, const std::vector<int> &exps) {
+  const int n = d->n;
+  if (n == 0) return 0;
+  struct Want { int e, bits; Lattice l; float h; };
+  std::vector<Want> joint, single;
+  for (int e : exps) {
+    if (d->ranks.count(e)) continue;
+    Want w;
+    w.e = e;
+    float ext[3];
+    for (int k = 0; k < 3; k++) ext[k] = d->bbmax[k] - d->bbmin[k];
+    float hsz = (e >= 1000) ? INFINITY : level_cell_size(e);
+    // keep at most 2^20 cells per axis
+    float emax = std::max(std::max(ext[0], ext[1]), ext[2]);
+    if (std::isfinite(hsz) && emax / hsz > 1048000.f) hsz = emax / 1048000.f;
+    w.h = hsz;
+    w.l.inv_h = std::isfinite(hsz) ? 1.f / hsz : 0.f;
+    w.l.ox = d->bbmin[0]; w.l.oy = d->bbmin[1]; w.l.oz = d->bbmin[2];
+    w.l.dimx = std::isfinite(hsz) ? (int)std::floor(ext[0] * w.l.inv_h) + 1 : 1;
+    w.l.dimy = std::isfinite(hsz) ? (int)std::floor(ext[1] * w.l.inv_h) + 1 : 1;
+    w.l.dimz = std::isfinite(hsz) ? (int)std::floor(ext[2] * w.l.inv_h) + 1 : 1;
+    const double cells = (double)w.l.dimx * w.l.dimy * w.l.dimz;
+    w.bits = 1;
+    while (w.bits < 63 && std::ldexp(1.0, w.bits) < cells) w.bits++;
+    (w.bits <= 27 ? joint : single).push_back(w);
+  }
+  auto build = [&](const Want *w, int count) -> int {
+    int bits = 1, lattice_bits = 0;
+    for (int q = 0; q < count; q++) bits = std::max(bits, w[q].bits);
+    while ((1 << lattice_bits) < count) lattice_bits++;
+    const bool wide = bits + lattice_bits > 32;
+    const size_t N = (size_t)n * count;
+    unsigned int *key = nullptr;
+    int *arrays = nullptr;
+    CVO_CUDA_TRY(h, cudaMalloc((void **)&arrays, sizeof(int) * 3 * N));
+    d->rank_allocs.push_back(arrays);
+    CVO_CUDA_TRY(h, cudaMallocAsync((void **)&key, sizeof(int) * 5 * N, h->stream));
+    unsigned int *key_tmp = key + N, *hi = key_tmp + N;
+    int *val = reinterpret_cast<int *>(hi + N), *val_tmp = val + N;
+    Lattices L;
+    memset(&L, 0, sizeof(L));
+    for (int q = 0; q < count; q++) L.l[q] = w[q].l;
+    const unsigned blocks = (unsigned)((N + 255) / 256);
+    k_rank_keys<<<blocks, 256, 0, h->stream>>>(d->pos, n, L, count, bits, key, wide ? hi : nullptr, val);
+    int rc = radix_sort_pairs(h, key, val, key_tmp, val_tmp, (int)N, wide ? 32 : bits + lattice_bits);
+    if (!rc && wide) {
+      k_rank_upper<<<blocks, 256, 0, h->stream>>>(hi, val, n, key);
+      h->launches++;
+      rc = radix_sort_pairs(h, key, val, key_tmp, val_tmp, n, bits - 32);
+    }
+    if (!rc) {
+      k_rank_arrays<<<blocks, 256, 0, h->stream>>>(val, n, count, arrays);
+      k_rank_tiles<<<blocks, 256, 0, h->stream>>>(d->sperm, n, count, arrays);
+    }
+    h->launches += 3;
+    CVO_CUDA_TRY(h, cudaFreeAsync(key, h->stream));
+    if (rc) return rc;
+    for (int q = 0; q < count; q++) {
+      int *a = arrays + 3 * (size_t)q * n;
+      d->ranks[w[q].e] = RankLevel{w[q].h, a, a + n, a + 2 * (size_t)n};
+    }
+    return 0;
+  };
+  // at most 2^25 keys in one sort
+  const int most = std::max(1, std::min({kMaxLattices, 16, (1 << 25) / n}));
+  for (size_t q = 0; q < joint.size(); q += most)
+    if (int rc = build(&joint[q], (int)std::min<size_t>(most, joint.size() - q))) return rc;
+  for (const Want &w : single)
+    if (int rc = build(&w, 1)) return rc;
+  return 0;
 }
 
 }  // namespace cvo_gb

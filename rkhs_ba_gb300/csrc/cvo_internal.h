@@ -30,11 +30,22 @@ inline int group_count(int n) { return (n + kGroup - 1) / kGroup; }
 // Feature chunks (float4) of a bounding box: the association takes at most two.
 inline int box_chunks(int FP) { return FP / 4 < 2 ? FP / 4 : 2; }
 
+// An order of a target cloud's points: by the cells of a lattice over the bounding box (z, then
+// y, then x), inside a cell by index.  The align loop keeps the entries of a kernel-matrix
+// row in this order and adds them up in it, with the lattice that follows the search radius.
+struct RankLevel {
+  float h;                // cell size
+  int *index;             // rank -> original index
+  int *of_index;          // original index -> rank
+  int *of_tile;           // tile-order position -> rank
+};
+
 struct DevCloud {
   int n = 0, F = 0, C = 0, FP = 0, CP = 0;
   bool has_geo = false;
   float bbmin[3] = {0, 0, 0}, bbmax[3] = {0, 0, 0};
   float max_norm = 0.f;
+  float tile_ext = 0.f;          // mean bounding-box diagonal of 128 consecutive tile-order points
   // original order
   float4 *pos = nullptr;
   float *feat = nullptr;
@@ -49,6 +60,8 @@ struct DevCloud {
   // bounding boxes of the groups, then of the supergroups: float4 planes (position low,
   // high, feature low, feature high; box_planes of them) of one entry per group
   float4 *gbox = nullptr, *sbox = nullptr;
+  std::map<int, RankLevel> ranks;          // by quantised cell size 2^(e/2), device arrays
+  std::vector<void *> rank_allocs;
 };
 
 // ----------------------------------------------------------- kernel params
@@ -101,6 +114,13 @@ struct PairDev {
   const float *tf, *tl;           // target features / labels, original order (float4 chunks)
   const float2 *tg;               // target geometric types, original order
   int *nnz_row;                   // n
+  float *row_sums;                // align: n * 8, omega(3)/c, v(3)/d
+  // align: orders of the target's points, finest lattice first, and the largest search radius
+  // each serves; a row that kept more than cap + order_cap pairs stays in index order
+  const RankLevel *levels;
+  float level_r[24];
+  int nlevels, level, order_cap;
+  float src_norm;                 // largest |x| of the source
   double *part;                   // block partials
   unsigned int *counter;          // last-block counters [2]
   int F, C;                       // feature / label dimensions (source and target agree)
@@ -136,9 +156,11 @@ struct BatchDev {
   const int *item_off;            // npairs + 1 (prefix of work items)
   const int *tgt_off;             // npairs + 1 (prefix of m)
   int *err;                       // error word (0 ok)
+  const int *row_off;             // npairs + 1 (prefix of n)
   const int *rblk_off;            // row-pass blocks per pair (prefix)
+  const int *gblk_off;            // k_reduce blocks per pair (prefix)
   const int *sblk_off;            // step blocks per pair (prefix)
-  int total_rblocks, total_sblocks;
+  int total_rblocks, total_gblocks, total_sblocks;
   int *active;                    // number of pairs not done
   int *active_iters;              // iterations that started with an active pair
   double *assoc_bytes;            // algorithmic bytes of the association passes
@@ -208,6 +230,10 @@ int cloud_upload(Handle *h, const cvo_cloud *c, DevCloud **out);
 int cloud_from_device(Handle *h, int n, int F, int C, const float *xyz_d, const float *feat_d, const float *lab_d,
                       const float2 *geo_d, DevCloud **out);
 void cloud_free(DevCloud *c);
+float level_cell_size(int level_exp);
+int level_for_radius(float r);
+// Orders of the cloud by the lattices of the given exponents (built once per cloud).
+int cloud_ranks(Handle *h, DevCloud *c, const std::vector<int> &exps);
 
 // radix sort / scan (cvo_sort.cu)
 int radix_sort_pairs(Handle *h, unsigned int *keys, int *vals, unsigned int *keys_tmp, int *vals_tmp,

@@ -7,8 +7,9 @@
 //                position and colour, then a tensor-core test of the 32 x 32 pairs of
 //                the groups that remain; one bit per pair that may be kept
 //   k_rows       each row's candidates in ascending target index: exact kernel value,
-//                threshold, the first cap kept ones to the ELL row, gradient sums
-//                                            (CvoGPU.cu:951-1099, 2001-2120)
+//                threshold, the first cap kept ones to the ELL row    (CvoGPU.cu:951-1099)
+//   k_rowsum, k_reduce   gradient sums of the rows and of the pair (CvoGPU.cu:2001-2120);
+//                single passes sum in k_rows instead
 //   k_step       Taylor step-size terms over the ELL rows; the last block of each pair
 //                runs the scalar tail of the iteration: cubic roots, step clamp,
 //                Exp_SEK3 pose update, SE(3) distance, lengthscale schedule, cap update
@@ -21,8 +22,8 @@ namespace cvo_gb {
 
 enum { MODE_ALIGN = 0, MODE_IP = 1, MODE_EXPORT = 2 };
 constexpr int kStepThreads = 256;
-constexpr int kStepRows = 16;           // rows of a block of k_step
-constexpr int kStepLanes = 16;          // lanes sharing one of them
+constexpr int kReduceRows = 1024;
+constexpr int kReduceThreads = 256;
 constexpr int kPartStride = 12;
 
 // ------------------------------------------------------------ pair value
@@ -446,31 +447,6 @@ __global__ void __launch_bounds__(32 * kCandWarps) k_cand(BatchDev B, KParams K)
 }
 
 // --------------------------------------------------------------- row pass
-// Sum of each of 8 values over the warp: lane l returns value l >> 2 (three folding
-// steps halve the values a lane carries, two more finish the sum).
-__device__ __forceinline__ float warp_sum8(const float (&v)[8], int lane) {
-  float a[4], b[2], c;
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const bool up = lane & 16;
-    const float keep = up ? v[k + 4] : v[k], give = up ? v[k] : v[k + 4];
-    a[k] = keep + __shfl_xor_sync(FULLMASK, give, 16);
-  }
-#pragma unroll
-  for (int k = 0; k < 2; k++) {
-    const bool up = lane & 8;
-    const float keep = up ? a[k + 2] : a[k], give = up ? a[k] : a[k + 2];
-    b[k] = keep + __shfl_xor_sync(FULLMASK, give, 8);
-  }
-  {
-    const bool up = lane & 4;
-    const float keep = up ? b[1] : b[0], give = up ? b[0] : b[1];
-    c = keep + __shfl_xor_sync(FULLMASK, give, 4);
-  }
-  c += __shfl_xor_sync(FULLMASK, c, 2);
-  return c + __shfl_xor_sync(FULLMASK, c, 1);
-}
-
 __device__ __forceinline__ int warp_excl_scan(int v, int lane, int &total) {
   int incl = v;
 #pragma unroll
@@ -489,9 +465,16 @@ __device__ __forceinline__ int warp_excl_scan(int v, int lane, int &total) {
 // flight.  The reference scans the targets by index and stops at cap kept pairs
 // (src/cvo/CvoGPU.cu:994-996): here the row stops there too, so no pair beyond cap is
 // evaluated or stored.  A row whose entries did not fit, or a call without a candidate
-// test, scans all targets in index order instead.  Gradient partials: FP32 per lane and
-// row, summed over the lanes, FP64 from there (CvoGPU.cu:2001-2062); the last block of a
-// pair adds the blocks' sums in a fixed order and normalises the gradient.
+// test, scans all targets in index order instead.
+// ROWS_SUM (single passes): FP32 sums per lane and row, over the lanes, FP64 from there; the
+// last block of a pair adds the blocks' sums in a fixed order.
+// ROWS_ALIGN: the entries of a row go to the order of the pair's level (RankLevel), in which
+// k_rowsum and k_step add them one by one.  The align loop turns a different last bit of the
+// gradient into a visibly different pose some tens of iterations later, so the order is part
+// of the result and is kept whatever finds the pairs.  A row with no more than cap candidates
+// is sorted and evaluated by rank from the start; a longer one is cut by index first and its
+// kept entries are then put in order.  One that kept more than cap + order_cap pairs stays in
+// index order.
 // Bounds: latency of the dependent steps entry -> permutation -> bitmap -> record, hidden
 // by 16-28 resident warps per SM (the bitmap's shared memory sets the number).  The rows'
 // FP64 constants are computed 32 rows at a time: once per warp and row they took most of
@@ -503,18 +486,60 @@ constexpr int kRowWindow = 65536;       // most target indices of one bitmap win
 constexpr int kRowQueue = 512;          // sorted candidates of one round
 constexpr int kRowSorted = 128;         // most candidates a sorting network puts in order
 
+// Whether a kernel instance serves single passes (and sums there) or the align loop.
+enum { ROWS_SUM = 0, ROWS_ALIGN = 1 };
+
 // Words of one warp's bitmap for targets of up to m points: an odd number per lane, so
 // that the lanes' runs start in different banks.
 __host__ __device__ inline int row_window_words(int m) {
   return 32 * ((((m < kRowWindow ? m : kRowWindow) + 1023) / 1024) | 1);
 }
+// Ints of its queue; also a 16-bit count before each word of the bitmap.
+__host__ __device__ inline int row_queue_ints(int window_words) {
+  return window_words / 2 > kRowQueue ? window_words / 2 : kRowQueue;
+}
 __host__ __device__ inline size_t row_smem_bytes(int m) {
-  return (size_t)kRowWarps * sizeof(uint32_t) * (row_window_words(m) + kRowQueue);
+  return (size_t)kRowWarps * sizeof(uint32_t) * (row_window_words(m) + row_queue_ints(row_window_words(m)));
 }
 
-// 1 / (2 l^2) of the step-size terms (compute_step_size_xi), in double, rounded once.
-__device__ __forceinline__ float step_coef(float l) {
-  return __double2float_rn(__ddiv_rn(1.0, dm(dm(2.0, (double)l), (double)l)));
+// Puts the z entries of an ELL row, which are in index order, in the order of the ranks:
+// their bits in a bitmap over the ranks, a count before every word, and each entry's slot is
+// the number of bits below its own.  tmp: z entries.  All lanes call it.
+__device__ __forceinline__ void order_row(int *Aj, float *Av, int z, const int *rank, int m, uint32_t *bits, int window_words,
+                                          unsigned short *before, uint2 *tmp, int lane) {
+  const int wl = window_words >> 5;
+  int base = 0;
+  for (int w0 = 0; w0 < m && base < z; w0 += 32 * window_words) {
+    __syncwarp();
+    for (int i = lane; i < window_words / 4; i += 32) reinterpret_cast<uint4 *>(bits)[i] = make_uint4(0u, 0u, 0u, 0u);
+    __syncwarp();
+    for (int c = lane; c < z; c += 32) {
+      const uint32_t k = (uint32_t)(__ldg(&rank[Aj[c]]) - w0);
+      if (k < 32u * (uint32_t)window_words) atomicOr(&bits[k >> 5], 1u << (k & 31));
+    }
+    __syncwarp();
+    int run = 0, total;
+    for (int i = 0; i < wl; i++) run += __popc(bits[lane * wl + i]);
+    run = warp_excl_scan(run, lane, total);
+    for (int i = 0; i < wl; i++) {
+      before[lane * wl + i] = (unsigned short)run;      // within the window: below 65536
+      run += __popc(bits[lane * wl + i]);
+    }
+    __syncwarp();
+    for (int c = lane; c < z; c += 32) {
+      const int j = Aj[c];
+      const uint32_t k = (uint32_t)(__ldg(&rank[j]) - w0);
+      if (k < 32u * (uint32_t)window_words)
+        tmp[base + before[k >> 5] + __popc(bits[k >> 5] & ((1u << (k & 31)) - 1u))] = make_uint2((uint32_t)j, __float_as_uint(Av[c]));
+    }
+    base += total;
+  }
+  __syncwarp();
+  for (int c = lane; c < z; c += 32) {
+    const uint2 v = tmp[c];
+    Aj[c] = (int)v.x;
+    Av[c] = __uint_as_float(v.y);
+  }
 }
 
 // Sorts queue[0 .. count), count <= 32 R, in ascending order: a bitonic network over element
@@ -550,21 +575,30 @@ __device__ __forceinline__ void warp_sort(int *queue, int count, int lane) {
   for (int r = 0; r < R; r++) queue[32 * r + lane] = v[r];
 }
 
-// Block sums -> part; the last block of the pair finishes the pass.
-__device__ __forceinline__ void rows_finish(const BatchDev &B, const KParams &K, PairDev *P, int b, int nb, double lane_sum,
-                                            long long nnz, int mx) {
-  __shared__ double sh[kRowWarps][9];
+// Totals of an association pass.  Algorithmic bytes: every source and target record once, the
+// per-row count, and the ELL entries when they are written.
+__device__ __forceinline__ void pass_finished(const BatchDev &B, PairDev *P, double asum, double nnz, double mx) {
+  atomicAdd(B.assoc_bytes, (double)(P->n + P->m) * B.record_bytes + 4.0 * P->n + (P->mode != MODE_IP ? 8.0 * nnz : 0.0));
+  P->asum = asum;
+  P->nnz_sum = (long long)nnz;
+  P->max_row = (int)mx;
+}
+
+// Sums of a single pass (value, kept pairs, longest row) -> part; the last block of the pair
+// finishes the pass.
+__device__ __forceinline__ void rows_finish(const BatchDev &B, PairDev *P, int b, int nb, double sum, long long nnz, int mx) {
+  __shared__ double sh[kRowWarps][3];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if ((lane & 3) == 0 && lane < 28) sh[w][lane >> 2] = lane_sum;
   if (lane == 0) {
-    sh[w][7] = (double)nnz;
-    sh[w][8] = (double)mx;
+    sh[w][0] = sum;
+    sh[w][1] = (double)nnz;
+    sh[w][2] = (double)mx;
   }
   __syncthreads();
-  if (threadIdx.x < 9) {
+  if (threadIdx.x < 3) {
     double t = sh[0][threadIdx.x];
-    for (int q = 1; q < kRowWarps; q++) t = threadIdx.x < 8 ? t + sh[q][threadIdx.x] : fmax(t, sh[q][threadIdx.x]);
+    for (int q = 1; q < kRowWarps; q++) t = threadIdx.x < 2 ? t + sh[q][threadIdx.x] : fmax(t, sh[q][threadIdx.x]);
     P->part[(size_t)b * kPartStride + threadIdx.x] = t;
     __threadfence();
   }
@@ -573,51 +607,30 @@ __device__ __forceinline__ void rows_finish(const BatchDev &B, const KParams &K,
   __syncthreads();
   if (!last) return;
   __threadfence();
-  double t[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  double t[3] = {0, 0, 0};
   for (int q = threadIdx.x; q < nb; q += 32 * kRowWarps) {
     const double *pv = P->part + (size_t)q * kPartStride;
-#pragma unroll
-    for (int k = 0; k < 8; k++) t[k] += __ldcg(pv + k);
-    t[8] = fmax(t[8], __ldcg(pv + 8));
+    t[0] += __ldcg(pv);
+    t[1] += __ldcg(pv + 1);
+    t[2] = fmax(t[2], __ldcg(pv + 2));
   }
+  t[0] = warp_sum(t[0]);
+  t[1] = warp_sum(t[1]);
 #pragma unroll
-  for (int k = 0; k < 8; k++) t[k] = warp_sum(t[k]);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) t[8] = fmax(t[8], __shfl_xor_sync(FULLMASK, t[8], o));
+  for (int o = 16; o > 0; o >>= 1) t[2] = fmax(t[2], __shfl_xor_sync(FULLMASK, t[2], o));
   if (lane == 0)
-    for (int k = 0; k < 9; k++) sh[w][k] = t[k];
+    for (int k = 0; k < 3; k++) sh[w][k] = t[k];
   __syncthreads();
   if (threadIdx.x != 0) return;
-  double tot[9];
-  for (int k = 0; k < 9; k++) {
-    tot[k] = sh[0][k];
-    for (int q = 1; q < kRowWarps; q++) tot[k] = k < 8 ? tot[k] + sh[q][k] : fmax(tot[k], sh[q][k]);
+  for (int k = 0; k < 3; k++) {
+    t[k] = sh[0][k];
+    for (int q = 1; q < kRowWarps; q++) t[k] = k < 2 ? t[k] + sh[q][k] : fmax(t[k], sh[q][k]);
   }
   P->counter[0] = 0;
-  // algorithmic bytes of this pair's association pass: every source and target
-  // record once, the per-row count, and the ELL entries when they are written
-  atomicAdd(B.assoc_bytes, (double)(P->n + P->m) * B.record_bytes + 4.0 * P->n +
-                               (P->mode != MODE_IP ? 8.0 * tot[7] : 0.0));
-  for (int k = 0; k < 6; k++) P->grad[k] = P->mode == MODE_ALIGN ? tot[k] : 0.0;
-  P->asum = tot[6];
-  P->nnz_sum = (long long)tot[7];
-  P->max_row = (int)tot[8];
-  if (P->mode == MODE_ALIGN) {
-    // float normalisation of the stacked gradient (CvoGPU.cu:2096-2104)
-    float f[6];
-    for (int k = 0; k < 6; k++) f[k] = (float)tot[k];
-    float s = 0.f;
-    for (int k = 0; k < 6; k++) s = fa(s, fm(f[k], f[k]));
-    if (s > 0.f) {
-      float nr = __fsqrt_rn(s);
-      for (int k = 0; k < 6; k++) f[k] = __fdiv_rn(f[k], nr);
-    }
-    for (int k = 0; k < 6; k++) P->xi[k] = f[k];
-    P->step_coef = step_coef(P->ell);   // FP64 division: once here, not per row
-  }
+  pass_finished(B, P, t[0], t[1], t[2]);
 }
 
-template <int FCH, int LCH, bool GT>
+template <int FCH, int LCH, bool GT, int KIND>
 __global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams K, int window_words) {
   extern __shared__ __align__(16) uint32_t row_smem[];
   __shared__ float4 sh_rc[kRowsPerBlock];                  // l, d2 threshold, 1 / (2 l^2)
@@ -627,7 +640,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams 
   __shared__ int sh_keepj[kRowWarps][64];
   constexpr int FP = FCH > 0 ? FCH : 1;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  uint32_t *bits = row_smem + (size_t)w * (window_words + kRowQueue);
+  uint32_t *bits = row_smem + (size_t)w * (window_words + row_queue_ints(window_words));
   int *queue = reinterpret_cast<int *>(bits + window_words);
   const int blk = blockIdx.x;
   if (blk >= B.total_rblocks) return;
@@ -665,7 +678,9 @@ __global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams 
     }
     __syncthreads();
   }
-  double lane_sum = 0.0;
+  const int order_cap = KIND == ROWS_ALIGN ? P->order_cap : 0;
+  const RankLevel *lv = KIND == ROWS_ALIGN ? P->levels + P->level : nullptr;
+  double row_total = 0.0;
   long long nnz = 0;
   int mx = 0;
   for (int r = w; r < kRowsPerBlock; r += kRowWarps) {
@@ -691,27 +706,26 @@ __global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams 
       }
       return at ? __ldg(at) : make_uint2(0u, 0u);
     };
+    // by rank from the start if the row cannot be cut; otherwise by index, and on past cap only
+    // to tell whether the row keeps more than cap + order_cap
+    const bool ranked = KIND == ROWS_ALIGN && entries > 0 && cands <= cap;
+    const int *perm = ranked ? lv->of_tile : tperm;
+    const int stop = KIND == ROWS_ALIGN && (entries < 0 || cands > cap + order_cap) ? cap + order_cap + 1 : cap;
     int kept = 0;
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    // 32 kept pairs to the ELL row and the gradient: lane l takes slots l, l + 32, ..., so
-    // the sums depend on the kept pairs alone, not on the candidates beside them
+    float acc = 0.f;
+    // 32 kept pairs to the ELL row and the sum: lane l takes slots l, l + 32, ..., so the
+    // sum depends on the kept pairs alone, not on the candidates beside them
     int flushed = 0;
     float4 *keep = sh_keep[w];
     int *keepj = sh_keepj[w];
     auto flush = [&](bool on) {
       const float4 v = keep[(flushed + lane) & 63];
       if (on) {
-        if (mode != MODE_IP) {
+        if (KIND == ROWS_ALIGN || mode != MODE_IP) {
           P->A_j[(size_t)s * P->ld + flushed + lane] = keepj[(flushed + lane) & 63];
           P->A_v[(size_t)s * P->ld + flushed + lane] = v.w;
         }
-        acc[0] = fmaf(v.w, fs(fm(x.y, v.z), fm(x.z, v.y)), acc[0]);
-        acc[1] = fmaf(v.w, fs(fm(x.z, v.x), fm(x.x, v.z)), acc[1]);
-        acc[2] = fmaf(v.w, fs(fm(x.x, v.y), fm(x.y, v.x)), acc[2]);
-        acc[3] = fmaf(v.w, v.x - x.x, acc[3]);
-        acc[4] = fmaf(v.w, v.y - x.y, acc[4]);
-        acc[5] = fmaf(v.w, v.z - x.z, acc[5]);
-        acc[6] += v.w;
+        acc += v.w;
       }
       flushed += 32;
       __syncwarp();
@@ -729,7 +743,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams 
           const uint2 v = entry(e0 + lane);
           int o, add;
           o = count + warp_excl_scan(__popc(v.y), lane, add);
-          for (uint32_t mk = v.y; mk; mk &= mk - 1) queue[o++] = __ldg(&tperm[32 * (int)v.x + __ffs(mk) - 1]);
+          for (uint32_t mk = v.y; mk; mk &= mk - 1) queue[o++] = __ldg(&perm[32 * (int)v.x + __ffs(mk) - 1]);
           count += add;
         }
         __syncwarp();
@@ -750,7 +764,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams 
             for (int i = 0; i < here; i++) {
               const uint32_t g = __shfl_sync(FULLMASK, v.x, i), mk = __shfl_sync(FULLMASK, v.y, i);
               if ((mk >> lane) & 1u) {
-                const uint32_t k = (uint32_t)(__ldg(&tperm[32 * (int)g + lane]) - w0);
+                const uint32_t k = (uint32_t)(__ldg(&perm[32 * (int)g + lane]) - w0);
                 if (k < 32u * (uint32_t)window_words) atomicOr(&bits[k >> 5], 1u << (k & 31));
               }
             }
@@ -788,12 +802,13 @@ __global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams 
       auto load = [&](int i) {
         if (i >= count) return;
         j = direct ? i : queue[i];
+        if (ranked) j = __ldg(&lv->index[j]);
         y = __ldg(&yorig[j]);
 #pragma unroll
         for (int q = 0; q < FCH; q++) yf[q] = __ldg(tf + (size_t)j * FCH + q);
       };
       load(lane);
-      for (int i0 = 0; i0 < count && kept < cap; i0 += 32) {
+      for (int i0 = 0; i0 < count && kept < stop; i0 += 32) {
         const bool has = i0 + lane < count;
         const float4 yc = y;
         float4 fc[FP];
@@ -816,7 +831,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams 
         if (min(kept, cap) - flushed >= 32) flush(true);
       }
       __syncwarp();
-      if (kept >= cap || entries < 0 || cands <= kRowSorted) break;
+      if (kept >= stop || entries < 0 || cands <= kRowSorted) break;
       if (base >= total) {
         w0 += 32 * window_words;
         if (w0 >= m) break;
@@ -826,13 +841,81 @@ __global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams 
     const int z = min(kept, cap);
     if (flushed < z) flush(lane < z - flushed);
     if (lane == 0) P->nnz_row[s] = z;
+    if (KIND == ROWS_ALIGN) {
+      if (!ranked && z > 1 && kept <= cap + order_cap && K.use_geo)
+        order_row(P->A_j + (size_t)s * P->ld, P->A_v + (size_t)s * P->ld, z, lv->of_index, m, bits, window_words,
+                  reinterpret_cast<unsigned short *>(queue), P->cand + (size_t)s * P->cand_pitch, lane);
+      __syncwarp();
+      continue;
+    }
     nnz += z;
     mx = max(mx, z);
-    const float sum = warp_sum8(acc, lane);
-    const int k = lane >> 2;
-    lane_sum += (double)(k < 3 ? __fdiv_rn(sum, K.c) : (k < 6 ? __fdiv_rn(sum, K.d) : sum));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(FULLMASK, acc, o);
+    row_total += (double)acc;
   }
-  rows_finish(B, K, P, b, nb, lane_sum, nnz, mx);
+  if (KIND == ROWS_SUM) rows_finish(B, P, b, nb, row_total, nnz, mx);
+}
+
+// Calls add(a, y) for the z entries of ELL row s in slot order.
+template <class Add>
+__device__ __forceinline__ void row_entries(const PairDev *P, int s, int z, Add add) {
+  const int *__restrict__ Aj = P->A_j + (size_t)s * P->ld;
+  const float *__restrict__ Av = P->A_v + (size_t)s * P->ld;
+  const float4 *__restrict__ yorig = P->yorig;
+  int c = 0;
+  if (z >= 8) {
+    int4 j0 = *reinterpret_cast<const int4 *>(Aj), j1 = *reinterpret_cast<const int4 *>(Aj + 4);
+    for (; c + 8 <= z; c += 8) {
+      const float4 y0 = __ldg(&yorig[j0.x]), y1 = __ldg(&yorig[j0.y]), y2 = __ldg(&yorig[j0.z]), y3 = __ldg(&yorig[j0.w]);
+      const float4 y4 = __ldg(&yorig[j1.x]), y5 = __ldg(&yorig[j1.y]), y6 = __ldg(&yorig[j1.z]), y7 = __ldg(&yorig[j1.w]);
+      const float4 a = *reinterpret_cast<const float4 *>(Av + c), b = *reinterpret_cast<const float4 *>(Av + c + 4);
+      if (c + 16 <= z) {
+        j0 = *reinterpret_cast<const int4 *>(Aj + c + 8);
+        j1 = *reinterpret_cast<const int4 *>(Aj + c + 12);
+      }
+      add(a.x, y0); add(a.y, y1); add(a.z, y2); add(a.w, y3);
+      add(b.x, y4); add(b.y, y5); add(b.z, y6); add(b.w, y7);
+    }
+  }
+  if (c + 4 <= z) {
+    const int4 j = *reinterpret_cast<const int4 *>(Aj + c);
+    const float4 a = *reinterpret_cast<const float4 *>(Av + c);
+    const float4 y0 = __ldg(&yorig[j.x]), y1 = __ldg(&yorig[j.y]), y2 = __ldg(&yorig[j.z]), y3 = __ldg(&yorig[j.w]);
+    add(a.x, y0); add(a.y, y1); add(a.z, y2); add(a.w, y3);
+    c += 4;
+  }
+  for (; c < z; c++) add(Av[c], __ldg(&yorig[Aj[c]]));
+}
+
+// Row partials of the align loop from the final ELL entries, one after the other in slot
+// order (thread per row): omega = sum a (x cross y), v = sum a (y - x), sum a
+// (CvoGPU.cu:2001-2062 computes the same sums from the sparse kernel matrix).  The order is
+// part of the result (see k_rows), so a row is one thread's chain of additions; the loads
+// run ahead of it: eight entries' indices one step, their targets' positions in one batch.
+// Bounds: L2 latency of index -> position, one round trip per eight entries.
+__global__ void __launch_bounds__(128) k_rowsum(BatchDev B, KParams K) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= B.total_rows) return;
+  const int p = find_segment(B.row_off, B.npairs, g);
+  const PairDev *P = &B.pairs[p];
+  if (P->done) return;
+  const int s = g - B.row_off[p];
+  const int z = P->nnz_row[s];
+  const float4 x = __ldg(&P->xs[s]);
+  float w0 = 0.f, w1 = 0.f, w2 = 0.f, v0 = 0.f, v1 = 0.f, v2 = 0.f, as = 0.f;
+  row_entries(P, s, z, [&](float a, const float4 &y) {
+    w0 = fmaf(a, fs(fm(x.y, y.z), fm(x.z, y.y)), w0);
+    w1 = fmaf(a, fs(fm(x.z, y.x), fm(x.x, y.z)), w1);
+    w2 = fmaf(a, fs(fm(x.x, y.y), fm(x.y, y.x)), w2);
+    v0 = fmaf(a, y.x - x.x, v0);
+    v1 = fmaf(a, y.y - x.y, v1);
+    v2 = fmaf(a, y.z - x.z, v2);
+    as += a;
+  });
+  float4 *rs = reinterpret_cast<float4 *>(P->row_sums + (size_t)s * 8);
+  rs[0] = make_float4(__fdiv_rn(w0, K.c), __fdiv_rn(w1, K.c), __fdiv_rn(w2, K.c), __fdiv_rn(v0, K.d));
+  rs[1] = make_float4(__fdiv_rn(v1, K.d), __fdiv_rn(v2, K.d), as, 0.f);
 }
 
 }  // namespace cvo_gb
