@@ -285,7 +285,7 @@ int run_association_adaptive(Handle *h, DevCloud *src, DevCloud *tgt, const floa
   k_ad_xform<<<(n + 255) / 256, 256, 0, h->stream>>>(n, src->spos, b.Id, b.xs);
   h->launches++;
   std::vector<EdgeAssoc> E;
-  int rc = run_association_edges(h, {src}, {tgt}, {b.xs}, std::vector<float>(Q, Q + 12), {ell}, {kAdCap},
+  int rc = run_association_edges(h, {src}, {tgt}, {b.xs}, {0.f}, std::vector<float>(Q, Q + 12), {ell}, {kAdCap},
                                  kAdCap, &E, &K);
   if (rc) return rc;
   const int ld = E[0].ld;
@@ -358,7 +358,7 @@ int run_align_adaptive(Handle *h, DevCloud *src, DevCloud *tgt, const float T_in
     poses.insert(poses.end(), kIdentity12, kIdentity12 + 12);
     poses.insert(poses.end(), Q, Q + 12);
     std::vector<EdgeAssoc> E;
-    int rc = run_association_edges(h, {src, src, tgt}, {tgt, src, tgt}, {b.xs, b.xs, b.ys}, poses,
+    int rc = run_association_edges(h, {src, src, tgt}, {tgt, src, tgt}, {b.xs, b.xs, b.ys}, {0.f, 0.f, 0.f}, poses,
                                    {ell, ell, ell}, {kAdCap, kAdCap, kAdCap}, kAdCap, &E, &K);
     if (rc) return rc;
     const Ell A{E[0].A_j, E[0].A_v, E[0].nnz_row, E[0].ld}, X{E[1].A_j, E[1].A_v, E[1].nnz_row, E[1].ld};

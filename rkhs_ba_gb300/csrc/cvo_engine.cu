@@ -323,7 +323,7 @@ using RowsFn = void (*)(BatchDev, KParams, int);
 
 struct AssocKernels {
   CandFn cand = nullptr;
-  RowsFn rows = nullptr, align_rows = nullptr;
+  RowsFn rows = nullptr, ordered_rows = nullptr;
 };
 
 // Feature rows are stored as ceil(F/4) float4 chunks; label rows as 5 or 9
@@ -333,9 +333,9 @@ template <int FC, int LC, bool G>
 static int pick_assoc(AssocKernels *a) {
   a->cand = k_cand<FC>;
   a->rows = k_rows<FC, LC, G, ROWS_SUM>;
-  a->align_rows = k_rows<FC, LC, G, ROWS_ALIGN>;
+  a->ordered_rows = k_rows<FC, LC, G, ROWS_ORDERED>;
   // opt in above the 48 KB default (setting it again is harmless)
-  for (RowsFn f : {a->rows, a->align_rows})
+  for (RowsFn f : {a->rows, a->ordered_rows})
     if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem_bytes(kRowWindow)) != cudaSuccess) {
       cudaGetLastError();
       return CVO_ERR_CUDA;
@@ -477,6 +477,13 @@ static float host_radius(const KParams &K, float ell, float norm) {
   return std::sqrt(std::max(d2t, 0.f));
 }
 
+// The finest of the pair's lattices that serves search radius r.
+static int level_for(const PairDev &P, float r) {
+  for (int i = 0; i < P.nlevels; i++)
+    if (P.level_r[i] >= r) return i;
+  return P.nlevels - 1;
+}
+
 long long tune_items(long long rows) { return (rows + 127) / 128; }
 
 long long tune_key(int F, int C, long long rows) {
@@ -496,6 +503,7 @@ struct BatchHost {
   int cand_blocks = 0, xform_blocks = 0;
   int window_words = 0;
   size_t row_smem = 0;
+  bool ordered = false;             // rows in the order of the targets' lattice (RankLevel)
 };
 
 // Work items that keep the candidate test's warps busy: about two per resident warp slot,
@@ -543,16 +551,17 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
   const double want = (tc.blocks_per_sm > 0 ? 4.0 * tc.blocks_per_sm * sms : (double)kCandItems) *
                       (tc.cell_div_r / 4.0) * (tc.cell_div_ext / 8.0);
   const int splits = (int)std::min<double>(kMaxSplits, std::max(1.0, std::ceil(want / (double)std::max<long long>(tiles, 1))));
-  // orders of the targets (align): the lattices of every radius the lengthscale may reach
+  // orders of the targets (align and edges): the lattices of every radius the lengthscale may reach
+  bh->ordered = mode == MODE_ALIGN || mode == MODE_EDGES;
   std::vector<std::vector<RankLevel>> lv(np);
   std::vector<std::vector<float>> lr(np);
-  for (int p = 0; p < np && mode == MODE_ALIGN; p++) {
+  for (int p = 0; p < np && bh->ordered; p++) {
     const float ext = srcs[p]->tile_ext;
     std::vector<int> exps;
     if (!K.use_geo) {
       exps.push_back(1000);
     } else {
-      const float ell_hi = ell0[p], ell_lo = std::min(K.ell_min, ell_hi);
+      const float ell_hi = ell0[p], ell_lo = mode == MODE_ALIGN ? std::min(K.ell_min, ell_hi) : ell_hi;
       const float r_hi = host_radius(K, ell_hi, srcs[p]->max_norm), r_lo = host_radius(K, ell_lo, 0.f);
       int e_hi = level_for_radius(cell_for_radius(r_hi, ext)), e_lo = level_for_radius(cell_for_radius(r_lo, ext));
       if (e_hi - e_lo + 1 > 24) e_lo = e_hi - 23;
@@ -589,8 +598,8 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     sp[p] = std::max(1, std::min(splits, ns));
     caps[p] = std::max(1, std::min(kGroup * ((ns + sp[p] - 1) / sp[p]), most / sp[p]));
     if (!K.use_mma) sp[p] = caps[p] = 1;
-    // an align row's kept entries pass through its candidate entries' place (order_row)
-    pitch[p] = std::max(sp[p] * caps[p], mode == MODE_ALIGN ? std::min(capmax, m) : 0);
+    // an ordered row's kept entries pass through its candidate entries' place (order_row)
+    pitch[p] = std::max(sp[p] * caps[p], bh->ordered ? std::min(capmax, m) : 0);
     bh->item_off[p + 1] = bh->item_off[p] + group_count(n) * sp[p];
     bh->tgt_off[p + 1] = bh->tgt_off[p] + m;
     int rb = (n + kRowsPerBlock - 1) / kRowsPerBlock, sb = (n + kStepThreads - 1) / kStepThreads;
@@ -604,10 +613,8 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     add(ell ? sizeof(int) * (size_t)n * ell_ld : 0);             // ELL
     add(ell ? sizeof(float) * (size_t)n * ell_ld : 0);
     add(sizeof(uint2) * (size_t)n * pitch[p]);                   // candidate entries
-    if (mode == MODE_ALIGN) {
-      add(sizeof(float) * 8 * (size_t)n);                        // row_sums
-      add(sizeof(RankLevel) * lv[p].size());
-    }
+    if (mode == MODE_ALIGN) add(sizeof(float) * 8 * (size_t)n);  // row_sums
+    add(sizeof(RankLevel) * lv[p].size());
     add(sizeof(int2) * (size_t)n * sp[p]);                       // entry counts
     add(sizeof(int) * n);                                        // nnz_row
     add(sizeof(double) * kPartStride * (size_t)std::max(rb, sb)); // partials
@@ -664,17 +671,14 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     P.cap = capmax;
     P.order_cap = order_cap;
     P.src_norm = s->max_norm;
-    if (mode == MODE_ALIGN) {
-      P.row_sums = ar.take<float>(8 * (size_t)s->n);
+    if (mode == MODE_ALIGN) P.row_sums = ar.take<float>(8 * (size_t)s->n);
+    if (bh->ordered) {
       RankLevel *levels = ar.take<RankLevel>(lv[p].size());
       CVO_CUDA_TRY(h, cudaMemcpyAsync(levels, lv[p].data(), sizeof(RankLevel) * lv[p].size(), cudaMemcpyHostToDevice, h->stream));
       P.levels = levels;
       P.nlevels = (int)lv[p].size();
       for (int i = 0; i < P.nlevels && i < 24; i++) P.level_r[i] = lr[p][i];
-      const float r0 = host_radius(K, P.ell, s->max_norm);
-      P.level = P.nlevels - 1;
-      for (int i = 0; i < P.nlevels; i++)
-        if (P.level_r[i] >= r0) { P.level = i; break; }
+      P.level = level_for(P, host_radius(K, P.ell, s->max_norm));
     }
     P.done = (s->n == 0 || t->n == 0) ? 1 : 0;
     if (!P.done) active++;
@@ -743,7 +747,7 @@ void launch_association(Handle *h, BatchHost *bh, const KParams &K, bool align =
     h->launches++;
   }
   mark(h, ev, 5);
-  const RowsFn rows = align ? bh->fn.align_rows : bh->fn.rows;
+  const RowsFn rows = bh->ordered ? bh->fn.ordered_rows : bh->fn.rows;
   rows<<<std::max(B.total_rblocks, 1), 32 * kRowWarps, bh->row_smem, h->stream>>>(B, K, bh->window_words);
   h->launches += 2;
   mark(h, ev, 6);
@@ -1181,7 +1185,8 @@ int replay_association(Handle *h, BatchHost *bh, const KParams &K, AssocGraph *g
 }  // namespace
 
 int run_association_edges(Handle *h, const std::vector<DevCloud *> &srcs, const std::vector<DevCloud *> &tgts,
-                          const std::vector<const float4 *> &src_world, const std::vector<float> &tgt_pose, const std::vector<float> &ells,
+                          const std::vector<const float4 *> &src_world, const std::vector<float> &src_world_norm,
+                          const std::vector<float> &tgt_pose, const std::vector<float> &ells,
                           const std::vector<int> &caps, int capmax, std::vector<EdgeAssoc> *out,
                           const KParams *kparams, AssocGraph *graph) {
   NvtxRange nvtx_range("association_edges");
@@ -1192,7 +1197,7 @@ int run_association_edges(Handle *h, const std::vector<DevCloud *> &srcs, const 
   std::vector<float> Tid(16 * (size_t)ne, 0.f);
   for (int e = 0; e < ne; e++) Tid[16 * e] = Tid[16 * e + 5] = Tid[16 * e + 10] = Tid[16 * e + 15] = 1.f;
   BatchHost bh;
-  int rc = build_batch(h, K, srcs, tgts, Tid, MODE_EXPORT, capmax, ells, &bh);
+  int rc = build_batch(h, K, srcs, tgts, Tid, MODE_EDGES, capmax, ells, &bh);
   if (rc) return rc;
   for (int e = 0; e < ne; e++) {
     PairDev &P = bh.pairs[e];
@@ -1208,6 +1213,7 @@ int run_association_edges(Handle *h, const std::vector<DevCloud *> &srcs, const 
     for (int r = 0; r < 3; r++)
       for (int c = 0; c < 3; c++) P.R[3 * r + c] = Q[4 * c + r];
     for (int r = 0; r < 3; r++) P.T[r] = -(P.R[3 * r] * Q[3] + P.R[3 * r + 1] * Q[7] + P.R[3 * r + 2] * Q[11]);
+    P.level = level_for(P, host_radius(K, ells[e], src_world_norm[e]));
   }
   if (graph && !h->prof.on) {
     if ((rc = replay_association(h, &bh, K, graph))) return rc;

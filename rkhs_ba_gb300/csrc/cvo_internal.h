@@ -31,8 +31,9 @@ inline int group_count(int n) { return (n + kGroup - 1) / kGroup; }
 inline int box_chunks(int FP) { return FP / 4 < 2 ? FP / 4 : 2; }
 
 // An order of a target cloud's points: by the cells of a lattice over the bounding box (z, then
-// y, then x), inside a cell by index.  The align loop keeps the entries of a kernel-matrix
-// row in this order and adds them up in it, with the lattice that follows the search radius.
+// y, then x), inside a cell by index.  The align loop and the window solve keep the entries
+// of a kernel-matrix row in this order and add them up in it, with the lattice that follows
+// the search radius.
 struct RankLevel {
   float h;                // cell size
   int *index;             // rank -> original index
@@ -115,7 +116,7 @@ struct PairDev {
   const float2 *tg;               // target geometric types, original order
   int *nnz_row;                   // n
   float *row_sums;                // align: n * 8, omega(3)/c, v(3)/d
-  // align: orders of the target's points, finest lattice first, and the largest search radius
+  // align and edges: orders of the target's points, finest lattice first, and the largest search radius
   // each serves; a row that kept more than cap + order_cap pairs stays in index order
   const RankLevel *levels;
   float level_r[24];
@@ -125,7 +126,7 @@ struct PairDev {
   unsigned int *counter;          // last-block counters [2]
   int F, C;                       // feature / label dimensions (source and target agree)
   int capmax;
-  int mode;                       // 0 align, 1 inner product, 2 export
+  int mode;                       // 0 align, 1 inner product, 2 export, 3 edges of a window
   // iteration state
   float R[9], T[3];               // internal pose
   float Ri[9], Ti[3];             // target transform R^T, -R^T T
@@ -264,7 +265,7 @@ int run_inner_product_pairs(Handle *h, const std::vector<DevCloud *> &srcs, cons
 
 // One association pass per edge between world-frame clouds (multi-frame solver).
 // src_world: per edge, the source frame's points already in world coordinates in
-// tile order ({x, y, z, ||x||}); tgt_pose: per edge 12 floats, the target frame's
+// tile order ({x, y, z, ||x||}) and an upper bound of their norms; tgt_pose: per edge 12 floats, the target frame's
 // pose (row-major 3x4, frame -> world) applied to the target points.  The result
 // arrays stay valid until the next batch is built on the handle.
 struct EdgeAssoc {
@@ -296,7 +297,8 @@ struct AssocGraph {
   ~AssocGraph();
 };
 int run_association_edges(Handle *h, const std::vector<DevCloud *> &srcs, const std::vector<DevCloud *> &tgts,
-                          const std::vector<const float4 *> &src_world, const std::vector<float> &tgt_pose, const std::vector<float> &ells,
+                          const std::vector<const float4 *> &src_world, const std::vector<float> &src_world_norm,
+                          const std::vector<float> &tgt_pose, const std::vector<float> &ells,
                           const std::vector<int> &caps, int capmax, std::vector<EdgeAssoc> *out,
                           const KParams *kparams = nullptr, AssocGraph *graph = nullptr);
 

@@ -9,8 +9,8 @@
 // reference's analytic Jacobian (IRLS_Cost_CPU.hpp:260-371) composed with the SE(3)
 // local parameterisation (local_parameterization_se3.hpp:13-100).  The reference
 // hands that solve to Ceres (LM, SPARSE_NORMAL_CHOLESKY, IRLS.cpp:273-290); here the
-// normal equations are accumulated on the GPU (the kernel-matrix entries are read once per
-// outer iteration and reduced to moments per row) and the 6F x 6F system is solved on the host, with the LM iteration
+// normal equations are accumulated on the GPU (one pass over all kernel-matrix entries
+// of all edges) and the 6F x 6F system is solved on the host, with the LM iteration
 // stated in oracle/cvo_oracle.c (lm_solve).
 #include <cmath>
 #include <cstring>
@@ -24,10 +24,8 @@
 namespace cvo_gb {
 namespace {
 
-constexpr int kIrlsWarps = 4;
-constexpr int kIrlsRows = 32 * kIrlsWarps;   // rows per block: one tile of 32 per warp
-constexpr int kNormTerms = 28;   // S (6), S K^T (9), K S K^T (6), q (3), K q (3), cost
-constexpr int kMoments = 40;     // floats a row's entries are reduced to, see k_irls_moments
+constexpr int kIrlsThreads = 128;
+constexpr int kNormTerms = 91;   // 78 upper-triangle Hessian terms (12x12), 12 gradient, 1 cost
 
 // frame points (tile order, local) -> world with the float pose, canonical order
 __global__ void k_world(const float4 *local, int n, const float *pose, float4 *world) {
@@ -52,228 +50,111 @@ struct IrlsEdge {
   int n, lim;         // rows, entries used per row
   int f1, f2;
   int blk0;           // first block of this edge
-  float *mom;         // kMoments planes of n floats
 };
 
-// The edge of a block.
-__device__ __forceinline__ IrlsEdge edge_of(const IrlsEdge *E, int ne, int blk) {
+// Accumulates, per block, the cost and (WANT_J) the 12x12 J^T J and J^T r of the
+// residuals of one edge.  One thread per row; the row's point is moved with the FP64
+// poses once, every entry is then single precision (see the residual below); per-row
+// sums in FP32, block sums in FP64.
+template <bool WANT_J>
+__global__ void __launch_bounds__(kIrlsThreads) k_irls_accum(const IrlsEdge *E, int ne, const double *poses,
+                                                              double *partial) {
+  __shared__ double sh[kIrlsThreads / 32][kNormTerms];
   int lo = 0, hi = ne - 1;
   while (lo < hi) {
     int mid = (lo + hi + 1) >> 1;
-    if (E[mid].blk0 <= blk) lo = mid; else hi = mid - 1;
+    if (E[mid].blk0 <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
   }
-  return E[lo];
-}
-
-// The row's point in the target frame, p' = R2^T (T1 p1 - t2), in double.
-__device__ __forceinline__ void row_point(const double *poses, const IrlsEdge &ed, int s, double (&pd)[3]) {
-  const double *T1 = poses + 12 * ed.f1, *T2 = poses + 12 * ed.f2;
-  const float4 a1 = __ldg(&ed.p1[s]);
-  const double p1[3] = {a1.x, a1.y, a1.z};
-  double q1[3];
-  for (int r = 0; r < 3; r++) q1[r] = T1[4 * r] * p1[0] + T1[4 * r + 1] * p1[1] + T1[4 * r + 2] * p1[2] + T1[4 * r + 3];
-  for (int r = 0; r < 3; r++)
-    pd[r] = T2[r] * (q1[0] - T2[3]) + T2[4 + r] * (q1[1] - T2[7]) + T2[8 + r] * (q1[2] - T2[11]);
-}
-
-// A row's share of the normal equations is a polynomial in its point p': with c = p' when
-// the kernel matrix was made, e = p2 - c per entry and x = p' - c, an entry's difference is
-// d = x - e and, with r = a |d|^2,
-//   sum d d^T   = n x x^T - x N1^T - N1 x^T + N2
-//   sum r d     = |x|^2 x A0 - |x|^2 A1 - 2 (x.A1) x + 2 A2 x + tr(A2) x - A3
-//   sum r^2     = |x|^4 M0 + 4 x^T M2 x + M4 - 4 |x|^2 x.M1 + 2 |x|^2 tr(M2) - 4 x.M3
-// with N, A, M the moments of e weighted by 1, a and a^2 (N2 = sum e e^T, A3 = sum a |e|^2 e,
-// ...).  So the entries are read once per outer iteration (37 sums) and every evaluation of
-// the solve, some forty per outer iteration, reads 40 floats a row.  e and x are small
-// against the coordinates (c is the rounded double p', e is exact to its own rounding), so
-// the sums keep the accuracy of summing each entry's r anew.
-// Planes: c (3), n, N1 (3), N2 (6), A0, A1 (3), A2 (6), A3 (3), M0, M1 (3), M2 (6), M3 (3), M4.
-// Eight lanes share a row and a warp runs four rows at a time: the rows' entries differ
-// widely (0 to cap), and one row per warp left too few gathers in flight.
-// Bounds: L2 latency of entry -> point.
-__global__ void __launch_bounds__(32 * kIrlsWarps) k_irls_moments(const IrlsEdge *E, int ne, const double *poses) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, sub = lane & 7;
-  const IrlsEdge ed = edge_of(E, ne, blockIdx.x);
-  const int t0 = ((int)blockIdx.x - ed.blk0) * kIrlsRows + 32 * w;
-  const int s = t0 + lane;
-  const int z = s < ed.n ? min(__ldg(&ed.nnz_row[s]), ed.lim) : 0;
-  if (s < ed.n) ed.mom[3 * (size_t)ed.n + s] = (float)z;
-  if (!__any_sync(FULLMASK, z > 0)) return;
-  float c[3] = {0.f, 0.f, 0.f};
-  if (z > 0) {
-    double pd[3];
-    row_point(poses, ed, s, pd);
-    for (int r = 0; r < 3; r++) {
-      c[r] = (float)pd[r];
-      ed.mom[r * (size_t)ed.n + s] = c[r];
-    }
-  }
-  for (int r0 = 0; r0 < 32; r0 += 4) {
-    const int r = r0 + (lane >> 3);
-    const int zr = __shfl_sync(FULLMASK, z, r);
-    if (!__any_sync(FULLMASK, zr > 0)) continue;
-    const float c0 = __shfl_sync(FULLMASK, c[0], r), c1 = __shfl_sync(FULLMASK, c[1], r), c2 = __shfl_sync(FULLMASK, c[2], r);
-    const int *__restrict__ Aj = ed.A_j + (size_t)(t0 + r) * ed.ld;
-    const float *__restrict__ Av = ed.A_v + (size_t)(t0 + r) * ed.ld;
-    float v[36];      // all but n
-#pragma unroll
-    for (int k = 0; k < 36; k++) v[k] = 0.f;
-#pragma unroll 4
-    for (int i = sub; i < zr; i += 8) {
-      const float a = __ldg(Av + i);
-      const float4 b2 = __ldg(&ed.p2[__ldg(Aj + i)]);
-      const float e[3] = {b2.x - c0, b2.y - c1, b2.z - c2};
-      const float e2 = e[0] * e[0] + e[1] * e[1] + e[2] * e[2];
-      const float ae[3] = {a * e[0], a * e[1], a * e[2]};
-      const float be[3] = {a * ae[0], a * ae[1], a * ae[2]}, be2 = a * a * e2;
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        v[k] += e[k];
-        v[10 + k] += ae[k];
-        v[19 + k] = fmaf(e2, ae[k], v[19 + k]);
-        v[23 + k] += be[k];
-        v[32 + k] = fmaf(e2, be[k], v[32 + k]);
-      }
-      v[9] += a;
-      v[22] = fmaf(a, a, v[22]);
-      v[35] = fmaf(be2, e2, v[35]);
-      int k = 0;
-#pragma unroll
-      for (int p = 0; p < 3; p++)
-#pragma unroll
-        for (int q = p; q < 3; q++, k++) {
-          v[3 + k] = fmaf(e[p], e[q], v[3 + k]);
-          v[13 + k] = fmaf(ae[p], e[q], v[13 + k]);
-          v[26 + k] = fmaf(be[p], e[q], v[26 + k]);
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < 36; k++) {
-      v[k] += __shfl_xor_sync(FULLMASK, v[k], 4);
-      v[k] += __shfl_xor_sync(FULLMASK, v[k], 2);
-      v[k] += __shfl_xor_sync(FULLMASK, v[k], 1);
-    }
-    if (sub == 0 && zr > 0) {
-#pragma unroll
-      for (int k = 0; k < 36; k++) ed.mom[(4 + k) * (size_t)ed.n + t0 + r] = v[k];
-    }
-  }
-}
-
-// Sums of the normal equations of one edge, per block.  With p' = R2^T (T1 p1 - t2) (the
-// row's point in the target frame), d = p' - p2, r = a |d|^2, K = [p']x and t' = R2^T (t1 - t2),
-// the Jacobian row of the residual is linear in d,
-//   J = [R12 d, p1 x R12 d, -d, -p2 x d] = B [d, p' x d],   R12 = R1^T R2,
-//   B = [R12 0; -R12 [t']x R12; -I 0; 0 -I]   (p2 x d = p' x d, p1 x R12 d = R12 ((p' - t') x d)),
-// and B is the edge's, p' the row's.  So a row adds G = [I; K] S [I; K]^T and [q; K q] with
-// S = sum d d^T, q = sum r d (27 terms), and the host forms J^T J = B G B^T and J^T r once
-// per edge, in FP64.  S, q and the cost come from the row's moments.  FP32 per row, FP64
-// over rows.
-// Bounds: reading 160 bytes a row, and the FP64 sums.  Summing 91 FP32 terms per entry in
-// one thread per row took 468 us an evaluation with the Jacobian and 250 without for 28
-// edges of 20k-60k rows.
-template <bool WANT_J>
-__global__ void __launch_bounds__(32 * kIrlsWarps) k_irls_accum(const IrlsEdge *E, int ne, const double *poses,
-                                                                double *partial) {
+  const IrlsEdge ed = E[lo];
+  const int s = ((int)blockIdx.x - ed.blk0) * kIrlsThreads + threadIdx.x;
   constexpr int NT = WANT_J ? kNormTerms : 1;
-  __shared__ double red[NT][32 * kIrlsWarps + 1];
-  const IrlsEdge ed = edge_of(E, ne, blockIdx.x);
-  const int s = ((int)blockIdx.x - ed.blk0) * kIrlsRows + threadIdx.x;
-  const size_t n = ed.n;
-  const float *__restrict__ m = ed.mom + s;
-  const float z = s < ed.n ? __ldg(m + 3 * n) : 0.f;
-  if (!__syncthreads_or(z > 0.f)) {
-    for (int k = threadIdx.x; k < NT; k += blockDim.x) partial[(size_t)blockIdx.x * kNormTerms + k] = 0.0;
-    return;
-  }
-  double acc[NT];
+  float acc[NT];
 #pragma unroll
-  for (int k = 0; k < NT; k++) acc[k] = 0.0;
-  if (z > 0.f) {
-    double pd[3];
-    row_point(poses, ed, s, pd);
-    auto M = [&](int k) { return __ldg(m + k * n); };
-    const float x[3] = {(float)(pd[0] - (double)M(0)), (float)(pd[1] - (double)M(1)), (float)(pd[2] - (double)M(2))};
-    const float x2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2];
-    const float B[6] = {M(30), M(31), M(32), M(33), M(34), M(35)};
-    const float Bx[3] = {B[0] * x[0] + B[1] * x[1] + B[2] * x[2], B[1] * x[0] + B[3] * x[1] + B[4] * x[2],
-                         B[2] * x[0] + B[4] * x[1] + B[5] * x[2]};
-    const float c2 = 4.f * (x[0] * Bx[0] + x[1] * Bx[1] + x[2] * Bx[2]) + 2.f * x2 * (B[0] + B[3] + B[5]);
-    const float c1 = x[0] * M(36) + x[1] * M(37) + x[2] * M(38), c3 = x[0] * M(27) + x[1] * M(28) + x[2] * M(29);
-    const float cost = 0.5f * (M(39) - 4.f * c1 + c2 - 4.f * x2 * c3 + x2 * x2 * M(26));
-    if (WANT_J) {
-      const float n1[3] = {M(4), M(5), M(6)}, A[6] = {M(17), M(18), M(19), M(20), M(21), M(22)}, a1[3] = {M(14), M(15), M(16)};
-      float S[3][3];
-      S[0][0] = M(7) - 2.f * x[0] * n1[0] + z * x[0] * x[0];
-      S[0][1] = S[1][0] = M(8) - x[0] * n1[1] - x[1] * n1[0] + z * x[0] * x[1];
-      S[0][2] = S[2][0] = M(9) - x[0] * n1[2] - x[2] * n1[0] + z * x[0] * x[2];
-      S[1][1] = M(10) - 2.f * x[1] * n1[1] + z * x[1] * x[1];
-      S[1][2] = S[2][1] = M(11) - x[1] * n1[2] - x[2] * n1[1] + z * x[1] * x[2];
-      S[2][2] = M(12) - 2.f * x[2] * n1[2] + z * x[2] * x[2];
-      const float xa = x[0] * a1[0] + x[1] * a1[1] + x[2] * a1[2], tr = A[0] + A[3] + A[5], a0 = M(13);
-      const float Ax[3] = {A[0] * x[0] + A[1] * x[1] + A[2] * x[2], A[1] * x[0] + A[3] * x[1] + A[4] * x[2],
-                           A[2] * x[0] + A[4] * x[1] + A[5] * x[2]};
-      float q[3];
-#pragma unroll
-      for (int k = 0; k < 3; k++) q[k] = (2.f * Ax[k] + tr * x[k] - M(23 + k)) + (x2 * (x[k] * a0 - a1[k]) - 2.f * xa * x[k]);
-      const float px = (float)pd[0], py = (float)pd[1], pz = (float)pd[2];
-      // K v = p' x v; W = S K^T has rows p' x (row of S), X = K S K^T columns p' x (column of W)
-      float W[3][3], X[3][3];
-#pragma unroll
-      for (int i = 0; i < 3; i++) {
-        W[i][0] = py * S[i][2] - pz * S[i][1];
-        W[i][1] = pz * S[i][0] - px * S[i][2];
-        W[i][2] = px * S[i][1] - py * S[i][0];
-      }
-#pragma unroll
-      for (int j = 0; j < 3; j++) {
-        X[0][j] = py * W[2][j] - pz * W[1][j];
-        X[1][j] = pz * W[0][j] - px * W[2][j];
-        X[2][j] = px * W[1][j] - py * W[0][j];
-      }
-      const float t[kNormTerms] = {S[0][0], S[0][1], S[0][2], S[1][1], S[1][2], S[2][2],
-                                   W[0][0], W[0][1], W[0][2], W[1][0], W[1][1], W[1][2], W[2][0], W[2][1], W[2][2],
-                                   X[0][0], X[0][1], X[0][2], X[1][1], X[1][2], X[2][2],
-                                   q[0], q[1], q[2], py * q[2] - pz * q[1], pz * q[0] - px * q[2], px * q[1] - py * q[0], cost};
-#pragma unroll
-      for (int k = 0; k < NT; k++) acc[k] = (double)t[k];
-    } else {
-      acc[0] = (double)cost;
+  for (int k = 0; k < NT; k++) acc[k] = 0.f;
+  double cost = 0.0;
+  if (s < ed.n) {
+    const double *T1 = poses + 12 * ed.f1, *T2 = poses + 12 * ed.f2;
+    const int z = min(ed.nnz_row[s], ed.lim);
+    const float4 a1 = ed.p1[s];
+    // The residual vector e = T1 p1 - T2 p2 (world frame) is a difference of two points
+    // tens of metres out that lie centimetres apart.  Per row, p1 is taken to the target
+    // frame in double, p1' = R2^T (T1 p1 - t2), and split into float hi + lo; per entry
+    // d = (hi - p2) + lo is then exact to float rounding of d itself (hi - p2 cancels
+    // without error for nearby points), e = R2 d, |e| = |d|, R2^T e = d and
+    // R1^T e = (R1^T R2) d.  So the per-entry arithmetic is single precision without the
+    // cancellation a float e = q1 - q2 would suffer.
+    const double p1[3] = {a1.x, a1.y, a1.z};
+    double q1[3], pd[3];
+    for (int r = 0; r < 3; r++) q1[r] = T1[4 * r] * p1[0] + T1[4 * r + 1] * p1[1] + T1[4 * r + 2] * p1[2] + T1[4 * r + 3];
+    for (int r = 0; r < 3; r++)
+      pd[r] = T2[r] * (q1[0] - T2[3]) + T2[4 + r] * (q1[1] - T2[7]) + T2[8 + r] * (q1[2] - T2[11]);
+    float ph[3], pl[3], R12[9];
+    for (int r = 0; r < 3; r++) {
+      ph[r] = (float)pd[r];
+      pl[r] = (float)(pd[r] - (double)ph[r]);
     }
-  }
+    for (int r = 0; r < 3; r++)
+      for (int c = 0; c < 3; c++)
+        R12[3 * r + c] = (float)(T1[r] * T2[c] + T1[4 + r] * T2[4 + c] + T1[8 + r] * T2[8 + c]);
+    float cost_f = 0.f;
+    for (int c = 0; c < z; c++) {
+      const int j = ed.A_j[(size_t)s * ed.ld + c];
+      const float a = ed.A_v[(size_t)s * ed.ld + c];
+      const float4 b2 = __ldg(&ed.p2[j]);
+      const float d[3] = {(ph[0] - b2.x) + pl[0], (ph[1] - b2.y) + pl[1], (ph[2] - b2.z) + pl[2]};
+      const float rr = a * (d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+      cost_f = fmaf(0.5f * rr, rr, cost_f);
+      if (WANT_J) {
+        float u1[3], J[12];
+        const float *u2 = d;                                                        // R2^T e
+        for (int r = 0; r < 3; r++) u1[r] = R12[3 * r] * d[0] + R12[3 * r + 1] * d[1] + R12[3 * r + 2] * d[2];   // R1^T e
+        const float x1 = a1.x, y1 = a1.y, z1 = a1.z, x2 = b2.x, y2 = b2.y, z2 = b2.z;
+        J[0] = u1[0]; J[1] = u1[1]; J[2] = u1[2];
+        J[3] = y1 * u1[2] - z1 * u1[1]; J[4] = z1 * u1[0] - x1 * u1[2]; J[5] = x1 * u1[1] - y1 * u1[0];
+        J[6] = -u2[0]; J[7] = -u2[1]; J[8] = -u2[2];
+        J[9] = -(y2 * u2[2] - z2 * u2[1]); J[10] = -(z2 * u2[0] - x2 * u2[2]); J[11] = -(x2 * u2[1] - y2 * u2[0]);
+        const float rf = rr;
+        int k = 0;
 #pragma unroll
-  for (int k = 0; k < NT; k++) red[k][threadIdx.x] = acc[k];
-  __syncthreads();
-  // four threads per term, 32 rows each
-  if (threadIdx.x < 4 * NT) {
-    double t = 0.0;
-    const int k = threadIdx.x >> 2, q = threadIdx.x & 3;
-#pragma unroll 8
-    for (int i = 0; i < 32; i++) t += red[k][32 * q + i];
-    red[k][32 * q] = t;
+        for (int p = 0; p < 12; p++)
+#pragma unroll
+          for (int q = p; q < 12; q++, k++) acc[k] = fmaf(J[p], J[q], acc[k]);
+#pragma unroll
+        for (int p = 0; p < 12; p++) acc[78 + p] = fmaf(J[p], rf, acc[78 + p]);
+      }
+    }
+    cost = (double)cost_f;
+  }
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (WANT_J) {
+#pragma unroll
+    for (int k = 0; k < 90; k++) {
+      double v = warp_sum((double)acc[k]);
+      if (lane == 0) sh[w][k] = v;
+    }
+    double v = warp_sum(cost);
+    if (lane == 0) sh[w][90] = v;
+  } else {
+    double v = warp_sum(cost);
+    if (lane == 0) sh[w][0] = v;
   }
   __syncthreads();
-  if (threadIdx.x < NT)
-    partial[(size_t)blockIdx.x * kNormTerms + threadIdx.x] =
-        (red[threadIdx.x][0] + red[threadIdx.x][32]) + (red[threadIdx.x][64] + red[threadIdx.x][96]);
+  const int nt = WANT_J ? kNormTerms : 1;
+  for (int k = threadIdx.x; k < nt; k += blockDim.x) {
+    double t = 0.0;
+    for (int ww = 0; ww < kIrlsThreads / 32; ww++) t += sh[ww][k];
+    partial[(size_t)blockIdx.x * kNormTerms + k] = t;
+  }
 }
 
-// per edge: sum of its blocks' partials, eight threads per term in a fixed order
-__global__ void __launch_bounds__(256) k_irls_sum(const IrlsEdge *E, int ne, int total_blocks, int nt, const double *partial,
-                                                  double *out) {
-  __shared__ double sh[8][32];
+// per edge: sum of its blocks' partials in block order
+__global__ void k_irls_sum(const IrlsEdge *E, int ne, int total_blocks, int nt, const double *partial, double *out) {
   const int e = blockIdx.x;
   if (e >= ne) return;
   const int b0 = E[e].blk0, b1 = (e + 1 < ne) ? E[e + 1].blk0 : total_blocks;
-  const int k = threadIdx.x & 31, g = threadIdx.x >> 5;
-  double t = 0.0;
-  if (k < nt)
-#pragma unroll 4
-    for (int b = b0 + g; b < b1; b += 8) t += partial[(size_t)b * kNormTerms + k];
-  sh[g][k] = t;
-  __syncthreads();
-  if (g == 0 && k < nt) {
-    for (int q = 1; q < 8; q++) t += sh[q][k];
+  for (int k = threadIdx.x; k < nt; k += blockDim.x) {
+    double t = 0.0;
+    for (int b = b0; b < b1; b++) t += partial[(size_t)b * kNormTerms + k];
     out[(size_t)e * kNormTerms + k] = t;
   }
 }
@@ -364,8 +245,6 @@ struct Normal {
   double *poses_d = nullptr;
   double *partial_d = nullptr;
   double *out_d = nullptr;
-  float *mom_d = nullptr;         // moments of every edge's rows
-  size_t mom_cap = 0;
   double *poses_pin = nullptr;    // 12 nf
   double *out_pin = nullptr;      // kNormTerms per edge
   int out_pin_edges = 0;
@@ -381,7 +260,6 @@ struct Normal {
       if (e) cudaGraphExecDestroy(e);
     cudaFree(partial_d);
     cudaFree(out_d);
-    cudaFree(mom_d);
     cudaFree(edges_d);
     cudaFree(poses_d);
     cudaFreeHost(poses_pin);
@@ -407,9 +285,9 @@ struct Normal {
     exec[w] = nullptr;
     CVO_CUDA_TRY(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t e1 = cudaMemcpyAsync(poses_d, poses_pin, sizeof(double) * 12 * nf, cudaMemcpyHostToDevice, h->stream);
-    if (want) k_irls_accum<true><<<total_blocks, 32 * kIrlsWarps, 0, h->stream>>>(edges_d, ne, poses_d, partial_d);
-    else k_irls_accum<false><<<total_blocks, 32 * kIrlsWarps, 0, h->stream>>>(edges_d, ne, poses_d, partial_d);
-    k_irls_sum<<<ne, 256, 0, h->stream>>>(edges_d, ne, total_blocks, want ? kNormTerms : 1, partial_d, out_d);
+    if (want) k_irls_accum<true><<<total_blocks, kIrlsThreads, 0, h->stream>>>(edges_d, ne, poses_d, partial_d);
+    else k_irls_accum<false><<<total_blocks, kIrlsThreads, 0, h->stream>>>(edges_d, ne, poses_d, partial_d);
+    k_irls_sum<<<ne, 128, 0, h->stream>>>(edges_d, ne, total_blocks, want ? kNormTerms : 1, partial_d, out_d);
     cudaError_t e2 = cudaMemcpyAsync(out_pin, out_d, sizeof(double) * ne * kNormTerms, cudaMemcpyDeviceToHost,
                                      h->stream);
     cudaGraph_t g = nullptr;
@@ -424,63 +302,6 @@ struct Normal {
       }
     key[w] = k;
     return 0;
-  }
-
-  // the rows' moments at the poses of the kernel matrices
-  int moments(const double *poses) {
-    if (edges.empty()) return 0;
-    memcpy(poses_pin, poses, sizeof(double) * 12 * nf);
-    CVO_CUDA_TRY(h, cudaMemcpyAsync(poses_d, poses_pin, sizeof(double) * 12 * nf, cudaMemcpyHostToDevice, h->stream));
-    k_irls_moments<<<total_blocks, 32 * kIrlsWarps, 0, h->stream>>>(edges_d, (int)edges.size(), poses_d);
-    h->launches++;
-    CVO_CUDA_TRY(h, cudaStreamSynchronize(h->stream));   // poses_pin is rewritten by the first evaluation
-    return 0;
-  }
-
-  // J^T J = B G B^T and J^T r = B [q; K q] of one edge (see k_irls_accum) into H and g
-  static void add_edge(const double *T1, const double *T2, const double *o, int o1, int o2, int D, std::vector<double> *H,
-                       std::vector<double> *g) {
-    double R12[3][3], tp[3], B[12][6] = {}, G[6][6];
-    for (int r = 0; r < 3; r++) {
-      for (int c = 0; c < 3; c++) R12[r][c] = T1[r] * T2[c] + T1[4 + r] * T2[4 + c] + T1[8 + r] * T2[8 + c];
-      tp[r] = T2[r] * (T1[3] - T2[3]) + T2[4 + r] * (T1[7] - T2[7]) + T2[8 + r] * (T1[11] - T2[11]);
-    }
-    for (int r = 0; r < 3; r++) {
-      // row r of R12 [t']x is R12's row x t'
-      const double cr[3] = {R12[r][1] * tp[2] - R12[r][2] * tp[1], R12[r][2] * tp[0] - R12[r][0] * tp[2],
-                            R12[r][0] * tp[1] - R12[r][1] * tp[0]};
-      for (int c = 0; c < 3; c++) {
-        B[r][c] = B[3 + r][3 + c] = R12[r][c];
-        B[3 + r][c] = -cr[c];
-      }
-      B[6 + r][r] = B[9 + r][3 + r] = -1.0;
-    }
-    const int tri[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
-    for (int i = 0; i < 3; i++)
-      for (int j = 0; j < 3; j++) {
-        G[i][j] = o[tri[i][j]];
-        G[i][3 + j] = G[3 + j][i] = o[6 + 3 * i + j];
-        G[3 + i][3 + j] = o[15 + tri[i][j]];
-      }
-    double BG[12][6];
-    for (int p = 0; p < 12; p++)
-      for (int j = 0; j < 6; j++) {
-        BG[p][j] = 0.0;
-        for (int k = 0; k < 6; k++) BG[p][j] += B[p][k] * G[k][j];
-      }
-    for (int p = 0; p < 12; p++) {
-      const int ip = (p < 6 ? o1 : o2) + p % 6;
-      for (int q = p; q < 12; q++) {
-        const int iq = (q < 6 ? o1 : o2) + q % 6;
-        double v = 0.0;
-        for (int k = 0; k < 6; k++) v += BG[p][k] * B[q][k];
-        (*H)[(size_t)ip * D + iq] += v;
-        if (ip != iq || p != q) (*H)[(size_t)iq * D + ip] += v;
-      }
-      double v = 0.0;
-      for (int k = 0; k < 6; k++) v += B[p][k] * o[21 + k];
-      (*g)[ip] += v;
-    }
   }
 
   // cost (and, if want, H and g over all 6 nf parameters) at `poses`
@@ -502,8 +323,16 @@ struct Normal {
     for (int e = 0; e < ne; e++) {
       const double *o = &out_h[(size_t)e * kNormTerms];
       if (!want) { *cost += o[0]; continue; }
-      *cost += o[27];
-      add_edge(poses + 12 * edges[e].f1, poses + 12 * edges[e].f2, o, 6 * edges[e].f1, 6 * edges[e].f2, D, H, g);
+      *cost += o[90];
+      int off[2] = {6 * edges[e].f1, 6 * edges[e].f2};
+      int k = 0;
+      for (int p = 0; p < 12; p++)
+        for (int q = p; q < 12; q++, k++) {
+          int ip = off[p / 6] + p % 6, iq = off[q / 6] + q % 6;
+          (*H)[(size_t)ip * D + iq] += o[k];
+          if (ip != iq || p != q) (*H)[(size_t)iq * D + ip] += o[k];
+        }
+      for (int p = 0; p < 12; p++) (*g)[off[p / 6] + p % 6] += o[78 + p];
     }
     return 0;
   }
@@ -638,17 +467,21 @@ int run_align_multi(Handle *h, int nf, DevCloud *const *clouds, double *poses, c
     for (int t = 0; t < 12 * nf; t++) fpose[t] = (float)poses[t];
     if (cudaMemcpyAsync(pose_d, fpose.data(), sizeof(float) * 12 * nf, cudaMemcpyHostToDevice, h->stream) !=
         cudaSuccess) { cleanup(); return CVO_ERR_CUDA; }
+    std::vector<float> wnorm(nf, 0.f);
     for (int f = 0; f < nf; f++) {
       int n = clouds[f]->n;
       if (n > 0) {
         k_world<<<(n + 255) / 256, 256, 0, h->stream>>>(clouds[f]->spos, n, pose_d + 12 * f, world[f]);
         h->launches++;
       }
+      double tn = std::sqrt(poses[12 * f + 3] * poses[12 * f + 3] + poses[12 * f + 7] * poses[12 * f + 7] +
+                            poses[12 * f + 11] * poses[12 * f + 11]);
+      wnorm[f] = (float)(clouds[f]->max_norm + tn) * 1.0001f;
     }
     // association of every edge in one batch
     std::vector<DevCloud *> es(ne), et(ne);
     std::vector<const float4 *> ew(ne);
-    std::vector<float> epose(12 * (size_t)ne), eell(ne);
+    std::vector<float> enorm(ne), epose(12 * (size_t)ne), eell(ne);
     for (int e = 0; e < ne; e++) {
       int f1 = edges[2 * e], f2 = edges[2 * e + 1];
       nz_last[e] = prev_nnz[e];
@@ -656,11 +489,12 @@ int run_align_multi(Handle *h, int nf, DevCloud *const *clouds, double *poses, c
       es[e] = clouds[f1];
       et[e] = clouds[f2];
       ew[e] = world[f1];
+      enorm[e] = wnorm[f1];
       for (int t = 0; t < 12; t++) epose[12 * e + t] = fpose[12 * f2 + t];
       eell[e] = (float)ell[e];
     }
     std::vector<EdgeAssoc> EA;
-    if ((rc = run_association_edges(h, es, et, ew, epose, eell, nn, init_nn, &EA, nullptr, &ag))) {
+    if ((rc = run_association_edges(h, es, et, ew, enorm, epose, eell, nn, init_nn, &EA, nullptr, &ag))) {
       cleanup();
       return rc;
     }
@@ -682,7 +516,7 @@ int run_align_multi(Handle *h, int nf, DevCloud *const *clouds, double *poses, c
         E.lim = std::min(p.nearest_neighbors_max, nn[e]);
         E.f1 = edges[2 * e]; E.f2 = edges[2 * e + 1];
         E.blk0 = blk;
-        blk += (E.n + kIrlsRows - 1) / kIrlsRows;
+        blk += (E.n + kIrlsThreads - 1) / kIrlsThreads;
         N.edges.push_back(E);
       }
     }
@@ -701,30 +535,11 @@ int run_align_multi(Handle *h, int nf, DevCloud *const *clouds, double *poses, c
         return CVO_ERR_OUT_OF_MEMORY;
       }
     }
-    size_t rows = 0;
-    for (const IrlsEdge &E : N.edges) rows += E.n;
-    if (rows > N.mom_cap) {
-      cudaFree(N.mom_d);
-      N.mom_d = nullptr;
-      N.mom_cap = 0;
-      if (cudaMalloc((void **)&N.mom_d, sizeof(float) * kMoments * rows) != cudaSuccess) {
-        cudaGetLastError();
-        cleanup();
-        return CVO_ERR_OUT_OF_MEMORY;
-      }
-      N.mom_cap = rows;
-    }
-    float *mom = N.mom_d;
-    for (IrlsEdge &E : N.edges) {
-      E.mom = mom;
-      mom += (size_t)kMoments * E.n;
-    }
     if (!N.edges.empty() && cudaMemcpyAsync(N.edges_d, N.edges.data(), sizeof(IrlsEdge) * N.edges.size(),
                                             cudaMemcpyHostToDevice, h->stream) != cudaSuccess) {
       cleanup();
       return CVO_ERR_CUDA;
     }
-    if ((rc = N.moments(poses))) { cleanup(); return rc; }
     if ((rc = lm_solve(N, nf, poses, hold, p.multiframe_iterations_per_solve, &steps))) { cleanup(); return rc; }
     double change = 0.0;
     for (int f = 0; f < nf; f++) change += pose_change(&old[12 * f], poses + 12 * f);

@@ -20,7 +20,7 @@
 
 namespace cvo_gb {
 
-enum { MODE_ALIGN = 0, MODE_IP = 1, MODE_EXPORT = 2 };
+enum { MODE_ALIGN = 0, MODE_IP = 1, MODE_EXPORT = 2, MODE_EDGES = 3 };
 constexpr int kStepThreads = 256;
 constexpr int kReduceRows = 1024;
 constexpr int kReduceThreads = 256;
@@ -466,12 +466,12 @@ __device__ __forceinline__ int warp_excl_scan(int v, int lane, int &total) {
 // (src/cvo/CvoGPU.cu:994-996): here the row stops there too, so no pair beyond cap is
 // evaluated or stored.  A row whose entries did not fit, or a call without a candidate
 // test, scans all targets in index order instead.
-// ROWS_SUM (single passes): FP32 sums per lane and row, over the lanes, FP64 from there; the
-// last block of a pair adds the blocks' sums in a fixed order.
-// ROWS_ALIGN: the entries of a row go to the order of the pair's level (RankLevel), in which
-// k_rowsum and k_step add them one by one.  The align loop turns a different last bit of the
-// gradient into a visibly different pose some tens of iterations later, so the order is part
-// of the result and is kept whatever finds the pairs.  A row with no more than cap candidates
+// Sums (all but align): FP32 per lane and row, over the lanes, FP64 from there; the last block
+// of a pair adds the blocks' sums in a fixed order.
+// ROWS_ORDERED: the entries of a row go to the order of the pair's level (RankLevel), in which
+// k_rowsum, k_step and k_irls_accum add them one by one.  The align loop and the window solve
+// turn a different last bit of the gradient into a visibly different pose some tens of
+// iterations later, so the order is part of the result and is kept whatever finds the pairs.  A row with no more than cap candidates
 // is sorted and evaluated by rank from the start; a longer one is cut by index first and its
 // kept entries are then put in order.  One that kept more than cap + order_cap pairs stays in
 // index order.
@@ -486,8 +486,9 @@ constexpr int kRowWindow = 65536;       // most target indices of one bitmap win
 constexpr int kRowQueue = 512;          // sorted candidates of one round
 constexpr int kRowSorted = 128;         // most candidates a sorting network puts in order
 
-// Whether a kernel instance serves single passes (and sums there) or the align loop.
-enum { ROWS_SUM = 0, ROWS_ALIGN = 1 };
+// Whether a kernel instance leaves the rows' entries in index order (single passes) or puts
+// them in the order of the pair's level (the align loop, the edges of a window).
+enum { ROWS_SUM = 0, ROWS_ORDERED = 1 };
 
 // Words of one warp's bitmap for targets of up to m points: an odd number per lane, so
 // that the lanes' runs start in different banks.
@@ -678,8 +679,8 @@ __global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams 
     }
     __syncthreads();
   }
-  const int order_cap = KIND == ROWS_ALIGN ? P->order_cap : 0;
-  const RankLevel *lv = KIND == ROWS_ALIGN ? P->levels + P->level : nullptr;
+  const int order_cap = KIND == ROWS_ORDERED ? P->order_cap : 0;
+  const RankLevel *lv = KIND == ROWS_ORDERED ? P->levels + P->level : nullptr;
   double row_total = 0.0;
   long long nnz = 0;
   int mx = 0;
@@ -708,9 +709,9 @@ __global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams 
     };
     // by rank from the start if the row cannot be cut; otherwise by index, and on past cap only
     // to tell whether the row keeps more than cap + order_cap
-    const bool ranked = KIND == ROWS_ALIGN && entries > 0 && cands <= cap;
+    const bool ranked = KIND == ROWS_ORDERED && entries > 0 && cands <= cap;
     const int *perm = ranked ? lv->of_tile : tperm;
-    const int stop = KIND == ROWS_ALIGN && (entries < 0 || cands > cap + order_cap) ? cap + order_cap + 1 : cap;
+    const int stop = KIND == ROWS_ORDERED && (entries < 0 || cands > cap + order_cap) ? cap + order_cap + 1 : cap;
     int kept = 0;
     float acc = 0.f;
     // 32 kept pairs to the ELL row and the sum: lane l takes slots l, l + 32, ..., so the
@@ -721,7 +722,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams 
     auto flush = [&](bool on) {
       const float4 v = keep[(flushed + lane) & 63];
       if (on) {
-        if (KIND == ROWS_ALIGN || mode != MODE_IP) {
+        if (KIND == ROWS_ORDERED || mode != MODE_IP) {
           P->A_j[(size_t)s * P->ld + flushed + lane] = keepj[(flushed + lane) & 63];
           P->A_v[(size_t)s * P->ld + flushed + lane] = v.w;
         }
@@ -841,12 +842,12 @@ __global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams 
     const int z = min(kept, cap);
     if (flushed < z) flush(lane < z - flushed);
     if (lane == 0) P->nnz_row[s] = z;
-    if (KIND == ROWS_ALIGN) {
+    if (KIND == ROWS_ORDERED) {
       if (!ranked && z > 1 && kept <= cap + order_cap && K.use_geo)
         order_row(P->A_j + (size_t)s * P->ld, P->A_v + (size_t)s * P->ld, z, lv->of_index, m, bits, window_words,
                   reinterpret_cast<unsigned short *>(queue), P->cand + (size_t)s * P->cand_pitch, lane);
       __syncwarp();
-      continue;
+      if (mode == MODE_ALIGN) continue;
     }
     nnz += z;
     mx = max(mx, z);
@@ -854,7 +855,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams 
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(FULLMASK, acc, o);
     row_total += (double)acc;
   }
-  if (KIND == ROWS_SUM) rows_finish(B, P, b, nb, row_total, nnz, mx);
+  if (KIND == ROWS_SUM || mode != MODE_ALIGN) rows_finish(B, P, b, nb, row_total, nnz, mx);
 }
 
 // Calls add(a, y) for the z entries of ELL row s in slot order.
