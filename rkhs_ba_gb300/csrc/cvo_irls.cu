@@ -50,31 +50,124 @@ struct IrlsEdge {
   int n, lim;         // rows, entries used per row
   int f1, f2;
   int blk0;           // first block of this edge
+  int row0;           // first of the edge's rows in Rows::order
 };
+
+// The rows of all edges by falling number of entries inside an edge, in tiles of 32 (four to
+// a block), and the tiles' entries as {p2, a}: entry c of tile t's lane l at
+// [32 (start[t] + c) + l].
+struct Rows {
+  const int *order;       // at row0 + i: i-th longest row of the edge
+  const int *start;       // per tile
+  const float4 *entries;  // null: read from the ELL rows
+};
+
+// The edge of a block.
+__device__ __forceinline__ int edge_of(const IrlsEdge *E, int ne, int blk) {
+  int lo = 0, hi = ne - 1;
+  while (lo < hi) {
+    int mid = (lo + hi + 1) >> 1;
+    if (E[mid].blk0 <= blk) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
+// Row of this thread (-1: none) and its number of entries.
+__device__ __forceinline__ int row_of(const IrlsEdge &ed, const int *order, int &z) {
+  const int i = ((int)blockIdx.x - ed.blk0) * kIrlsThreads + threadIdx.x;
+  const int s = i < ed.n ? __ldg(order + ed.row0 + i) : -1;
+  z = s >= 0 ? min(__ldg(&ed.nnz_row[s]), ed.lim) : 0;
+  return s;
+}
+
+// Sort keys: edge, then falling number of entries (in steps of 2^drop).
+__global__ void __launch_bounds__(kIrlsThreads) k_irls_keys(const IrlsEdge *E, int ne, int most, int drop, int bits,
+                                                            unsigned int *key, int *val) {
+  const int e = edge_of(E, ne, blockIdx.x);
+  const IrlsEdge ed = E[e];
+  const int s = ((int)blockIdx.x - ed.blk0) * kIrlsThreads + threadIdx.x;
+  if (s >= ed.n) return;
+  key[ed.row0 + s] = ((unsigned)e << bits) | (unsigned)((most - min(__ldg(&ed.nnz_row[s]), ed.lim)) >> drop);
+  val[ed.row0 + s] = s;
+}
+
+// Entries of a tile's longest row; 0 after the last tile.
+__global__ void __launch_bounds__(kIrlsThreads) k_irls_widths(const IrlsEdge *E, int ne, const int *order, int tiles, int *width) {
+  const IrlsEdge ed = E[edge_of(E, ne, blockIdx.x)];
+  int z;
+  row_of(ed, order, z);
+  z = __reduce_max_sync(0xFFFFFFFFu, z);
+  const int tile = blockIdx.x * (kIrlsThreads / 32) + (threadIdx.x >> 5);
+  if ((threadIdx.x & 31) == 0) width[tile] = z;
+  if (tile == tiles - 1 && (threadIdx.x & 31) == 0) width[tiles] = 0;
+}
+
+// The tiles' entries, once per outer iteration.  Every evaluation of the solve (some twenty)
+// then streams 16 bytes an entry with full-width loads: an evaluation that reads an index, a
+// value and a scattered point per entry is bound by the gathers (32 lines a warp load).
+__global__ void __launch_bounds__(kIrlsThreads) k_irls_pack(const IrlsEdge *E, int ne, const int *order, const int *start,
+                                                            float4 *entries) {
+  const IrlsEdge ed = E[edge_of(E, ne, blockIdx.x)];
+  int z;
+  const int s = row_of(ed, order, z);
+  if (z == 0) return;
+  float4 *out = entries + 32 * (size_t)start[blockIdx.x * (kIrlsThreads / 32) + (threadIdx.x >> 5)] + (threadIdx.x & 31);
+  const int *Aj = ed.A_j + (size_t)s * ed.ld;     // rows are 16-byte aligned, ld a multiple of 4
+  const float *Av = ed.A_v + (size_t)s * ed.ld;
+  for (int c = 0; c < z; c += 4) {
+    const int4 j = *reinterpret_cast<const int4 *>(Aj + c);
+    const float4 a = *reinterpret_cast<const float4 *>(Av + c);
+    const int jj[4] = {j.x, j.y, j.z, j.w};
+    const float aa[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (c + k < z) {
+        const float4 p = __ldg(&ed.p2[jj[k]]);
+        out[32 * (c + k)] = make_float4(p.x, p.y, p.z, aa[k]);
+      }
+  }
+}
 
 // Accumulates, per block, the cost and (WANT_J) the 12x12 J^T J and J^T r of the
 // residuals of one edge.  One thread per row; the row's point is moved with the FP64
 // poses once, every entry is then single precision (see the residual below); per-row
-// sums in FP32, block sums in FP64.
+// sums in FP32, one entry after the other, block sums in FP64.
+// The solve turns a different last bit of a row's sums into poses that differ by up to
+// 1e-4 after six outer iterations (64-bit sums in the place of these do, too), so a row
+// stays one thread's chain of additions in the order of the ELL row.
+// Bounds: issue, about 130 instructions an entry with the Jacobian.  The rows of a warp have
+// nearly equal numbers of entries (Rows); the FP64 sums over a block's rows go through shared
+// memory, one addition a row and term: as shuffle trees they cost five a lane, on a unit with
+// two lanes a clock.
+// Window of 8 frames (20k-60k points, 28 edges, 6 outer iterations): 179 -> 56 ms with the
+// tiles and one evaluation per candidate instead of two.
 template <bool WANT_J>
-__global__ void __launch_bounds__(kIrlsThreads) k_irls_accum(const IrlsEdge *E, int ne, const double *poses,
-                                                              double *partial) {
-  __shared__ double sh[kIrlsThreads / 32][kNormTerms];
-  int lo = 0, hi = ne - 1;
-  while (lo < hi) {
-    int mid = (lo + hi + 1) >> 1;
-    if (E[mid].blk0 <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
-  }
-  const IrlsEdge ed = E[lo];
-  const int s = ((int)blockIdx.x - ed.blk0) * kIrlsThreads + threadIdx.x;
+__global__ void __launch_bounds__(kIrlsThreads) k_irls_accum(const IrlsEdge *E, int ne, Rows rows, const double *poses,
+                                                             double *partial) {
   constexpr int NT = WANT_J ? kNormTerms : 1;
+  __shared__ float red[NT][kIrlsThreads + 1];
+  __shared__ double sh_T[24];
+  __shared__ float sh_R[9];
+  const IrlsEdge ed = E[edge_of(E, ne, blockIdx.x)];
+  int z;
+  const int s = row_of(ed, rows.order, z);
+  if (!__syncthreads_or(z > 0)) {
+    for (int k = threadIdx.x; k < NT; k += kIrlsThreads) partial[(size_t)blockIdx.x * kNormTerms + k] = 0.0;
+    return;
+  }
+  if (threadIdx.x < 24) sh_T[threadIdx.x] = poses[12 * (threadIdx.x < 12 ? ed.f1 : ed.f2) + threadIdx.x % 12];
+  __syncthreads();
+  const double *T1 = sh_T, *T2 = sh_T + 12;
+  if (threadIdx.x < 9) {
+    const int r = threadIdx.x / 3, c = threadIdx.x % 3;
+    sh_R[threadIdx.x] = (float)(T1[r] * T2[c] + T1[4 + r] * T2[4 + c] + T1[8 + r] * T2[8 + c]);
+  }
+  __syncthreads();
   float acc[NT];
 #pragma unroll
   for (int k = 0; k < NT; k++) acc[k] = 0.f;
-  double cost = 0.0;
-  if (s < ed.n) {
-    const double *T1 = poses + 12 * ed.f1, *T2 = poses + 12 * ed.f2;
-    const int z = min(ed.nnz_row[s], ed.lim);
+  float cost_f = 0.f;
+  if (z > 0) {
     const float4 a1 = ed.p1[s];
     // The residual vector e = T1 p1 - T2 p2 (world frame) is a difference of two points
     // tens of metres out that lie centimetres apart.  Per row, p1 is taken to the target
@@ -93,14 +186,9 @@ __global__ void __launch_bounds__(kIrlsThreads) k_irls_accum(const IrlsEdge *E, 
       ph[r] = (float)pd[r];
       pl[r] = (float)(pd[r] - (double)ph[r]);
     }
-    for (int r = 0; r < 3; r++)
-      for (int c = 0; c < 3; c++)
-        R12[3 * r + c] = (float)(T1[r] * T2[c] + T1[4 + r] * T2[4 + c] + T1[8 + r] * T2[8 + c]);
-    float cost_f = 0.f;
-    for (int c = 0; c < z; c++) {
-      const int j = ed.A_j[(size_t)s * ed.ld + c];
-      const float a = ed.A_v[(size_t)s * ed.ld + c];
-      const float4 b2 = __ldg(&ed.p2[j]);
+    for (int r = 0; r < 9; r++) R12[r] = sh_R[r];
+    auto add = [&](const float4 &b2) {      // target point, kernel value
+      const float a = b2.w;
       const float d[3] = {(ph[0] - b2.x) + pl[0], (ph[1] - b2.y) + pl[1], (ph[2] - b2.z) + pl[2]};
       const float rr = a * (d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
       cost_f = fmaf(0.5f * rr, rr, cost_f);
@@ -122,39 +210,54 @@ __global__ void __launch_bounds__(kIrlsThreads) k_irls_accum(const IrlsEdge *E, 
 #pragma unroll
         for (int p = 0; p < 12; p++) acc[78 + p] = fmaf(J[p], rf, acc[78 + p]);
       }
+    };
+    if (rows.entries) {
+      const float4 *in = rows.entries + 32 * (size_t)rows.start[blockIdx.x * (kIrlsThreads / 32) + (threadIdx.x >> 5)] +
+                         (threadIdx.x & 31);
+      float4 n0 = __ldcs(in), n1 = 1 < z ? __ldcs(in + 32) : n0;      // two entries ahead
+      for (int c = 0; c < z; c++) {
+        const float4 b2 = n0;
+        n0 = n1;
+        if (c + 2 < z) n1 = __ldcs(in + 32 * (size_t)(c + 2));
+        add(b2);
+      }
+    } else {
+      for (int c = 0; c < z; c++) {
+        const float4 p = __ldg(&ed.p2[ed.A_j[(size_t)s * ed.ld + c]]);
+        add(make_float4(p.x, p.y, p.z, ed.A_v[(size_t)s * ed.ld + c]));
+      }
     }
-    cost = (double)cost_f;
   }
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (WANT_J) {
 #pragma unroll
-    for (int k = 0; k < 90; k++) {
-      double v = warp_sum((double)acc[k]);
-      if (lane == 0) sh[w][k] = v;
-    }
-    double v = warp_sum(cost);
-    if (lane == 0) sh[w][90] = v;
-  } else {
-    double v = warp_sum(cost);
-    if (lane == 0) sh[w][0] = v;
-  }
+  for (int k = 0; k < NT - 1; k++) red[k][threadIdx.x] = acc[k];
+  red[NT - 1][threadIdx.x] = cost_f;
   __syncthreads();
-  const int nt = WANT_J ? kNormTerms : 1;
-  for (int k = threadIdx.x; k < nt; k += blockDim.x) {
-    double t = 0.0;
-    for (int ww = 0; ww < kIrlsThreads / 32; ww++) t += sh[ww][k];
-    partial[(size_t)blockIdx.x * kNormTerms + k] = t;
+  if (threadIdx.x < NT) {
+    double t[4] = {0, 0, 0, 0};
+#pragma unroll 4
+    for (int i = 0; i < kIrlsThreads / 4; i++)
+#pragma unroll
+      for (int q = 0; q < 4; q++) t[q] += (double)red[threadIdx.x][q * (kIrlsThreads / 4) + i];
+    partial[(size_t)blockIdx.x * kNormTerms + threadIdx.x] = (t[0] + t[1]) + (t[2] + t[3]);
   }
 }
 
-// per edge: sum of its blocks' partials in block order
-__global__ void k_irls_sum(const IrlsEdge *E, int ne, int total_blocks, int nt, const double *partial, double *out) {
+// per edge: sum of its blocks' partials, eight threads per term in a fixed order
+__global__ void __launch_bounds__(256) k_irls_sum(const IrlsEdge *E, int ne, int total_blocks, int nt, const double *partial,
+                                                  double *out) {
+  __shared__ double sh[8][32];
   const int e = blockIdx.x;
   if (e >= ne) return;
   const int b0 = E[e].blk0, b1 = (e + 1 < ne) ? E[e + 1].blk0 : total_blocks;
-  for (int k = threadIdx.x; k < nt; k += blockDim.x) {
-    double t = 0.0;
-    for (int b = b0; b < b1; b++) t += partial[(size_t)b * kNormTerms + k];
+  const int k = 32 * blockIdx.y + (threadIdx.x & 31), g = threadIdx.x >> 5;
+  double t = 0.0;
+  if (k < nt)
+#pragma unroll 4
+    for (int b = b0 + g; b < b1; b += 8) t += partial[(size_t)b * kNormTerms + k];
+  sh[g][threadIdx.x & 31] = t;
+  __syncthreads();
+  if (g == 0 && k < nt) {
+    for (int q = 1; q < 8; q++) t += sh[q][threadIdx.x & 31];
     out[(size_t)e * kNormTerms + k] = t;
   }
 }
@@ -245,6 +348,11 @@ struct Normal {
   double *poses_d = nullptr;
   double *partial_d = nullptr;
   double *out_d = nullptr;
+  Rows rows{nullptr, nullptr, nullptr};
+  unsigned int *rows_d = nullptr; // sort buffers of the rows, tile widths and starts
+  size_t rows_cap = 0;
+  float4 *entries_d = nullptr;
+  size_t entries_cap = 0;         // tile entries (32 float4 each)
   double *poses_pin = nullptr;    // 12 nf
   double *out_pin = nullptr;      // kNormTerms per edge
   int out_pin_edges = 0;
@@ -261,6 +369,8 @@ struct Normal {
     cudaFree(partial_d);
     cudaFree(out_d);
     cudaFree(edges_d);
+    cudaFree(rows_d);
+    cudaFree(entries_d);
     cudaFree(poses_d);
     cudaFreeHost(poses_pin);
     cudaFreeHost(out_pin);
@@ -280,14 +390,16 @@ struct Normal {
     add(&total_blocks, sizeof(total_blocks));
     add(&nf, sizeof(nf));
     add(&h->stream, sizeof(h->stream));
+    add(&rows, sizeof(rows));
     if (exec[w] && key[w] == k) return 0;
     if (exec[w]) cudaGraphExecDestroy(exec[w]);
     exec[w] = nullptr;
     CVO_CUDA_TRY(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t e1 = cudaMemcpyAsync(poses_d, poses_pin, sizeof(double) * 12 * nf, cudaMemcpyHostToDevice, h->stream);
-    if (want) k_irls_accum<true><<<total_blocks, kIrlsThreads, 0, h->stream>>>(edges_d, ne, poses_d, partial_d);
-    else k_irls_accum<false><<<total_blocks, kIrlsThreads, 0, h->stream>>>(edges_d, ne, poses_d, partial_d);
-    k_irls_sum<<<ne, 128, 0, h->stream>>>(edges_d, ne, total_blocks, want ? kNormTerms : 1, partial_d, out_d);
+    if (want) k_irls_accum<true><<<total_blocks, kIrlsThreads, 0, h->stream>>>(edges_d, ne, rows, poses_d, partial_d);
+    else k_irls_accum<false><<<total_blocks, kIrlsThreads, 0, h->stream>>>(edges_d, ne, rows, poses_d, partial_d);
+    const int nt = want ? kNormTerms : 1;
+    k_irls_sum<<<dim3(ne, (nt + 31) / 32), 256, 0, h->stream>>>(edges_d, ne, total_blocks, nt, partial_d, out_d);
     cudaError_t e2 = cudaMemcpyAsync(out_pin, out_d, sizeof(double) * ne * kNormTerms, cudaMemcpyDeviceToHost,
                                      h->stream);
     cudaGraph_t g = nullptr;
@@ -301,6 +413,62 @@ struct Normal {
         return set_cuda_error(h, e, "normal-equation graph capture");
       }
     key[w] = k;
+    return 0;
+  }
+
+  // Orders the rows and lays out their entries for the evaluations of one solve (the edges
+  // are in edges_d).  Entries beyond 32 GB, or beyond the device's memory, are left out:
+  // the evaluations then read the ELL rows.
+  int prepare() {
+    const int ne = (int)edges.size();
+    rows = Rows{nullptr, nullptr, nullptr};
+    if (ne == 0) return 0;
+    const int tiles = total_blocks * (kIrlsThreads / 32);
+    int n = 0, most = 0, bits = 1, edge_bits = 0;
+    for (const IrlsEdge &E : edges) {
+      n += E.n;
+      most = std::max(most, E.lim);
+    }
+    while (bits < 31 && (1 << bits) <= most) bits++;
+    while ((1 << edge_bits) < ne) edge_bits++;
+    const int drop = std::max(0, bits + edge_bits - 32);
+    bits -= drop;
+    const size_t scratch = scan_scratch_ints(tiles + 1), words = 4 * (size_t)n + 2 * (size_t)(tiles + 1) + scratch;
+    if (words > rows_cap) {
+      cudaFree(rows_d);
+      rows_d = nullptr;
+      rows_cap = 0;
+      CVO_CUDA_TRY(h, cudaMalloc((void **)&rows_d, sizeof(int) * words));
+      rows_cap = words;
+    }
+    unsigned int *key = rows_d, *key_tmp = key + n;
+    int *val = reinterpret_cast<int *>(key_tmp + n), *val_tmp = val + n, *width = val_tmp + n, *start = width + tiles + 1;
+    k_irls_keys<<<total_blocks, kIrlsThreads, 0, h->stream>>>(edges_d, ne, most, drop, bits, key, val);
+    if (int rc = radix_sort_pairs(h, key, val, key_tmp, val_tmp, n, bits + edge_bits)) return rc;
+    k_irls_widths<<<total_blocks, kIrlsThreads, 0, h->stream>>>(edges_d, ne, val, tiles, width);
+    exclusive_scan_int(h, width, start, tiles + 1, start + tiles + 1, (int)scratch);
+    int total = 0;
+    CVO_CUDA_TRY(h, cudaMemcpyAsync(&total, start + tiles, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    CVO_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+    h->launches += 2;
+    rows.order = val;
+    rows.start = start;
+    constexpr size_t kMost = (32ull << 30) / (32 * sizeof(float4));
+    if ((size_t)total > entries_cap) {
+      cudaFree(entries_d);
+      entries_d = nullptr;
+      entries_cap = 0;
+      const size_t want = std::min(kMost, total + (size_t)total / 8);      // later iterations keep some pairs more
+      if ((size_t)total <= kMost) {
+        if (cudaMalloc((void **)&entries_d, 32 * sizeof(float4) * want) == cudaSuccess) entries_cap = want;
+        else cudaGetLastError();
+      }
+    }
+    if (entries_d && (size_t)total <= entries_cap) {
+      k_irls_pack<<<total_blocks, kIrlsThreads, 0, h->stream>>>(edges_d, ne, rows.order, rows.start, entries_d);
+      h->launches++;
+      rows.entries = entries_d;
+    }
     return 0;
   }
 
@@ -345,11 +513,15 @@ int lm_solve(Normal &N, int nf, double *poses, const uint8_t *hold, int max_iter
   int nfree = 0;
   for (int f = 0; f < nf; f++)
     for (int k = 0; k < 6; k++) idx[6 * f + k] = hold[f] ? -1 : nfree++;
-  std::vector<double> H, g, Hf((size_t)std::max(nfree, 1) * std::max(nfree, 1)), gf(std::max(nfree, 1)), A, b,
+  std::vector<double> H, g, Hn, gn, Hf((size_t)std::max(nfree, 1) * std::max(nfree, 1)), gf(std::max(nfree, 1)), A, b,
       cand(12 * (size_t)nf);
   double radius = 1e4, nu = 2.0, cost = 0.0;
   int rc = N.eval(poses, true, &H, &g, &cost);
   if (rc) return rc;
+  // A candidate is evaluated with its normal equations: nearly all are accepted and need them
+  // next, and the cost alone takes about half as long.  After a rejected one (the radius is
+  // being reduced) the cost comes first.
+  bool with_equations = true;
   for (int it = 0; it < max_iter && nfree > 0; it++) {
     for (int i = 0; i < D; i++) {
       if (idx[i] < 0) continue;
@@ -389,7 +561,7 @@ int lm_solve(Normal &N, int nf, double *poses, const uint8_t *hold, int max_iter
       compose(poses + 12 * f, X, &cand[12 * f]);
     }
     double cnew = 0.0;
-    if ((rc = N.eval(cand.data(), false, nullptr, nullptr, &cnew))) return rc;
+    if ((rc = N.eval(cand.data(), with_equations, &Hn, &gn, &cnew))) return rc;
     double rho = model > 0.0 ? (cost - cnew) / model : -1.0;
     if (rho > 1e-3) {
       memcpy(poses, cand.data(), sizeof(double) * 12 * nf);
@@ -401,8 +573,15 @@ int lm_solve(Normal &N, int nf, double *poses, const uint8_t *hold, int max_iter
       bool stop = rel <= 1e-5 * cost;
       cost = cnew;
       if (stop) break;
-      if ((rc = N.eval(poses, true, &H, &g, &cost))) return rc;
+      if (with_equations) {
+        H.swap(Hn);
+        g.swap(gn);
+      } else if ((rc = N.eval(poses, true, &H, &g, &cost))) {
+        return rc;
+      }
+      with_equations = true;
     } else {
+      with_equations = false;
       radius /= nu;
       nu *= 2.0;
     }
@@ -500,7 +679,7 @@ int run_align_multi(Handle *h, int nf, DevCloud *const *clouds, double *poses, c
     }
     int counter = 0;
     N.edges.clear();
-    int blk = 0;
+    int blk = 0, row = 0;
     for (int e = 0; e < ne; e++) {
       prev_nnz[e] = EA[e].nnz;
       prev_max[e] = EA[e].max_row;
@@ -516,6 +695,8 @@ int run_align_multi(Handle *h, int nf, DevCloud *const *clouds, double *poses, c
         E.lim = std::min(p.nearest_neighbors_max, nn[e]);
         E.f1 = edges[2 * e]; E.f2 = edges[2 * e + 1];
         E.blk0 = blk;
+        E.row0 = row;
+        row += E.n;
         blk += (E.n + kIrlsThreads - 1) / kIrlsThreads;
         N.edges.push_back(E);
       }
@@ -540,6 +721,7 @@ int run_align_multi(Handle *h, int nf, DevCloud *const *clouds, double *poses, c
       cleanup();
       return CVO_ERR_CUDA;
     }
+    if ((rc = N.prepare())) { cleanup(); return rc; }
     if ((rc = lm_solve(N, nf, poses, hold, p.multiframe_iterations_per_solve, &steps))) { cleanup(); return rc; }
     double change = 0.0;
     for (int f = 0; f < nf; f++) change += pose_change(&old[12 * f], poses + 12 * f);
