@@ -206,6 +206,7 @@ KParams adaptive_kparams(const cvo_params &p) {
   q.is_using_geometry = 1;       // the distance gate is unconditional on this path
   KParams k = make_kparams(q);
   k.use_gtype = 0;               // no geometric-type factor
+  k.sure_tau = 0.f;              // thresholds of this path's own
   k.d2_s_thres = INFINITY;       // no semantic gate
   if (k.use_int)
     k.d2_c_thres = (float)(-2.0 * (double)p.c_ell * (double)p.c_ell * (double)logf(p.sp_thres / p.c_sigma / p.c_sigma));

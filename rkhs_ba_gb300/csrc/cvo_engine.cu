@@ -21,6 +21,88 @@ namespace {
 
 constexpr int kChunk = 8;
 
+// ------------------------------------------------------------- transform
+// Writes the transformed targets twice: in tile order (read by k_cand) and in
+// original order (gathered by index by k_rows and k_step).
+__global__ void k_transform(BatchDev B) {
+  int gt = blockIdx.x * blockDim.x + threadIdx.x;
+  if (gt == 0 && *B.active > 0) *B.active_iters += 1;
+  if (gt >= B.total_targets) return;
+  int p = find_segment(B.tgt_off, B.npairs, gt);
+  PairDev *P = &B.pairs[p];
+  if (P->done) return;
+  int t = gt - B.tgt_off[p];
+  float4 y = __ldg(&P->tpos[t]);
+  float o0 = xform_row(&P->Ri[0], P->Ti[0], y.x, y.y, y.z);
+  float o1 = xform_row(&P->Ri[3], P->Ti[1], y.x, y.y, y.z);
+  float o2 = xform_row(&P->Ri[6], P->Ti[2], y.x, y.y, y.z);
+  float4 o = make_float4(o0, o1, o2, 0.f);
+  P->ycur[t] = o;
+  P->yorig[__ldg(&P->tperm[t])] = o;
+}
+
+// ---------------------------------------------------------------- row sums
+// Calls add(a, y) for the z entries of ELL row s in slot order.
+template <class Add>
+__device__ __forceinline__ void row_entries(const PairDev *P, int s, int z, Add add) {
+  const int *__restrict__ Aj = P->A_j + (size_t)s * P->ld;
+  const float *__restrict__ Av = P->A_v + (size_t)s * P->ld;
+  const float4 *__restrict__ yorig = P->yorig;
+  int c = 0;
+  if (z >= 8) {
+    int4 j0 = *reinterpret_cast<const int4 *>(Aj), j1 = *reinterpret_cast<const int4 *>(Aj + 4);
+    for (; c + 8 <= z; c += 8) {
+      const float4 y0 = __ldg(&yorig[j0.x]), y1 = __ldg(&yorig[j0.y]), y2 = __ldg(&yorig[j0.z]), y3 = __ldg(&yorig[j0.w]);
+      const float4 y4 = __ldg(&yorig[j1.x]), y5 = __ldg(&yorig[j1.y]), y6 = __ldg(&yorig[j1.z]), y7 = __ldg(&yorig[j1.w]);
+      const float4 a = *reinterpret_cast<const float4 *>(Av + c), b = *reinterpret_cast<const float4 *>(Av + c + 4);
+      if (c + 16 <= z) {
+        j0 = *reinterpret_cast<const int4 *>(Aj + c + 8);
+        j1 = *reinterpret_cast<const int4 *>(Aj + c + 12);
+      }
+      add(a.x, y0); add(a.y, y1); add(a.z, y2); add(a.w, y3);
+      add(b.x, y4); add(b.y, y5); add(b.z, y6); add(b.w, y7);
+    }
+  }
+  if (c + 4 <= z) {
+    const int4 j = *reinterpret_cast<const int4 *>(Aj + c);
+    const float4 a = *reinterpret_cast<const float4 *>(Av + c);
+    const float4 y0 = __ldg(&yorig[j.x]), y1 = __ldg(&yorig[j.y]), y2 = __ldg(&yorig[j.z]), y3 = __ldg(&yorig[j.w]);
+    add(a.x, y0); add(a.y, y1); add(a.z, y2); add(a.w, y3);
+    c += 4;
+  }
+  for (; c < z; c++) add(Av[c], __ldg(&yorig[Aj[c]]));
+}
+
+// Row partials of the align loop from the final ELL entries, one after the other in slot
+// order (thread per row): omega = sum a (x cross y), v = sum a (y - x), sum a
+// (CvoGPU.cu:2001-2062 computes the same sums from the sparse kernel matrix).  The order is
+// part of the result (see k_rows), so a row is one thread's chain of additions; the loads
+// run ahead of it: eight entries' indices one step, their targets' positions in one batch.
+// Bounds: L2 latency of index -> position, one round trip per eight entries.
+__global__ void __launch_bounds__(128) k_rowsum(BatchDev B, KParams K) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= B.total_rows) return;
+  const int p = find_segment(B.row_off, B.npairs, g);
+  const PairDev *P = &B.pairs[p];
+  if (P->done) return;
+  const int s = g - B.row_off[p];
+  const int z = P->nnz_row[s];
+  const float4 x = __ldg(&P->xs[s]);
+  float w0 = 0.f, w1 = 0.f, w2 = 0.f, v0 = 0.f, v1 = 0.f, v2 = 0.f, as = 0.f;
+  row_entries(P, s, z, [&](float a, const float4 &y) {
+    w0 = fmaf(a, fs(fm(x.y, y.z), fm(x.z, y.y)), w0);
+    w1 = fmaf(a, fs(fm(x.z, y.x), fm(x.x, y.z)), w1);
+    w2 = fmaf(a, fs(fm(x.x, y.y), fm(x.y, y.x)), w2);
+    v0 = fmaf(a, y.x - x.x, v0);
+    v1 = fmaf(a, y.y - x.y, v1);
+    v2 = fmaf(a, y.z - x.z, v2);
+    as += a;
+  });
+  float4 *rs = reinterpret_cast<float4 *>(P->row_sums + (size_t)s * 8);
+  rs[0] = make_float4(__fdiv_rn(w0, K.c), __fdiv_rn(w1, K.c), __fdiv_rn(w2, K.c), __fdiv_rn(v0, K.d));
+  rs[1] = make_float4(__fdiv_rn(v1, K.d), __fdiv_rn(v2, K.d), as, 0.f);
+}
+
 // ------------------------------------------------------------------ reduce
 // Sums of columns 0 .. NV-1 of the blocks' partials, each from block 0 upwards by one thread
 // (the order is part of the result); all threads bring the partials to shared memory first,
@@ -318,43 +400,15 @@ __global__ void k_export(const PairDev *P, const int *row_start, int *cols, floa
 }
 
 // --------------------------------------------------------- template dispatch
-using CandFn = void (*)(BatchDev, KParams);
-using RowsFn = void (*)(BatchDev, KParams, int);
-
-struct AssocKernels {
-  CandFn cand = nullptr;
-  RowsFn rows = nullptr, ordered_rows = nullptr;
-};
-
-// Feature rows are stored as ceil(F/4) float4 chunks; label rows as 5 or 9
-// chunks (C <= 20 or C <= 36, padded at upload), so the chunk counts below are
-// the storage strides of the clouds.
-template <int FC, int LC, bool G>
-static int pick_assoc(AssocKernels *a) {
-  a->cand = k_cand<FC>;
-  a->rows = k_rows<FC, LC, G, ROWS_SUM>;
-  a->ordered_rows = k_rows<FC, LC, G, ROWS_ORDERED>;
-  // opt in above the 48 KB default (setting it again is harmless)
-  for (RowsFn f : {a->rows, a->ordered_rows})
-    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem_bytes(kRowWindow)) != cudaSuccess) {
-      cudaGetLastError();
-      return CVO_ERR_CUDA;
-    }
-  return 0;
-}
-
 int select_kernels(const KParams &K, int F, int C, AssocKernels *a) {
   int fch = K.use_int ? (F + 3) / 4 : 0;
   int lch = K.use_sem ? label_chunks(C) : 0;
   bool gt = K.use_gtype != 0;
   if (fch > 2 || lch > 9) return CVO_ERR_UNSUPPORTED;
-#define CVO_PICK(FC, LC) \
-  if (fch == FC && lch == LC) return gt ? pick_assoc<FC, LC, true>(a) : pick_assoc<FC, LC, false>(a);
-  CVO_PICK(0, 0) CVO_PICK(1, 0) CVO_PICK(2, 0)
-  CVO_PICK(0, 5) CVO_PICK(1, 5) CVO_PICK(2, 5)
-  CVO_PICK(0, 9) CVO_PICK(1, 9) CVO_PICK(2, 9)
-#undef CVO_PICK
-  return CVO_ERR_UNSUPPORTED;
+  // the feature and label chunk counts are the storage strides of the clouds
+  if (lch == 0) return assoc_kernels_no_labels(fch, gt, a);
+  if (lch == 5) return assoc_kernels_labels5(fch, gt, a);
+  return lch == 9 ? assoc_kernels_labels9(fch, gt, a) : CVO_ERR_UNSUPPORTED;
 }
 
 // ------------------------------------------------------------ device arena
@@ -460,6 +514,12 @@ KParams make_kparams(const cvo_params &p) {
     if (k.val_scale > 0.f) lb += std::log((double)k.val_scale);
     k.mma_tau = (float)(lb + 1e-3);
     k.use_mma = 1;
+    // below this the value and each of its terms pass their thresholds
+    if (!k.use_sem && !k.use_gtype) {
+      if (k.use_geo) lb = std::min(lb, -(double)k.log_geo);
+      if (k.use_int) lb = std::min(lb, (double)k.d2_c_thres * (double)k.inv2c2);
+      k.sure_tau = (float)(lb - 2e-3);
+    }
   }
   return k;
 }
@@ -503,6 +563,7 @@ struct BatchHost {
   int cand_blocks = 0, xform_blocks = 0;
   int window_words = 0;
   size_t row_smem = 0;
+  bool split_rows = false;          // rows of few candidates in a launch of their own
   bool ordered = false;             // rows in the order of the targets' lattice (RankLevel)
 };
 
@@ -617,7 +678,7 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     add(sizeof(RankLevel) * lv[p].size());
     add(sizeof(int2) * (size_t)n * sp[p]);                       // entry counts
     add(sizeof(int) * n);                                        // nnz_row
-    add(sizeof(double) * kPartStride * (size_t)std::max(rb, sb)); // partials
+    add(sizeof(double) * kPartStride * (size_t)std::max(kRowSlots * rb, sb)); // partials
     add(sizeof(unsigned) * 2);
     bytes += 12 * 256;                                           // room for empty pieces
   }
@@ -652,7 +713,7 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     P.tf = t->feat; P.tl = t->lab; P.tg = t->geo;
     P.nnz_row = ar.take<int>(s->n);
     int rb = bh->rblk_off[p + 1] - bh->rblk_off[p], sb = bh->sblk_off[p + 1] - bh->sblk_off[p];
-    P.part = ar.take<double>(kPartStride * (size_t)std::max(rb, sb));
+    P.part = ar.take<double>(kPartStride * (size_t)std::max(kRowSlots * rb, sb));
     P.counter = ar.take<unsigned>(2);
     P.capmax = capmax;
     P.mode = mode;
@@ -669,7 +730,7 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     }
     P.ell = ell0[p];
     P.cap = capmax;
-    P.order_cap = order_cap;
+    P.order_cap = bh->ordered ? order_cap : 0;
     P.src_norm = s->max_norm;
     if (mode == MODE_ALIGN) P.row_sums = ar.take<float>(8 * (size_t)s->n);
     if (bh->ordered) {
@@ -725,6 +786,7 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
   bh->xform_blocks = (B.total_targets + 255) / 256;
   bh->window_words = row_window_words(maxm);
   bh->row_smem = row_smem_bytes(maxm);
+  bh->split_rows = K.use_mma && maxm > kRowSplitTargets;
   return 0;
 }
 
@@ -747,8 +809,13 @@ void launch_association(Handle *h, BatchHost *bh, const KParams &K, bool align =
     h->launches++;
   }
   mark(h, ev, 5);
-  const RowsFn rows = bh->ordered ? bh->fn.ordered_rows : bh->fn.rows;
-  rows<<<std::max(B.total_rblocks, 1), 32 * kRowWarps, bh->row_smem, h->stream>>>(B, K, bh->window_words);
+  const RowsFn *rows = bh->ordered ? bh->fn.ordered_rows : bh->fn.rows;
+  const int split = bh->split_rows ? 1 : 0, blocks = std::max(B.total_rblocks, 1);
+  if (split) {
+    rows[ROWS_LIGHT]<<<blocks, 32 * kRowWarps, sizeof(int) * kRowSorted * kRowWarps, h->stream>>>(B, K, 0, 1);
+    h->launches++;
+  }
+  rows[ROWS_ALL]<<<blocks * (kRowsPerBlock / kRowsHeavy), 32 * kRowWarps, bh->row_smem, h->stream>>>(B, K, bh->window_words, split);
   h->launches += 2;
   mark(h, ev, 6);
   if (align) {
@@ -780,6 +847,7 @@ void append_launch_key(const Handle *h, const BatchHost &bh, const KParams &K, s
   add(&bh.xform_blocks, sizeof(bh.xform_blocks));
   add(&bh.window_words, sizeof(bh.window_words));
   add(&bh.row_smem, sizeof(bh.row_smem));
+  add(&bh.split_rows, sizeof(bh.split_rows));
   add(&h->stream, sizeof(h->stream));
 }
 

@@ -81,6 +81,8 @@ struct KParams {
   // (mma_tau = ln(sigma^2 c_sigma^2 s_sigma^2 / sp_thres) + slack), see k_cand.
   float mma_tau;
   int use_mma;
+  // Pairs with the exponent below this are kept (0: semantic or geometric-type terms decide, too).
+  float sure_tau;
   // Value scale (1 on the two-view path; c_sigma for the adaptive path's geometric-only
   // values s^2 exp(-d2/2l^2) c_sigma) and the colour denominator 2 c_ell^2 of the exact
   // (double) value as each path rounds it.
@@ -107,8 +109,8 @@ struct PairDev {
   int *A_j; float *A_v;           // ELL, row-major: entry c of row s at [s * ld + c] (original target index)
   int ld;                         // ELL row pitch (capmax rounded up to a multiple of 4)
   // candidates: entry e of split q of row s at [s * cand_pitch + q * cap_split + e] =
-  // {group, bits of its 32 points}; cand_cnt[q * n + s] = {entries, candidates} (more than
-  // cap_split entries: not all stored)
+  // {group, bits of its 32 points}; cand_cnt[q * n + s] = {entries and pairs surely kept,
+  // candidates} (see kSureShift; more than cap_split entries: not all stored)
   uint2 *cand;
   int2 *cand_cnt;
   int splits, cap_split, cand_pitch;
@@ -167,6 +169,19 @@ struct BatchDev {
   double *assoc_bytes;            // algorithmic bytes of the association passes
   int record_bytes;               // packed bytes of one target record
 };
+
+// Kernels of the association for a batch's feature and label strides (cvo_assoc_*.cu).
+using CandFn = void (*)(BatchDev, KParams);
+using RowsFn = void (*)(BatchDev, KParams, int, int);
+
+struct AssocKernels {
+  CandFn cand = nullptr;
+  RowsFn rows[2] = {nullptr, nullptr}, ordered_rows[2] = {nullptr, nullptr};      // ROWS_ALL, ROWS_LIGHT
+};
+
+int assoc_kernels_no_labels(int fch, bool gt, AssocKernels *a);
+int assoc_kernels_labels5(int fch, bool gt, AssocKernels *a);
+int assoc_kernels_labels9(int fch, bool gt, AssocKernels *a);
 
 // ------------------------------------------------------------- host side
 struct Workspace;

@@ -105,26 +105,6 @@ __device__ __forceinline__ RowConst row_const(const KParams &K, float ell, float
   return rc;
 }
 
-// ------------------------------------------------------------- transform
-// Writes the transformed targets twice: in tile order (read by k_cand) and in
-// original order (gathered by index by k_rows and k_step).
-__global__ void k_transform(BatchDev B) {
-  int gt = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gt == 0 && *B.active > 0) *B.active_iters += 1;
-  if (gt >= B.total_targets) return;
-  int p = find_segment(B.tgt_off, B.npairs, gt);
-  PairDev *P = &B.pairs[p];
-  if (P->done) return;
-  int t = gt - B.tgt_off[p];
-  float4 y = __ldg(&P->tpos[t]);
-  float o0 = xform_row(&P->Ri[0], P->Ti[0], y.x, y.y, y.z);
-  float o1 = xform_row(&P->Ri[3], P->Ti[1], y.x, y.y, y.z);
-  float o2 = xform_row(&P->Ri[6], P->Ti[2], y.x, y.y, y.z);
-  float4 o = make_float4(o0, o1, o2, 0.f);
-  P->ycur[t] = o;
-  P->yorig[__ldg(&P->tperm[t])] = o;
-}
-
 // ---------------------------------------------------------- candidate test
 // A kept pair satisfies  u = g_s |x - y|^2 + c |xc - yc|^2 < tau  with
 // g_s = 1/(2 l_s^2), c = 1/(2 c_ell^2), tau = ln(sigma^2 c_sigma^2 s_sigma^2 / sp_thres)
@@ -141,8 +121,15 @@ __global__ void k_transform(BatchDev B) {
 // of the accumulator is the answer.  The bound is within 1-2 % of tau for tiles a few
 // lengthscales wide.  Only candidates go through the exact per-pair arithmetic
 // (eval_pair), so the kernel matrix does not depend on the test.
+// The same accumulators answer the opposite question: |a^ - b^|^2 below
+//   (sqrt(tau') - 2^-11 (2 A + sqrt(tau)))^2 - rounding,   tau' = K.sure_tau g_min / g_max,
+// means that the pair is kept (no term but position and colour, and u below the thresholds of
+// both: K.sure_tau > 0).  k_cand counts such pairs of dense groups, see k_rows.
 constexpr float kCandWide = 200.f;      // largest |a^| the f16 squares serve
 constexpr float kCandFar = 60000.f;     // |b^|^2 beyond which a candidate is rejected outright
+// cand_cnt's x: entries (a row has at most 2^17, one per target group), then the pairs that are
+// surely kept, as far as they were counted
+constexpr int kSureShift = 18, kSureMost = (1 << 13) - 1;
 
 __device__ __forceinline__ float f4_at(const float4 &v, int i) {
   return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w));
@@ -159,12 +146,12 @@ __device__ __forceinline__ void ldsm_x4(const void *p, uint32_t &r0, uint32_t &r
                : "memory");
 }
 
-__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, float c) {
   asm volatile(
       "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
       "{%10, %10, %10, %10};\n"
       : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c));
 }
 
 // The operand of one point: scaled coordinates v[11] rounded to f16, and the four
@@ -233,7 +220,7 @@ __device__ __forceinline__ bool box_near(const float4 *box, int count, int i, co
 constexpr int kCandWarps = 4;
 
 template <int FCH>
-__global__ void __launch_bounds__(32 * kCandWarps) k_cand(BatchDev B, KParams K) {
+__global__ void __launch_bounds__(32 * kCandWarps, 4) k_cand(BatchDev B, KParams K) {
   __shared__ __align__(16) uint4 apl_all[kCandWarps][2][32];
   __shared__ __align__(16) uint4 bpl_all[kCandWarps][2][32];
   constexpr int FP = FCH > 0 ? FCH : 1;
@@ -291,6 +278,7 @@ __global__ void __launch_bounds__(32 * kCandWarps) k_cand(BatchDev B, KParams K)
   const float sg = sqrtf(g), sc = sqrtf(cw);
   // the rows' operands
   bool wide, spread;
+  float sure_at = INFINITY;      // accumulators below -sure_at are kept pairs
   {
     float v[11];
     cand_coords<FCH>(v, x, xf, pc, fc, sg, sc);
@@ -305,10 +293,14 @@ __global__ void __launch_bounds__(32 * kCandWarps) k_cand(BatchDev B, KParams K)
     }
     const float A = sqrtf(warp_fmax(sa)), rt = sqrtf(fmaxf(tau, 0.f));
     wide = !(A <= kCandWide);
+    const float lmin = -warp_fmax(-l), rs = K.use_geo ? lmin / lmax : 1.f;
+    const float rv = sqrtf(fmaxf(K.sure_tau, 0.f)) * rs - 4.95e-4f * (2.f * A + rt) - 2e-6f;
     spread = K.use_geo && A > 3.f * rt;
     const float reach = 2.f * A + rt;
     const float rb = rt + 4.95e-4f * reach + 2e-6f;
     const float bound = rb * rb * 1.00001f + 4e-6f * reach * reach + 1e-6f;
+    const float inner = rv * rv * 0.9999f - 4e-6f * reach * reach - 1e-6f;
+    if (P->order_cap > 0 && K.sure_tau > 0.f && rv > 0.f && inner > 0.f) sure_at = bound - inner;
     const float d = valid ? sa - bound : kCandFar;
     const __half hi = __float2half_rn(d), one = __float2half_rn(1.f);
     cand_store(h, hi, __float2half_rn(d - __half2float(hi)), one, one, apl, lane);
@@ -322,7 +314,7 @@ __global__ void __launch_bounds__(32 * kCandWarps) k_cand(BatchDev B, KParams K)
   const int caps = P->cap_split;
   uint2 *out = P->cand + (size_t)si * P->cand_pitch + (size_t)sp * caps;
   const int ng = P->groups, ns = (ng + 31) >> 5;
-  int cnt = 0, cands = 0;
+  int cnt = 0, cands = 0, sure = 0;
   const int my_col = cand_col(lane);
   const int src0 = 4 * (lane & 7);
   const uint32_t sel = (uint32_t)(lane >> 3) | ((uint32_t)((lane >> 3) + 4) << 4);
@@ -394,28 +386,39 @@ __global__ void __launch_bounds__(32 * kCandWarps) k_cand(BatchDev B, KParams K)
           uint32_t b0[4], b1[4];
           ldsm_x4(&bpl[(lane >> 3) & 1][8 * (lane >> 4) + (lane & 7)], b0[0], b0[1], b0[2], b0[3]);
           ldsm_x4(&bpl[(lane >> 3) & 1][16 + 8 * (lane >> 4) + (lane & 7)], b1[0], b1[1], b1[2], b1[3]);
-          uint32_t wb[4];      // byte 2 mm + hh: rows 16 mm + 8 hh + lane / 4
+          // signs of the accumulators plus `at`: byte 2 mm + hh of a lane's word holds its
+          // columns of row 16 mm + 8 hh + lane / 4
+          auto signs = [&](float at) {
+            uint32_t wb[4];
 #pragma unroll
-          for (int mm = 0; mm < 2; mm++) {
-            uint32_t w0 = 0, w1 = 0;
+            for (int mm = 0; mm < 2; mm++) {
+              uint32_t w0 = 0, w1 = 0;
 #pragma unroll
-            for (int nn = 0; nn < 4; nn++) {
-              float d[4];
-              mma_16816(d, af[mm], nn < 2 ? b0[2 * nn] : b1[2 * nn - 4], nn < 2 ? b0[2 * nn + 1] : b1[2 * nn - 3]);
-              w0 = __funnelshift_l(__float_as_uint(d[0]), w0, 1);
-              w0 = __funnelshift_l(__float_as_uint(d[1]), w0, 1);
-              w1 = __funnelshift_l(__float_as_uint(d[2]), w1, 1);
-              w1 = __funnelshift_l(__float_as_uint(d[3]), w1, 1);
+              for (int nn = 0; nn < 4; nn++) {
+                float d[4];
+                mma_16816(d, af[mm], nn < 2 ? b0[2 * nn] : b1[2 * nn - 4], nn < 2 ? b0[2 * nn + 1] : b1[2 * nn - 3], at);
+                w0 = __funnelshift_l(__float_as_uint(d[0]), w0, 1);
+                w0 = __funnelshift_l(__float_as_uint(d[1]), w0, 1);
+                w1 = __funnelshift_l(__float_as_uint(d[2]), w1, 1);
+                w1 = __funnelshift_l(__float_as_uint(d[3]), w1, 1);
+              }
+              wb[2 * mm] = w0;
+              wb[2 * mm + 1] = w1;
             }
-            wb[2 * mm] = w0;
-            wb[2 * mm + 1] = w1;
-          }
-          const uint32_t word = __byte_perm(__byte_perm(wb[0], wb[1], 0x0040), __byte_perm(wb[2], wb[3], 0x0040), 0x5410);
-          if (!__any_sync(FULLMASK, word != 0)) continue;
-          uint32_t q4[4];
+            return __byte_perm(__byte_perm(wb[0], wb[1], 0x0040), __byte_perm(wb[2], wb[3], 0x0040), 0x5410);
+          };
+          // the word of row `lane`: its 32 columns in the candidates' order
+          auto row_mask = [&](uint32_t word) {
+            uint32_t q4[4];
 #pragma unroll
-          for (int t = 0; t < 4; t++) q4[t] = __shfl_sync(FULLMASK, word, src0 + t);
-          mask = __byte_perm(__byte_perm(q4[0], q4[1], sel), __byte_perm(q4[2], q4[3], sel), 0x5410);
+            for (int t = 0; t < 4; t++) q4[t] = __shfl_sync(FULLMASK, word, src0 + t);
+            return __byte_perm(__byte_perm(q4[0], q4[1], sel), __byte_perm(q4[2], q4[3], sel), 0x5410);
+          };
+          const uint32_t word = signs(0.f);
+          if (!__any_sync(FULLMASK, word != 0)) continue;
+          mask = row_mask(word);
+          // rows of thousands of candidates are made of dense groups
+          if (sure_at < INFINITY && __any_sync(FULLMASK, __popc(mask) >= 16)) sure += __popc(row_mask(signs(sure_at)));
         } else {
           // a tile many lengthscales wide: the same test in FP32, candidate by candidate
 #pragma unroll 1
@@ -443,7 +446,7 @@ __global__ void __launch_bounds__(32 * kCandWarps) k_cand(BatchDev B, KParams K)
       }
     }
   }
-  if (valid) P->cand_cnt[(size_t)sp * n + s] = make_int2(cnt, cands);
+  if (valid) P->cand_cnt[(size_t)sp * n + s] = make_int2(cnt | (min(sure, kSureMost) << kSureShift), cands);
 }
 
 // --------------------------------------------------------------- row pass
@@ -458,49 +461,58 @@ __device__ __forceinline__ int warp_excl_scan(int v, int lane, int &total) {
   return incl - v;
 }
 
-// One block of four warps per source tile, one warp per row.  The row's candidates
-// (entries of k_cand) are put in ascending target index -- up to 128 of them by a sorting
-// network over the lanes, more through a bitmap over a window of target indices in shared
-// memory -- and evaluated 32 at a time with the exact arithmetic, the next 32 records in
-// flight.  The reference scans the targets by index and stops at cap kept pairs
-// (src/cvo/CvoGPU.cu:994-996): here the row stops there too, so no pair beyond cap is
-// evaluated or stored.  A row whose entries did not fit, or a call without a candidate
-// test, scans all targets in index order instead.
+// One warp per row.  The row's candidates (entries of k_cand) are put in ascending target index
+// -- up to 128 of them by a sorting network over the lanes, more through a bitmap over a window
+// of target indices in shared memory -- and evaluated 32 at a time with the exact arithmetic,
+// the next 32 records in flight.  The reference scans the targets by index and stops at cap kept
+// pairs (src/cvo/CvoGPU.cu:994-996): here the row stops there too, so no pair beyond cap is
+// evaluated or stored.  A row whose entries did not fit, or a call without a candidate test,
+// scans all targets in index order instead.
 // Sums (all but align): FP32 per lane and row, over the lanes, FP64 from there; the last block
 // of a pair adds the blocks' sums in a fixed order.
 // ROWS_ORDERED: the entries of a row go to the order of the pair's level (RankLevel), in which
 // k_rowsum, k_step and k_irls_accum add them one by one.  The align loop and the window solve
 // turn a different last bit of the gradient into a visibly different pose some tens of
-// iterations later, so the order is part of the result and is kept whatever finds the pairs.  A row with no more than cap candidates
-// is sorted and evaluated by rank from the start; a longer one is cut by index first and its
-// kept entries are then put in order.  One that kept more than cap + order_cap pairs stays in
-// index order.
-// Bounds: latency of the dependent steps entry -> permutation -> bitmap -> record, hidden
-// by 16-28 resident warps per SM (the bitmap's shared memory sets the number).  The rows'
-// FP64 constants are computed 32 rows at a time: once per warp and row they took most of
-// a pass over rows without candidates.
+// iterations later, so the order is part of the result and is kept whatever finds the pairs.
+// A row with no more than cap candidates is sorted and evaluated by rank from the start; a
+// longer one is cut by index first and its kept entries are then put in order.  One that kept
+// more than cap + order_cap pairs stays in index order: nearly all such rows are told by the
+// pairs that k_cand is sure of; the rest are evaluated that far (eight pairs of 20k-50k
+// points had 7 % of the rows evaluated to 4,353 pairs, 60 % of all evaluations).
+// Two instances share the rows of large targets: ROWS_LIGHT those of up to 128 candidates, with
+// hardly any shared memory, 32 rows to a block; ROWS_ALL the others, or all rows of targets
+// whose bitmap is small anyway, eight rows to a block, handed to the warps one by one (rows of
+// 0 to cap pairs lie in clusters: blocks of 32 rows left a tail of a third of the launch).
+// Bounds: latency of the dependent steps entry -> permutation -> bitmap -> record, hidden by
+// the resident warps.  The rows' FP64 constants are computed up to 32 rows at a time: once per
+// warp and row they took most of a pass over rows without candidates.
 constexpr int kRowWarps = 4;
 constexpr int kRowsPerBlock = kGroup;
+constexpr int kRowsHeavy = 8;           // rows of a ROWS_ALL block
+constexpr int kRowSlots = 1 + kRowsPerBlock / kRowsHeavy;      // partial sums of 32 rows: ROWS_LIGHT, ROWS_ALL
 constexpr int kMaxSplits = 16;
-constexpr int kRowWindow = 65536;       // most target indices of one bitmap window
-constexpr int kRowQueue = 512;          // sorted candidates of one round
+constexpr int kRowWindow = 63 * 1024;   // most target indices of one bitmap window (the queue's 16 bits)
+constexpr int kRowBatch = 256;          // candidates taken from the bitmap before they are evaluated
 constexpr int kRowSorted = 128;         // most candidates a sorting network puts in order
+constexpr int kRowSplitTargets = 8192;  // larger targets: ROWS_LIGHT and ROWS_ALL
 
 // Whether a kernel instance leaves the rows' entries in index order (single passes) or puts
 // them in the order of the pair's level (the align loop, the edges of a window).
 enum { ROWS_SUM = 0, ROWS_ORDERED = 1 };
+enum { ROWS_ALL = 0, ROWS_LIGHT = 1 };
 
 // Words of one warp's bitmap for targets of up to m points: an odd number per lane, so
 // that the lanes' runs start in different banks.
 __host__ __device__ inline int row_window_words(int m) {
   return 32 * ((((m < kRowWindow ? m : kRowWindow) + 1023) / 1024) | 1);
 }
-// Ints of its queue; also a 16-bit count before each word of the bitmap.
-__host__ __device__ inline int row_queue_ints(int window_words) {
-  return window_words / 2 > kRowQueue ? window_words / 2 : kRowQueue;
+// Words of its queue (16 bits an index, a batch and the 1024 of one step more; or 128 sorted
+// candidates), which also holds a 16-bit count before each word of the bitmap.
+__host__ __device__ inline int row_queue_words(int window_words) {
+  return window_words / 2 > (kRowBatch + 1024) / 2 ? window_words / 2 : (kRowBatch + 1024) / 2;
 }
 __host__ __device__ inline size_t row_smem_bytes(int m) {
-  return (size_t)kRowWarps * sizeof(uint32_t) * (row_window_words(m) + row_queue_ints(row_window_words(m)));
+  return (size_t)kRowWarps * sizeof(uint32_t) * (row_window_words(m) + row_queue_words(row_window_words(m)));
 }
 
 // Puts the z entries of an ELL row, which are in index order, in the order of the ranks:
@@ -585,32 +597,26 @@ __device__ __forceinline__ void pass_finished(const BatchDev &B, PairDev *P, dou
   P->max_row = (int)mx;
 }
 
-// Sums of a single pass (value, kept pairs, longest row) -> part; the last block of the pair
-// finishes the pass.
-__device__ __forceinline__ void rows_finish(const BatchDev &B, PairDev *P, int b, int nb, double sum, long long nnz, int mx) {
+// Sums of a single pass (value, kept pairs, longest row) of one block -> slot; the last of nb
+// blocks adds the slots first .. first + slots - 1 and finishes the pass.
+__device__ __forceinline__ void rows_partial(PairDev *P, int slot, const double (&t)[3]) {
+  for (int k = 0; k < 3; k++) P->part[(size_t)slot * kPartStride + k] = t[k];
+}
+__device__ __forceinline__ void rows_finish(const BatchDev &B, PairDev *P, int nb, int first, int slots) {
   __shared__ double sh[kRowWarps][3];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) {
-    sh[w][0] = sum;
-    sh[w][1] = (double)nnz;
-    sh[w][2] = (double)mx;
-  }
-  __syncthreads();
-  if (threadIdx.x < 3) {
-    double t = sh[0][threadIdx.x];
-    for (int q = 1; q < kRowWarps; q++) t = threadIdx.x < 2 ? t + sh[q][threadIdx.x] : fmax(t, sh[q][threadIdx.x]);
-    P->part[(size_t)b * kPartStride + threadIdx.x] = t;
+  if (threadIdx.x == 0) {
     __threadfence();
+    last = atomicAdd(&P->counter[0], 1u) == (unsigned)(nb - 1);
   }
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(&P->counter[0], 1u) == (unsigned)(nb - 1);
   __syncthreads();
   if (!last) return;
   __threadfence();
   double t[3] = {0, 0, 0};
-  for (int q = threadIdx.x; q < nb; q += 32 * kRowWarps) {
-    const double *pv = P->part + (size_t)q * kPartStride;
+#pragma unroll 8
+  for (int q = threadIdx.x; q < slots; q += 32 * kRowWarps) {
+    const double *pv = P->part + (size_t)(first + q) * kPartStride;
     t[0] += __ldcg(pv);
     t[1] += __ldcg(pv + 1);
     t[2] = fmax(t[2], __ldcg(pv + 2));
@@ -631,19 +637,27 @@ __device__ __forceinline__ void rows_finish(const BatchDev &B, PairDev *P, int b
   pass_finished(B, P, t[0], t[1], t[2]);
 }
 
-template <int FCH, int LCH, bool GT, int KIND>
-__global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams K, int window_words) {
+// split: ROWS_LIGHT has taken the rows of up to 128 candidates.
+template <int FCH, int LCH, bool GT, int KIND, int PART>
+__global__ void __launch_bounds__(32 * kRowWarps, PART == ROWS_LIGHT && LCH == 0 ? 6 : 5)
+    k_rows(BatchDev B, KParams K, int window_words, int split) {
+  constexpr int RB = PART == ROWS_LIGHT ? kRowsPerBlock : kRowsHeavy;
   extern __shared__ __align__(16) uint32_t row_smem[];
-  __shared__ float4 sh_rc[kRowsPerBlock];                  // l, d2 threshold, 1 / (2 l^2)
-  __shared__ int2 sh_cnt[kMaxSplits][kRowsPerBlock];       // entries and candidates per split
-  __shared__ int2 sh_tot[kRowsPerBlock];                   // of the row; entries < 0: scan all targets
+  __shared__ float4 sh_rc[RB];                             // l, d2 threshold, 1 / (2 l^2)
+  __shared__ int2 sh_cnt[kMaxSplits][RB];                  // entries and candidates per split
+  __shared__ int4 sh_tot[RB];                              // of the row, and pairs surely kept; entries < 0: scan all targets
+  __shared__ double sh_sum[RB];                            // the rows' sums and kept pairs
+  __shared__ int sh_kept[RB];
+  __shared__ int next_row;
   __shared__ float4 sh_keep[kRowWarps][64];                // kept pairs by slot: y and value
   __shared__ int sh_keepj[kRowWarps][64];
   constexpr int FP = FCH > 0 ? FCH : 1;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  uint32_t *bits = row_smem + (size_t)w * (window_words + row_queue_ints(window_words));
-  int *queue = reinterpret_cast<int *>(bits + window_words);
-  const int blk = blockIdx.x;
+  constexpr int SUBS = kRowsPerBlock / RB;                 // blocks of a source tile
+  uint32_t *bits = row_smem + (size_t)w * (PART == ROWS_LIGHT ? kRowSorted : window_words + row_queue_words(window_words));
+  int *sorted = reinterpret_cast<int *>(PART == ROWS_LIGHT ? bits : bits + window_words);
+  unsigned short *queue = reinterpret_cast<unsigned short *>(sorted);
+  const int blk = blockIdx.x / SUBS, part = blockIdx.x % SUBS;
   if (blk >= B.total_rblocks) return;
   const int p = find_segment(B.rblk_off, B.npairs, blk);
   PairDev *P = &B.pairs[p];
@@ -654,40 +668,59 @@ __global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams 
   const float4 *__restrict__ tf = reinterpret_cast<const float4 *>(P->tf);
   const float4 *__restrict__ tl = reinterpret_cast<const float4 *>(P->tl);
   const int *__restrict__ tperm = P->tperm;
+  const int s0 = b * kRowsPerBlock + part * RB;
   {
-    const int s = b * kRowsPerBlock + lane;
-    if (w == 0) {
-      const RowConst rc = row_const(K, P->ell, s < n ? __ldg(&P->xs[s]).w : 0.f);
-      sh_rc[lane] = make_float4(rc.l, rc.d2t, rc.inv2l2, 0.f);
-    }
     if (K.use_mma)
-      for (int q = w; q < S; q += kRowWarps) sh_cnt[q][lane] = s < n ? __ldg(&P->cand_cnt[(size_t)q * n + s]) : make_int2(0, 0);
+      for (int i = threadIdx.x; i < S * RB; i += 32 * kRowWarps) {
+        const int q = i / RB, s = s0 + i % RB;
+        sh_cnt[q][i % RB] = s < n ? __ldg(&P->cand_cnt[(size_t)q * n + s]) : make_int2(0, 0);
+      }
+    if (threadIdx.x == 0) next_row = 0;
     __syncthreads();
-    if (w == 0) {
-      int2 t = make_int2(K.use_mma ? 0 : -1, 0);
+    bool here = false;
+    if (threadIdx.x < RB) {
+      const int s = s0 + lane;
+      int4 t = make_int4(K.use_mma ? 0 : -1, 0, 0, 0);
       bool fits = true;
       for (int q = 0; q < S && K.use_mma; q++) {
-        const int2 c = sh_cnt[q][lane];
+        int2 c = sh_cnt[q][lane];
+        t.z += c.x >> kSureShift;
+        c.x &= (1 << kSureShift) - 1;
+        sh_cnt[q][lane].x = c.x;
         fits = fits && c.x <= caps;
         t.x += c.x;
         t.y += c.y;
       }
       if (!fits) t.x = -1;
       if (cap <= 0 || s >= n) t.x = 0;
+      const bool light = t.x >= 0 && t.y <= kRowSorted;
+      if (s < n && t.x == 0 && (PART == ROWS_LIGHT || !split)) P->nnz_row[s] = 0;
+      if (PART == ROWS_LIGHT ? !light : split && light) t.x = 0;      // the other instance's
+      here = t.x != 0;
       sh_tot[lane] = t;
-      if (s < n && t.x == 0) P->nnz_row[s] = 0;
+      sh_sum[lane] = 0.0;
+      sh_kept[lane] = 0;
     }
-    __syncthreads();
+    const bool any = __syncthreads_or(here);
+    if (any && threadIdx.x < RB) {
+      const int s = s0 + lane;
+      const RowConst rc = row_const(K, P->ell, s < n ? __ldg(&P->xs[s]).w : 0.f);
+      sh_rc[lane] = make_float4(rc.l, rc.d2t, rc.inv2l2, 0.f);
+    }
+    if (any) __syncthreads();
+    else if (KIND == ROWS_ORDERED && mode == MODE_ALIGN) return;
   }
   const int order_cap = KIND == ROWS_ORDERED ? P->order_cap : 0;
   const RankLevel *lv = KIND == ROWS_ORDERED ? P->levels + P->level : nullptr;
-  double row_total = 0.0;
-  long long nnz = 0;
-  int mx = 0;
-  for (int r = w; r < kRowsPerBlock; r += kRowWarps) {
+  for (int r = w;; r += kRowWarps) {
+    if (PART == ROWS_ALL) {
+      if (lane == 0) r = atomicAdd(&next_row, 1);
+      r = __shfl_sync(FULLMASK, r, 0);
+    }
+    if (r >= RB) break;
     const int entries = sh_tot[r].x, cands = sh_tot[r].y;
     if (entries == 0) continue;
-    const int s = b * kRowsPerBlock + r;
+    const int s = s0 + r;
     const float4 x = __ldg(&P->xs[s]);
     float4 xf[FP];
 #pragma unroll
@@ -708,10 +741,11 @@ __global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams 
       return at ? __ldg(at) : make_uint2(0u, 0u);
     };
     // by rank from the start if the row cannot be cut; otherwise by index, and on past cap only
-    // to tell whether the row keeps more than cap + order_cap
+    // to tell whether the row keeps more than cap + order_cap (it may, and is not sure to)
     const bool ranked = KIND == ROWS_ORDERED && entries > 0 && cands <= cap;
     const int *perm = ranked ? lv->of_tile : tperm;
-    const int stop = KIND == ROWS_ORDERED && (entries < 0 || cands > cap + order_cap) ? cap + order_cap + 1 : cap;
+    const bool over = KIND == ROWS_ORDERED && sh_tot[r].z > cap + order_cap;
+    const int stop = KIND == ROWS_ORDERED && !over && (entries < 0 || cands > cap + order_cap) ? cap + order_cap + 1 : cap;
     int kept = 0;
     float acc = 0.f;
     // 32 kept pairs to the ELL row and the sum: lane l takes slots l, l + 32, ..., so the
@@ -731,29 +765,31 @@ __global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams 
       flushed += 32;
       __syncwarp();
     };
-    int w0 = 0, base = 0, total = 0, off = 0, bank = 0;      // bitmap window, rounds of its candidates
-    bool fresh = true;
-    const int wl = window_words >> 5;
+    // Rounds of n candidates in order: all of a sorted list, all targets, or a queue (relative to
+    // w0) taken from the bitmap 32 words at a time, one a lane: the indices of a row lie in
+    // clusters, and a run of words per lane left most lanes idle.
+    const bool direct = entries < 0, listed = !direct && cands <= kRowSorted;
+    int w0 = 0, pos = 0, qn = 0;
+    bool filled = false;
     while (true) {
-      int count = 0;
-      if (entries < 0) {
-        count = m;
-      } else if (cands <= kRowSorted) {
+      int n = m;
+      if (PART == ROWS_LIGHT || listed) {
         // one to four candidates in a lane, sorted by a bitonic network
+        n = 0;
         for (int e0 = 0; e0 < entries; e0 += 32) {
           const uint2 v = entry(e0 + lane);
           int o, add;
-          o = count + warp_excl_scan(__popc(v.y), lane, add);
-          for (uint32_t mk = v.y; mk; mk &= mk - 1) queue[o++] = __ldg(&perm[32 * (int)v.x + __ffs(mk) - 1]);
-          count += add;
+          o = n + warp_excl_scan(__popc(v.y), lane, add);
+          for (uint32_t mk = v.y; mk; mk &= mk - 1) sorted[o++] = __ldg(&perm[32 * (int)v.x + __ffs(mk) - 1]);
+          n += add;
         }
         __syncwarp();
-        if (count <= 32) warp_sort<1>(queue, count, lane);
-        else if (count <= 64) warp_sort<2>(queue, count, lane);
-        else warp_sort<4>(queue, count, lane);
+        if (n <= 32) warp_sort<1>(sorted, n, lane);
+        else if (n <= 64) warp_sort<2>(sorted, n, lane);
+        else warp_sort<4>(sorted, n, lane);
         __syncwarp();
-      } else {
-        if (fresh) {
+      } else if (!direct) {
+        if (!filled) {
           for (int i = lane; i < window_words / 4; i += 32) reinterpret_cast<uint4 *>(bits)[i] = make_uint4(0u, 0u, 0u, 0u);
           __syncwarp();
           uint2 next = entry(lane);
@@ -771,46 +807,35 @@ __global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams 
             }
           }
           __syncwarp();
-          // lane l owns words l * wl .. : their candidates follow those of the lanes before
-          bank = 0;
-          for (int i = 0; i < wl; i++) bank += __popc(bits[lane * wl + i]);
-          off = warp_excl_scan(bank, lane, total);
-          base = 0;
-          fresh = false;
+          filled = true;
+          pos = qn = 0;
         }
-        count = min(kRowQueue, total - base);
-        if (off < base + count && off + bank > base) {
-          int o = off - base;
-          for (int i = 0; i < wl && o < count; i++) {
-            uint32_t mk = bits[lane * wl + i];
-            if (o + __popc(mk) <= 0) {
-              o += __popc(mk);
-              continue;
-            }
-            for (; mk; mk &= mk - 1, o++)
-              if (o >= 0 && o < count) queue[o] = w0 + 32 * (lane * wl + i) + __ffs(mk) - 1;
-          }
+        for (; pos < window_words && qn < kRowBatch; pos += 32) {
+          uint32_t mk = bits[pos + lane];
+          if (!__any_sync(FULLMASK, mk != 0)) continue;
+          int add, o = qn + warp_excl_scan(__popc(mk), lane, add);
+          for (; mk; mk &= mk - 1) queue[o++] = (unsigned short)(32 * (pos + lane) + __ffs(mk) - 1);
+          qn += add;
         }
-        base += count;
         __syncwarp();
+        n = pos < window_words ? qn & ~31 : qn;      // whole rounds of 32, and the rest when the window ends
       }
-      // the round's candidates, 32 at a time
-      const bool direct = entries < 0;
       float4 y = make_float4(0.f, 0.f, 0.f, 0.f), yf[FP];
 #pragma unroll
       for (int q = 0; q < FP; q++) yf[q] = y;
       int j = 0;
       auto load = [&](int i) {
-        if (i >= count) return;
-        j = direct ? i : queue[i];
+        if (i >= n) return;
+        if (PART == ROWS_LIGHT || listed) j = sorted[i];
+        else j = direct ? i : w0 + queue[i];
         if (ranked) j = __ldg(&lv->index[j]);
         y = __ldg(&yorig[j]);
 #pragma unroll
         for (int q = 0; q < FCH; q++) yf[q] = __ldg(tf + (size_t)j * FCH + q);
       };
       load(lane);
-      for (int i0 = 0; i0 < count && kept < stop; i0 += 32) {
-        const bool has = i0 + lane < count;
+      for (int i0 = 0; i0 < n && kept < stop; i0 += 32) {
+        const bool has = i0 + lane < n;
         const float4 yc = y;
         float4 fc[FP];
 #pragma unroll
@@ -832,91 +857,48 @@ __global__ void __launch_bounds__(32 * kRowWarps, 5) k_rows(BatchDev B, KParams 
         if (min(kept, cap) - flushed >= 32) flush(true);
       }
       __syncwarp();
-      if (kept >= stop || entries < 0 || cands <= kRowSorted) break;
-      if (base >= total) {
+      if (PART == ROWS_LIGHT || listed || direct || kept >= stop) break;
+      if (pos < window_words) {
+        const unsigned short rest = n + lane < qn ? queue[n + lane] : (unsigned short)0;
+        __syncwarp();
+        queue[lane] = rest;
+        qn -= n;
+        __syncwarp();
+      } else {
         w0 += 32 * window_words;
         if (w0 >= m) break;
-        fresh = true;
+        filled = false;
       }
     }
     const int z = min(kept, cap);
     if (flushed < z) flush(lane < z - flushed);
     if (lane == 0) P->nnz_row[s] = z;
     if (KIND == ROWS_ORDERED) {
-      if (!ranked && z > 1 && kept <= cap + order_cap && K.use_geo)
-        order_row(P->A_j + (size_t)s * P->ld, P->A_v + (size_t)s * P->ld, z, lv->of_index, m, bits, window_words,
-                  reinterpret_cast<unsigned short *>(queue), P->cand + (size_t)s * P->cand_pitch, lane);
+      if (PART == ROWS_ALL && !ranked && z > 1 && !over && kept <= cap + order_cap && K.use_geo)
+        order_row(P->A_j + (size_t)s * P->ld, P->A_v + (size_t)s * P->ld, z, lv->of_index, m, bits, window_words, queue,
+                  P->cand + (size_t)s * P->cand_pitch, lane);
       __syncwarp();
       if (mode == MODE_ALIGN) continue;
     }
-    nnz += z;
-    mx = max(mx, z);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(FULLMASK, acc, o);
-    row_total += (double)acc;
-  }
-  if (KIND == ROWS_SUM || mode != MODE_ALIGN) rows_finish(B, P, b, nb, row_total, nnz, mx);
-}
-
-// Calls add(a, y) for the z entries of ELL row s in slot order.
-template <class Add>
-__device__ __forceinline__ void row_entries(const PairDev *P, int s, int z, Add add) {
-  const int *__restrict__ Aj = P->A_j + (size_t)s * P->ld;
-  const float *__restrict__ Av = P->A_v + (size_t)s * P->ld;
-  const float4 *__restrict__ yorig = P->yorig;
-  int c = 0;
-  if (z >= 8) {
-    int4 j0 = *reinterpret_cast<const int4 *>(Aj), j1 = *reinterpret_cast<const int4 *>(Aj + 4);
-    for (; c + 8 <= z; c += 8) {
-      const float4 y0 = __ldg(&yorig[j0.x]), y1 = __ldg(&yorig[j0.y]), y2 = __ldg(&yorig[j0.z]), y3 = __ldg(&yorig[j0.w]);
-      const float4 y4 = __ldg(&yorig[j1.x]), y5 = __ldg(&yorig[j1.y]), y6 = __ldg(&yorig[j1.z]), y7 = __ldg(&yorig[j1.w]);
-      const float4 a = *reinterpret_cast<const float4 *>(Av + c), b = *reinterpret_cast<const float4 *>(Av + c + 4);
-      if (c + 16 <= z) {
-        j0 = *reinterpret_cast<const int4 *>(Aj + c + 8);
-        j1 = *reinterpret_cast<const int4 *>(Aj + c + 12);
-      }
-      add(a.x, y0); add(a.y, y1); add(a.z, y2); add(a.w, y3);
-      add(b.x, y4); add(b.y, y5); add(b.z, y6); add(b.w, y7);
+    if (lane == 0) {
+      sh_sum[r] = (double)acc;
+      sh_kept[r] = z;
     }
   }
-  if (c + 4 <= z) {
-    const int4 j = *reinterpret_cast<const int4 *>(Aj + c);
-    const float4 a = *reinterpret_cast<const float4 *>(Av + c);
-    const float4 y0 = __ldg(&yorig[j.x]), y1 = __ldg(&yorig[j.y]), y2 = __ldg(&yorig[j.z]), y3 = __ldg(&yorig[j.w]);
-    add(a.x, y0); add(a.y, y1); add(a.z, y2); add(a.w, y3);
-    c += 4;
+  if (KIND == ROWS_ORDERED && mode == MODE_ALIGN) return;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t[3] = {0.0, 0.0, 0.0};
+    for (int r = 0; r < RB; r++) {
+      t[0] += sh_sum[r];
+      t[1] += (double)sh_kept[r];
+      t[2] = fmax(t[2], (double)sh_kept[r]);
+    }
+    rows_partial(P, PART == ROWS_LIGHT ? b : nb + SUBS * b + part, t);
   }
-  for (; c < z; c++) add(Av[c], __ldg(&yorig[Aj[c]]));
-}
-
-// Row partials of the align loop from the final ELL entries, one after the other in slot
-// order (thread per row): omega = sum a (x cross y), v = sum a (y - x), sum a
-// (CvoGPU.cu:2001-2062 computes the same sums from the sparse kernel matrix).  The order is
-// part of the result (see k_rows), so a row is one thread's chain of additions; the loads
-// run ahead of it: eight entries' indices one step, their targets' positions in one batch.
-// Bounds: L2 latency of index -> position, one round trip per eight entries.
-__global__ void __launch_bounds__(128) k_rowsum(BatchDev B, KParams K) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= B.total_rows) return;
-  const int p = find_segment(B.row_off, B.npairs, g);
-  const PairDev *P = &B.pairs[p];
-  if (P->done) return;
-  const int s = g - B.row_off[p];
-  const int z = P->nnz_row[s];
-  const float4 x = __ldg(&P->xs[s]);
-  float w0 = 0.f, w1 = 0.f, w2 = 0.f, v0 = 0.f, v1 = 0.f, v2 = 0.f, as = 0.f;
-  row_entries(P, s, z, [&](float a, const float4 &y) {
-    w0 = fmaf(a, fs(fm(x.y, y.z), fm(x.z, y.y)), w0);
-    w1 = fmaf(a, fs(fm(x.z, y.x), fm(x.x, y.z)), w1);
-    w2 = fmaf(a, fs(fm(x.x, y.y), fm(x.y, y.x)), w2);
-    v0 = fmaf(a, y.x - x.x, v0);
-    v1 = fmaf(a, y.y - x.y, v1);
-    v2 = fmaf(a, y.z - x.z, v2);
-    as += a;
-  });
-  float4 *rs = reinterpret_cast<float4 *>(P->row_sums + (size_t)s * 8);
-  rs[0] = make_float4(__fdiv_rn(w0, K.c), __fdiv_rn(w1, K.c), __fdiv_rn(w2, K.c), __fdiv_rn(v0, K.d));
-  rs[1] = make_float4(__fdiv_rn(v1, K.d), __fdiv_rn(v2, K.d), as, 0.f);
+  if (PART == ROWS_ALL) rows_finish(B, P, SUBS * nb, split ? 0 : nb, (split ? kRowSlots : kRowSlots - 1) * nb);
 }
 
 }  // namespace cvo_gb

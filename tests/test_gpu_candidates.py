@@ -63,3 +63,30 @@ def test_terms_switched_off(cuda_device, geometry, intensity):
     p.is_using_geometry, p.is_using_intensity, p.nearest_neighbors_max = geometry, intensity, 50
     total, _ = _check(p, _cloud(rng, 70, 3.0), _cloud(rng, 1500, 3.0), T, 0.4)
     assert total > 0
+
+
+@pytest.mark.parametrize("n, m, cap", [(300, 8192, 64), (300, 8193, 64), (70, 20001, 200)])
+def test_targets_that_take_a_launch_for_the_rows_of_few_candidates(cuda_device, n, m, cap):
+    """Rows of 0 to thousands of candidates on both sides of the 8,192 targets."""
+    rng = np.random.default_rng(m)
+    p = CvoParams(params_path("geometric"))
+    p.nearest_neighbors_max = cap
+    src, tgt = (CvoPointCloud(np.abs(rng.normal(size=(k, 3))) ** 3) for k in (n, m))
+    total, most = _check(p, src, tgt, T, 0.1)
+    assert total > 0 and most == cap
+
+
+@pytest.mark.parametrize("m, cap", [(4127, 32), (4128, 32), (4129, 32), (6000, 7), (9000, 300)])
+def test_align_of_rows_longer_than_those_put_in_order(cuda_device, m, cap):
+    """Every target lies within the radius of every source: rows that keep about 4,096 pairs
+    more than cap.  Three iterations against the oracle's, 1e-5 rad / 1e-5 m (the kept pairs are
+    the same, FP32 sums of them in another order: 1e-6 relative, steps of at most 1 cm)."""
+    rng = np.random.default_rng(m)
+    p = CvoParams(params_path("color"))
+    p.nearest_neighbors_max, p.MAX_ITER = cap, 3
+    src, tgt = (CvoPointCloud(rng.uniform(0, 1, (k, 3)) + 2, rng.uniform(0.49, 0.51, (k, 5))) for k in (65, m))
+    ret, Tg, _, _, it = CvoGPU(params=p).align(src, tgt, T)
+    ret_o, To, it_o, _ = orc.align(p, src, tgt, T)
+    assert (ret, it) == (ret_o, it_o)
+    R = Tg[:3, :3].T.astype(np.float64) @ To[:3, :3].astype(np.float64)
+    assert np.linalg.norm(R - R.T) / 2 < 1e-5 and np.linalg.norm(Tg[:3, 3] - To[:3, 3]) < 1e-5
