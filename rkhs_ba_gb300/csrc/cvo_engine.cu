@@ -27,6 +27,7 @@ constexpr int kChunk = 8;
 __global__ void k_transform(BatchDev B) {
   int gt = blockIdx.x * blockDim.x + threadIdx.x;
   if (gt == 0 && *B.active > 0) *B.active_iters += 1;
+  if (gt < 2) B.heavy_ctr[gt] = 0;
   if (gt >= B.total_targets) return;
   int p = find_segment(B.tgt_off, B.npairs, gt);
   PairDev *P = &B.pairs[p];
@@ -41,143 +42,180 @@ __global__ void k_transform(BatchDev B) {
   P->yorig[__ldg(&P->tperm[t])] = o;
 }
 
+// Totals of the single passes whose rows took two launches, a block per pair.
+__global__ void __launch_bounds__(32 * kRowWarps) k_rows_total(BatchDev B) {
+  PairDev *P = &B.pairs[blockIdx.x];
+  if (P->done) return;
+  sum_slots(B, P, 0, kRowSlots * (B.rblk_off[blockIdx.x + 1] - B.rblk_off[blockIdx.x]));
+}
+
 // ---------------------------------------------------------------- row sums
-// Calls add(a, y) for the z entries of ELL row s in slot order.
-template <class Add>
-__device__ __forceinline__ void row_entries(const PairDev *P, int s, int z, Add add) {
+// Sums over the z entries of ELL row s of NV terms: X[t] of an entry from term(y, X),
+// acc[t] = a X[t] + acc[t], one entry after the other in slot order.  The order is part of the
+// result (see k_rows), so a sum is one lane's chain of fused multiply-adds; but what is added
+// does not depend on it.  G lanes share a row: they compute the terms of G entries, one each,
+// and lane t < NV then adds the G entries' X[t].  A thread per row was as slow as the longest
+// of its warp's 32 rows and left most of the chip without a warp.
+// The positions of the next entries and the indices of those after them are in flight.
+// buf: the warp's; per row NV + 1 lists (the last: a) of G floats, spaced so that the lanes'
+// stores hit distinct banks.  Returns acc[lane % G].  All lanes call it; z is the own row's.
+template <int G>
+struct RowLists {
+  static constexpr int kPitch = G == 8 ? 12 : 4;       // floats from list to list
+  static constexpr int kRow = G == 8 ? 104 : 20;       // from row to row
+  static constexpr int kWarp = 32 / G * kRow;
+};
+
+template <int G, int NV, class Term>
+__device__ __forceinline__ float row_sums(const PairDev *P, int s, int z, float *buf, Term term) {
+  using L = RowLists<G>;
+  const int lane = threadIdx.x & 31, sub = lane % G;
   const int *__restrict__ Aj = P->A_j + (size_t)s * P->ld;
   const float *__restrict__ Av = P->A_v + (size_t)s * P->ld;
   const float4 *__restrict__ yorig = P->yorig;
-  int c = 0;
-  if (z >= 8) {
-    int4 j0 = *reinterpret_cast<const int4 *>(Aj), j1 = *reinterpret_cast<const int4 *>(Aj + 4);
-    for (; c + 8 <= z; c += 8) {
-      const float4 y0 = __ldg(&yorig[j0.x]), y1 = __ldg(&yorig[j0.y]), y2 = __ldg(&yorig[j0.z]), y3 = __ldg(&yorig[j0.w]);
-      const float4 y4 = __ldg(&yorig[j1.x]), y5 = __ldg(&yorig[j1.y]), y6 = __ldg(&yorig[j1.z]), y7 = __ldg(&yorig[j1.w]);
-      const float4 a = *reinterpret_cast<const float4 *>(Av + c), b = *reinterpret_cast<const float4 *>(Av + c + 4);
-      if (c + 16 <= z) {
-        j0 = *reinterpret_cast<const int4 *>(Aj + c + 8);
-        j1 = *reinterpret_cast<const int4 *>(Aj + c + 12);
-      }
-      add(a.x, y0); add(a.y, y1); add(a.z, y2); add(a.w, y3);
-      add(b.x, y4); add(b.y, y5); add(b.z, y6); add(b.w, y7);
+  float *row = buf + lane / G * L::kRow;
+  const float4 *mine = reinterpret_cast<const float4 *>(row + min(sub, NV) * L::kPitch);
+  const float4 *val = reinterpret_cast<const float4 *>(row + NV * L::kPitch);
+  const int most = __reduce_max_sync(FULLMASK, z);
+  int j1 = 0;
+  float a0 = 0.f, a1 = 0.f, acc = 0.f;
+  float4 y0 = make_float4(0.f, 0.f, 0.f, 0.f), y1 = y0;
+  if (sub < z) {
+    y0 = __ldg(&yorig[Aj[sub]]);
+    a0 = Av[sub];
+  }
+  if (G + sub < z) {
+    j1 = Aj[G + sub];
+    a1 = Av[G + sub];
+  }
+  for (int c = 0; c < most; c += G) {
+    if (c + G + sub < z) y1 = __ldg(&yorig[j1]);
+    float a2 = 0.f;
+    if (c + 2 * G + sub < z) {
+      j1 = Aj[c + 2 * G + sub];
+      a2 = Av[c + 2 * G + sub];
     }
+    float X[NV];
+    term(y0, X);
+    __syncwarp();
+#pragma unroll
+    for (int t = 0; t < NV; t++) row[t * L::kPitch + sub] = X[t];
+    row[NV * L::kPitch + sub] = a0;
+    __syncwarp();
+    const int here = z - c;
+#pragma unroll
+    for (int e = 0; e < G; e += 4) {
+      const float4 v = mine[e / 4], a = val[e / 4];
+      if (e < here) acc = fmaf(a.x, v.x, acc);
+      if (e + 1 < here) acc = fmaf(a.y, v.y, acc);
+      if (e + 2 < here) acc = fmaf(a.z, v.z, acc);
+      if (e + 3 < here) acc = fmaf(a.w, v.w, acc);
+    }
+    y0 = y1;
+    a0 = a1;
+    a1 = a2;
   }
-  if (c + 4 <= z) {
-    const int4 j = *reinterpret_cast<const int4 *>(Aj + c);
-    const float4 a = *reinterpret_cast<const float4 *>(Av + c);
-    const float4 y0 = __ldg(&yorig[j.x]), y1 = __ldg(&yorig[j.y]), y2 = __ldg(&yorig[j.z]), y3 = __ldg(&yorig[j.w]);
-    add(a.x, y0); add(a.y, y1); add(a.z, y2); add(a.w, y3);
-    c += 4;
-  }
-  for (; c < z; c++) add(Av[c], __ldg(&yorig[Aj[c]]));
+  __syncwarp();
+  return acc;
 }
 
-// Row partials of the align loop from the final ELL entries, one after the other in slot
-// order (thread per row): omega = sum a (x cross y), v = sum a (y - x), sum a
-// (CvoGPU.cu:2001-2062 computes the same sums from the sparse kernel matrix).  The order is
-// part of the result (see k_rows), so a row is one thread's chain of additions; the loads
-// run ahead of it: eight entries' indices one step, their targets' positions in one batch.
-// Bounds: L2 latency of index -> position, one round trip per eight entries.
-__global__ void __launch_bounds__(128) k_rowsum(BatchDev B, KParams K) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= B.total_rows) return;
-  const int p = find_segment(B.row_off, B.npairs, g);
-  const PairDev *P = &B.pairs[p];
-  if (P->done) return;
-  const int s = g - B.row_off[p];
-  const int z = P->nnz_row[s];
-  const float4 x = __ldg(&P->xs[s]);
-  float w0 = 0.f, w1 = 0.f, w2 = 0.f, v0 = 0.f, v1 = 0.f, v2 = 0.f, as = 0.f;
-  row_entries(P, s, z, [&](float a, const float4 &y) {
-    w0 = fmaf(a, fs(fm(x.y, y.z), fm(x.z, y.y)), w0);
-    w1 = fmaf(a, fs(fm(x.z, y.x), fm(x.x, y.z)), w1);
-    w2 = fmaf(a, fs(fm(x.x, y.y), fm(x.y, y.x)), w2);
-    v0 = fmaf(a, y.x - x.x, v0);
-    v1 = fmaf(a, y.y - x.y, v1);
-    v2 = fmaf(a, y.z - x.z, v2);
-    as += a;
-  });
-  float4 *rs = reinterpret_cast<float4 *>(P->row_sums + (size_t)s * 8);
-  rs[0] = make_float4(__fdiv_rn(w0, K.c), __fdiv_rn(w1, K.c), __fdiv_rn(w2, K.c), __fdiv_rn(v0, K.d));
-  rs[1] = make_float4(__fdiv_rn(v1, K.d), __fdiv_rn(v2, K.d), as, 0.f);
-}
-
-// ------------------------------------------------------------------ reduce
-// Sums of columns 0 .. NV-1 of the blocks' partials, each from block 0 upwards by one thread
-// (the order is part of the result); all threads bring the partials to shared memory first,
-// where a chain of loads costs 30 cycles a step instead of an L2 round trip.  Column NV-1 is a
-// maximum if MAX.  buf: kReduceThreads * NV doubles; out: NV.
-template <int NV, bool MAX>
-__device__ __forceinline__ void sum_partials(const double *part, int nb, double *buf, double *out) {
-  double t = 0.0;
-  for (int q0 = 0; q0 < nb; q0 += kReduceThreads) {
-    const int here = min(kReduceThreads, nb - q0);
-    __syncthreads();
-    for (int i = threadIdx.x; i < here * NV; i += blockDim.x)
-      buf[i] = __ldcg(part + (size_t)(q0 + i / NV) * kPartStride + i % NV);
-    __syncthreads();
-    if (threadIdx.x < NV)
-      for (int q = 0; q < here; q++) {
-        const double v = buf[q * NV + threadIdx.x];
-        t = MAX && threadIdx.x == NV - 1 ? fmax(t, v) : t + v;
-      }
-  }
-  if (threadIdx.x < NV) out[threadIdx.x] = t;
-  __syncthreads();
-}
-
-// Per-pair FP64 sums of the per-row partials written by k_rowsum.
-__global__ void __launch_bounds__(kReduceThreads) k_reduce(BatchDev B, KParams K) {
-  __shared__ double sh[kReduceThreads / 32][10];
-  __shared__ double buf[kReduceThreads * 9], tot[9];
+// The block's FP64 sums of NV terms (lane t < NV of G holds term t in acc) -> part; whether
+// this is the pair's last block, whose tot then holds the sums over all blocks.
+template <int G, int NV>
+__device__ __forceinline__ bool sum_blocks(PairDev *P, double acc, int b, int nb, unsigned int *counter, double *tot) {
+  __shared__ double sh[kStepThreads / 32][8];
   __shared__ bool last;
-  const int blk = blockIdx.x;
-  if (blk >= B.total_gblocks) return;
-  const int p = find_segment(B.gblk_off, B.npairs, blk);
-  PairDev *P = &B.pairs[p];
-  if (P->done) return;
-  const int b = blk - B.gblk_off[p];
-  const int nb = B.gblk_off[p + 1] - B.gblk_off[p];
-  const int n = P->n;
-  double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-  int mx = 0;
-  for (int r = b * kReduceRows + threadIdx.x; r < min(n, (b + 1) * kReduceRows); r += kReduceThreads) {
-    const float4 *rs = reinterpret_cast<const float4 *>(P->row_sums + (size_t)r * 8);
-    float4 a0 = rs[0], a1 = rs[1];
-    acc[0] += a0.x; acc[1] += a0.y; acc[2] += a0.z; acc[3] += a0.w;
-    acc[4] += a1.x; acc[5] += a1.y; acc[6] += a1.z;
-    int z = P->nnz_row[r];
-    acc[7] += (double)z;
-    mx = max(mx, z);
-  }
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
-  for (int k = 0; k < 8; k++) acc[k] = warp_sum(acc[k]);
+  for (int o = G; o < 32; o <<= 1) acc += __shfl_xor_sync(FULLMASK, acc, o);
+  if (lane < G) sh[w][lane] = acc;
+  __syncthreads();
+  if (threadIdx.x < NV) {
+    double t = sh[0][threadIdx.x];
+    for (int q = 1; q < kStepThreads / 32; q++) t += sh[q][threadIdx.x];
+    P->part[(size_t)b * kPartStride + threadIdx.x] = t;
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(counter, 1u) == (unsigned)(nb - 1);
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  // lane t of eight takes term t of every 32nd block
+  acc = 0.0;
+  const int k = threadIdx.x & 7;
+  if (k < NV)
+#pragma unroll 8
+    for (int q = threadIdx.x >> 3; q < nb; q += kStepThreads / 8) acc += __ldcg(P->part + (size_t)q * kPartStride + k);
+  acc += __shfl_xor_sync(FULLMASK, acc, 8);
+  acc += __shfl_xor_sync(FULLMASK, acc, 16);
+  if (lane < 8) sh[w][lane] = acc;
+  __syncthreads();
+  if (threadIdx.x < NV) {
+    double t = sh[0][threadIdx.x];
+    for (int q = 1; q < kStepThreads / 32; q++) t += sh[q][threadIdx.x];
+    tot[threadIdx.x] = t;
+  }
+  __syncthreads();
+  return true;
+}
+
+// The gradient from the final ELL entries: omega = sum a (x cross y) / c, v = sum a (y - x) / d
+// and sum a, FP32 per row, FP64 over rows (CvoGPU.cu:2001-2120 computes the same sums from the
+// sparse kernel matrix).  The last block of a pair finishes the pass and normalises.
+// Bounds: issue and L2 latency of index -> position, see row_sums.
+__global__ void __launch_bounds__(kStepThreads) k_gradient(BatchDev B, KParams K) {
+  constexpr int G = 8;
+  __shared__ __align__(16) float buf[kStepThreads / 32][RowLists<G>::kWarp];
+  __shared__ double tot[7];
+  const int blk = blockIdx.x;
+  if (blk >= B.total_sblocks) return;
+  const int p = find_segment(B.sblk_off, B.npairs, blk);
+  PairDev *P = &B.pairs[p];
+  if (P->done) return;
+  const int b = blk - B.sblk_off[p], nb = B.sblk_off[p + 1] - B.sblk_off[p], n = P->n;
+  const int sub = threadIdx.x % G;
+  double acc = 0.0;
+  int nnz = 0, mx = 0;
+  for (int s = b * B.step_rows + (int)threadIdx.x / G; s - (int)threadIdx.x / G < min(n, (b + 1) * B.step_rows);
+       s += kStepThreads / G) {
+    const bool has = s < n;
+    const int z = has ? P->nnz_row[s] : 0;
+    const float4 x = has ? __ldg(&P->xs[s]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float t = row_sums<G, 7>(P, has ? s : 0, z, buf[threadIdx.x >> 5], [&](const float4 &y, float (&X)[7]) {
+      X[0] = fs(fm(x.y, y.z), fm(x.z, y.y));
+      X[1] = fs(fm(x.z, y.x), fm(x.x, y.z));
+      X[2] = fs(fm(x.x, y.y), fm(x.y, y.x));
+      X[3] = y.x - x.x;
+      X[4] = y.y - x.y;
+      X[5] = y.z - x.z;
+      X[6] = 1.f;
+    });
+    acc += (double)(sub < 3 ? __fdiv_rn(t, K.c) : sub < 6 ? __fdiv_rn(t, K.d) : t);
+    if (sub == 0) nnz += z;
+    mx = max(mx, z);
+  }
+  // kept pairs and the longest row
+  __shared__ unsigned int sh_nnz, sh_mx;
+  if (threadIdx.x == 0) sh_nnz = sh_mx = 0u;
+  __syncthreads();
+  nnz = __reduce_add_sync(FULLMASK, nnz);
   mx = __reduce_max_sync(FULLMASK, mx);
-  if (lane == 0) {
-    for (int k = 0; k < 8; k++) sh[w][k] = acc[k];
-    sh[w][8] = (double)mx;
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(&sh_nnz, (unsigned)nnz);
+    atomicMax(&sh_mx, (unsigned)mx);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    double out[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int ww = 0; ww < kReduceThreads / 32; ww++) {
-      for (int k = 0; k < 8; k++) out[k] += sh[ww][k];
-      out[8] = fmax(out[8], sh[ww][8]);
-    }
-    for (int k = 0; k < 9; k++) P->part[(size_t)b * kPartStride + k] = out[k];
-    __threadfence();
-    unsigned prev = atomicAdd(&P->counter[0], 1u);
-    last = (prev == (unsigned)(nb - 1));
+    atomicAdd(&P->run_nnz, (unsigned long long)sh_nnz);
+    atomicMax(&P->run_max, sh_mx);
   }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  sum_partials<9, true>(P->part, nb, buf, tot);
+  if (!sum_blocks<G, 7>(P, acc, b, nb, &P->counter[0], tot)) return;
   if (threadIdx.x != 0) return;
   P->counter[0] = 0;
-  pass_finished(B, P, tot[6], tot[7], tot[8]);
+  pass_finished(B, P, tot[6], (double)__ldcg(&P->run_nnz), (double)__ldcg(&P->run_max));
+  P->run_nnz = 0ull;
+  P->run_max = 0u;
   for (int k = 0; k < 6; k++) P->grad[k] = tot[k];
   // float normalisation of the stacked gradient (CvoGPU.cu:2096-2104)
   float f[6];
@@ -302,32 +340,39 @@ __device__ void finalize_iteration(BatchDev &B, PairDev *P, const KParams &K) {
 }
 
 // -------------------------------------------------------------------- step
+// 1 / (2 l^2), rounded from double.
+__device__ __forceinline__ float step_coef(float l) {
+  return __double2float_rn(__ddiv_rn(1.0, dm(dm(2.0, (double)l), (double)l)));
+}
+
 // Taylor step-size terms (compute_step_size_xi + compute_step_size_poly_coeff,
-// src/cvo/CvoGPU.cu:333-462) per ELL row in FP32, one entry after the other (see k_rowsum),
+// src/cvo/CvoGPU.cu:333-462) per ELL row in FP32, one entry after the other (see row_sums),
 // FP64 across rows; the last block of a pair adds the blocks' sums and finishes the iteration.
-// Bounds: L2 latency of index -> position, then the scalar tail in FP64.
+// Bounds: issue (some 100 instructions per 32 entries), then the scalar tail.
+template <int G>
 __global__ void __launch_bounds__(kStepThreads) k_step(BatchDev B, KParams K) {
-  __shared__ double sh[kStepThreads / 32][4];
-  __shared__ double buf[kReduceThreads * 4], tot[4];
-  __shared__ bool last;
+  __shared__ __align__(16) float buf[kStepThreads / 32][RowLists<G>::kWarp];
+  __shared__ double tot[4];
+  __shared__ float sh_coef;
   const int blk = blockIdx.x;
   if (blk >= B.total_sblocks) return;
   const int p = find_segment(B.sblk_off, B.npairs, blk);
   PairDev *P = &B.pairs[p];
   if (P->done) return;
-  const int b = blk - B.sblk_off[p];
-  const int nb = B.sblk_off[p + 1] - B.sblk_off[p];
-  const int n = P->n;
-  const int s = b * kStepThreads + threadIdx.x;
-  float Bs = 0.f, Cs = 0.f, Ds = 0.f, Es = 0.f;
-  if (s < n) {
-    const float w0 = P->xi[0], w1 = P->xi[1], w2 = P->xi[2];
-    const float u0v = P->xi[3], u1v = P->xi[4], u2v = P->xi[5];
-    float4 x = __ldg(&P->xs[s]);
-    float tl = K.use_range_ell_step ? range_ell(P->ell, x.w) : P->ell;
-    float coef = __double2float_rn(__ddiv_rn(1.0, dm(dm(2.0, (double)tl), (double)tl)));
-    const int z = P->nnz_row[s];
-    auto add = [&](float a, const float4 &y) {
+  const int b = blk - B.sblk_off[p], nb = B.sblk_off[p + 1] - B.sblk_off[p], n = P->n;
+  const float w0 = P->xi[0], w1 = P->xi[1], w2 = P->xi[2];
+  const float u0v = P->xi[3], u1v = P->xi[4], u2v = P->xi[5];
+  if (threadIdx.x == 0) sh_coef = step_coef(P->ell);
+  __syncthreads();
+  const float coef0 = sh_coef;
+  double sum = 0.0;
+  for (int s = b * B.step_rows + (int)threadIdx.x / G; s - (int)threadIdx.x / G < min(n, (b + 1) * B.step_rows);
+       s += kStepThreads / G) {
+    const bool has = s < n;
+    const int z = has ? P->nnz_row[s] : 0;
+    const float4 x = has ? __ldg(&P->xs[s]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float coef = K.use_range_ell_step ? step_coef(range_ell(P->ell, x.w)) : coef0;
+    sum += (double)row_sums<G, 4>(P, has ? s : 0, z, buf[threadIdx.x >> 5], [&](const float4 &y, float (&X)[4]) {
       float ux = w1 * y.z - w2 * y.y + u0v, uy = w2 * y.x - w0 * y.z + u1v, uz = w0 * y.y - w1 * y.x + u2v;
       float px = w1 * uz - w2 * uy, py = w2 * ux - w0 * uz, pz = w0 * uy - w1 * ux;          // xi^2 z
       float qx = w1 * pz - w2 * py, qy = w2 * px - w0 * pz, qz = w0 * py - w1 * px;          // xi^3 z
@@ -341,33 +386,13 @@ __global__ void __launch_bounds__(kStepThreads) k_step(BatchDev B, KParams K) {
       float delta = 2.f * coef * (xiz_dot_xi2z - (qx * dx + qy * dy + qz * dz));
       float epsil = -coef * (epsil_const + 2.f * (rx * dx + ry * dy + rz * dz));
       float b2 = beta * beta;
-      Bs += a * beta;
-      Cs += a * (gamma + 0.5f * b2);
-      Ds += a * (delta + beta * gamma + b2 * beta * (1.f / 6.f));
-      Es += a * (epsil + beta * delta + 0.5f * b2 * gamma + 0.5f * gamma * gamma + b2 * b2 * (1.f / 24.f));
-    };
-    row_entries(P, s, z, add);
+      X[0] = beta;
+      X[1] = gamma + 0.5f * b2;
+      X[2] = delta + beta * gamma + b2 * beta * (1.f / 6.f);
+      X[3] = epsil + beta * delta + 0.5f * b2 * gamma + 0.5f * gamma * gamma + b2 * b2 * (1.f / 24.f);
+    });
   }
-  double v[4] = {Bs, Cs, Ds, Es};
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < 4; k++) v[k] = warp_sum(v[k]);
-  if (lane == 0)
-    for (int k = 0; k < 4; k++) sh[w][k] = v[k];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double o[4] = {0, 0, 0, 0};
-    for (int ww = 0; ww < kStepThreads / 32; ww++)
-      for (int k = 0; k < 4; k++) o[k] += sh[ww][k];
-    for (int k = 0; k < 4; k++) P->part[(size_t)b * kPartStride + k] = o[k];
-    __threadfence();
-    unsigned prev = atomicAdd(&P->counter[1], 1u);
-    last = (prev == (unsigned)(nb - 1));
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  sum_partials<4, false>(P->part, nb, buf, tot);
+  if (!sum_blocks<G, 4>(P, sum, b, nb, &P->counter[1], tot)) return;
   // The scalar tail is one thread's chain of dependent reads and writes of the pair's state:
   // in shared memory they cost 30 cycles instead of an L2 round trip each.
   __shared__ PairDev state;
@@ -558,7 +583,7 @@ namespace {
 struct BatchHost {
   BatchDev B;
   std::vector<PairDev> pairs;
-  std::vector<int> item_off, tgt_off, row_off, rblk_off, gblk_off, sblk_off;
+  std::vector<int> item_off, tgt_off, rblk_off, sblk_off;
   AssocKernels fn;
   int cand_blocks = 0, xform_blocks = 0;
   int window_words = 0;
@@ -637,8 +662,6 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
   }
   // sizes
   bh->item_off.assign(np + 1, 0);
-  bh->row_off.assign(np + 1, 0);
-  bh->gblk_off.assign(np + 1, 0);
   bh->tgt_off.assign(np + 1, 0);
   bh->rblk_off.assign(np + 1, 0);
   bh->sblk_off.assign(np + 1, 0);
@@ -653,6 +676,10 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
   const int order_cap = rows_all > 0 ? (int)std::min<long long>(4096, (16ll << 30) / (8ll * rows_all)) & ~3 : 0;
   const bool ell = mode != MODE_IP;                    // an inner product needs no kernel matrix
   std::vector<int> sp(np), caps(np), pitch(np);
+  // rows of a k_gradient or k_step block: 32 (four to a warp), or of large batches multiples of
+  // 64, so that some eight blocks per SM leave their sums to the last one
+  const long long per_block = rows_all / (8ll * sms);
+  const int step_rows = per_block <= kStepRows ? kStepRows : 64 * (int)((per_block + 63) / 64);
   for (int p = 0; p < np; p++) {
     int n = srcs[p]->n, m = tgts[p]->n;
     const int ns = group_count(group_count(m));
@@ -663,18 +690,14 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     pitch[p] = std::max(sp[p] * caps[p], bh->ordered ? std::min(capmax, m) : 0);
     bh->item_off[p + 1] = bh->item_off[p] + group_count(n) * sp[p];
     bh->tgt_off[p + 1] = bh->tgt_off[p] + m;
-    int rb = (n + kRowsPerBlock - 1) / kRowsPerBlock, sb = (n + kStepThreads - 1) / kStepThreads;
+    int rb = (n + kRowsPerBlock - 1) / kRowsPerBlock, sb = (n + step_rows - 1) / step_rows;
     bh->rblk_off[p + 1] = bh->rblk_off[p] + rb;
-    const int gb = (n + kReduceRows - 1) / kReduceRows;
-    bh->row_off[p + 1] = bh->row_off[p] + n;
-    bh->gblk_off[p + 1] = bh->gblk_off[p] + gb;
     bh->sblk_off[p + 1] = bh->sblk_off[p] + sb;
     add(sizeof(float4) * m);                                     // ycur
     add(sizeof(float4) * m);                                     // yorig
     add(ell ? sizeof(int) * (size_t)n * ell_ld : 0);             // ELL
     add(ell ? sizeof(float) * (size_t)n * ell_ld : 0);
     add(sizeof(uint2) * (size_t)n * pitch[p]);                   // candidate entries
-    if (mode == MODE_ALIGN) add(sizeof(float) * 8 * (size_t)n);  // row_sums
     add(sizeof(RankLevel) * lv[p].size());
     add(sizeof(int2) * (size_t)n * sp[p]);                       // entry counts
     add(sizeof(int) * n);                                        // nnz_row
@@ -683,8 +706,9 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     bytes += 12 * 256;                                           // room for empty pieces
   }
   add(sizeof(PairDev) * np);
-  add(sizeof(int) * (np + 1) * 6);
-  add(sizeof(int) * 4);
+  add(sizeof(int) * (np + 1) * 4);
+  add(sizeof(int) * 8);
+  add(sizeof(int) * (kRowsPerBlock / kRowsHeavy) * (size_t)bh->rblk_off[np]);      // groups of long rows
   add(sizeof(double));
   if ((rc = ensure_workspace(h, bytes))) return rc;
   Arena ar;
@@ -732,7 +756,6 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     P.cap = capmax;
     P.order_cap = bh->ordered ? order_cap : 0;
     P.src_norm = s->max_norm;
-    if (mode == MODE_ALIGN) P.row_sums = ar.take<float>(8 * (size_t)s->n);
     if (bh->ordered) {
       RankLevel *levels = ar.take<RankLevel>(lv[p].size());
       CVO_CUDA_TRY(h, cudaMemcpyAsync(levels, lv[p].data(), sizeof(RankLevel) * lv[p].size(), cudaMemcpyHostToDevice, h->stream));
@@ -745,16 +768,17 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     if (!P.done) active++;
   }
   PairDev *pairs_d = ar.take<PairDev>(np);
-  int *offs_d = ar.take<int>((size_t)(np + 1) * 6);
-  int *ctr_d = ar.take<int>(4);
+  int *offs_d = ar.take<int>((size_t)(np + 1) * 4);
+  int *ctr_d = ar.take<int>(8);
+  int *heavy_d = ar.take<int>((kRowsPerBlock / kRowsHeavy) * (size_t)bh->rblk_off[np]);
   double *bytes_d = ar.take<double>(1);
   // zero counters of every pair
   for (int p = 0; p < np; p++) CVO_CUDA_TRY(h, cudaMemsetAsync(bh->pairs[p].counter, 0, 2 * sizeof(unsigned), h->stream));
   CVO_CUDA_TRY(h, cudaMemcpyAsync(pairs_d, bh->pairs.data(), sizeof(PairDev) * np, cudaMemcpyHostToDevice, h->stream));
   std::vector<int> offs;
-  for (auto *v : {&bh->item_off, &bh->tgt_off, &bh->rblk_off, &bh->sblk_off, &bh->row_off, &bh->gblk_off}) offs.insert(offs.end(), v->begin(), v->end());
+  for (auto *v : {&bh->item_off, &bh->tgt_off, &bh->rblk_off, &bh->sblk_off}) offs.insert(offs.end(), v->begin(), v->end());
   CVO_CUDA_TRY(h, cudaMemcpyAsync(offs_d, offs.data(), sizeof(int) * offs.size(), cudaMemcpyHostToDevice, h->stream));
-  int ctr_h[4] = {0, 0, active, 0};
+  int ctr_h[8] = {0, 0, active, 0, 0, 0, 0, 0};
   CVO_CUDA_TRY(h, cudaMemcpyAsync(ctr_d, ctr_h, sizeof(ctr_h), cudaMemcpyHostToDevice, h->stream));
   CVO_CUDA_TRY(h, cudaMemsetAsync(bytes_d, 0, sizeof(double), h->stream));
   CVO_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
@@ -762,21 +786,20 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
   memset(&B, 0, sizeof(B));
   B.npairs = np;
   B.total_items = bh->item_off[np];
-  B.total_rows = (int)rows_all;
+  B.step_rows = step_rows;
   B.total_targets = bh->tgt_off[np];
   B.pairs = pairs_d;
   B.item_off = offs_d;
   B.tgt_off = offs_d + (np + 1);
   B.rblk_off = offs_d + 2 * (np + 1);
   B.sblk_off = offs_d + 3 * (np + 1);
-  B.row_off = offs_d + 4 * (np + 1);
-  B.gblk_off = offs_d + 5 * (np + 1);
-  B.total_gblocks = bh->gblk_off[np];
   B.total_rblocks = bh->rblk_off[np];
   B.total_sblocks = bh->sblk_off[np];
   B.err = ctr_d + 1;
   B.active = ctr_d + 2;
   B.active_iters = ctr_d + 3;
+  B.heavy = heavy_d;
+  B.heavy_ctr = ctr_d + 4;
   B.assoc_bytes = bytes_d;
   {
     int fch = K.use_int ? (F + 3) / 4 : 0, lch = K.use_sem ? label_chunks(C) : 0;
@@ -815,21 +838,28 @@ void launch_association(Handle *h, BatchHost *bh, const KParams &K, bool align =
     rows[ROWS_LIGHT]<<<blocks, 32 * kRowWarps, sizeof(int) * kRowSorted * kRowWarps, h->stream>>>(B, K, 0, 1);
     h->launches++;
   }
-  rows[ROWS_ALL]<<<blocks * (kRowsPerBlock / kRowsHeavy), 32 * kRowWarps, bh->row_smem, h->stream>>>(B, K, bh->window_words, split);
+  const int groups = blocks * (kRowsPerBlock / kRowsHeavy), resident = 5 * (h->num_sms > 0 ? h->num_sms : 152);
+  rows[ROWS_ALL]<<<split ? std::min(groups, resident) : groups, 32 * kRowWarps, bh->row_smem, h->stream>>>(B, K, bh->window_words, split);
   h->launches += 2;
+  if (split && !align) {
+    k_rows_total<<<B.npairs, 32 * kRowWarps, 0, h->stream>>>(B);
+    h->launches++;
+  }
   mark(h, ev, 6);
   if (align) {
-    k_rowsum<<<std::max((B.total_rows + 127) / 128, 1), 128, 0, h->stream>>>(B, K);
     mark(h, ev, 2);
-    k_reduce<<<std::max(B.total_gblocks, 1), kReduceThreads, 0, h->stream>>>(B, K);
-    h->launches += 2;
+    k_gradient<<<std::max(B.total_sblocks, 1), kStepThreads, 0, h->stream>>>(B, K);
+    h->launches++;
   }
   mark(h, ev, 3);
 }
 
 void launch_iteration(Handle *h, BatchHost *bh, const KParams &K, const cudaEvent_t *ev = nullptr) {
   launch_association(h, bh, K, true, ev);
-  k_step<<<std::max(bh->B.total_sblocks, 1), kStepThreads, 0, h->stream>>>(bh->B, K);
+  // Four lanes a row take fewer instructions per entry (lane t adds term t, and there are four);
+  // eight lanes keep the SMs busy when the rows are few.
+  const bool few = bh->B.step_rows == kStepRows;
+  (few ? k_step<8> : k_step<4>)<<<std::max(bh->B.total_sblocks, 1), kStepThreads, 0, h->stream>>>(bh->B, K);
   mark(h, ev, 4);
   h->launches += 1;
 }

@@ -117,7 +117,6 @@ struct PairDev {
   const float *tf, *tl;           // target features / labels, original order (float4 chunks)
   const float2 *tg;               // target geometric types, original order
   int *nnz_row;                   // n
-  float *row_sums;                // align: n * 8, omega(3)/c, v(3)/d
   // align and edges: orders of the target's points, finest lattice first, and the largest search radius
   // each serves; a row that kept more than cap + order_cap pairs stays in index order
   const RankLevel *levels;
@@ -126,13 +125,15 @@ struct PairDev {
   float src_norm;                 // largest |x| of the source
   double *part;                   // block partials
   unsigned int *counter;          // last-block counters [2]
+  unsigned long long run_nnz;     // kept pairs and longest row of the pass so far
+  unsigned int run_max;
   int F, C;                       // feature / label dimensions (source and target agree)
   int capmax;
   int mode;                       // 0 align, 1 inner product, 2 export, 3 edges of a window
   // iteration state
   float R[9], T[3];               // internal pose
   float Ri[9], Ti[3];             // target transform R^T, -R^T T
-  float ell, step_coef;           // step_coef: 1 / (2 ell^2), rounded from double
+  float ell;
   int cap;
   int iter, done, ret;
   float xi[6];
@@ -153,17 +154,16 @@ struct PairDev {
 struct BatchDev {
   int npairs;
   int total_items;                // work items of k_cand over all pairs (tiles x splits)
-  int total_rows;                 // sum of n
+  int step_rows;                  // rows of a k_gradient or k_step block
   int total_targets;              // sum of m
   PairDev *pairs;                 // device array
   const int *item_off;            // npairs + 1 (prefix of work items)
   const int *tgt_off;             // npairs + 1 (prefix of m)
   int *err;                       // error word (0 ok)
-  const int *row_off;             // npairs + 1 (prefix of n)
   const int *rblk_off;            // row-pass blocks per pair (prefix)
-  const int *gblk_off;            // k_reduce blocks per pair (prefix)
-  const int *sblk_off;            // step blocks per pair (prefix)
-  int total_rblocks, total_gblocks, total_sblocks;
+  const int *sblk_off;            // k_gradient and k_step blocks per pair (prefix)
+  int total_rblocks, total_sblocks;
+  int *heavy, *heavy_ctr;         // groups of long rows (see k_rows); their number, the next one
   int *active;                    // number of pairs not done
   int *active_iters;              // iterations that started with an active pair
   double *assoc_bytes;            // algorithmic bytes of the association passes

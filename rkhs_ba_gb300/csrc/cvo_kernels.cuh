@@ -8,7 +8,7 @@
 //                the groups that remain; one bit per pair that may be kept
 //   k_rows       each row's candidates in ascending target index: exact kernel value,
 //                threshold, the first cap kept ones to the ELL row    (CvoGPU.cu:951-1099)
-//   k_rowsum, k_reduce   gradient sums of the rows and of the pair (CvoGPU.cu:2001-2120);
+//   k_gradient   gradient sums of the rows and of the pair (CvoGPU.cu:2001-2120);
 //                single passes sum in k_rows instead
 //   k_step       Taylor step-size terms over the ELL rows; the last block of each pair
 //                runs the scalar tail of the iteration: cubic roots, step clamp,
@@ -22,8 +22,7 @@ namespace cvo_gb {
 
 enum { MODE_ALIGN = 0, MODE_IP = 1, MODE_EXPORT = 2, MODE_EDGES = 3 };
 constexpr int kStepThreads = 256;
-constexpr int kReduceRows = 1024;
-constexpr int kReduceThreads = 256;
+constexpr int kStepRows = 32;           // fewest rows of a block of the gradient and step kernels
 constexpr int kPartStride = 12;
 
 // ------------------------------------------------------------ pair value
@@ -471,7 +470,7 @@ __device__ __forceinline__ int warp_excl_scan(int v, int lane, int &total) {
 // Sums (all but align): FP32 per lane and row, over the lanes, FP64 from there; the last block
 // of a pair adds the blocks' sums in a fixed order.
 // ROWS_ORDERED: the entries of a row go to the order of the pair's level (RankLevel), in which
-// k_rowsum, k_step and k_irls_accum add them one by one.  The align loop and the window solve
+// k_gradient, k_step and k_irls_accum add them one by one.  The align loop and the window solve
 // turn a different last bit of the gradient into a visibly different pose some tens of
 // iterations later, so the order is part of the result and is kept whatever finds the pairs.
 // A row with no more than cap candidates is sorted and evaluated by rank from the start; a
@@ -480,9 +479,10 @@ __device__ __forceinline__ int warp_excl_scan(int v, int lane, int &total) {
 // pairs that k_cand is sure of; the rest are evaluated that far (eight pairs of 20k-50k
 // points had 7 % of the rows evaluated to 4,353 pairs, 60 % of all evaluations).
 // Two instances share the rows of large targets: ROWS_LIGHT those of up to 128 candidates, with
-// hardly any shared memory, 32 rows to a block; ROWS_ALL the others, or all rows of targets
-// whose bitmap is small anyway, eight rows to a block, handed to the warps one by one (rows of
-// 0 to cap pairs lie in clusters: blocks of 32 rows left a tail of a third of the launch).
+// hardly any shared memory, 32 rows to a block; ROWS_ALL the others, which ROWS_LIGHT lists by
+// groups of eight rows, or all rows of targets whose bitmap is small anyway.  Its blocks take
+// eight rows at a time and hand them to their warps one by one (rows of 0 to cap pairs lie in
+// clusters: blocks of 32 rows left a tail of a third of the launch).
 // Bounds: latency of the dependent steps entry -> permutation -> bitmap -> record, hidden by
 // the resident warps.  The rows' FP64 constants are computed up to 32 rows at a time: once per
 // warp and row they took most of a pass over rows without candidates.
@@ -491,7 +491,7 @@ constexpr int kRowsPerBlock = kGroup;
 constexpr int kRowsHeavy = 8;           // rows of a ROWS_ALL block
 constexpr int kRowSlots = 1 + kRowsPerBlock / kRowsHeavy;      // partial sums of 32 rows: ROWS_LIGHT, ROWS_ALL
 constexpr int kMaxSplits = 16;
-constexpr int kRowWindow = 63 * 1024;   // most target indices of one bitmap window (the queue's 16 bits)
+constexpr int kRowWindow = 15 * 4096;   // most target indices of one bitmap window (the queue's 16 bits)
 constexpr int kRowBatch = 256;          // candidates taken from the bitmap before they are evaluated
 constexpr int kRowSorted = 128;         // most candidates a sorting network puts in order
 constexpr int kRowSplitTargets = 8192;  // larger targets: ROWS_LIGHT and ROWS_ALL
@@ -501,22 +501,21 @@ constexpr int kRowSplitTargets = 8192;  // larger targets: ROWS_LIGHT and ROWS_A
 enum { ROWS_SUM = 0, ROWS_ORDERED = 1 };
 enum { ROWS_ALL = 0, ROWS_LIGHT = 1 };
 
-// Words of one warp's bitmap for targets of up to m points: an odd number per lane, so
-// that the lanes' runs start in different banks.
+// Words of one warp's bitmap for targets of up to m points: four times an odd number per lane,
+// so that 16-byte loads of the lanes' runs meet distinct banks.
 __host__ __device__ inline int row_window_words(int m) {
-  return 32 * ((((m < kRowWindow ? m : kRowWindow) + 1023) / 1024) | 1);
+  return 32 * 4 * ((((m < kRowWindow ? m : kRowWindow) + 4095) / 4096) | 1);
 }
-// Words of its queue (16 bits an index, a batch and the 1024 of one step more; or 128 sorted
-// candidates), which also holds a 16-bit count before each word of the bitmap.
-__host__ __device__ inline int row_queue_words(int window_words) {
-  return window_words / 2 > (kRowBatch + 1024) / 2 ? window_words / 2 : (kRowBatch + 1024) / 2;
-}
+// Words of its queue: 16 bits an index, a batch and the 1024 of one step more; also 128 sorted
+// candidates, and a 16-bit count before every four words of the bitmap.
+constexpr int kRowQueueWords = (kRowBatch + 1024) / 2;
+
 __host__ __device__ inline size_t row_smem_bytes(int m) {
-  return (size_t)kRowWarps * sizeof(uint32_t) * (row_window_words(m) + row_queue_words(row_window_words(m)));
+  return (size_t)kRowWarps * sizeof(uint32_t) * (row_window_words(m) + kRowQueueWords);
 }
 
 // Puts the z entries of an ELL row, which are in index order, in the order of the ranks:
-// their bits in a bitmap over the ranks, a count before every word, and each entry's slot is
+// their bits in a bitmap over the ranks, a count before every four words, and each entry's slot is
 // the number of bits below its own.  tmp: z entries.  All lanes call it.
 __device__ __forceinline__ void order_row(int *Aj, float *Av, int z, const int *rank, int m, uint32_t *bits, int window_words,
                                           unsigned short *before, uint2 *tmp, int lane) {
@@ -531,19 +530,28 @@ __device__ __forceinline__ void order_row(int *Aj, float *Av, int z, const int *
       if (k < 32u * (uint32_t)window_words) atomicOr(&bits[k >> 5], 1u << (k & 31));
     }
     __syncwarp();
+    const uint4 *run_bits = reinterpret_cast<const uint4 *>(bits + lane * wl);
     int run = 0, total;
-    for (int i = 0; i < wl; i++) run += __popc(bits[lane * wl + i]);
+    for (int i = 0; i < wl / 4; i++) {
+      const uint4 v = run_bits[i];
+      run += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
+    }
     run = warp_excl_scan(run, lane, total);
-    for (int i = 0; i < wl; i++) {
-      before[lane * wl + i] = (unsigned short)run;      // within the window: below 65536
-      run += __popc(bits[lane * wl + i]);
+    for (int i = 0; i < wl / 4; i++) {
+      const uint4 v = run_bits[i];
+      before[lane * (wl / 4) + i] = (unsigned short)run;      // below 65536
+      run += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
     }
     __syncwarp();
     for (int c = lane; c < z; c += 32) {
       const int j = Aj[c];
       const uint32_t k = (uint32_t)(__ldg(&rank[j]) - w0);
-      if (k < 32u * (uint32_t)window_words)
-        tmp[base + before[k >> 5] + __popc(bits[k >> 5] & ((1u << (k & 31)) - 1u))] = make_uint2((uint32_t)j, __float_as_uint(Av[c]));
+      if (k < 32u * (uint32_t)window_words) {
+        const uint4 v = reinterpret_cast<const uint4 *>(bits)[k >> 7];
+        const uint32_t w = (k >> 5) & 3u, own = w == 0 ? v.x : w == 1 ? v.y : w == 2 ? v.z : v.w;
+        const int lower = (w > 0 ? __popc(v.x) : 0) + (w > 1 ? __popc(v.y) : 0) + (w > 2 ? __popc(v.z) : 0);
+        tmp[base + before[k >> 7] + lower + __popc(own & ((1u << (k & 31)) - 1u))] = make_uint2((uint32_t)j, __float_as_uint(Av[c]));
+      }
     }
     base += total;
   }
@@ -597,22 +605,14 @@ __device__ __forceinline__ void pass_finished(const BatchDev &B, PairDev *P, dou
   P->max_row = (int)mx;
 }
 
-// Sums of a single pass (value, kept pairs, longest row) of one block -> slot; the last of nb
-// blocks adds the slots first .. first + slots - 1 and finishes the pass.
+// Sums of a single pass (value, kept pairs, longest row) of one block -> slot; sum_slots adds the
+// slots first .. first + slots - 1 and finishes the pass.
 __device__ __forceinline__ void rows_partial(PairDev *P, int slot, const double (&t)[3]) {
   for (int k = 0; k < 3; k++) P->part[(size_t)slot * kPartStride + k] = t[k];
 }
-__device__ __forceinline__ void rows_finish(const BatchDev &B, PairDev *P, int nb, int first, int slots) {
+__device__ __forceinline__ void sum_slots(const BatchDev &B, PairDev *P, int first, int slots) {
   __shared__ double sh[kRowWarps][3];
-  __shared__ bool last;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (threadIdx.x == 0) {
-    __threadfence();
-    last = atomicAdd(&P->counter[0], 1u) == (unsigned)(nb - 1);
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
   double t[3] = {0, 0, 0};
 #pragma unroll 8
   for (int q = threadIdx.x; q < slots; q += 32 * kRowWarps) {
@@ -633,8 +633,20 @@ __device__ __forceinline__ void rows_finish(const BatchDev &B, PairDev *P, int n
     t[k] = sh[0][k];
     for (int q = 1; q < kRowWarps; q++) t[k] = k < 2 ? t[k] + sh[q][k] : fmax(t[k], sh[q][k]);
   }
-  P->counter[0] = 0;
   pass_finished(B, P, t[0], t[1], t[2]);
+}
+// Without ROWS_LIGHT: the last of the pair's nb blocks.
+__device__ __forceinline__ void rows_finish(const BatchDev &B, PairDev *P, int nb, int first, int slots) {
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(&P->counter[0], 1u) == (unsigned)(nb - 1);
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  sum_slots(B, P, first, slots);
+  if (threadIdx.x == 0) P->counter[0] = 0;
 }
 
 // split: ROWS_LIGHT has taken the rows of up to 128 candidates.
@@ -648,16 +660,26 @@ __global__ void __launch_bounds__(32 * kRowWarps, PART == ROWS_LIGHT && LCH == 0
   __shared__ int4 sh_tot[RB];                              // of the row, and pairs surely kept; entries < 0: scan all targets
   __shared__ double sh_sum[RB];                            // the rows' sums and kept pairs
   __shared__ int sh_kept[RB];
-  __shared__ int next_row;
+  __shared__ int next_row, item;
   __shared__ float4 sh_keep[kRowWarps][64];                // kept pairs by slot: y and value
   __shared__ int sh_keepj[kRowWarps][64];
   constexpr int FP = FCH > 0 ? FCH : 1;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   constexpr int SUBS = kRowsPerBlock / RB;                 // blocks of a source tile
-  uint32_t *bits = row_smem + (size_t)w * (PART == ROWS_LIGHT ? kRowSorted : window_words + row_queue_words(window_words));
+  uint32_t *bits = row_smem + (size_t)w * (PART == ROWS_LIGHT ? kRowSorted : window_words + kRowQueueWords);
   int *sorted = reinterpret_cast<int *>(PART == ROWS_LIGHT ? bits : bits + window_words);
   unsigned short *queue = reinterpret_cast<unsigned short *>(sorted);
-  const int blk = blockIdx.x / SUBS, part = blockIdx.x % SUBS;
+  while (true) {
+  // ROWS_ALL after ROWS_LIGHT: the next listed group of rows; otherwise the block's own
+  int group = blockIdx.x;
+  if (PART == ROWS_ALL && split) {
+    __syncthreads();      // the last item's shared memory has been read
+    if (threadIdx.x == 0) item = atomicAdd(&B.heavy_ctr[1], 1);
+    __syncthreads();
+    if (item >= __ldcg(&B.heavy_ctr[0])) return;
+    group = __ldcg(&B.heavy[item]);
+  }
+  const int blk = group / SUBS, part = group % SUBS;
   if (blk >= B.total_rblocks) return;
   const int p = find_segment(B.rblk_off, B.npairs, blk);
   PairDev *P = &B.pairs[p];
@@ -694,6 +716,16 @@ __global__ void __launch_bounds__(32 * kRowWarps, PART == ROWS_LIGHT && LCH == 0
       if (!fits) t.x = -1;
       if (cap <= 0 || s >= n) t.x = 0;
       const bool light = t.x >= 0 && t.y <= kRowSorted;
+      if (PART == ROWS_LIGHT) {
+        constexpr int groups = kRowsPerBlock / kRowsHeavy;
+        const unsigned heavy = __ballot_sync(FULLMASK, t.x != 0 && !light);
+        if (lane < groups) {
+          if (heavy >> (kRowsHeavy * lane) & ((1u << kRowsHeavy) - 1u))
+            B.heavy[atomicAdd(&B.heavy_ctr[0], 1)] = groups * blk + lane;
+          else if (mode != MODE_ALIGN)
+            for (int k = 0; k < 3; k++) P->part[(size_t)(nb + groups * b + lane) * kPartStride + k] = 0.0;
+        }
+      }
       if (s < n && t.x == 0 && (PART == ROWS_LIGHT || !split)) P->nnz_row[s] = 0;
       if (PART == ROWS_LIGHT ? !light : split && light) t.x = 0;      // the other instance's
       here = t.x != 0;
@@ -780,9 +812,11 @@ __global__ void __launch_bounds__(32 * kRowWarps, PART == ROWS_LIGHT && LCH == 0
           const uint2 v = entry(e0 + lane);
           int o, add;
           o = n + warp_excl_scan(__popc(v.y), lane, add);
-          for (uint32_t mk = v.y; mk; mk &= mk - 1) sorted[o++] = __ldg(&perm[32 * (int)v.x + __ffs(mk) - 1]);
+          for (uint32_t mk = v.y; mk; mk &= mk - 1) sorted[o++] = 32 * (int)v.x + __ffs(mk) - 1;
           n += add;
         }
+        __syncwarp();
+        for (int i = lane; i < n; i += 32) sorted[i] = __ldg(&perm[sorted[i]]);      // not in the loop over bits: a chain of loads
         __syncwarp();
         if (n <= 32) warp_sort<1>(sorted, n, lane);
         else if (n <= 64) warp_sort<2>(sorted, n, lane);
@@ -814,7 +848,18 @@ __global__ void __launch_bounds__(32 * kRowWarps, PART == ROWS_LIGHT && LCH == 0
           uint32_t mk = bits[pos + lane];
           if (!__any_sync(FULLMASK, mk != 0)) continue;
           int add, o = qn + warp_excl_scan(__popc(mk), lane, add);
-          for (; mk; mk &= mk - 1) queue[o++] = (unsigned short)(32 * (pos + lane) + __ffs(mk) - 1);
+          uint32_t words = __ballot_sync(FULLMASK, mk != 0);
+          if (__popc(words) <= __reduce_max_sync(FULLMASK, __popc(mk))) {
+            // few words, some of them dense: word by word, a bit a lane
+            for (; words; words &= words - 1) {
+              const int src = __ffs(words) - 1;
+              const uint32_t v = __shfl_sync(FULLMASK, mk, src);
+              const int at = __shfl_sync(FULLMASK, o, src);
+              if ((v >> lane) & 1u) queue[at + __popc(v & ((1u << lane) - 1u))] = (unsigned short)(32 * (pos + src) + lane);
+            }
+          } else {
+            for (; mk; mk &= mk - 1) queue[o++] = (unsigned short)(32 * (pos + lane) + __ffs(mk) - 1);
+          }
           qn += add;
         }
         __syncwarp();
@@ -887,7 +932,10 @@ __global__ void __launch_bounds__(32 * kRowWarps, PART == ROWS_LIGHT && LCH == 0
       sh_kept[r] = z;
     }
   }
-  if (KIND == ROWS_ORDERED && mode == MODE_ALIGN) return;
+  if (KIND == ROWS_ORDERED && mode == MODE_ALIGN) {
+    if (PART == ROWS_ALL && split) continue;
+    return;
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
     double t[3] = {0.0, 0.0, 0.0};
@@ -898,7 +946,10 @@ __global__ void __launch_bounds__(32 * kRowWarps, PART == ROWS_LIGHT && LCH == 0
     }
     rows_partial(P, PART == ROWS_LIGHT ? b : nb + SUBS * b + part, t);
   }
-  if (PART == ROWS_ALL) rows_finish(B, P, SUBS * nb, split ? 0 : nb, (split ? kRowSlots : kRowSlots - 1) * nb);
+  if (PART == ROWS_ALL && split) continue;      // k_rows_total adds the slots
+  if (PART == ROWS_ALL) rows_finish(B, P, SUBS * nb, nb, (kRowSlots - 1) * nb);
+  return;
+  }
 }
 
 }  // namespace cvo_gb
