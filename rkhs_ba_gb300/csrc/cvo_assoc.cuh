@@ -14,12 +14,6 @@ inline int assoc_instances(AssocKernels *a) {
   a->rows[ROWS_LIGHT] = k_rows<FC, LC, G, ROWS_SUM, ROWS_LIGHT>;
   a->ordered_rows[ROWS_ALL] = k_rows<FC, LC, G, ROWS_ORDERED, ROWS_ALL>;
   a->ordered_rows[ROWS_LIGHT] = k_rows<FC, LC, G, ROWS_ORDERED, ROWS_LIGHT>;
-  // opt in above the 48 KB default (setting it again is harmless)
-  for (RowsFn f : {a->rows[ROWS_ALL], a->ordered_rows[ROWS_ALL]})
-    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem_bytes(kRowWindow)) != cudaSuccess) {
-      cudaGetLastError();
-      return CVO_ERR_CUDA;
-    }
   return 0;
 }
 

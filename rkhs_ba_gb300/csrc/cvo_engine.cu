@@ -586,8 +586,6 @@ struct BatchHost {
   std::vector<int> item_off, tgt_off, rblk_off, sblk_off;
   AssocKernels fn;
   int cand_blocks = 0, xform_blocks = 0;
-  int window_words = 0;
-  size_t row_smem = 0;
   bool split_rows = false;          // rows of few candidates in a launch of their own
   bool ordered = false;             // rows in the order of the targets' lattice (RankLevel)
 };
@@ -722,7 +720,7 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     DevCloud *s = srcs[p], *t = tgts[p];
     P.n = s->n; P.m = t->n; P.F = F; P.C = C;
     P.xs = s->spos; P.xf = s->sfeat; P.xl = s->slab; P.xg = s->sgeo; P.sbox = s->gbox;
-    P.tpos = t->spos; P.tperm = t->sperm; P.tfs = t->sfeat; P.tbox = t->gbox; P.tsup = t->sbox;
+    P.tpos = t->spos; P.tperm = t->sperm; P.tfs = t->sfeat; P.tbox = t->gbox; P.tsup = t->sbox; P.trange = t->grange;
     P.groups = group_count(t->n);
     P.ycur = ar.take<float4>(t->n);
     P.yorig = ar.take<float4>(t->n);
@@ -807,8 +805,6 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
   }
   bh->cand_blocks = K.use_mma ? (B.total_items + kCandWarps - 1) / kCandWarps : 0;
   bh->xform_blocks = (B.total_targets + 255) / 256;
-  bh->window_words = row_window_words(maxm);
-  bh->row_smem = row_smem_bytes(maxm);
   bh->split_rows = K.use_mma && maxm > kRowSplitTargets;
   return 0;
 }
@@ -835,11 +831,11 @@ void launch_association(Handle *h, BatchHost *bh, const KParams &K, bool align =
   const RowsFn *rows = bh->ordered ? bh->fn.ordered_rows : bh->fn.rows;
   const int split = bh->split_rows ? 1 : 0, blocks = std::max(B.total_rblocks, 1);
   if (split) {
-    rows[ROWS_LIGHT]<<<blocks, 32 * kRowWarps, sizeof(int) * kRowSorted * kRowWarps, h->stream>>>(B, K, 0, 1);
+    rows[ROWS_LIGHT]<<<blocks, 32 * kRowWarps, 0, h->stream>>>(B, K, 1);
     h->launches++;
   }
   const int groups = blocks * (kRowsPerBlock / kRowsHeavy), resident = 5 * (h->num_sms > 0 ? h->num_sms : 152);
-  rows[ROWS_ALL]<<<split ? std::min(groups, resident) : groups, 32 * kRowWarps, bh->row_smem, h->stream>>>(B, K, bh->window_words, split);
+  rows[ROWS_ALL]<<<split ? std::min(groups, resident) : groups, 32 * kRowWarps, 0, h->stream>>>(B, K, split);
   h->launches += 2;
   if (split && !align) {
     k_rows_total<<<B.npairs, 32 * kRowWarps, 0, h->stream>>>(B);
@@ -875,8 +871,6 @@ void append_launch_key(const Handle *h, const BatchHost &bh, const KParams &K, s
   add(&bh.fn, sizeof(bh.fn));
   add(&bh.cand_blocks, sizeof(bh.cand_blocks));
   add(&bh.xform_blocks, sizeof(bh.xform_blocks));
-  add(&bh.window_words, sizeof(bh.window_words));
-  add(&bh.row_smem, sizeof(bh.row_smem));
   add(&bh.split_rows, sizeof(bh.split_rows));
   add(&h->stream, sizeof(h->stream));
 }

@@ -177,6 +177,15 @@ int dalloc(Handle *h, T **p, size_t count) {
   return 0;
 }
 
+// Lowest and highest original index of each group's points, a warp per group.
+__global__ void k_group_range(const int *sperm, int n, int ng, int2 *range) {
+  const int g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, i = 32 * g + (threadIdx.x & 31);
+  if (g >= ng) return;
+  const int j = i < n ? sperm[i] : sperm[n - 1];
+  const int lo = __reduce_min_sync(0xFFFFFFFFu, j), hi = __reduce_max_sync(0xFFFFFFFFu, j);
+  if ((threadIdx.x & 31) == 0) range[g] = make_int2(lo, hi);
+}
+
 }  // namespace
 
 // Device part of a cloud's construction from staged device arrays (xyz with stride
@@ -227,13 +236,15 @@ static int cloud_build(Handle *h, DevCloud *d, const float *xyz_d, int stride, c
   // boxes of the groups and supergroups
   const int ng = group_count(n), ns = group_count(ng), ch = box_chunks(d->FP);
   if ((rc = dalloc(h, &d->gbox, (size_t)(2 + 2 * ch) * ng)) || (rc = dalloc(h, &d->sbox, (size_t)(2 + 2 * ch) * ns))) return rc;
+  if ((rc = dalloc(h, &d->grange, ng))) return rc;
+  k_group_range<<<(ng + 3) / 4, 128, 0, h->stream>>>(d->sperm, n, ng, d->grange);
   k_boxes<0><<<(ng + 3) / 4, 128, 0, h->stream>>>(d->spos, reinterpret_cast<const float4 *>(d->sfeat), d->FP / 4, n, ch,
                                                   d->gbox, ng);
   k_boxes<1><<<(ns + 3) / 4, 128, 0, h->stream>>>(d->gbox, nullptr, 0, ng, ch, d->sbox, ns);
   const int tiles = (n + 127) / 128;
   float *ext_d = reinterpret_cast<float *>(keys);
   k_tile_extent<<<(tiles + 127) / 128, 128, 0, h->stream>>>(d->gbox, ng, tiles, ext_d);
-  h->launches += 3;
+  h->launches += 4;
   std::vector<float> ext_h(tiles);
   CVO_CUDA_TRY(h, cudaMemcpyAsync(ext_h.data(), ext_d, sizeof(float) * tiles, cudaMemcpyDeviceToHost, h->stream));
   CVO_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
@@ -370,7 +381,7 @@ void cloud_free(DevCloud *d) {
   if (!d) return;
   cudaFree(d->pos); cudaFree(d->feat); cudaFree(d->lab); cudaFree(d->geo);
   cudaFree(d->sperm); cudaFree(d->spos); cudaFree(d->sfeat); cudaFree(d->slab); cudaFree(d->sgeo);
-  cudaFree(d->gbox); cudaFree(d->sbox);
+  cudaFree(d->gbox); cudaFree(d->sbox); cudaFree(d->grange);
   for (void *p : d->rank_allocs) cudaFree(p);
   delete d;
 }

@@ -61,6 +61,7 @@ struct DevCloud {
   // bounding boxes of the groups, then of the supergroups: float4 planes (position low,
   // high, feature low, feature high; box_planes of them) of one entry per group
   float4 *gbox = nullptr, *sbox = nullptr;
+  int2 *grange = nullptr;        // lowest and highest original index of a group's points
   std::map<int, RankLevel> ranks;          // by quantised cell size 2^(e/2), device arrays
   std::vector<void *> rank_allocs;
 };
@@ -103,6 +104,7 @@ struct PairDev {
   const int *tperm;               // tile-order position -> original index
   const float *tfs;
   const float4 *tbox, *tsup;      // boxes of groups and supergroups
+  const int2 *trange;             // lowest and highest original index of a group's points
   int groups;
   float4 *ycur;                   // transformed targets, tile order
   float4 *yorig;                  // transformed targets, original order
@@ -172,7 +174,7 @@ struct BatchDev {
 
 // Kernels of the association for a batch's feature and label strides (cvo_assoc_*.cu).
 using CandFn = void (*)(BatchDev, KParams);
-using RowsFn = void (*)(BatchDev, KParams, int, int);
+using RowsFn = void (*)(BatchDev, KParams, int);
 
 struct AssocKernels {
   CandFn cand = nullptr;

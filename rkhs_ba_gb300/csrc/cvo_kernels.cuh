@@ -15,6 +15,7 @@
 //                Exp_SEK3 pose update, SE(3) distance, lengthscale schedule, cap update
 //                                                               (CvoGPU.cu:333-544, 547-665, 1339-1433)
 #pragma once
+#include <climits>
 #include <cuda_fp16.h>
 #include "cvo_device.cuh"
 
@@ -461,7 +462,7 @@ __device__ __forceinline__ int warp_excl_scan(int v, int lane, int &total) {
 }
 
 // One warp per row.  The row's candidates (entries of k_cand) are put in ascending target index
-// -- up to 128 of them by a sorting network over the lanes, more through a bitmap over a window
+// -- up to 256 of them by a sorting network over the lanes, more through a bitmap over a window
 // of target indices in shared memory -- and evaluated 32 at a time with the exact arithmetic,
 // the next 32 records in flight.  The reference scans the targets by index and stops at cap kept
 // pairs (src/cvo/CvoGPU.cu:994-996): here the row stops there too, so no pair beyond cap is
@@ -473,8 +474,8 @@ __device__ __forceinline__ int warp_excl_scan(int v, int lane, int &total) {
 // k_gradient, k_step and k_irls_accum add them one by one.  The align loop and the window solve
 // turn a different last bit of the gradient into a visibly different pose some tens of
 // iterations later, so the order is part of the result and is kept whatever finds the pairs.
-// A row with no more than cap candidates is sorted and evaluated by rank from the start; a
-// longer one is cut by index first and its kept entries are then put in order.  One that kept
+// A row of up to 256 candidates and no more than cap is sorted and evaluated by rank from the
+// start; another is cut by index first and its kept entries are then put in order.  One that kept
 // more than cap + order_cap pairs stays in index order: nearly all such rows are told by the
 // pairs that k_cand is sure of; the rest are evaluated that far (eight pairs of 20k-50k
 // points had 7 % of the rows evaluated to 4,353 pairs, 60 % of all evaluations).
@@ -491,9 +492,13 @@ constexpr int kRowsPerBlock = kGroup;
 constexpr int kRowsHeavy = 8;           // rows of a ROWS_ALL block
 constexpr int kRowSlots = 1 + kRowsPerBlock / kRowsHeavy;      // partial sums of 32 rows: ROWS_LIGHT, ROWS_ALL
 constexpr int kMaxSplits = 16;
-constexpr int kRowWindow = 15 * 4096;   // most target indices of one bitmap window (the queue's 16 bits)
+// Target indices of one bitmap window.  Only the groups whose indices meet the window are
+// entered, and a row that is cut needs the first windows alone.  Small: 20 bitmaps of 60k
+// targets left the SM 6 KB of L1, and neighbouring rows read the same targets.
+constexpr int kRowWindow = 20 * 1024;
 constexpr int kRowBatch = 256;          // candidates taken from the bitmap before they are evaluated
-constexpr int kRowSorted = 128;         // most candidates a sorting network puts in order
+constexpr int kRowSorted = 256;         // most candidates a sorting network puts in order
+constexpr int kRowLight = 128;          // most candidates of a row of ROWS_LIGHT
 constexpr int kRowSplitTargets = 8192;  // larger targets: ROWS_LIGHT and ROWS_ALL
 
 // Whether a kernel instance leaves the rows' entries in index order (single passes) or puts
@@ -501,25 +506,85 @@ constexpr int kRowSplitTargets = 8192;  // larger targets: ROWS_LIGHT and ROWS_A
 enum { ROWS_SUM = 0, ROWS_ORDERED = 1 };
 enum { ROWS_ALL = 0, ROWS_LIGHT = 1 };
 
-// Words of one warp's bitmap for targets of up to m points: four times an odd number per lane,
-// so that 16-byte loads of the lanes' runs meet distinct banks.
-__host__ __device__ inline int row_window_words(int m) {
-  return 32 * 4 * ((((m < kRowWindow ? m : kRowWindow) + 4095) / 4096) | 1);
-}
-// Words of its queue: 16 bits an index, a batch and the 1024 of one step more; also 128 sorted
-// candidates, and a 16-bit count before every four words of the bitmap.
+// A warp's bitmap: four times an odd number of words per lane, so that 16-byte loads of the
+// lanes' runs meet distinct banks.  Its queue: 16 bits an index, a batch and the 1024 of one step
+// more; also sorted candidates, and a 16-bit count before every four words of the bitmap.
+constexpr int kRowWindowWords = kRowWindow / 32;
 constexpr int kRowQueueWords = (kRowBatch + 1024) / 2;
+static_assert(kRowWindow <= 65536 && kRowWindowWords / 32 % 8 == 4, "16-bit queue, banks");
 
-__host__ __device__ inline size_t row_smem_bytes(int m) {
-  return (size_t)kRowWarps * sizeof(uint32_t) * (row_window_words(m) + kRowQueueWords);
+// Sorts v: element 32 r + lane in register r of each lane, ascending, by a bitonic network.
+template <int R, class T>
+__device__ __forceinline__ void warp_sort(T (&v)[R], int lane) {
+#pragma unroll
+  for (int k = 2; k <= 32 * R; k <<= 1)
+#pragma unroll
+    for (int d = k >> 1; d > 0; d >>= 1) {
+      if (d >= 32) {
+#pragma unroll
+        for (int r = 0; r < R; r++)
+          if ((r & (d >> 5)) == 0) {
+            const T a = v[r], b = v[r | (d >> 5)];
+            const bool up = ((32 * r) & k) == 0;
+            v[r] = up ? min(a, b) : max(a, b);
+            v[r | (d >> 5)] = up ? max(a, b) : min(a, b);
+          }
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+          const T o = __shfl_xor_sync(FULLMASK, v[r], d);
+          const bool up = ((32 * r + lane) & k) == 0;
+          v[r] = ((lane & d) == 0) == up ? min(v[r], o) : max(v[r], o);
+        }
+      }
+    }
 }
 
-// Puts the z entries of an ELL row, which are in index order, in the order of the ranks:
+// Sorts list[0 .. count), count <= 32 R.
+template <int R>
+__device__ __forceinline__ void sort_list(int *list, int count, int lane) {
+  int v[R];
+#pragma unroll
+  for (int r = 0; r < R; r++) v[r] = 32 * r + lane < count ? list[32 * r + lane] : 0x7FFFFFFF;
+  warp_sort<R>(v, lane);
+#pragma unroll
+  for (int r = 0; r < R; r++) list[32 * r + lane] = v[r];
+}
+
+// Puts the z <= 32 R <= 512 entries of an ELL row, which are in index order, in the order of the
+// ranks: rank (22 bits) and slot sorted as one key.
+template <int R>
+__device__ __forceinline__ void order_row(int *Aj, float *Av, int z, const int *rank, int lane) {
+  uint32_t v[R];
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    const int c = 32 * r + lane;
+    v[r] = c < z ? (uint32_t)__ldg(&rank[Aj[c]]) << 9 | (uint32_t)c : 0xFFFFFFFFu;
+  }
+  warp_sort<R>(v, lane);
+  int j[R];
+  float a[R];
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    const bool has = 32 * r + lane < z;
+    j[r] = has ? Aj[v[r] & 511u] : 0;
+    a[r] = has ? Av[v[r] & 511u] : 0.f;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < R; r++)
+    if (32 * r + lane < z) {
+      Aj[32 * r + lane] = j[r];
+      Av[32 * r + lane] = a[r];
+    }
+}
+
+// The same for rows of more entries:
 // their bits in a bitmap over the ranks, a count before every four words, and each entry's slot is
 // the number of bits below its own.  tmp: z entries.  All lanes call it.
-__device__ __forceinline__ void order_row(int *Aj, float *Av, int z, const int *rank, int m, uint32_t *bits, int window_words,
-                                          unsigned short *before, uint2 *tmp, int lane) {
-  const int wl = window_words >> 5;
+__device__ __forceinline__ void order_long_row(int *Aj, float *Av, int z, const int *rank, int m, uint32_t *bits,
+                                               unsigned short *before, uint2 *tmp, int lane) {
+  constexpr int window_words = kRowWindowWords, wl = window_words >> 5;
   int base = 0;
   for (int w0 = 0; w0 < m && base < z; w0 += 32 * window_words) {
     __syncwarp();
@@ -561,39 +626,6 @@ __device__ __forceinline__ void order_row(int *Aj, float *Av, int z, const int *
     Aj[c] = (int)v.x;
     Av[c] = __uint_as_float(v.y);
   }
-}
-
-// Sorts queue[0 .. count), count <= 32 R, in ascending order: a bitonic network over element
-// 32 r + lane in register r of each lane.
-template <int R>
-__device__ __forceinline__ void warp_sort(int *queue, int count, int lane) {
-  int v[R];
-#pragma unroll
-  for (int r = 0; r < R; r++) v[r] = 32 * r + lane < count ? queue[32 * r + lane] : 0x7FFFFFFF;
-#pragma unroll
-  for (int k = 2; k <= 32 * R; k <<= 1)
-#pragma unroll
-    for (int d = k >> 1; d > 0; d >>= 1) {
-      if (d >= 32) {
-#pragma unroll
-        for (int r = 0; r < R; r++)
-          if ((r & (d >> 5)) == 0) {
-            const int a = v[r], b = v[r | (d >> 5)];
-            const bool up = ((32 * r) & k) == 0;
-            v[r] = up ? min(a, b) : max(a, b);
-            v[r | (d >> 5)] = up ? max(a, b) : min(a, b);
-          }
-      } else {
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-          const int o = __shfl_xor_sync(FULLMASK, v[r], d);
-          const bool up = ((32 * r + lane) & k) == 0;
-          v[r] = ((lane & d) == 0) == up ? min(v[r], o) : max(v[r], o);
-        }
-      }
-    }
-#pragma unroll
-  for (int r = 0; r < R; r++) queue[32 * r + lane] = v[r];
 }
 
 // Totals of an association pass.  Algorithmic bytes: every source and target record once, the
@@ -652,9 +684,10 @@ __device__ __forceinline__ void rows_finish(const BatchDev &B, PairDev *P, int n
 // split: ROWS_LIGHT has taken the rows of up to 128 candidates.
 template <int FCH, int LCH, bool GT, int KIND, int PART>
 __global__ void __launch_bounds__(32 * kRowWarps, PART == ROWS_LIGHT && LCH == 0 ? 6 : 5)
-    k_rows(BatchDev B, KParams K, int window_words, int split) {
+    k_rows(BatchDev B, KParams K, int split) {
   constexpr int RB = PART == ROWS_LIGHT ? kRowsPerBlock : kRowsHeavy;
-  extern __shared__ __align__(16) uint32_t row_smem[];
+  constexpr int kWords = PART == ROWS_LIGHT ? kRowLight : kRowWindowWords + kRowQueueWords;
+  __shared__ __align__(16) uint32_t row_smem[kRowWarps][kWords];      // bitmap and queue
   __shared__ float4 sh_rc[RB];                             // l, d2 threshold, 1 / (2 l^2)
   __shared__ int2 sh_cnt[kMaxSplits][RB];                  // entries and candidates per split
   __shared__ int4 sh_tot[RB];                              // of the row, and pairs surely kept; entries < 0: scan all targets
@@ -666,8 +699,8 @@ __global__ void __launch_bounds__(32 * kRowWarps, PART == ROWS_LIGHT && LCH == 0
   constexpr int FP = FCH > 0 ? FCH : 1;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   constexpr int SUBS = kRowsPerBlock / RB;                 // blocks of a source tile
-  uint32_t *bits = row_smem + (size_t)w * (PART == ROWS_LIGHT ? kRowSorted : window_words + kRowQueueWords);
-  int *sorted = reinterpret_cast<int *>(PART == ROWS_LIGHT ? bits : bits + window_words);
+  uint32_t *bits = row_smem[w];
+  int *sorted = reinterpret_cast<int *>(PART == ROWS_LIGHT ? bits : bits + kRowWindowWords);
   unsigned short *queue = reinterpret_cast<unsigned short *>(sorted);
   while (true) {
   // ROWS_ALL after ROWS_LIGHT: the next listed group of rows; otherwise the block's own
@@ -690,6 +723,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, PART == ROWS_LIGHT && LCH == 0
   const float4 *__restrict__ tf = reinterpret_cast<const float4 *>(P->tf);
   const float4 *__restrict__ tl = reinterpret_cast<const float4 *>(P->tl);
   const int *__restrict__ tperm = P->tperm;
+  const int2 *__restrict__ trange = P->trange;
   const int s0 = b * kRowsPerBlock + part * RB;
   {
     if (K.use_mma)
@@ -715,7 +749,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, PART == ROWS_LIGHT && LCH == 0
       }
       if (!fits) t.x = -1;
       if (cap <= 0 || s >= n) t.x = 0;
-      const bool light = t.x >= 0 && t.y <= kRowSorted;
+      const bool light = t.x >= 0 && t.y <= kRowLight;
       if (PART == ROWS_LIGHT) {
         constexpr int groups = kRowsPerBlock / kRowsHeavy;
         const unsigned heavy = __ballot_sync(FULLMASK, t.x != 0 && !light);
@@ -774,7 +808,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, PART == ROWS_LIGHT && LCH == 0
     };
     // by rank from the start if the row cannot be cut; otherwise by index, and on past cap only
     // to tell whether the row keeps more than cap + order_cap (it may, and is not sure to)
-    const bool ranked = KIND == ROWS_ORDERED && entries > 0 && cands <= cap;
+    const bool ranked = KIND == ROWS_ORDERED && entries > 0 && cands <= min(cap, kRowSorted);
     const int *perm = ranked ? lv->of_tile : tperm;
     const bool over = KIND == ROWS_ORDERED && sh_tot[r].z > cap + order_cap;
     const int stop = KIND == ROWS_ORDERED && !over && (entries < 0 || cands > cap + order_cap) ? cap + order_cap + 1 : cap;
@@ -801,7 +835,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, PART == ROWS_LIGHT && LCH == 0
     // w0) taken from the bitmap 32 words at a time, one a lane: the indices of a row lie in
     // clusters, and a run of words per lane left most lanes idle.
     const bool direct = entries < 0, listed = !direct && cands <= kRowSorted;
-    int w0 = 0, pos = 0, qn = 0;
+    int w0 = -1, w1 = 0, pos = 0, qn = 0;      // window, the next one, words read, queue
     bool filled = false;
     while (true) {
       int n = m;
@@ -818,33 +852,52 @@ __global__ void __launch_bounds__(32 * kRowWarps, PART == ROWS_LIGHT && LCH == 0
         __syncwarp();
         for (int i = lane; i < n; i += 32) sorted[i] = __ldg(&perm[sorted[i]]);      // not in the loop over bits: a chain of loads
         __syncwarp();
-        if (n <= 32) warp_sort<1>(sorted, n, lane);
-        else if (n <= 64) warp_sort<2>(sorted, n, lane);
-        else warp_sort<4>(sorted, n, lane);
+        if (n <= 32) sort_list<1>(sorted, n, lane);
+        else if (n <= 64) sort_list<2>(sorted, n, lane);
+        else if (PART == ROWS_LIGHT || n <= 128) sort_list<4>(sorted, n, lane);
+        else sort_list<8>(sorted, n, lane);
         __syncwarp();
       } else if (!direct) {
         if (!filled) {
-          for (int i = lane; i < window_words / 4; i += 32) reinterpret_cast<uint4 *>(bits)[i] = make_uint4(0u, 0u, 0u, 0u);
+          if (w0 < 0) {      // the first window starts at the row's lowest index
+            int low = INT_MAX;
+            for (int e0 = 0; e0 < entries; e0 += 32) {
+              const uint2 v = entry(e0 + lane);
+              if (v.y) low = min(low, __ldg(&trange[v.x]).x);
+            }
+            w0 = __reduce_min_sync(FULLMASK, low) & ~31;
+          }
+          for (int i = lane; i < kRowWindowWords / 4; i += 32) reinterpret_cast<uint4 *>(bits)[i] = make_uint4(0u, 0u, 0u, 0u);
           __syncwarp();
-          uint2 next = entry(lane);
+          w1 = INT_MAX;
           for (int e0 = 0; e0 < entries; e0 += 32) {
-            const uint2 v = next;
-            if (e0 + 32 < entries) next = entry(e0 + 32 + lane);
-            const int here = min(32, entries - e0);
-#pragma unroll 8
-            for (int i = 0; i < here; i++) {
-              const uint32_t g = __shfl_sync(FULLMASK, v.x, i), mk = __shfl_sync(FULLMASK, v.y, i);
-              if ((mk >> lane) & 1u) {
-                const uint32_t k = (uint32_t)(__ldg(&perm[32 * (int)g + lane]) - w0);
-                if (k < 32u * (uint32_t)window_words) atomicOr(&bits[k >> 5], 1u << (k & 31));
+            const uint2 v = entry(e0 + lane);
+            const int2 range = v.y ? __ldg(&trange[v.x]) : make_int2(0, -1);
+            if (range.y >= w0 + kRowWindow) w1 = min(w1, max(range.x, w0 + kRowWindow));
+            uint32_t todo = __ballot_sync(FULLMASK, range.y >= w0 && range.x < w0 + kRowWindow);
+            while (todo) {
+              // eight groups' indices in flight: a load under its own branch waits for the last one
+              uint32_t k[8];
+#pragma unroll
+              for (int u = 0; u < 8; u++) {
+                const int src = todo ? __ffs(todo) - 1 : 0;
+                const int g = __shfl_sync(FULLMASK, (int)v.x, src);
+                const uint32_t mk = __shfl_sync(FULLMASK, todo ? v.y : 0u, src);
+                const uint32_t at = (uint32_t)(__ldg(&tperm[min(32 * g + lane, m - 1)]) - w0);
+                k[u] = (mk >> lane) & 1u ? at : 0xFFFFFFFFu;
+                todo &= todo - 1;
               }
+#pragma unroll
+              for (int u = 0; u < 8; u++)
+                if (k[u] < (uint32_t)kRowWindow) atomicOr(&bits[k[u] >> 5], 1u << (k[u] & 31));
             }
           }
+          w1 = __reduce_min_sync(FULLMASK, w1);
           __syncwarp();
           filled = true;
           pos = qn = 0;
         }
-        for (; pos < window_words && qn < kRowBatch; pos += 32) {
+        for (; pos < kRowWindowWords && qn < kRowBatch; pos += 32) {
           uint32_t mk = bits[pos + lane];
           if (!__any_sync(FULLMASK, mk != 0)) continue;
           int add, o = qn + warp_excl_scan(__popc(mk), lane, add);
@@ -863,7 +916,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, PART == ROWS_LIGHT && LCH == 0
           qn += add;
         }
         __syncwarp();
-        n = pos < window_words ? qn & ~31 : qn;      // whole rounds of 32, and the rest when the window ends
+        n = pos < kRowWindowWords ? qn & ~31 : qn;      // whole rounds of 32, and the rest when the window ends
       }
       float4 y = make_float4(0.f, 0.f, 0.f, 0.f), yf[FP];
 #pragma unroll
@@ -903,15 +956,15 @@ __global__ void __launch_bounds__(32 * kRowWarps, PART == ROWS_LIGHT && LCH == 0
       }
       __syncwarp();
       if (PART == ROWS_LIGHT || listed || direct || kept >= stop) break;
-      if (pos < window_words) {
+      if (pos < kRowWindowWords) {
         const unsigned short rest = n + lane < qn ? queue[n + lane] : (unsigned short)0;
         __syncwarp();
         queue[lane] = rest;
         qn -= n;
         __syncwarp();
       } else {
-        w0 += 32 * window_words;
-        if (w0 >= m) break;
+        if (w1 == INT_MAX) break;
+        w0 = w1 & ~31;
         filled = false;
       }
     }
@@ -919,9 +972,15 @@ __global__ void __launch_bounds__(32 * kRowWarps, PART == ROWS_LIGHT && LCH == 0
     if (flushed < z) flush(lane < z - flushed);
     if (lane == 0) P->nnz_row[s] = z;
     if (KIND == ROWS_ORDERED) {
-      if (PART == ROWS_ALL && !ranked && z > 1 && !over && kept <= cap + order_cap && K.use_geo)
-        order_row(P->A_j + (size_t)s * P->ld, P->A_v + (size_t)s * P->ld, z, lv->of_index, m, bits, window_words, queue,
-                  P->cand + (size_t)s * P->cand_pitch, lane);
+      if (!ranked && z > 1 && !over && kept <= cap + order_cap && K.use_geo) {
+        int *Aj = P->A_j + (size_t)s * P->ld;
+        float *Av = P->A_v + (size_t)s * P->ld;
+        __syncwarp();
+        if (PART == ROWS_LIGHT) order_row<4>(Aj, Av, z, lv->of_index, lane);
+        else if (z <= 256) order_row<8>(Aj, Av, z, lv->of_index, lane);
+        else if (z <= 512) order_row<16>(Aj, Av, z, lv->of_index, lane);
+        else order_long_row(Aj, Av, z, lv->of_index, m, bits, queue, P->cand + (size_t)s * P->cand_pitch, lane);
+      }
       __syncwarp();
       if (mode == MODE_ALIGN) continue;
     }
