@@ -11,10 +11,11 @@
 // thresholds; the geometric type is off.  Each row keeps its first `cap` pairs in
 // ascending target index (fill_in_A_mat_gpu_dense_mat_kernel, :719-830).
 //
-// Without a distance threshold there is no spatial pruning, so this is an
-// index-ordered scan of all targets per source row: a block of 128 rows stages 128
-// targets at a time in shared memory (coalesced loads), every thread tests its row
-// against them, and the block stops as soon as all of its rows hold `cap` pairs.
+// Without a distance threshold there is no spatial pruning, so this is an index-ordered scan of
+// all targets per source row.  A warp takes four rows and tests them against 32 targets at a
+// time, one a lane, colour first (few pairs pass it); a row's kept pairs are the set bits in
+// order, and the warp stops as soon as its rows hold `cap` pairs.  A thread per row left five
+// warps in six of the SMs' slots empty and ran every pair's whole arithmetic in some lane.
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -24,7 +25,7 @@
 namespace cvo_gb {
 namespace {
 
-constexpr int kAnisoRows = 128;
+constexpr int kAnisoWarps = 4, kAnisoRows = 4;      // warps of a block, rows of a warp
 
 struct AnisoParams {
   KParams K;
@@ -64,106 +65,112 @@ __device__ __forceinline__ void aniso_row_matrix(const float *Ki, float x0, floa
     for (int j = 0; j < 3; j++) M[3 * i + j] = fa(fa(fm(P[i][0], U[j][0]), fm(P[i][1], U[j][1])), fm(P[i][2], U[j][2]));
 }
 
-// One pair: kept?  Value in a (FP32 fast path, FP64 re-evaluation near sp_thres).
+// Bounds: issue, some 25 instructions per row and 32 targets, and 80 more where a colour passes.
 template <int FCH, int LCH>
-__device__ __forceinline__ bool aniso_pair(const KParams &K, int F, int C, const float (&M)[9], const float4 &x,
-                                           const float4 (&xf)[FCH > 0 ? FCH : 1], const float4 (&xl)[LCH > 0 ? LCH : 1],
-                                           const float4 &y, const float4 *yf, const float4 *yl, float &a) {
-  float d2 = 0.f;
-  if (K.use_geo) {
-    const float d0 = fs(x.x, y.x), d1 = fs(x.y, y.y), dd = fs(x.z, y.z);
-    float v[3];
+__global__ void __launch_bounds__(32 * kAnisoWarps) k_assoc_aniso(AnisoParams A, const float4 *xpos, const float *xfeat,
+                                                                  const float *xlab, const float4 *ytr, const float *yfeat,
+                                                                  const float *ylab, int *ell_j, float *ell_v, int *nnz) {
+  constexpr int FP = FCH > 0 ? FCH : 1;
+  __shared__ float4 sh_x[kAnisoWarps][kAnisoRows], sh_f[kAnisoWarps][kAnisoRows][FP];
+  __shared__ float sh_M[kAnisoWarps][kAnisoRows][9];
+  const KParams &K = A.K;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int i0 = (blockIdx.x * kAnisoWarps + w) * kAnisoRows;
+  if (i0 >= A.n) return;
+  if (lane < kAnisoRows) {
+    const int i = min(i0 + lane, A.n - 1);
+    const float4 x = xpos[i];
+    sh_x[w][lane] = x;
 #pragma unroll
-    for (int j = 0; j < 3; j++) v[j] = fa(fa(fm(d0, M[j]), fm(d1, M[3 + j])), fm(dd, M[6 + j]));
-    d2 = fa(fa(fm(v[0], d0), fm(v[1], d1)), fm(v[2], dd));
+    for (int q = 0; q < FCH; q++) sh_f[w][lane][q] = reinterpret_cast<const float4 *>(xfeat)[(size_t)i * FCH + q];
+    float M[9];
+    aniso_row_matrix(A.Ki, x.x, x.y, x.z, M);
+#pragma unroll
+    for (int k = 0; k < 9; k++) sh_M[w][lane][k] = M[k];
   }
-  float d2c = 0.f;
-  if (K.use_int) {
+  __syncwarp();
+  int cnt[kAnisoRows];
 #pragma unroll
-    for (int q = 0; q < (FCH > 0 ? FCH : 1); q++) {
-      if (FCH == 0) break;
-      const float av[4] = {xf[q].x, xf[q].y, xf[q].z, xf[q].w};
-      const float4 b4 = yf[q];
-      const float bv[4] = {b4.x, b4.y, b4.z, b4.w};
+  for (int r = 0; r < kAnisoRows; r++) cnt[r] = i0 + r < A.n ? 0 : A.cap;
+  float4 y = make_float4(0.f, 0.f, 0.f, 0.f), yf[FP];
 #pragma unroll
-      for (int r = 0; r < 4; r++)
-        if (4 * q + r < F) { const float t = fs(av[r], bv[r]); d2c = fa(d2c, fm(t, t)); }
-    }
-    if (!(d2c < K.d2_c_thres)) return false;
-  }
-  float d2s = 0.f;
-  if (K.use_sem) {
+  for (int q = 0; q < FP; q++) yf[q] = y;
+  auto load = [&](int j) {
+    if (j >= A.m) return;
+    y = __ldg(&ytr[j]);
 #pragma unroll
-    for (int q = 0; q < (LCH > 0 ? LCH : 1); q++) {
-      if (LCH == 0) break;
-      const float av[4] = {xl[q].x, xl[q].y, xl[q].z, xl[q].w};
-      const float4 b4 = yl[q];
-      const float bv[4] = {b4.x, b4.y, b4.z, b4.w};
+    for (int q = 0; q < FCH; q++) yf[q] = __ldg(reinterpret_cast<const float4 *>(yfeat) + (size_t)j * FCH + q);
+  };
+  load(lane);
+  for (int j0 = 0; j0 < A.m; j0 += 32) {
+    const int j = j0 + lane;
+    const float4 yc = y;
+    float4 fc[FP];
 #pragma unroll
-      for (int r = 0; r < 4; r++)
-        if (4 * q + r < C) { const float t = fs(av[r], bv[r]); d2s = fa(d2s, fm(t, t)); }
-    }
-    if (!(d2s < K.d2_s_thres)) return false;
-  }
-  const float kf = K.use_geo ? fm(K.sigma2, __expf(fm(-d2, 0.5f))) : 1.f;
-  const float ckf = K.use_int ? fm(K.c_sigma2, __expf(fm(-d2c, K.inv2c2))) : 1.f;
-  const float skf = K.use_sem ? fm(K.s_sigma_sq, __expf(fm(-d2s, __frcp_rn(fm(fm(2.f, K.s_ell), K.s_ell))))) : 1.f;
-  float af = fm(fm(fm(ckf, kf), skf), 1.f);
-  // sigma^2 exp(-d2 / 2) is the isotropic value with l = 1
-  if (fabsf(fs(af, K.sp_thres)) <= kBand * K.sp_thres) af = exact_value(K, 1.f, d2, d2c, d2s, 1.f);
-  a = af;
-  return af > K.sp_thres;
-}
-
-template <int FCH, int LCH>
-__global__ void __launch_bounds__(kAnisoRows) k_assoc_aniso(AnisoParams A, const float4 *xpos, const float *xfeat,
-                                                            const float *xlab, const float4 *ytr, const float *yfeat,
-                                                            const float *ylab, int *ell_j, float *ell_v, int *nnz) {
-  constexpr int FP = FCH > 0 ? FCH : 1, LP = LCH > 0 ? LCH : 1;
-  __shared__ float4 cpos[kAnisoRows];
-  __shared__ float4 cfeat[kAnisoRows * FP];
-  __shared__ float4 clab[kAnisoRows * LP];
-  const int tid = threadIdx.x;
-  const int i = blockIdx.x * kAnisoRows + tid;
-  const bool valid = i < A.n;
-  const float4 x = valid ? xpos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 xf[FP], xl[LP];
+    for (int q = 0; q < FP; q++) fc[q] = yf[q];
+    load(j + 32);
+    bool full = true;
 #pragma unroll
-  for (int q = 0; q < FP; q++)
-    xf[q] = (FCH > 0 && valid) ? reinterpret_cast<const float4 *>(xfeat)[(size_t)i * FCH + q] : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int r = 0; r < kAnisoRows; r++) {
+      if (cnt[r] >= A.cap) continue;
+      full = false;
+      bool pass = j < A.m;
+      float d2c = 0.f;
+      if (K.use_int) {
 #pragma unroll
-  for (int q = 0; q < LP; q++)
-    xl[q] = (LCH > 0 && valid) ? reinterpret_cast<const float4 *>(xlab)[(size_t)i * LCH + q] : make_float4(0.f, 0.f, 0.f, 0.f);
-  float M[9];
-  aniso_row_matrix(A.Ki, x.x, x.y, x.z, M);
-  int cnt = 0;
-  for (int j0 = 0; j0 < A.m; j0 += kAnisoRows) {
-    if (__syncthreads_and(!valid || cnt >= A.cap)) break;   // every row of the block is full
-    const int j = j0 + tid;
-    const bool has = j < A.m;
-    cpos[tid] = has ? ytr[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int q = 0; q < FCH; q++) {
+          const float4 f = sh_f[w][r][q];
+          const float av[4] = {f.x, f.y, f.z, f.w}, bv[4] = {fc[q].x, fc[q].y, fc[q].z, fc[q].w};
 #pragma unroll
-    for (int q = 0; q < FP; q++)
-      cfeat[tid * FP + q] = (FCH > 0 && has) ? reinterpret_cast<const float4 *>(yfeat)[(size_t)j * FCH + q]
-                                             : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int q = 0; q < LP; q++)
-      clab[tid * LP + q] = (LCH > 0 && has) ? reinterpret_cast<const float4 *>(ylab)[(size_t)j * LCH + q]
-                                            : make_float4(0.f, 0.f, 0.f, 0.f);
-    __syncthreads();
-    const int nk = min(kAnisoRows, A.m - j0);
-    if (valid) {
-      for (int k = 0; k < nk && cnt < A.cap; k++) {
-        float a;
-        if (aniso_pair<FCH, LCH>(A.K, A.F, A.C, M, x, xf, xl, cpos[k], &cfeat[k * FP], &clab[k * LP], a)) {
-          ell_j[(size_t)i * A.cap + cnt] = j0 + k;
-          ell_v[(size_t)i * A.cap + cnt] = a;
-          cnt++;
+          for (int k = 0; k < 4; k++)
+            if (4 * q + k < A.F) { const float t = fs(av[k], bv[k]); d2c = fa(d2c, fm(t, t)); }
         }
+        pass = pass && d2c < K.d2_c_thres;
       }
+      if (!__any_sync(0xFFFFFFFFu, pass)) continue;
+      float d2s = 0.f;
+      if (K.use_sem) {
+#pragma unroll
+        for (int q = 0; q < LCH; q++) {
+          const float4 l = __ldg(reinterpret_cast<const float4 *>(xlab) + (size_t)(i0 + r) * LCH + q);
+          const float4 o = pass ? __ldg(reinterpret_cast<const float4 *>(ylab) + (size_t)j * LCH + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+          const float av[4] = {l.x, l.y, l.z, l.w}, bv[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+          for (int k = 0; k < 4; k++)
+            if (4 * q + k < A.C) { const float t = fs(av[k], bv[k]); d2s = fa(d2s, fm(t, t)); }
+        }
+        pass = pass && d2s < K.d2_s_thres;
+      }
+      float d2 = 0.f;
+      if (K.use_geo) {
+        const float4 x = sh_x[w][r];
+        const float *M = sh_M[w][r];
+        const float d0 = fs(x.x, yc.x), d1 = fs(x.y, yc.y), dd = fs(x.z, yc.z);
+        float v[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) v[k] = fa(fa(fm(d0, M[k]), fm(d1, M[3 + k])), fm(dd, M[6 + k]));
+        d2 = fa(fa(fm(v[0], d0), fm(v[1], d1)), fm(v[2], dd));
+      }
+      const float kf = K.use_geo ? fm(K.sigma2, __expf(fm(-d2, 0.5f))) : 1.f;
+      const float ckf = K.use_int ? fm(K.c_sigma2, __expf(fm(-d2c, K.inv2c2))) : 1.f;
+      const float skf = K.use_sem ? fm(K.s_sigma_sq, __expf(fm(-d2s, __frcp_rn(fm(fm(2.f, K.s_ell), K.s_ell))))) : 1.f;
+      float af = fm(fm(fm(ckf, kf), skf), 1.f);
+      // sigma^2 exp(-d2 / 2) is the isotropic value with l = 1
+      if (pass && fabsf(fs(af, K.sp_thres)) <= kBand * K.sp_thres) af = exact_value(K, 1.f, d2, d2c, d2s, 1.f);
+      pass = pass && af > K.sp_thres;
+      const unsigned kept = __ballot_sync(0xFFFFFFFFu, pass);
+      const int c = cnt[r] + __popc(kept & ((1u << lane) - 1u));
+      if (pass && c < A.cap) {
+        ell_j[(size_t)(i0 + r) * A.cap + c] = j;
+        ell_v[(size_t)(i0 + r) * A.cap + c] = af;
+      }
+      cnt[r] = min(cnt[r] + __popc(kept), A.cap);
     }
+    if (full) break;
   }
-  if (valid) nnz[i] = cnt;
+#pragma unroll
+  for (int r = 0; r < kAnisoRows; r++)
+    if (lane == 0 && i0 + r < A.n) nnz[i0 + r] = cnt[r];
 }
 
 using AnisoFn = void (*)(AnisoParams, const float4 *, const float *, const float *, const float4 *, const float *,
@@ -237,27 +244,13 @@ int run_association_aniso(Handle *h, DevCloud *src, DevCloud *tgt, const float T
     return CVO_ERR_OUT_OF_MEMORY;
   }
   k_aniso_transform<<<(m + 255) / 256, 256, 0, h->stream>>>(tgt->pos, m, A, ytr);
-  fn<<<(n + kAnisoRows - 1) / kAnisoRows, kAnisoRows, 0, h->stream>>>(A, src->pos, src->feat, src->lab, ytr, tgt->feat,
+  constexpr int rows = kAnisoRows * kAnisoWarps;
+  fn<<<(n + rows - 1) / rows, 32 * kAnisoWarps, 0, h->stream>>>(A, src->pos, src->feat, src->lab, ytr, tgt->feat,
                                                                       tgt->lab, ej, ev, nz);
   h->launches += 2;
-  std::vector<int> nzh(n);
-  std::vector<int> jh((size_t)n * cap);
-  std::vector<float> vh((size_t)n * cap);
-  cudaError_t e = cudaMemcpyAsync(nzh.data(), nz, sizeof(int) * n, cudaMemcpyDeviceToHost, h->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(jh.data(), ej, sizeof(int) * jh.size(), cudaMemcpyDeviceToHost, h->stream);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(vh.data(), ev, sizeof(float) * vh.size(), cudaMemcpyDeviceToHost, h->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+  const int rc = csr_to_host(h, n, nz, nullptr, cap, ej, ev, rowptr, col, val);
   release();
-  if (e != cudaSuccess) return set_cuda_error(h, e, "association (non-isotropic kernel)");
-  for (int i = 0; i < n; i++) (*rowptr)[i + 1] = (*rowptr)[i] + nzh[i];
-  col->resize((size_t)(*rowptr)[n]);
-  val->resize((size_t)(*rowptr)[n]);
-  for (int i = 0; i < n; i++)
-    for (int t = 0; t < nzh[i]; t++) {
-      (*col)[(size_t)(*rowptr)[i] + t] = jh[(size_t)i * cap + t];
-      (*val)[(size_t)(*rowptr)[i] + t] = vh[(size_t)i * cap + t];
-    }
-  return CVO_OK;
+  return rc;
 }
 
 }  // namespace cvo_gb

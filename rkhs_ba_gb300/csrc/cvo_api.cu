@@ -6,6 +6,7 @@
 #include <cstring>
 #include <cctype>
 #include <string>
+#include <utility>
 #include <vector>
 #include <algorithm>
 #include <chrono>
@@ -454,21 +455,19 @@ void rigid_inverse(const float *T, float *out) {
   out[15] = 1.f;
 }
 
-void fill_assoc(cvo_assoc *a, int rows, int cols, const std::vector<int> &rowptr, const std::vector<int> &col,
-                const std::vector<float> &val) {
+void fill_assoc(cvo_assoc *a, int rows, int cols, const std::vector<int> &rowptr, std::vector<int> &&col,
+                std::vector<float> &&val) {
   a->rows = rows;
   a->cols = cols;
   a->row_ptr.assign(rowptr.begin(), rowptr.end());
-  a->col = col;
-  a->val = val;
+  a->col = std::move(col);
+  a->val = std::move(val);
   a->source_inliers.clear();
-  a->target_inliers.clear();
   // gpu_association_to_cpu (src/cvo/CvoGPU_impl.cu:370-431): rows with any
   // pair are source inliers; every pair's column is appended to the target list
-  for (int i = 0; i < rows; i++) {
+  for (int i = 0; i < rows; i++)
     if (rowptr[i + 1] > rowptr[i]) a->source_inliers.push_back(i);
-    for (int k = rowptr[i]; k < rowptr[i + 1]; k++) a->target_inliers.push_back(col[k]);
-  }
+  a->target_inliers = a->col;
 }
 
 }  // namespace
@@ -538,7 +537,7 @@ static int align_dev_impl(cvo_handle *H, DevCloud *s, DevCloud *t, const float T
   copy16(&r.T_out[0], T_out);
   if (iters) *iters = r.iters[0];
   if (secs) *secs += gsecs;
-  if (want) fill_assoc(assoc, s->n, t->n, ar[0], ac[0], av[0]);
+  if (want) fill_assoc(assoc, s->n, t->n, ar[0], std::move(ac[0]), std::move(av[0]));
   return r.ret[0] == -1 ? CVO_ZERO_GRADIENT : CVO_OK;
 }
 
@@ -834,7 +833,7 @@ extern "C" int cvo_compute_association(cvo_handle *H, const cvo_cloud *src, cons
   rc = run_inner_product_batch(&H->h, s->d, t->d, Tv, ell, H->h.params.nearest_neighbors_max, &asum, &nnz, true,
                                &rowptr, &col, &val);
   if (rc) return rc;
-  fill_assoc(out, src->n, tgt->n, rowptr, col, val);
+  fill_assoc(out, src->n, tgt->n, rowptr, std::move(col), std::move(val));
   return CVO_OK;
 } catch (...) {
   return status_from_exception();
@@ -849,7 +848,7 @@ extern "C" int cvo_compute_association_aniso_dev(cvo_handle *H, const cvo_gpu_cl
   int rc = run_association_aniso(&H->h, src->d, tgt->d, T, kernel, H->h.params.nearest_neighbors_max, &rowptr, &col,
                                  &val);
   if (rc) return rc;
-  fill_assoc(out, src->d->n, tgt->d->n, rowptr, col, val);
+  fill_assoc(out, src->d->n, tgt->d->n, rowptr, std::move(col), std::move(val));
   return CVO_OK;
 } catch (...) {
   return status_from_exception();
@@ -1225,7 +1224,7 @@ extern "C" int cvo_compute_association_adaptive(cvo_handle *H, const cvo_cloud *
   std::vector<int> rp, col;
   std::vector<float> val;
   if ((rc = run_association_adaptive(&H->h, s->d, t->d, T, ell, &rp, &col, &val))) return rc;
-  fill_assoc(out, src->n, tgt->n, rp, col, val);
+  fill_assoc(out, src->n, tgt->n, rp, std::move(col), std::move(val));
   return CVO_OK;
 } catch (...) {
   return status_from_exception();

@@ -411,16 +411,22 @@ __global__ void __launch_bounds__(kStepThreads) k_step(BatchDev B, KParams K) {
 }
 
 // ----------------------------------------------------- association export
-// Rows of the last association as (original row, original column, value),
-// written into a compact buffer at row offsets computed on the host.
-__global__ void k_export(const PairDev *P, const int *row_start, int *cols, float *vals) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= P->n) return;
-  int z = P->nnz_row[s];
-  int o = row_start[s];
-  for (int c = 0; c < z; c++) {
-    cols[o + c] = P->A_j[(size_t)s * P->ld + c];
-    vals[o + c] = P->A_v[(size_t)s * P->ld + c];
+// Entries of each row (ELL row s is row perm[s], or s), and 0 after the last.
+__global__ void k_csr_counts(int n, const int *nnz, const int *perm, int *count) {
+  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s < n) count[perm ? perm[s] : s] = nnz[s];
+  if (s == 0) count[n] = 0;
+}
+
+// ELL rows to CSR, a warp per row.
+__global__ void __launch_bounds__(128) k_csr_rows(int n, const int *nnz, const int *perm, int ld, const int *ell_j, const float *ell_v,
+                                                  const int *rowptr, int *col, float *val) {
+  const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (s >= n) return;
+  const int z = nnz[s], o = rowptr[perm ? perm[s] : s];
+  for (int c = lane; c < z; c += 32) {
+    col[o + c] = ell_j[(size_t)s * ld + c];
+    val[o + c] = ell_v[(size_t)s * ld + c];
   }
 }
 
@@ -891,54 +897,65 @@ int check_err(Handle *h, BatchHost *bh) {
 
 // Exports the association of pair p into per-row CSR on the host (rows =
 // original source indices, columns ascending).
-int export_pair(Handle *h, BatchHost *bh, int p, DevCloud *src, DevCloud *tgt, std::vector<int> *rowptr,
-                std::vector<int> *cols, std::vector<float> *vals) {
-  PairDev &P = bh->pairs[p];
-  int n = P.n;
-  std::vector<int> nnz(n);
-  CVO_CUDA_TRY(h, cudaMemcpyAsync(nnz.data(), P.nnz_row, sizeof(int) * n, cudaMemcpyDeviceToHost, h->stream));
-  std::vector<int> sperm(n);
-  CVO_CUDA_TRY(h, cudaMemcpyAsync(sperm.data(), src->sperm, sizeof(int) * n, cudaMemcpyDeviceToHost, h->stream));
-  CVO_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-  std::vector<int> start(n + 1, 0);
-  for (int s = 0; s < n; s++) start[s + 1] = start[s] + nnz[s];
-  int total = start[n];
-  int *start_d = nullptr, *cols_d = nullptr;
-  float *vals_d = nullptr;
-  CVO_CUDA_TRY(h, cudaMalloc((void **)&start_d, sizeof(int) * (n + 1)));
-  CVO_CUDA_TRY(h, cudaMalloc((void **)&cols_d, sizeof(int) * std::max(total, 1)));
-  CVO_CUDA_TRY(h, cudaMalloc((void **)&vals_d, sizeof(float) * std::max(total, 1)));
-  CVO_CUDA_TRY(h, cudaMemcpyAsync(start_d, start.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, h->stream));
-  (void)tgt;
-  PairDev *pd = bh->B.pairs + p;
-  k_export<<<(n + 255) / 256, 256, 0, h->stream>>>(pd, start_d, cols_d, vals_d);
-  h->launches++;
-  std::vector<int> c(total);
-  std::vector<float> v(total);
-  CVO_CUDA_TRY(h, cudaMemcpyAsync(c.data(), cols_d, sizeof(int) * total, cudaMemcpyDeviceToHost, h->stream));
-  CVO_CUDA_TRY(h, cudaMemcpyAsync(v.data(), vals_d, sizeof(float) * total, cudaMemcpyDeviceToHost, h->stream));
-  CVO_CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-  cudaFree(start_d); cudaFree(cols_d); cudaFree(vals_d);
-  // reorder rows to original order and sort columns
-  std::vector<int> cnt(n, 0);
-  for (int s = 0; s < n; s++) cnt[sperm[s]] = nnz[s];
-  rowptr->assign(n + 1, 0);
-  for (int i = 0; i < n; i++) (*rowptr)[i + 1] = (*rowptr)[i] + cnt[i];
-  cols->assign(total, 0);
-  vals->assign(total, 0.f);
+int export_pair(Handle *h, BatchHost *bh, int p, DevCloud *src, std::vector<int> *rowptr, std::vector<int> *cols,
+                std::vector<float> *vals) {
+  const PairDev &P = bh->pairs[p];
+  if (P.n == 0 || P.m == 0) {      // nothing was associated
+    rowptr->assign((size_t)P.n + 1, 0);
+    cols->clear();
+    vals->clear();
+    return 0;
+  }
+  if (int rc = csr_to_host(h, P.n, P.nnz_row, src->sperm, P.ld, P.A_j, P.A_v, rowptr, cols, vals)) return rc;
+  if (!bh->ordered) return 0;
+  // rows in the order of the lattice: by column
   std::vector<std::pair<int, float>> tmp;
-  for (int s = 0; s < n; s++) {
-    int i = sperm[s];
-    tmp.clear();
-    for (int k = start[s]; k < start[s + 1]; k++) tmp.push_back({c[k], v[k]});
+  for (int i = 0; i < P.n; i++) {
+    const int o = (*rowptr)[i], z = (*rowptr)[i + 1] - o;
+    tmp.resize(z);
+    for (int k = 0; k < z; k++) tmp[k] = {(*cols)[o + k], (*vals)[o + k]};
     std::sort(tmp.begin(), tmp.end(), [](const std::pair<int, float> &a, const std::pair<int, float> &b) { return a.first < b.first; });
-    int o = (*rowptr)[i];
-    for (size_t k = 0; k < tmp.size(); k++) { (*cols)[o + k] = tmp[k].first; (*vals)[o + k] = tmp[k].second; }
+    for (int k = 0; k < z; k++) { (*cols)[o + k] = tmp[k].first; (*vals)[o + k] = tmp[k].second; }
   }
   return 0;
 }
 
 }  // namespace
+
+// Only the kept entries cross to the host, in place: copying whole ELL rows and laying out the
+// CSR there took most of an export.
+int csr_to_host(Handle *h, int n, const int *nnz, const int *perm, int ld, const int *ell_j, const float *ell_v,
+                std::vector<int> *rowptr, std::vector<int> *col, std::vector<float> *val) {
+  rowptr->assign((size_t)n + 1, 0);
+  col->clear();
+  val->clear();
+  if (n == 0) return 0;
+  const size_t scr = scan_scratch_ints(n + 1);
+  int *buf = nullptr, *out = nullptr;
+  CVO_CUDA_TRY(h, cudaMallocAsync((void **)&buf, sizeof(int) * (2 * (size_t)(n + 1) + scr), h->stream));
+  int *count = buf, *start = buf + n + 1;
+  k_csr_counts<<<(n + 255) / 256, 256, 0, h->stream>>>(n, nnz, perm, count);
+  exclusive_scan_int(h, count, start, n + 1, start + n + 1, (int)scr);
+  h->launches++;
+  cudaError_t e = cudaMemcpyAsync(rowptr->data(), start, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost, h->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+  const size_t total = e == cudaSuccess ? (*rowptr)[n] : 0;
+  if (total > 0) e = cudaMallocAsync((void **)&out, sizeof(int) * 2 * total, h->stream);
+  if (e == cudaSuccess && total > 0) {
+    float *out_v = reinterpret_cast<float *>(out + total);
+    k_csr_rows<<<(n + 3) / 4, 128, 0, h->stream>>>(n, nnz, perm, ld, ell_j, ell_v, start, out, out_v);
+    h->launches++;
+    col->resize(total);
+    val->resize(total);
+    e = cudaMemcpyAsync(col->data(), out, sizeof(int) * total, cudaMemcpyDeviceToHost, h->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(val->data(), out_v, sizeof(float) * total, cudaMemcpyDeviceToHost, h->stream);
+  }
+  if (out) cudaFreeAsync(out, h->stream);
+  cudaFreeAsync(buf, h->stream);
+  const cudaError_t es = cudaStreamSynchronize(h->stream);
+  if (e == cudaSuccess) e = es;
+  return e == cudaSuccess ? 0 : set_cuda_error(h, e, "association export");
+}
 
 // Runs the align loop for every pair of the batch until all pairs stop.
 int run_align_batch(Handle *h, const std::vector<DevCloud *> &srcs, const std::vector<DevCloud *> &tgts,
@@ -1075,7 +1092,7 @@ int run_align_batch(Handle *h, const std::vector<DevCloud *> &srcs, const std::v
   if (export_assoc && a_rows) {
     a_rows->resize(np); a_cols->resize(np); a_vals->resize(np);
     for (int p = 0; p < np; p++)
-      if ((rc = export_pair(h, &bh, p, srcs[p], tgts[p], &(*a_rows)[p], &(*a_cols)[p], &(*a_vals)[p]))) return rc;
+      if ((rc = export_pair(h, &bh, p, srcs[p], &(*a_rows)[p], &(*a_cols)[p], &(*a_vals)[p]))) return rc;
   }
   return 0;
 }
@@ -1200,7 +1217,7 @@ int run_inner_product_batch(Handle *h, DevCloud *src, DevCloud *tgt, const std::
   nnz->assign(np, 0);
   for (int p = 0; p < np; p++) { (*asum)[p] = bh.pairs[p].asum; (*nnz)[p] = bh.pairs[p].nnz_sum; }
   if (export_assoc && np == 1)
-    if ((rc = export_pair(h, &bh, 0, src, tgt, a_rowptr, a_cols, a_vals))) return rc;
+    if ((rc = export_pair(h, &bh, 0, src, a_rowptr, a_cols, a_vals))) return rc;
   return 0;
 }
 

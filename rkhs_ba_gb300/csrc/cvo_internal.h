@@ -319,6 +319,11 @@ int run_association_edges(Handle *h, const std::vector<DevCloud *> &srcs, const 
                           const std::vector<int> &caps, int capmax, std::vector<EdgeAssoc> *out,
                           const KParams *kparams = nullptr, AssocGraph *graph = nullptr);
 
+// ELL rows on the device (ELL row s is row perm[s], or s if perm is null; nnz[s] entries at s * ld)
+// to CSR on the host.
+int csr_to_host(Handle *h, int n, const int *nnz, const int *perm, int ld, const int *ell_j, const float *ell_v,
+                std::vector<int> *rowptr, std::vector<int> *col, std::vector<float> *val);
+
 // Non-isotropic association (cvo_aniso.cu): CSR of the kernel matrix with a 3x3
 // geometric kernel (column-major), first `cap` pairs per row in index order.
 void kernel_inverse3(const float K[9], float Ki[9]);
