@@ -131,35 +131,29 @@ int cloud_from_rgbd(Handle *h, const uint8_t *image, int rows, int cols, int cha
   float *xyz = nullptr, *feat = nullptr, *lab = nullptr, *oxyz = nullptr, *ofeat = nullptr, *olab = nullptr;
   float2 *geo = nullptr, *ogeo = nullptr;
   int *uv_d = nullptr, *flag = nullptr, *pos = nullptr, *scratch = nullptr;
-  auto release = [&]() {
-    cudaFree(img_d); cudaFree(dep_d); cudaFree(gray); cudaFree(grad); cudaFree(sem_d); cudaFree(geo_in);
-    cudaFree(xyz); cudaFree(feat); cudaFree(lab); cudaFree(oxyz); cudaFree(ofeat); cudaFree(olab);
-    cudaFree(geo); cudaFree(ogeo); cudaFree(uv_d); cudaFree(flag); cudaFree(pos); cudaFree(scratch);
-  };
-  const size_t scr = scan_scratch_ints(ns);
-  bool ok = cudaMalloc((void **)&img_d, total * channels) == cudaSuccess &&
-            cudaMalloc((void **)&dep_d, sizeof(float) * total) == cudaSuccess &&
-            cudaMalloc((void **)&gray, sizeof(float) * total) == cudaSuccess &&
-            cudaMalloc((void **)&grad, sizeof(float) * 2 * total) == cudaSuccess &&
-            cudaMalloc((void **)&sem_d, sizeof(float) * (num_classes > 0 ? total * num_classes : 1)) == cudaSuccess &&
-            cudaMalloc((void **)&geo_in, sizeof(float) * 2 * ns) == cudaSuccess &&
-            cudaMalloc((void **)&xyz, sizeof(float) * 3 * ns) == cudaSuccess &&
-            cudaMalloc((void **)&feat, sizeof(float) * A.F * ns) == cudaSuccess &&
-            cudaMalloc((void **)&lab, sizeof(float) * (num_classes > 0 ? (size_t)num_classes * ns : 1)) == cudaSuccess &&
-            cudaMalloc((void **)&oxyz, sizeof(float) * 3 * ns) == cudaSuccess &&
-            cudaMalloc((void **)&ofeat, sizeof(float) * A.F * ns) == cudaSuccess &&
-            cudaMalloc((void **)&olab, sizeof(float) * (num_classes > 0 ? (size_t)num_classes * ns : 1)) == cudaSuccess &&
-            cudaMalloc((void **)&geo, sizeof(float2) * ns) == cudaSuccess &&
-            cudaMalloc((void **)&ogeo, sizeof(float2) * ns) == cudaSuccess &&
-            cudaMalloc((void **)&uv_d, sizeof(int) * 2 * ns) == cudaSuccess &&
-            cudaMalloc((void **)&flag, sizeof(int) * ns) == cudaSuccess &&
-            cudaMalloc((void **)&pos, sizeof(int) * (ns + 1)) == cudaSuccess &&
-            cudaMalloc((void **)&scratch, sizeof(int) * (scr > 0 ? scr : 1)) == cudaSuccess;
-  if (!ok) {
-    cudaGetLastError();
-    release();
-    return CVO_ERR_OUT_OF_MEMORY;
-  }
+  char *work = nullptr;
+  auto release = [&]() { cudaFree(work); };
+  const size_t scr = scan_scratch_ints(ns), classes = (size_t)num_classes;
+  Pieces pieces;      // one allocation: eighteen took longer than the kernels
+  pieces.take(&img_d, total * channels);
+  pieces.take(&dep_d, total);
+  pieces.take(&gray, total);
+  pieces.take(&grad, 2 * total);
+  pieces.take(&sem_d, total * classes);
+  pieces.take(&geo_in, 2 * (size_t)ns);
+  pieces.take(&xyz, 3 * (size_t)ns);
+  pieces.take(&feat, (size_t)A.F * ns);
+  pieces.take(&lab, classes * ns);
+  pieces.take(&oxyz, 3 * (size_t)ns);
+  pieces.take(&ofeat, (size_t)A.F * ns);
+  pieces.take(&olab, classes * ns);
+  pieces.take(&geo, ns);
+  pieces.take(&ogeo, ns);
+  pieces.take(&uv_d, 2 * (size_t)ns);
+  pieces.take(&flag, ns);
+  pieces.take(&pos, (size_t)ns + 1);
+  pieces.take(&scratch, scr);
+  if (int rc = pieces.allocate(h, &work)) return rc;
   cudaStream_t st = h->stream;
   cudaError_t e = cudaMemcpyAsync(img_d, image, total * channels, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(dep_d, depth, sizeof(float) * total, cudaMemcpyHostToDevice, st);

@@ -188,6 +188,15 @@ __global__ void k_group_range(const int *sperm, int n, int ng, int2 *range) {
 
 }  // namespace
 
+int Pieces::allocate(Handle *h, char **base) {
+  CVO_CUDA_TRY(h, cudaMalloc((void **)base, bytes > 0 ? bytes : 256));
+  for (auto &p : at) {
+    char *q = *base + p.second;
+    memcpy(p.first, &q, sizeof(q));
+  }
+  return 0;
+}
+
 // Device part of a cloud's construction from staged device arrays (xyz with stride
 // 3 or 4, features n x F, labels n x C, geometric types n float2 or null) and its
 // bounding box: packed original-order records, Morton tile order, tile extents.
@@ -195,16 +204,32 @@ static int cloud_build(Handle *h, DevCloud *d, const float *xyz_d, int stride, c
                        const float *lab_in, const float2 *geo_in, const float mn[3], const float mx[3]) {
   const int n = d->n;
   int rc = 0;
-  int *perm_vals = nullptr, *perm_tmp = nullptr;
-  unsigned int *keys = nullptr, *keys_tmp = nullptr;
-  if ((rc = dalloc(h, &d->pos, n)) || (rc = dalloc(h, &d->feat, (size_t)n * d->FP)) ||
-      (rc = dalloc(h, &d->lab, (size_t)n * d->CP)) || (rc = dalloc(h, &d->sperm, n)) ||
-      (rc = dalloc(h, &d->spos, n)) || (rc = dalloc(h, &d->sfeat, (size_t)n * d->FP)) ||
-      (rc = dalloc(h, &d->slab, (size_t)n * d->CP)))
-    return rc;
+  // one allocation for everything that the cloud keeps and one for the sort: an allocation or a
+  // release costs as much as several of the kernels below
+  const int ng = group_count(n), ns = group_count(ng), ch = box_chunks(d->FP);
+  Pieces keep, tmp;
+  keep.take(&d->pos, n);
+  keep.take(&d->feat, (size_t)n * d->FP);
+  keep.take(&d->lab, (size_t)n * d->CP);
+  keep.take(&d->sperm, n);
+  keep.take(&d->spos, n);
+  keep.take(&d->sfeat, (size_t)n * d->FP);
+  keep.take(&d->slab, (size_t)n * d->CP);
   if (d->has_geo) {
-    if ((rc = dalloc(h, &d->geo, n)) || (rc = dalloc(h, &d->sgeo, n))) return rc;
+    keep.take(&d->geo, n);
+    keep.take(&d->sgeo, n);
   }
+  keep.take(&d->gbox, (size_t)(2 + 2 * ch) * ng);
+  keep.take(&d->sbox, (size_t)(2 + 2 * ch) * ns);
+  keep.take(&d->grange, ng);
+  if ((rc = keep.allocate(h, &d->base))) return rc;
+  unsigned int *keys = nullptr, *keys_tmp = nullptr;
+  int *perm_tmp = nullptr;
+  char *tmp_d = nullptr;
+  tmp.take(&keys, n);
+  tmp.take(&keys_tmp, n);
+  tmp.take(&perm_tmp, n);
+  if ((rc = tmp.allocate(h, &tmp_d))) return rc;
   k_pack_positions<<<(n + 255) / 256, 256, 0, h->stream>>>(xyz_d, stride, n, d->pos);
   h->launches++;
   if (d->FP > 0) {
@@ -221,22 +246,18 @@ static int cloud_build(Handle *h, DevCloud *d, const float *xyz_d, int stride, c
     CVO_CUDA_TRY(h, cudaMemcpyAsync(d->geo, geo_in, sizeof(float2) * n, cudaMemcpyDeviceToDevice, h->stream));
 
   // tile order: Morton order of a 1024^3 lattice over the bounding box
-  if ((rc = dalloc(h, &keys, n)) || (rc = dalloc(h, &keys_tmp, n)) || (rc = dalloc(h, &perm_vals, n)) ||
-      (rc = dalloc(h, &perm_tmp, n)))
-    return rc;
   float ext = std::max(std::max(mx[0] - mn[0], mx[1] - mn[1]), mx[2] - mn[2]);
   float inv = ext > 0 ? 1023.999f / ext : 0.f;
-  k_morton<<<(n + 255) / 256, 256, 0, h->stream>>>(d->pos, n, mn[0], mn[1], mn[2], inv, keys, perm_vals);
+  k_morton<<<(n + 255) / 256, 256, 0, h->stream>>>(d->pos, n, mn[0], mn[1], mn[2], inv, keys, d->sperm);
   h->launches++;
-  if ((rc = radix_sort_pairs(h, keys, perm_vals, keys_tmp, perm_tmp, n, 30))) return rc;
-  CVO_CUDA_TRY(h, cudaMemcpyAsync(d->sperm, perm_vals, sizeof(int) * n, cudaMemcpyDeviceToDevice, h->stream));
+  if ((rc = radix_sort_pairs(h, keys, d->sperm, keys_tmp, perm_tmp, n, 30))) {
+    cudaFree(tmp_d);
+    return rc;
+  }
   k_gather_source<<<(n + 255) / 256, 256, 0, h->stream>>>(d->sperm, n, d->pos, d->feat, d->FP, d->lab, d->CP, d->geo,
                                                          d->spos, d->sfeat, d->slab, d->sgeo);
   h->launches++;
   // boxes of the groups and supergroups
-  const int ng = group_count(n), ns = group_count(ng), ch = box_chunks(d->FP);
-  if ((rc = dalloc(h, &d->gbox, (size_t)(2 + 2 * ch) * ng)) || (rc = dalloc(h, &d->sbox, (size_t)(2 + 2 * ch) * ns))) return rc;
-  if ((rc = dalloc(h, &d->grange, ng))) return rc;
   k_group_range<<<(ng + 3) / 4, 128, 0, h->stream>>>(d->sperm, n, ng, d->grange);
   k_boxes<0><<<(ng + 3) / 4, 128, 0, h->stream>>>(d->spos, reinterpret_cast<const float4 *>(d->sfeat), d->FP / 4, n, ch,
                                                   d->gbox, ng);
@@ -251,7 +272,7 @@ static int cloud_build(Handle *h, DevCloud *d, const float *xyz_d, int stride, c
   double es = 0.0;
   for (float e : ext_h) es += e;
   d->tile_ext = tiles > 0 ? (float)(es / tiles) : 0.f;
-  cudaFree(keys); cudaFree(keys_tmp); cudaFree(perm_vals); cudaFree(perm_tmp);
+  cudaFree(tmp_d);
   return 0;
 }
 
@@ -299,25 +320,25 @@ int cloud_upload(Handle *h, const cvo_cloud *c, DevCloud **out) {
 
   float *xyz_d = nullptr, *feat_in = nullptr, *lab_in = nullptr;
   float2 *geo_in = nullptr;
+  char *staged = nullptr;
   int rc = 0;
-  auto release = [&]() { cudaFree(xyz_d); cudaFree(feat_in); cudaFree(lab_in); cudaFree(geo_in); };
-  if ((rc = dalloc(h, &xyz_d, (size_t)n * c->xyz_stride))) { release(); return rc; }
+  Pieces in;
+  in.take(&xyz_d, (size_t)n * c->xyz_stride);
+  in.take(&feat_in, (size_t)n * c->F);
+  in.take(&lab_in, (size_t)n * c->C);
+  if (d->has_geo) in.take(&geo_in, n);
+  if ((rc = in.allocate(h, &staged))) return rc;
+  auto release = [&]() { cudaFree(staged); };
   CVO_CUDA_TRY(h, cudaMemcpyAsync(xyz_d, c->xyz, sizeof(float) * (size_t)n * c->xyz_stride, cudaMemcpyHostToDevice,
                                   h->stream));
-  if (d->FP > 0) {
-    if ((rc = dalloc(h, &feat_in, (size_t)n * c->F))) { release(); return rc; }
+  if (d->FP > 0)
     CVO_CUDA_TRY(h, cudaMemcpyAsync(feat_in, c->features, sizeof(float) * (size_t)n * c->F, cudaMemcpyHostToDevice,
                                     h->stream));
-  }
-  if (d->CP > 0) {
-    if ((rc = dalloc(h, &lab_in, (size_t)n * c->C))) { release(); return rc; }
+  if (d->CP > 0)
     CVO_CUDA_TRY(h, cudaMemcpyAsync(lab_in, c->labels, sizeof(float) * (size_t)n * c->C, cudaMemcpyHostToDevice,
                                     h->stream));
-  }
-  if (d->has_geo) {
-    if ((rc = dalloc(h, &geo_in, n))) { release(); return rc; }
+  if (d->has_geo)
     CVO_CUDA_TRY(h, cudaMemcpyAsync(geo_in, c->geom_type, sizeof(float2) * n, cudaMemcpyHostToDevice, h->stream));
-  }
   rc = cloud_build(h, d, xyz_d, c->xyz_stride, feat_in, lab_in, geo_in, mn, mx);
   release();
   return rc;
@@ -379,9 +400,7 @@ int cloud_from_device(Handle *h, int n, int F, int C, const float *xyz_d, const 
 
 void cloud_free(DevCloud *d) {
   if (!d) return;
-  cudaFree(d->pos); cudaFree(d->feat); cudaFree(d->lab); cudaFree(d->geo);
-  cudaFree(d->sperm); cudaFree(d->spos); cudaFree(d->sfeat); cudaFree(d->slab); cudaFree(d->sgeo);
-  cudaFree(d->gbox); cudaFree(d->sbox); cudaFree(d->grange);
+  cudaFree(d->base);
   for (void *p : d->rank_allocs) cudaFree(p);
   delete d;
 }

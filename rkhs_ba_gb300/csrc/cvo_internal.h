@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <string>
+#include <utility>
 #include <vector>
 #include <map>
 #include <new>
@@ -30,6 +31,8 @@ inline int group_count(int n) { return (n + kGroup - 1) / kGroup; }
 // Feature chunks (float4) of a bounding box: the association takes at most two.
 inline int box_chunks(int FP) { return FP / 4 < 2 ? FP / 4 : 2; }
 
+struct Handle;
+
 // An order of a target cloud's points: by the cells of a lattice over the bounding box (z, then
 // y, then x), inside a cell by index.  The align loop and the window solve keep the entries
 // of a kernel-matrix row in this order and add them up in it, with the lattice that follows
@@ -41,7 +44,21 @@ struct RankLevel {
   int *of_tile;           // tile-order position -> rank
 };
 
+// Device arrays that share one allocation, each on a 256-byte boundary: take() notes an array's
+// pointer and size, allocate() sets the pointers.
+struct Pieces {
+  size_t bytes = 0;
+  std::vector<std::pair<void *, size_t>> at;
+  template <class T>
+  void take(T **p, size_t count) {
+    at.emplace_back(static_cast<void *>(p), bytes);
+    bytes += (sizeof(T) * count + 255) & ~(size_t)255;
+  }
+  int allocate(Handle *h, char **base);      // the status of the allocation; base owns it
+};
+
 struct DevCloud {
+  char *base = nullptr;          // of the arrays below
   int n = 0, F = 0, C = 0, FP = 0, CP = 0;
   bool has_geo = false;
   float bbmin[3] = {0, 0, 0}, bbmax[3] = {0, 0, 0};
