@@ -42,15 +42,15 @@ UNIT = "registrations/s"
 
 def _capture_value(key):
     """A per-pair figure of the committed association capture
-    (profiles/k_assoc_cta_global50k.json, written by rkhs_ba_gb300.profiling), or None."""
+    (profiles/k_rows_global50k.json: the candidate test and the row pass of a pass), or None."""
     from rkhs_ba_gb300 import profiling
-    d = profiling.load("k_assoc_cta_global50k.json")
+    d = profiling.load("k_rows_global50k.json")
     return None if d is None else d.get(key)
 
 
 def issue_roofline(inst_per_pair, pair_passes, launches, avg_launch_s, sms, sm_mhz):
-    """Instruction-issue bound of the association phase: k_assoc_cta's warp instructions
-    per launch (the ncu capture's count per pair-launch times this run's mean pairs per
+    """Instruction-issue bound of the association phase: its kernels' warp instructions
+    per pass (the ncu capture's count per pair-launch times this run's mean pairs per
     launch) over the event-timed phase duration, against one warp instruction per
     cycle on each of an SM's 4 schedulers at the sampled SM clock.  None when an input
     is missing."""
@@ -62,7 +62,7 @@ def issue_roofline(inst_per_pair, pair_passes, launches, avg_launch_s, sms, sm_m
     peak = sms * 4 * sm_mhz * 1e6 / 1e9
     return {"achieved": round(achieved, 2), "peak": round(peak, 2), "unit": "G warp instructions/s",
             "frac": round(achieved / peak, 4), "warp_instructions_per_launch": round(inst),
-            "note": "k_assoc_cta instructions per pair from the committed ncu capture summary over the whole "
+            "note": "k_cand and k_rows instructions per pair from the committed ncu capture summary over the whole "
                     "association phase's duration; peak = SMs x 4 schedulers x SM clock"}
 
 

@@ -1,7 +1,7 @@
 // cvo_sort.cu -- stable LSD radix sort of (uint32 key, int value) pairs and an
-// exclusive prefix scan.  Used to build the spatial-hash grids and the source
-// tile order (the reference builds a kd-tree with per-node thrust::sort,
-// thirdparty/cugicp/cukdtree/cukdtree.cuh:236-284; this replaces it).
+// exclusive prefix scan.  Used for the tile order of the clouds, the orders of their
+// lattices and the rows of a window solve (the reference builds a kd-tree with per-node
+// thrust::sort, thirdparty/cugicp/cukdtree/cukdtree.cuh:236-284; this replaces it).
 #include "cvo_internal.h"
 
 namespace cvo_gb {

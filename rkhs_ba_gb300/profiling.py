@@ -6,8 +6,8 @@ the association kernel issues (roofline.issue).  Both come from one `ncu` captur
 the same kernel on a small case of the workload, scaled per pair.  This module turns
 that capture into profiles/<kernel>_<workload>.json:
 
-  python -m rkhs_ba_gb300.profiling <capture.ncu-rep> --kernel k_assoc_cta --pairs 2 \
-      --command "<the ncu command that made the capture>" --out profiles/k_assoc_cta_global50k.json
+  python -m rkhs_ba_gb300.profiling <capture.ncu-rep> --kernel k_rows --pairs 2 \
+      --command "<the ncu command that made the capture>" --out profiles/k_rows_global50k.json
 
 It runs `ncu -i <capture> --page raw --csv` (no GPU needed) and averages the metrics
 over the captured launches of the kernel.
@@ -76,7 +76,7 @@ def load(name: str) -> dict | None:
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("capture")
-    ap.add_argument("--kernel", default="k_assoc_cta")
+    ap.add_argument("--kernel", default="k_rows")
     ap.add_argument("--pairs", type=int, required=True)
     ap.add_argument("--command", required=True)
     ap.add_argument("--out", required=True)
