@@ -119,21 +119,53 @@ __device__ __forceinline__ float row_sums(const PairDev *P, int s, int z, float 
   return acc;
 }
 
-// The block's FP64 sums of NV terms (lane t < NV of G holds term t in acc) -> part; whether
-// this is the pair's last block, whose tot then holds the sums over all blocks.
+// FP64 sums over a pair's rows.  Four rows, 32 (a unit) and the units of a slot are added up in a
+// fixed tree, and the slots' sums by the last block: how many slots a block takes and how many
+// lanes a row follow the batch, the sums do not, so that a pair's result is the same alone and
+// in a batch.
+constexpr int kMostUnits = 4;           // units of a block
+
+// One pass of the block over its rows (lane t < NV of G holds term t of its row in v): the sums
+// of four rows each -> quads.
 template <int G, int NV>
-__device__ __forceinline__ bool sum_blocks(PairDev *P, double acc, int b, int nb, unsigned int *counter, double *tot) {
+__device__ __forceinline__ void keep_quads(double v, int pass, double (*quads)[8][NV]) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  v += __shfl_xor_sync(FULLMASK, v, G);
+  v += __shfl_xor_sync(FULLMASK, v, 2 * G);
+  constexpr int L = 4 * G;              // lanes of four rows: a warp, or half of one
+  const int quad = 32 / L * w + lane / L;
+  if (lane % L < NV) quads[(32 / L) * pass + quad / 8][quad % 8][lane % L] = v;
+}
+
+// The sums of the block's `rows` rows -> part; whether this is the pair's last block, whose tot
+// then holds the sums over all rows.  The groups g are read before the rows: a load after a
+// fence waits for L2.
+template <int NV>
+__device__ __forceinline__ bool sum_blocks(PairDev *P, double (*quads)[8][NV], SumGroups g, int rows, int b, int nb,
+                                           unsigned int *counter, double *tot) {
   __shared__ double sh[kStepThreads / 32][8];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = G; o < 32; o <<= 1) acc += __shfl_xor_sync(FULLMASK, acc, o);
-  if (lane < G) sh[w][lane] = acc;
+  const int units = (rows + kUnitRows - 1) / kUnitRows;
+  const int unit = threadIdx.x / NV, k0 = threadIdx.x % NV;
+  double t = 0.0;
   __syncthreads();
-  if (threadIdx.x < NV) {
-    double t = sh[0][threadIdx.x];
-    for (int q = 1; q < kStepThreads / 32; q++) t += sh[q][threadIdx.x];
-    P->part[(size_t)b * kPartStride + threadIdx.x] = t;
+  if (unit < units) {
+    t = quads[unit][0][k0];
+    for (int i = 1; i < 8; i++) t += quads[unit][i][k0];
+    if (g.slot_units > 1) quads[unit][0][k0] = t;
+  }
+  if (g.slot_units > 1) {
+    if (units * NV > 32) __syncthreads();
+    else __syncwarp();                  // one warp has them all
+    const int u0 = unit * g.slot_units, u1 = min(units, u0 + g.slot_units);
+    if (u0 < u1) {
+      t = quads[u0][0][k0];
+      for (int u = u0 + 1; u < u1; u++) t += quads[u][0][k0];
+    }
+  }
+  if (unit * g.slot_units < units) {
+    P->part[(size_t)(b * g.block_slots + unit) * kPartStride + k0] = t;
     __threadfence();
   }
   __syncthreads();
@@ -141,12 +173,12 @@ __device__ __forceinline__ bool sum_blocks(PairDev *P, double acc, int b, int nb
   __syncthreads();
   if (!last) return false;
   __threadfence();
-  // lane t of eight takes term t of every 32nd block
-  acc = 0.0;
+  // lane t of eight takes term t of every 32nd slot
+  double acc = 0.0;
   const int k = threadIdx.x & 7;
   if (k < NV)
 #pragma unroll 8
-    for (int q = threadIdx.x >> 3; q < nb; q += kStepThreads / 8) acc += __ldcg(P->part + (size_t)q * kPartStride + k);
+    for (int q = threadIdx.x >> 3; q < g.slots; q += kStepThreads / 8) acc += __ldcg(P->part + (size_t)q * kPartStride + k);
   acc += __shfl_xor_sync(FULLMASK, acc, 8);
   acc += __shfl_xor_sync(FULLMASK, acc, 16);
   if (lane < 8) sh[w][lane] = acc;
@@ -167,18 +199,19 @@ __device__ __forceinline__ bool sum_blocks(PairDev *P, double acc, int b, int nb
 __global__ void __launch_bounds__(kStepThreads) k_gradient(BatchDev B, KParams K) {
   constexpr int G = 8;
   __shared__ __align__(16) float buf[kStepThreads / 32][RowLists<G>::kWarp];
-  __shared__ double tot[7];
+  __shared__ double quads[kMostUnits][8][7], tot[7];
   const int blk = blockIdx.x;
   if (blk >= B.total_sblocks) return;
   const int p = find_segment(B.sblk_off, B.npairs, blk);
   PairDev *P = &B.pairs[p];
   if (P->done) return;
   const int b = blk - B.sblk_off[p], nb = B.sblk_off[p + 1] - B.sblk_off[p], n = P->n;
+  const SumGroups g = P->sums;
+  const int block_rows = g.block_slots * g.slot_units * kUnitRows, s0 = b * block_rows, rows = min(n - s0, block_rows);
   const int sub = threadIdx.x % G;
-  double acc = 0.0;
   int nnz = 0, mx = 0;
-  for (int s = b * B.step_rows + (int)threadIdx.x / G; s - (int)threadIdx.x / G < min(n, (b + 1) * B.step_rows);
-       s += kStepThreads / G) {
+  for (int pass = 0; pass * (kStepThreads / G) < rows; pass++) {
+    const int s = s0 + pass * (kStepThreads / G) + (int)threadIdx.x / G;
     const bool has = s < n;
     const int z = has ? P->nnz_row[s] : 0;
     const float4 x = has ? __ldg(&P->xs[s]) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -191,7 +224,7 @@ __global__ void __launch_bounds__(kStepThreads) k_gradient(BatchDev B, KParams K
       X[5] = y.z - x.z;
       X[6] = 1.f;
     });
-    acc += (double)(sub < 3 ? __fdiv_rn(t, K.c) : sub < 6 ? __fdiv_rn(t, K.d) : t);
+    keep_quads<G, 7>((double)(sub < 3 ? __fdiv_rn(t, K.c) : sub < 6 ? __fdiv_rn(t, K.d) : t), pass, quads);
     if (sub == 0) nnz += z;
     mx = max(mx, z);
   }
@@ -210,7 +243,7 @@ __global__ void __launch_bounds__(kStepThreads) k_gradient(BatchDev B, KParams K
     atomicAdd(&P->run_nnz, (unsigned long long)sh_nnz);
     atomicMax(&P->run_max, sh_mx);
   }
-  if (!sum_blocks<G, 7>(P, acc, b, nb, &P->counter[0], tot)) return;
+  if (!sum_blocks<7>(P, quads, g, rows, b, nb, &P->counter[0], tot)) return;
   if (threadIdx.x != 0) return;
   P->counter[0] = 0;
   pass_finished(B, P, tot[6], (double)__ldcg(&P->run_nnz), (double)__ldcg(&P->run_max));
@@ -350,9 +383,9 @@ __device__ __forceinline__ float step_coef(float l) {
 // FP64 across rows; the last block of a pair adds the blocks' sums and finishes the iteration.
 // Bounds: issue (some 100 instructions per 32 entries), then the scalar tail.
 template <int G>
-__global__ void __launch_bounds__(kStepThreads) k_step(BatchDev B, KParams K) {
+__global__ void __launch_bounds__(kStepThreads, 4) k_step(BatchDev B, KParams K) {
   __shared__ __align__(16) float buf[kStepThreads / 32][RowLists<G>::kWarp];
-  __shared__ double tot[4];
+  __shared__ double quads[kMostUnits][8][4], tot[4];
   __shared__ float sh_coef;
   const int blk = blockIdx.x;
   if (blk >= B.total_sblocks) return;
@@ -365,14 +398,15 @@ __global__ void __launch_bounds__(kStepThreads) k_step(BatchDev B, KParams K) {
   if (threadIdx.x == 0) sh_coef = step_coef(P->ell);
   __syncthreads();
   const float coef0 = sh_coef;
-  double sum = 0.0;
-  for (int s = b * B.step_rows + (int)threadIdx.x / G; s - (int)threadIdx.x / G < min(n, (b + 1) * B.step_rows);
-       s += kStepThreads / G) {
+  const SumGroups g = P->sums;
+  const int block_rows = g.block_slots * g.slot_units * kUnitRows, s0 = b * block_rows, rows = min(n - s0, block_rows);
+  for (int pass = 0; pass * (kStepThreads / G) < rows; pass++) {
+    const int s = s0 + pass * (kStepThreads / G) + (int)threadIdx.x / G;
     const bool has = s < n;
     const int z = has ? P->nnz_row[s] : 0;
     const float4 x = has ? __ldg(&P->xs[s]) : make_float4(0.f, 0.f, 0.f, 0.f);
     const float coef = K.use_range_ell_step ? step_coef(range_ell(P->ell, x.w)) : coef0;
-    sum += (double)row_sums<G, 4>(P, has ? s : 0, z, buf[threadIdx.x >> 5], [&](const float4 &y, float (&X)[4]) {
+    const float t = row_sums<G, 4>(P, has ? s : 0, z, buf[threadIdx.x >> 5], [&](const float4 &y, float (&X)[4]) {
       float ux = w1 * y.z - w2 * y.y + u0v, uy = w2 * y.x - w0 * y.z + u1v, uz = w0 * y.y - w1 * y.x + u2v;
       float px = w1 * uz - w2 * uy, py = w2 * ux - w0 * uz, pz = w0 * uy - w1 * ux;          // xi^2 z
       float qx = w1 * pz - w2 * py, qy = w2 * px - w0 * pz, qz = w0 * py - w1 * px;          // xi^3 z
@@ -391,8 +425,9 @@ __global__ void __launch_bounds__(kStepThreads) k_step(BatchDev B, KParams K) {
       X[2] = delta + beta * gamma + b2 * beta * (1.f / 6.f);
       X[3] = epsil + beta * delta + 0.5f * b2 * gamma + 0.5f * gamma * gamma + b2 * b2 * (1.f / 24.f);
     });
+    keep_quads<G, 4>((double)t, pass, quads);
   }
-  if (!sum_blocks<G, 4>(P, sum, b, nb, &P->counter[1], tot)) return;
+  if (!sum_blocks<4>(P, quads, g, rows, b, nb, &P->counter[1], tot)) return;
   // The scalar tail is one thread's chain of dependent reads and writes of the pair's state:
   // in shared memory they cost 30 cycles instead of an L2 round trip each.
   __shared__ PairDev state;
@@ -593,6 +628,7 @@ struct BatchHost {
   AssocKernels fn;
   int cand_blocks = 0, xform_blocks = 0;
   bool split_rows = false;          // rows of few candidates in a launch of their own
+  bool few_rows = false;            // k_step with eight lanes a row
   bool ordered = false;             // rows in the order of the targets' lattice (RankLevel)
 };
 
@@ -680,10 +716,18 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
   const int order_cap = rows_all > 0 ? (int)std::min<long long>(4096, (16ll << 30) / (8ll * rows_all)) & ~3 : 0;
   const bool ell = mode != MODE_IP;                    // an inner product needs no kernel matrix
   std::vector<int> sp(np), caps(np), pitch(np);
-  // rows of a k_gradient or k_step block: 32 (four to a warp), or of large batches multiples of
-  // 64, so that some eight blocks per SM leave their sums to the last one
-  const long long per_block = rows_all / (8ll * sms);
-  const int step_rows = per_block <= kStepRows ? kStepRows : 64 * (int)((per_block + 63) / 64);
+  // Rows of a k_gradient or k_step block: 32 (four to a warp), or of large batches multiples of
+  // 64, up to kMostUnits units, so that some eight blocks per SM leave their sums to the last
+  // one.  A pair's slots (groups of its FP64 sums) are the blocks that its own rows ask for.
+  auto share = [&](long long rows) {
+    const long long per_block = rows / (8ll * sms);
+    return per_block <= kUnitRows ? kUnitRows : (int)std::min<long long>(64 * ((per_block + 63) / 64), kMostUnits * kUnitRows);
+  };
+  auto groups_of = [&](int n) {
+    const int slot = share(n);
+    return SumGroups{slot / kUnitRows, (n + slot - 1) / slot, share(rows_all) / slot};
+  };
+  bh->few_rows = share(rows_all) == kUnitRows;
   for (int p = 0; p < np; p++) {
     int n = srcs[p]->n, m = tgts[p]->n;
     const int ns = group_count(group_count(m));
@@ -694,7 +738,8 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     pitch[p] = std::max(sp[p] * caps[p], bh->ordered ? std::min(capmax, m) : 0);
     bh->item_off[p + 1] = bh->item_off[p] + group_count(n) * sp[p];
     bh->tgt_off[p + 1] = bh->tgt_off[p] + m;
-    int rb = (n + kRowsPerBlock - 1) / kRowsPerBlock, sb = (n + step_rows - 1) / step_rows;
+    const SumGroups g = groups_of(n);
+    int rb = (n + kRowsPerBlock - 1) / kRowsPerBlock, sb = (g.slots + g.block_slots - 1) / g.block_slots;
     bh->rblk_off[p + 1] = bh->rblk_off[p] + rb;
     bh->sblk_off[p + 1] = bh->sblk_off[p] + sb;
     add(sizeof(float4) * m);                                     // ycur
@@ -705,7 +750,7 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     add(sizeof(RankLevel) * lv[p].size());
     add(sizeof(int2) * (size_t)n * sp[p]);                       // entry counts
     add(sizeof(int) * n);                                        // nnz_row
-    add(sizeof(double) * kPartStride * (size_t)std::max(kRowSlots * rb, sb)); // partials
+    add(sizeof(double) * kPartStride * (size_t)std::max(kRowSlots * rb, g.slots)); // partials
     add(sizeof(unsigned) * 2);
     bytes += 12 * 256;                                           // room for empty pieces
   }
@@ -740,8 +785,9 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     P.cand_cnt = ar.take<int2>((size_t)s->n * sp[p]);
     P.tf = t->feat; P.tl = t->lab; P.tg = t->geo;
     P.nnz_row = ar.take<int>(s->n);
-    int rb = bh->rblk_off[p + 1] - bh->rblk_off[p], sb = bh->sblk_off[p + 1] - bh->sblk_off[p];
-    P.part = ar.take<double>(kPartStride * (size_t)std::max(kRowSlots * rb, sb));
+    P.sums = groups_of(s->n);
+    const int rb = bh->rblk_off[p + 1] - bh->rblk_off[p];
+    P.part = ar.take<double>(kPartStride * (size_t)std::max(kRowSlots * rb, P.sums.slots));
     P.counter = ar.take<unsigned>(2);
     P.capmax = capmax;
     P.mode = mode;
@@ -790,7 +836,6 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
   memset(&B, 0, sizeof(B));
   B.npairs = np;
   B.total_items = bh->item_off[np];
-  B.step_rows = step_rows;
   B.total_targets = bh->tgt_off[np];
   B.pairs = pairs_d;
   B.item_off = offs_d;
@@ -860,8 +905,7 @@ void launch_iteration(Handle *h, BatchHost *bh, const KParams &K, const cudaEven
   launch_association(h, bh, K, true, ev);
   // Four lanes a row take fewer instructions per entry (lane t adds term t, and there are four);
   // eight lanes keep the SMs busy when the rows are few.
-  const bool few = bh->B.step_rows == kStepRows;
-  (few ? k_step<8> : k_step<4>)<<<std::max(bh->B.total_sblocks, 1), kStepThreads, 0, h->stream>>>(bh->B, K);
+  (bh->few_rows ? k_step<8> : k_step<4>)<<<std::max(bh->B.total_sblocks, 1), kStepThreads, 0, h->stream>>>(bh->B, K);
   mark(h, ev, 4);
   h->launches += 1;
 }
@@ -878,6 +922,7 @@ void append_launch_key(const Handle *h, const BatchHost &bh, const KParams &K, s
   add(&bh.cand_blocks, sizeof(bh.cand_blocks));
   add(&bh.xform_blocks, sizeof(bh.xform_blocks));
   add(&bh.split_rows, sizeof(bh.split_rows));
+  add(&bh.few_rows, sizeof(bh.few_rows));
   add(&h->stream, sizeof(h->stream));
 }
 

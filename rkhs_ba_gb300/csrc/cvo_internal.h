@@ -108,10 +108,17 @@ struct KParams {
   double two_c2;
 };
 
+// Groups of the FP64 sums over a pair's rows (k_gradient, k_step): units of 32 rows in a slot,
+// slots of the pair, slots of a block.
+struct SumGroups {
+  int slot_units, slots, block_slots;
+};
+
 // Per-pair device state.  One struct per pair, in device memory.
 struct PairDev {
   // problem
   int n, m;                       // source rows, target points
+  SumGroups sums;
   const float4 *xs;               // source, tile order (x,y,z,||x||)
   const float *xf, *xl;
   const float2 *xg;
@@ -173,7 +180,6 @@ struct PairDev {
 struct BatchDev {
   int npairs;
   int total_items;                // work items of k_cand over all pairs (tiles x splits)
-  int step_rows;                  // rows of a k_gradient or k_step block
   int total_targets;              // sum of m
   PairDev *pairs;                 // device array
   const int *item_off;            // npairs + 1 (prefix of work items)

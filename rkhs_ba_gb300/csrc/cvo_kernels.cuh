@@ -23,7 +23,7 @@ namespace cvo_gb {
 
 enum { MODE_ALIGN = 0, MODE_IP = 1, MODE_EXPORT = 2, MODE_EDGES = 3 };
 constexpr int kStepThreads = 256;
-constexpr int kStepRows = 32;           // fewest rows of a block of the gradient and step kernels
+constexpr int kUnitRows = 32;           // fewest rows of a block of the gradient and step kernels
 constexpr int kPartStride = 12;
 
 // ------------------------------------------------------------ pair value
