@@ -713,7 +713,12 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
   for (int p = 0; p < np; p++) rows_all += srcs[p]->n;
   const int most = rows_all > 0 ? (int)std::min<long long>(1 << 20, (16ll << 30) / (8ll * rows_all)) : 1;
   const int ell_ld = (std::max(capmax, 1) + 3) & ~3;   // 16-byte aligned ELL rows
-  const int order_cap = rows_all > 0 ? (int)std::min<long long>(4096, (16ll << 30) / (8ll * rows_all)) & ~3 : 0;
+  // An ordered row that keeps more than cap + order_cap pairs stays in index order.  A pair of an
+  // align batch has one rule whatever the batch, so that its pose is the same alone.  A window is
+  // one problem, and another order of some rows moves its poses by up to 3e-5: there the value
+  // shrinks beyond 524,288 rows, as it always has.
+  const int order_cap = mode != MODE_EDGES || rows_all == 0 ? kOrderCap
+                                                            : (int)std::min<long long>(kOrderCap, (16ll << 30) / (8ll * rows_all)) & ~3;
   const bool ell = mode != MODE_IP;                    // an inner product needs no kernel matrix
   std::vector<int> sp(np), caps(np), pitch(np);
   // Rows of a k_gradient or k_step block: 32 (four to a warp), or of large batches multiples of

@@ -25,6 +25,9 @@ namespace cvo_gb {
 constexpr int kWarp = 32;
 constexpr int kMaxIndicatorWindow = 128;
 constexpr int kMaxTargetBits = 22;          // targets per cloud <= 4M
+// A row of an align or a window edge that keeps more than cap + order_cap pairs stays in index order
+// (order_cap: kOrderCap, or less in large windows).
+constexpr int kOrderCap = 4096;
 constexpr int kGroup = 32;                  // points of a group, groups of a supergroup
 
 inline int group_count(int n) { return (n + kGroup - 1) / kGroup; }
@@ -144,7 +147,7 @@ struct PairDev {
   const float2 *tg;               // target geometric types, original order
   int *nnz_row;                   // n
   // align and edges: orders of the target's points, finest lattice first, and the largest search radius
-  // each serves; a row that kept more than cap + order_cap pairs stays in index order
+  // each serves; order_cap as at kOrderCap, 0 for single passes (all rows in index order)
   const RankLevel *levels;
   float level_r[24];
   int nlevels, level, order_cap;

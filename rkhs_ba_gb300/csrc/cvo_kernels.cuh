@@ -465,9 +465,9 @@ __device__ __forceinline__ int warp_excl_scan(int v, int lane, int &total) {
 // -- up to 256 of them by a sorting network over the lanes, more through a bitmap over a window
 // of target indices in shared memory -- and evaluated 32 at a time with the exact arithmetic,
 // the next 32 records in flight.  The reference scans the targets by index and stops at cap kept
-// pairs (src/cvo/CvoGPU.cu:994-996): here the row stops there too, so no pair beyond cap is
-// evaluated or stored.  A row whose entries did not fit, or a call without a candidate test,
-// scans all targets in index order instead.
+// pairs (src/cvo/CvoGPU.cu:994-996): here the row stops there too, and no pair beyond cap is
+// stored (nor, but for some rows of ROWS_ORDERED, evaluated).  A row whose entries did not fit,
+// or a call without a candidate test, scans all targets in index order instead.
 // Sums (all but align): FP32 per lane and row, over the lanes, FP64 from there; the last block
 // of a pair adds the blocks' sums in a fixed order.
 // ROWS_ORDERED: the entries of a row go to the order of the pair's level (RankLevel), in which

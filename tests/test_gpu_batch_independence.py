@@ -33,3 +33,14 @@ def test_batches_of_more_rows_than_their_pairs(cuda_device, sizes):
     p.MAX_ITER, p.ell_init, p.nearest_neighbors_max = 5, 0.1, 24
     clouds = [(_mirrored(rng, n), _mirrored(rng, 4000, 1.0)) for n in sizes]
     _alone_and_in_batch(p, *zip(*clouds), range(len(sizes)))
+
+
+def test_batch_of_more_than_half_a_million_rows(cuda_device):
+    """Rows that keep 4,000 pairs at a cap of 200 are added up in the same order alone and beside a
+    pair of 600,000 rows."""
+    rng = np.random.default_rng(5)
+    p = CvoParams(params_path("color"))
+    p.MAX_ITER, p.nearest_neighbors_max = 20, 200
+    src, tgt = (CvoPointCloud(rng.uniform(0, 1.6, (n, 3)) + 2, rng.uniform(0.495, 0.505, (n, 5))) for n in (300, 4000))
+    many, one = (CvoPointCloud(rng.uniform(0, 30, (n, 3)), rng.uniform(0.4, 0.6, (n, 5))) for n in (600000, 1))
+    _alone_and_in_batch(p, [src, many], [tgt, one], [0])
