@@ -626,7 +626,7 @@ struct BatchHost {
   std::vector<PairDev> pairs;
   std::vector<int> item_off, tgt_off, rblk_off, sblk_off;
   AssocKernels fn;
-  int cand_blocks = 0, xform_blocks = 0;
+  int cand_blocks = 0, xform_blocks = 0, rows_blocks = 0;
   bool split_rows = false;          // rows of few candidates in a launch of their own
   bool few_rows = false;            // k_step with eight lanes a row
   bool ordered = false;             // rows in the order of the targets' lattice (RankLevel)
@@ -720,7 +720,7 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
   const int order_cap = mode != MODE_EDGES || rows_all == 0 ? kOrderCap
                                                             : (int)std::min<long long>(kOrderCap, (16ll << 30) / (8ll * rows_all)) & ~3;
   const bool ell = mode != MODE_IP;                    // an inner product needs no kernel matrix
-  std::vector<int> sp(np), caps(np), pitch(np);
+  std::vector<int> sp(np), caps(np);
   // Rows of a k_gradient or k_step block: 32 (four to a warp), or of large batches multiples of
   // 64, up to kMostUnits units, so that some eight blocks per SM leave their sums to the last
   // one.  A pair's slots (groups of its FP64 sums) are the blocks that its own rows ask for.
@@ -739,8 +739,6 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     sp[p] = std::max(1, std::min(splits, ns));
     caps[p] = std::max(1, std::min(kGroup * ((ns + sp[p] - 1) / sp[p]), most / sp[p]));
     if (!K.use_mma) sp[p] = caps[p] = 1;
-    // an ordered row's kept entries pass through its candidate entries' place (order_row)
-    pitch[p] = std::max(sp[p] * caps[p], bh->ordered ? std::min(capmax, m) : 0);
     bh->item_off[p + 1] = bh->item_off[p] + group_count(n) * sp[p];
     bh->tgt_off[p + 1] = bh->tgt_off[p] + m;
     const SumGroups g = groups_of(n);
@@ -751,7 +749,7 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     add(sizeof(float4) * m);                                     // yorig
     add(ell ? sizeof(int) * (size_t)n * ell_ld : 0);             // ELL
     add(ell ? sizeof(float) * (size_t)n * ell_ld : 0);
-    add(sizeof(uint2) * (size_t)n * pitch[p]);                   // candidate entries
+    add(sizeof(uint2) * (size_t)n * sp[p] * caps[p]);            // candidate entries
     add(sizeof(RankLevel) * lv[p].size());
     add(sizeof(int2) * (size_t)n * sp[p]);                       // entry counts
     add(sizeof(int) * n);                                        // nnz_row
@@ -762,7 +760,18 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
   add(sizeof(PairDev) * np);
   add(sizeof(int) * (np + 1) * 4);
   add(sizeof(int) * 8);
-  add(sizeof(int) * (kRowsPerBlock / kRowsHeavy) * (size_t)bh->rblk_off[np]);      // groups of long rows
+  const int groups = (kRowsPerBlock / kRowsHeavy) * bh->rblk_off[np];
+  add(sizeof(int) * (size_t)groups);                                               // groups of long rows
+  // Ordered rows of more than kRowOrdered entries pass through room of their own: each row's, or
+  // beyond kRowRoom (room in every row would double the kernel matrix) each resident warp's, with
+  // the rows listed as those of large targets are.  Listing them anyway is up to a fourth slower
+  // (20 iterations on 8k colour points at a cap of 2,000: 4.8 against 6.0 ms).
+  const int longest = std::min(capmax, maxm);
+  const bool long_rows = bh->ordered && longest > kRowOrdered;
+  bh->split_rows = (K.use_mma && maxm > kRowSplitTargets) || (long_rows && sizeof(uint2) * rows_all * longest > kRowRoom);
+  bh->rows_blocks = std::max(1, bh->split_rows ? std::min(groups, 5 * sms) : groups);
+  const size_t long_room = !long_rows ? 0 : (size_t)longest * (bh->split_rows ? (long long)bh->rows_blocks * kRowWarps : rows_all);
+  add(sizeof(uint2) * long_room);
   add(sizeof(double));
   if ((rc = ensure_workspace(h, bytes))) return rc;
   Arena ar;
@@ -785,7 +794,7 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     P.ld = ell_ld;
     P.splits = sp[p];
     P.cap_split = caps[p];
-    P.cand_pitch = pitch[p];
+    P.cand_pitch = sp[p] * caps[p];
     P.cand = ar.take<uint2>((size_t)s->n * P.cand_pitch);
     P.cand_cnt = ar.take<int2>((size_t)s->n * sp[p]);
     P.tf = t->feat; P.tl = t->lab; P.tg = t->geo;
@@ -825,7 +834,13 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
   PairDev *pairs_d = ar.take<PairDev>(np);
   int *offs_d = ar.take<int>((size_t)(np + 1) * 4);
   int *ctr_d = ar.take<int>(8);
-  int *heavy_d = ar.take<int>((kRowsPerBlock / kRowsHeavy) * (size_t)bh->rblk_off[np]);
+  int *heavy_d = ar.take<int>(groups);
+  uint2 *long_d = ar.take<uint2>(long_room);
+  if (long_rows)
+    for (int p = 0, row = 0; p < np; row += bh->pairs[p++].n) {
+      bh->pairs[p].long_rows = long_d + (bh->split_rows ? 0 : (size_t)row * longest);
+      bh->pairs[p].long_pitch = longest;
+    }
   double *bytes_d = ar.take<double>(1);
   // zero counters of every pair
   for (int p = 0; p < np; p++) CVO_CUDA_TRY(h, cudaMemsetAsync(bh->pairs[p].counter, 0, 2 * sizeof(unsigned), h->stream));
@@ -861,7 +876,6 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
   }
   bh->cand_blocks = K.use_mma ? (B.total_items + kCandWarps - 1) / kCandWarps : 0;
   bh->xform_blocks = (B.total_targets + 255) / 256;
-  bh->split_rows = K.use_mma && maxm > kRowSplitTargets;
   return 0;
 }
 
@@ -890,8 +904,7 @@ void launch_association(Handle *h, BatchHost *bh, const KParams &K, bool align =
     rows[ROWS_LIGHT]<<<blocks, 32 * kRowWarps, 0, h->stream>>>(B, K, 1);
     h->launches++;
   }
-  const int groups = blocks * (kRowsPerBlock / kRowsHeavy), resident = 5 * (h->num_sms > 0 ? h->num_sms : 152);
-  rows[ROWS_ALL]<<<split ? std::min(groups, resident) : groups, 32 * kRowWarps, 0, h->stream>>>(B, K, split);
+  rows[ROWS_ALL]<<<bh->rows_blocks, 32 * kRowWarps, 0, h->stream>>>(B, K, split);
   h->launches += 2;
   if (split && !align) {
     k_rows_total<<<B.npairs, 32 * kRowWarps, 0, h->stream>>>(B);
@@ -927,6 +940,7 @@ void append_launch_key(const Handle *h, const BatchHost &bh, const KParams &K, s
   add(&bh.cand_blocks, sizeof(bh.cand_blocks));
   add(&bh.xform_blocks, sizeof(bh.xform_blocks));
   add(&bh.split_rows, sizeof(bh.split_rows));
+  add(&bh.rows_blocks, sizeof(bh.rows_blocks));
   add(&bh.few_rows, sizeof(bh.few_rows));
   add(&h->stream, sizeof(h->stream));
 }

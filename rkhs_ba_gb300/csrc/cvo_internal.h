@@ -152,6 +152,8 @@ struct PairDev {
   float level_r[24];
   int nlevels, level, order_cap;
   float src_norm;                 // largest |x| of the source
+  uint2 *long_rows;               // room to order rows of more than kRowOrdered entries (see build_batch)
+  int long_pitch;
   double *part;                   // block partials
   unsigned int *counter;          // last-block counters [2]
   unsigned long long run_nnz;     // kept pairs and longest row of the pass so far

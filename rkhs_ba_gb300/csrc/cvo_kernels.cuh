@@ -500,6 +500,8 @@ constexpr int kRowBatch = 256;          // candidates taken from the bitmap befo
 constexpr int kRowSorted = 256;         // most candidates a sorting network puts in order
 constexpr int kRowLight = 128;          // most candidates of a row of ROWS_LIGHT
 constexpr int kRowSplitTargets = 8192;  // larger targets: ROWS_LIGHT and ROWS_ALL
+constexpr int kRowOrdered = 512;        // most entries that order_row puts in order
+constexpr size_t kRowRoom = 1ull << 30; // most bytes to order longer rows with, see build_batch
 
 // Whether a kernel instance leaves the rows' entries in index order (single passes) or puts
 // them in the order of the pair's level (the align loop, the edges of a window).
@@ -551,7 +553,7 @@ __device__ __forceinline__ void sort_list(int *list, int count, int lane) {
   for (int r = 0; r < R; r++) list[32 * r + lane] = v[r];
 }
 
-// Puts the z <= 32 R <= 512 entries of an ELL row, which are in index order, in the order of the
+// Puts the z <= 32 R <= kRowOrdered entries of an ELL row, which are in index order, in the order of the
 // ranks: rank (22 bits) and slot sorted as one key.
 template <int R>
 __device__ __forceinline__ void order_row(int *Aj, float *Av, int z, const int *rank, int lane) {
@@ -581,7 +583,7 @@ __device__ __forceinline__ void order_row(int *Aj, float *Av, int z, const int *
 
 // The same for rows of more entries:
 // their bits in a bitmap over the ranks, a count before every four words, and each entry's slot is
-// the number of bits below its own.  tmp: z entries.  All lanes call it.
+// the number of bits below its own.  tmp: z entries of the warp's own.  All lanes call it.
 __device__ __forceinline__ void order_long_row(int *Aj, float *Av, int z, const int *rank, int m, uint32_t *bits,
                                                unsigned short *before, uint2 *tmp, int lane) {
   constexpr int window_words = kRowWindowWords, wl = window_words >> 5;
@@ -978,8 +980,8 @@ __global__ void __launch_bounds__(32 * kRowWarps, PART == ROWS_LIGHT && LCH == 0
         __syncwarp();
         if (PART == ROWS_LIGHT) order_row<4>(Aj, Av, z, lv->of_index, lane);
         else if (z <= 256) order_row<8>(Aj, Av, z, lv->of_index, lane);
-        else if (z <= 512) order_row<16>(Aj, Av, z, lv->of_index, lane);
-        else order_long_row(Aj, Av, z, lv->of_index, m, bits, queue, P->cand + (size_t)s * P->cand_pitch, lane);
+        else if (z <= kRowOrdered) order_row<16>(Aj, Av, z, lv->of_index, lane);
+        else order_long_row(Aj, Av, z, lv->of_index, m, bits, queue, P->long_rows + (size_t)(split ? blockIdx.x * kRowWarps + w : s) * P->long_pitch, lane);
       }
       __syncwarp();
       if (mode == MODE_ALIGN) continue;
