@@ -514,6 +514,11 @@ static int ensure_workspace(Handle *h, size_t bytes) {
   if (w->align_exec) { cudaGraphExecDestroy(w->align_exec); w->align_exec = nullptr; w->align_key.clear(); }
   size_t want = bytes + bytes / 4 + (1 << 20);
   cudaError_t e = cudaMalloc((void **)&w->dev, want);
+  if (e == cudaErrorMemoryAllocation) {      // without room to grow
+    cudaGetLastError();
+    want = bytes;
+    e = cudaMalloc((void **)&w->dev, want);
+  }
   if (e != cudaSuccess) {
     set_cuda_error(h, e, "workspace");
     return e == cudaErrorMemoryAllocation ? CVO_ERR_OUT_OF_MEMORY : CVO_ERR_CUDA;
@@ -707,11 +712,8 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
   bh->sblk_off.assign(np + 1, 0);
   size_t bytes = 0;
   auto add = [&](size_t b) { bytes += (b + 255) & ~(size_t)255; };
-  // candidate entries per row: one per target group, at most 16 GB for the batch (a row
-  // that needs more is evaluated by an index-ordered scan of the targets)
   long long rows_all = 0;
   for (int p = 0; p < np; p++) rows_all += srcs[p]->n;
-  const int most = rows_all > 0 ? (int)std::min<long long>(1 << 20, (16ll << 30) / (8ll * rows_all)) : 1;
   const int ell_ld = (std::max(capmax, 1) + 3) & ~3;   // 16-byte aligned ELL rows
   // An ordered row that keeps more than cap + order_cap pairs stays in index order.  A pair of an
   // align batch has one rule whatever the batch, so that its pose is the same alone.  A window is
@@ -737,8 +739,7 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     int n = srcs[p]->n, m = tgts[p]->n;
     const int ns = group_count(group_count(m));
     sp[p] = std::max(1, std::min(splits, ns));
-    caps[p] = std::max(1, std::min(kGroup * ((ns + sp[p] - 1) / sp[p]), most / sp[p]));
-    if (!K.use_mma) sp[p] = caps[p] = 1;
+    if (!K.use_mma) sp[p] = 1;
     bh->item_off[p + 1] = bh->item_off[p] + group_count(n) * sp[p];
     bh->tgt_off[p + 1] = bh->tgt_off[p] + m;
     const SumGroups g = groups_of(n);
@@ -749,7 +750,6 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
     add(sizeof(float4) * m);                                     // yorig
     add(ell ? sizeof(int) * (size_t)n * ell_ld : 0);             // ELL
     add(ell ? sizeof(float) * (size_t)n * ell_ld : 0);
-    add(sizeof(uint2) * (size_t)n * sp[p] * caps[p]);            // candidate entries
     add(sizeof(RankLevel) * lv[p].size());
     add(sizeof(int2) * (size_t)n * sp[p]);                       // entry counts
     add(sizeof(int) * n);                                        // nnz_row
@@ -773,7 +773,24 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
   const size_t long_room = !long_rows ? 0 : (size_t)longest * (bh->split_rows ? (long long)bh->rows_blocks * kRowWarps : rows_all);
   add(sizeof(uint2) * long_room);
   add(sizeof(double));
-  if ((rc = ensure_workspace(h, bytes))) return rc;
+  // Candidate entries per row: one per target group, at most 16 GB for the batch, and fewer if the
+  // device has no such room (a row that needs more is evaluated by an index-ordered scan of the
+  // targets).
+  auto candidates = [&](long long most) {
+    size_t sum = 0;
+    for (int p = 0; p < np; p++) {
+      const int ns = group_count(group_count(tgts[p]->n));
+      caps[p] = !K.use_mma ? 1 : std::max(1, (int)std::min<long long>(kGroup * ((ns + sp[p] - 1) / sp[p]), most / sp[p]));
+      sum += (sizeof(uint2) * (size_t)srcs[p]->n * sp[p] * caps[p] + 255) & ~(size_t)255;
+    }
+    return sum;
+  };
+  long long most = std::min<long long>(group_count(maxm) + kGroup * kMaxSplits, (16ll << 30) / (8ll * std::max(rows_all, 1ll)));
+  const std::string error = h->last_error;
+  rc = ensure_workspace(h, bytes + candidates(most));
+  while (rc == CVO_ERR_OUT_OF_MEMORY && K.use_mma && most > kGroup) rc = ensure_workspace(h, bytes + candidates(most /= 2));
+  if (rc) return rc;
+  h->last_error = error;
   Arena ar;
   ar.base = h->ws->dev;
   ar.cap = h->ws->dev_cap;

@@ -42,3 +42,18 @@ def test_align_with_long_rows_needs_one_kernel_matrix(cuda_device):
     with _free_memory(6 << 30):
         T = cvo.align(gs, gt, np.eye(4))[1]
     assert np.array_equal(T, T0)
+
+
+def test_inner_product_with_little_room_for_candidates(cuda_device):
+    """A candidate entry per row and group of 32 targets would be 1 GB; rows that need more entries than
+    there is room for scan the targets."""
+    rng = np.random.default_rng(2)
+    cvo = CvoGPU(params=CvoParams(params_path("geometric")))
+    src, tgt = _uniform(rng, 20000, 20.0), _uniform(rng, 200000, 20.0)
+    want = cvo.inner_product_gpu(src, tgt, np.eye(4), 0.25)
+    for size in (1 << 30, 400 << 20, 100 << 20):
+        small = CvoGPU(params=cvo.get_params())
+        gs, gt = small.upload(src), small.upload(tgt)
+        with _free_memory(size):
+            got = small.inner_product_gpu(gs, gt, np.eye(4), 0.25)
+        assert abs(got - want) <= 1e-6 * want
