@@ -644,9 +644,8 @@ struct BatchHost {
 constexpr long long kCandItems = 10240;
 
 // Lays out every device buffer of a batch in the handle's workspace.
-int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs, const std::vector<DevCloud *> &tgts,
-                const std::vector<float> &T_init, int mode, int capmax, const std::vector<float> &ell0,
-                BatchHost *bh) {
+int lay_out_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs, const std::vector<DevCloud *> &tgts,
+                  const std::vector<float> &T_init, int mode, int capmax, const std::vector<float> &ell0, BatchHost *bh) {
   const int np = (int)srcs.size();
   int F = srcs[0]->F, C = srcs[0]->C;
   for (int p = 0; p < np; p++) {
@@ -894,6 +893,15 @@ int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs
   bh->cand_blocks = K.use_mma ? (B.total_items + kCandWarps - 1) / kCandWarps : 0;
   bh->xform_blocks = (B.total_targets + 255) / 256;
   return 0;
+}
+
+// A batch that is refused may have built orders of a target already, which the cloud keeps: they
+// are complete when it returns, since the next batch may run on another handle's stream.
+int build_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &srcs, const std::vector<DevCloud *> &tgts,
+                const std::vector<float> &T_init, int mode, int capmax, const std::vector<float> &ell0, BatchHost *bh) {
+  const int rc = lay_out_batch(h, K, srcs, tgts, T_init, mode, capmax, ell0, bh);
+  if (rc) cudaStreamSynchronize(h->stream);
+  return rc;
 }
 
 // Inside stream capture an event becomes a record node of the graph only with

@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 from rkhs_ba_gb300 import CvoGPU, CvoParams, CvoPointCloud, params_path
+from rkhs_ba_gb300._lib import CvoError
 
 pytestmark = pytest.mark.gpu
 
@@ -57,3 +58,22 @@ def test_inner_product_with_little_room_for_candidates(cuda_device):
         with _free_memory(size):
             got = small.inner_product_gpu(gs, gt, np.eye(4), 0.25)
         assert abs(got - want) <= 1e-6 * want
+
+
+def test_clouds_of_a_refused_align_are_ready_on_another_stream(cuda_device):
+    """A kernel matrix that no device holds: the align is refused after the targets' orders were built, and
+    the next one, of another handle on a stream of its own, may use them at once."""
+    rng = np.random.default_rng(3)
+    p = CvoParams(params_path("geometric"))
+    p.MAX_ITER = 3
+    src, tgt = _uniform(rng, 300000, 30.0), _uniform(rng, 300000, 30.0)
+    cvo = CvoGPU(params=p)
+    want = cvo.align(src, tgt, np.eye(4))[1]
+    greedy = p.copy()
+    greedy.nearest_neighbors_max = 1 << 22
+    first, second = CvoGPU(params=greedy), CvoGPU(params=p)
+    for _ in range(3):
+        gs, gt = first.upload(src), first.upload(tgt)
+        with pytest.raises(CvoError):
+            first.align(gs, gt, np.eye(4))
+        assert np.array_equal(second.align(gs, gt, np.eye(4))[1], want)
