@@ -692,7 +692,7 @@ int run_align_multi(Handle *h, int nf, DevCloud *const *clouds, double *poses, c
         E.p1 = clouds[edges[2 * e]]->spos;
         E.p2 = clouds[edges[2 * e + 1]]->pos;
         E.n = EA[e].n;
-        E.lim = std::min(p.nearest_neighbors_max, nn[e]);
+        E.lim = std::max(0, std::min(p.nearest_neighbors_max, nn[e]));      // the rows' sort keys count down to it
         E.f1 = edges[2 * e]; E.f2 = edges[2 * e + 1];
         E.blk0 = blk;
         E.row0 = row;
