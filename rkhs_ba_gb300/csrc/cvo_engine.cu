@@ -694,6 +694,7 @@ int lay_out_batch(Handle *h, const KParams &K, const std::vector<DevCloud *> &sr
       const float ell_hi = ell0[p], ell_lo = mode == MODE_ALIGN ? std::min(K.ell_min, ell_hi) : ell_hi;
       const float r_hi = host_radius(K, ell_hi, srcs[p]->max_norm), r_lo = host_radius(K, ell_lo, 0.f);
       int e_hi = level_for_radius(cell_for_radius(r_hi, ext)), e_lo = level_for_radius(cell_for_radius(r_lo, ext));
+      if (e_lo > e_hi) std::swap(e_lo, e_hi);      // a negative ell_min: its square counts
       if (e_hi - e_lo + 1 > 24) e_lo = e_hi - 23;
       for (int e = e_lo; e <= e_hi; e++) exps.push_back(e);
     }
