@@ -11,11 +11,14 @@
 // thresholds; the geometric type is off.  Each row keeps its first `cap` pairs in
 // ascending target index (fill_in_A_mat_gpu_dense_mat_kernel, :719-830).
 //
-// Without a distance threshold there is no spatial pruning, so this is an index-ordered scan of
-// all targets per source row.  A warp takes four rows and tests them against 32 targets at a
-// time, one a lane, colour first (few pairs pass it); a row's kept pairs are the set bits in
-// order, and the warp stops as soon as its rows hold `cap` pairs.  A thread per row left five
-// warps in six of the SMs' slots empty and ran every pair's whole arithmetic in some lane.
+// There is no distance threshold and an indefinite kernel has no bound by position, so this is an
+// index-ordered scan of all targets per source row (a positive-definite kernel would have one:
+// the columns of U are orthogonal and no shorter than 1, so that (a-b)^T M (a-b) is at least the
+// smallest eigenvalue of K^-1 times |a-b|^2; not used).  A warp takes four rows and tests them
+// against 32 targets at a time, one a lane, colour first (few pairs pass it); a row's kept pairs
+// are the set bits in order, and the warp stops as soon as its rows hold `cap` pairs.  A thread
+// per row left five warps in six of the SMs' slots empty and ran every pair's whole arithmetic in
+// some lane.
 #include <cmath>
 #include <cstring>
 #include <vector>

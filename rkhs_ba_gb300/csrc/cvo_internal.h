@@ -189,7 +189,7 @@ struct BatchDev {
   PairDev *pairs;                 // device array
   const int *item_off;            // npairs + 1 (prefix of work items)
   const int *tgt_off;             // npairs + 1 (prefix of m)
-  int *err;                       // error word (0 ok)
+  int *err;                       // error word (0 ok; no kernel of the engine sets it)
   const int *rblk_off;            // row-pass blocks per pair (prefix)
   const int *sblk_off;            // k_gradient and k_step blocks per pair (prefix)
   int total_rblocks, total_sblocks;
@@ -220,7 +220,7 @@ struct Profile {
   bool on = false;
   double assoc_ms = 0.0;
   double kernel_ms[5] = {0, 0, 0, 0, 0};   // transform, assoc, reduce, step, all four
-  double assoc_split_ms[3] = {0, 0, 0};    // association kernel, selection, row sums
+  double assoc_split_ms[3] = {0, 0, 0};    // candidate test, row pass, 0 (row sums: part of reduce)
   long long assoc_launches = 0;
   double assoc_bytes = 0.0;
   long long iterations = 0;
@@ -335,7 +335,6 @@ struct AssocGraph {
   PairDev *pin_in = nullptr, *pin_out = nullptr;
   int *pin_err = nullptr;
   int pin_pairs = 0;
-  int captures = 0, replays = 0;
   AssocGraph() = default;
   AssocGraph(const AssocGraph &) = delete;
   AssocGraph &operator=(const AssocGraph &) = delete;

@@ -230,6 +230,7 @@ class CvoGPU:
         L.check(L.lib().cvo_profile_assoc_split(self._h, sp), "cvo_profile_assoc_split")
         return {"assoc_ms": ms.value, "assoc_launches": n.value, "assoc_bytes": b.value, "iterations": it.value,
                 "kernel_ms": {names[i]: k[i] for i in range(5)},
+                # candidate test, row pass, and 0 (the row sums are part of "reduce")
                 "assoc_split_ms": {"kernel": sp[0], "select": sp[1], "rowsum": sp[2]}}
 
     def upload(self, cloud: CvoPointCloud) -> GpuCloud:
@@ -467,10 +468,11 @@ class CvoGPU:
 
     # -- autotuner -----------------------------------------------------
     def autotune(self, source: GpuCloud, target: GpuCloud, T=None, ell: float = 0.0, reps: int = 3) -> dict:
-        """Times the association's cell-size configurations on one pair, then the best one
-        with 1-3 resident blocks per SM, and keeps the fastest for later batches of the same
-        (F, C, size) key.  Returns {"configs": [(div_r, div_ext, blocks_per_sm, ms), ...],
-        "best": index}; blocks_per_sm 0 = as many as the occupancy allows."""
+        """Times divisions of the association's candidate test among warps on one pair (12 pairs of
+        factors, whose product counts: 8 divisions), then the best one with work items for 1-3
+        blocks per SM, and keeps the fastest for later batches of the same (F, C, size) key.
+        Returns {"configs": [(div_r, div_ext, blocks_per_sm, ms), ...], "best": index};
+        blocks_per_sm 0 = the default, about two items per resident warp."""
         Ti = _m16(np.eye(4) if T is None else T)
         n = C.c_int()
         dr, de, ms = np.zeros(32, np.float32), np.zeros(32, np.float32), np.zeros(32, np.float32)

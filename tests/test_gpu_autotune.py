@@ -1,5 +1,5 @@
 """The association autotuner (cvo_autotune_launch_dev): every candidate configuration --
-12 cell sizes, then 1-3 resident blocks per SM -- gives the same kernel matrix (identical
+12 divisions of the candidate test, then items for 1-3 blocks per SM -- gives the same kernel matrix (identical
 columns per row, values within 1e-6 relative) and the same inner product (1e-5
 relative: row sums may add in another order); the fastest configuration is kept for
 later batches of the same key."""

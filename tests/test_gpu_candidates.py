@@ -1,7 +1,7 @@
 """The association's candidate test and row pass at the sizes where their tiling can go
 wrong, against the CPU oracle: identical columns per row, values within 1e-5 relative (FP32
 exp against the oracle's double).  Sizes straddle the tile of 32 rows, the group of 32 and
-the supergroup of 1,024 targets and the bitmap window of 65,536; caps below and above the
+the supergroup of 1,024 targets (the bitmap window of 20,480: test_gpu_long_rows.py); caps below and above the
 rows' counts; tiles many lengthscales wide; and the kernels without a geometric term."""
 import numpy as np
 import pytest

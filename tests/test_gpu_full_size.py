@@ -5,8 +5,8 @@ with a grid and runs on all host threads):
 
 * 10,000-point geometric room pair (geometric.yaml, lengthscale 0.25);
 * 50,000-point colour stereo pair (color.yaml, lengthscale 0.4, identity pose): about
-  5 M kept pairs, 20 k rows above the 256-pair cap, so the index-ordered selection
-  (k_select / k_rescan) runs on tens of thousands of rows;
+  5 M kept pairs, 20 k rows above the 256-pair cap, so the row pass cuts
+  tens of thousands of rows at the cap;
 * 128,000-point semantic LiDAR scan pair (lidar_semantic.yaml, 19 classes,
   lengthscale 1.0).
 

@@ -1,5 +1,5 @@
 """The window solve's normal equations where their tiling can go wrong (rows around the warp's
-32 and the block's 1,024, entries per row around 32, edges of very different sizes) against the
+32 and the block's 128, entries per row around 32, edges of very different sizes) against the
 oracle's FP64 solve: one outer iteration within 1e-5 rad / 1e-5 m, the bound of the window tests."""
 import numpy as np
 import pytest
